@@ -106,6 +106,182 @@ __global__ void __launch_bounds__(kTj * kTk) k_extrapolate_tile(float *__restric
     }
 }
 
+// set_unknown and one extrapolation pass of the three face arrays in one
+// kernel, from the level set.  Inside the cell grid all three axes share the
+// flag phi >= 0 of set_unknown, so one staging of phi serves them; only the
+// last face layer of each array (i == nx of u, j == ny of v, k == nz of w)
+// takes its flag from the caller's arrays, patched in by the tiles that reach
+// it.
+//
+// A block owns kPi x kPj x kPk faces.  "Known" and "to extrapolate" are one
+// bit per face (a ballot per 32 faces along k, with a one-face halo of known
+// bits); a thread per word finds the faces that border a known one, and only
+// those load face values.  The other unknown faces are written as 0 from the
+// bits alone.
+constexpr int kPi = 8, kPj = 8, kPk = 128, kPWords = kPk / 32;
+constexpr int kPRows = (kPi + 2) * (kPj + 2);
+constexpr int kPThreads = kPi * kPj * kPWords;  // one word each in the second step
+
+struct ExtrapArgs {
+    float *q[3];
+    int32_t *t[3];
+    const float *phi;
+    int nx, ny, nz;
+};
+
+struct ExtrapTile {
+    // of each row: words 1 .. kPWords cover the tile's k range; word 0 holds
+    // the face below it in bit 31, word kPWords + 1 the face above it in bit 0
+    uint32_t known[kPRows][kPWords + 2], todo[kPRows][kPWords + 2];
+    uint32_t near[kPi * kPj][kPWords];  // a known face in the 3x3x3 block around
+};
+
+// Row (ra, rb) of the halo: the known and to-extrapolate bits of its faces,
+// from state(k) = bit 0 known, bit 1 to extrapolate.  One warp.
+template <typename F>
+__device__ __forceinline__ void extrap_row(ExtrapTile &T, int row, int lane, F state) {
+    unsigned st[kPWords];
+#pragma unroll
+    for (int w = 0; w < kPWords; w++) st[w] = state(32 * w + lane);
+    const unsigned edge = lane < 2 ? state(lane ? kPk : -1) : 0u;
+#pragma unroll
+    for (int w = 0; w < kPWords; w++) {
+        const uint32_t kn = __ballot_sync(0xffffffffu, st[w] & 1u), td = __ballot_sync(0xffffffffu, st[w] & 2u);
+        if (lane == 0) {
+            T.known[row][w + 1] = kn;
+            T.todo[row][w + 1] = td;
+        }
+    }
+    if (lane == 0) T.known[row][0] = (edge & 1u) << 31;
+    if (lane == 1) T.known[row][kPWords + 1] = edge & 1u;
+}
+
+// The last face layer of axis d from the caller's flags (set), or without a
+// face again for the next axis (!set).
+__device__ __forceinline__ void extrap_patch(ExtrapTile &T, const ExtrapArgs &A, int d, int i0, int j0, int k0,
+                                             bool set) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int fy = A.ny + (d == 1), fz = A.nz + (d == 2);
+    auto flag = [&](int a, int b, int c) -> unsigned {
+        const int32_t fl = __ldg(A.t[d] + ((int64_t)a * fy + b) * fz + c);
+        return fl == 0 ? 1u : (fl == 1 ? 2u : 0u);
+    };
+    if (d < 2) {
+        for (int row = warp; row < kPRows; row += kPThreads / 32) {
+            const int a = i0 - 1 + row / (kPj + 2), b = j0 - 1 + row % (kPj + 2);
+            if ((d == 0 ? a != A.nx : b != A.ny)) continue;
+            const bool in = set && (d == 0 ? b >= 0 && b < A.ny : a >= 0 && a < A.nx);
+            extrap_row(T, row, lane, [&](int x) -> unsigned {
+                const int c = k0 + x;
+                return in && c >= 0 && c < A.nz ? flag(a, b, c) : 0u;
+            });
+        }
+        return;
+    }
+    const int pos = A.nz - k0 + 32;  // bit pos & 31 of word pos / 32 of every row
+    if (pos < 31 || pos > kPk + 32) return;
+    for (int row = threadIdx.x; row < kPRows; row += kPThreads) {
+        const int a = i0 - 1 + row / (kPj + 2), b = j0 - 1 + row % (kPj + 2);
+        const unsigned st = set && a >= 0 && a < A.nx && b >= 0 && b < A.ny ? flag(a, b, A.nz) : 0u;
+        const uint32_t bit = 1u << (pos & 31);
+        uint32_t &kn = T.known[row][pos >> 5], &td = T.todo[row][pos >> 5];
+        kn = (st & 1u) ? kn | bit : kn & ~bit;
+        td = (st & 2u) ? td | bit : td & ~bit;
+    }
+}
+
+// One word per thread: the faces of tile row threadIdx.x / kPWords with a
+// known face among their 3x3x3 neighbours.
+__device__ __forceinline__ void extrap_near(ExtrapTile &T) {
+    const int w = threadIdx.x % kPWords, o = threadIdx.x / kPWords;
+    const int rc = (o / kPj + 1) * (kPj + 2) + o % kPj + 1;
+    uint32_t lo = 0u, mid = 0u, hi = 0u;
+#pragma unroll
+    for (int m = 0; m < 9; m++) {
+        const uint32_t *r = T.known[rc + (m / 3 - 1) * (kPj + 2) + m % 3 - 1] + w;
+        lo |= r[0];
+        mid |= r[1];
+        hi |= r[2];
+    }
+    T.near[o][w] = mid | (mid << 1) | (lo >> 31) | (mid >> 1) | (hi << 31);
+}
+
+__global__ void __launch_bounds__(kPThreads) k_extrapolate_phi(const ExtrapArgs A) {
+    __shared__ ExtrapTile T;
+    const int i0 = blockIdx.z * kPi, j0 = blockIdx.y * kPj, k0 = blockIdx.x * kPk;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int row = warp; row < kPRows; row += kPThreads / 32) {
+        const int a = i0 - 1 + row / (kPj + 2), b = j0 - 1 + row % (kPj + 2);
+        const bool in = a >= 0 && a < A.nx && b >= 0 && b < A.ny;
+        const float *pr = A.phi + ((int64_t)(in ? a : 0) * A.ny + (in ? b : 0)) * A.nz;
+        extrap_row(T, row, lane, [&](int x) -> unsigned {
+            const int c = k0 + x;
+            return in && c >= 0 && c < A.nz ? (__ldg(pr + c) >= 0.0f ? 2u : 1u) : 0u;
+        });
+    }
+    __syncthreads();
+    extrap_near(T);
+    __syncthreads();
+    bool patched = false;
+    for (int d = 0; d < 3; d++) {
+        const bool last = d == 0 ? i0 + kPi >= A.nx : (d == 1 ? j0 + kPj >= A.ny : k0 + kPk >= A.nz);
+        if (patched || last) {
+            __syncthreads();
+            if (patched) extrap_patch(T, A, d - 1, i0, j0, k0, false);
+            if (patched && last) __syncthreads();
+            if (last) extrap_patch(T, A, d, i0, j0, k0, true);
+            __syncthreads();
+            extrap_near(T);
+            __syncthreads();
+            patched = last;
+        }
+        const int fx = A.nx + (d == 0), fy = A.ny + (d == 1), fz = A.nz + (d == 2);
+        float *q = A.q[d];
+        int32_t *t = A.t[d];
+        for (int o = warp; o < kPi * kPj; o += kPThreads / 32) {
+            const int i = i0 + o / kPj, j = j0 + o % kPj;
+            if (i >= fx || j >= fy) continue;
+            const int rc = (o / kPj + 1) * (kPj + 2) + o % kPj + 1;
+            const int64_t f = ((int64_t)i * fy + j) * fz + k0 + lane;
+            const bool flags = i < A.nx && j < A.ny;
+#pragma unroll
+            for (int w = 0; w < kPWords; w++) {
+                const int k = k0 + 32 * w + lane;
+                const uint32_t td = T.todo[rc][w + 1], nr = T.near[o][w];
+                const bool mine = (td >> lane) & 1u;
+                if (flags && k < A.nz) t[f + 32 * w] = mine ? 1 : 0;  // set_unknown
+                if (mine && !((nr >> lane) & 1u)) q[f + 32 * w] = 0.0f;
+                if ((td & nr) == 0u) continue;
+                if (!((td & nr) >> lane & 1u)) continue;
+                int n = 0;
+                float s = 0.0f;
+                // nine loads at a time in flight, summed in (ii, jj, kk) order
+#pragma unroll 1
+                for (int ii = -1; ii <= 1; ii++) {
+                    float v[9];
+                    unsigned have = 0u;
+#pragma unroll
+                    for (int jj = -1; jj <= 1; jj++) {
+                        const uint32_t *r = T.known[rc + ii * (kPj + 2) + jj] + w;
+                        const uint64_t bits =
+                            (uint64_t)(r[0] >> 31) | ((uint64_t)r[1] << 1) | ((uint64_t)(r[2] & 1u) << 33);
+                        const unsigned b3 = (unsigned)(bits >> lane) & 7u;  // the row's faces k - 1, k, k + 1
+                        const float *qr = q + f + 32 * w + ((int64_t)ii * fy + jj) * fz;
+                        have |= b3 << (3 * (jj + 1));
+#pragma unroll
+                        for (int kk = 0; kk < 3; kk++) v[3 * (jj + 1) + kk] = (b3 & (1u << kk)) ? qr[kk - 1] : 0.0f;
+                    }
+                    n += __popc(have);
+#pragma unroll
+                    for (int m = 0; m < 9; m++)
+                        if (have & (1u << m)) s = __fadd_rn(s, v[m]);
+                }
+                q[f + 32 * w] = __fdiv_rn(s, (float)n);
+            }
+        }
+    }
+}
+
 static inline dim3 tile_grid(int fx, int fy, int fz) {
     return dim3((unsigned)((fz + kTk - 1) / kTk), (unsigned)((fy + kTj - 1) / kTj), (unsigned)((fx + kTi - 1) / kTi));
 }
@@ -155,11 +331,19 @@ int flub_extrapolate(float *u, float *v, float *w, int32_t *tu, int32_t *tv, int
     FLUB_REQUIRE(nx > 0 && ny > 0 && nz > 0 && nx < 65535 && ny < 65535, "flub_extrapolate: bad shape");
     FLUB_REQUIRE(n_passes >= 0, "flub_extrapolate: n_passes must be >= 0");
     cudaStream_t s = as_stream(stream);
-    if (phi) {
+    // A pass leaves the flags as they were (the flush turns its -1 back into
+    // 1), never writes a known face and reads no other, so every further pass
+    // writes the values the first one wrote: one pass gives the result of
+    // n_passes >= 1 for any input.
+    if (phi && n_passes > 0) {
+        ExtrapArgs A{{u, v, w}, {tu, tv, tw}, phi, nx, ny, nz};
+        k_extrapolate_phi<<<dim3((unsigned)(nz / kPk + 1), (unsigned)(ny / kPj + 1), (unsigned)(nx / kPi + 1)),
+                            kPThreads, 0, s>>>(A);
+        FLUB_CHECK_LAUNCH();
+    } else if (phi) {
         k_set_unknown<<<row_grid(nx, ny, nz), kRowThreads, 0, s>>>(phi, tu, tv, tw, nx, ny, nz);
         FLUB_CHECK_LAUNCH();
-    }
-    for (int p = 0; p < n_passes; p++) {
+    } else if (n_passes > 0) {
         k_extrapolate_tile<false><<<tile_grid(nx + 1, ny, nz), dim3(kTk, kTj), 0, s>>>(u, tu, nx + 1, ny, nz);
         FLUB_CHECK_LAUNCH();
         k_extrapolate_tile<false><<<tile_grid(nx, ny + 1, nz), dim3(kTk, kTj), 0, s>>>(v, tv, nx, ny + 1, nz);

@@ -167,8 +167,8 @@ int flub_flush_unknown(int32_t *unk, int64_t n, void *stream);
 /* water_3d.py:70-73 extrapolate: set_unknown (skipped when phi is NULL), then
  * n_passes of extrapolate_by_1 (extrapolate.py:39-47) on the three axes.  Each
  * pass leaves the flags as the reference's flush does (extrapolated faces
- * back to 1), so the faces extrapolated and their values are the reference's
- * pass for pass. */
+ * back to 1), so every pass after the first writes the same values again:
+ * n_passes >= 1 runs one. */
 int flub_extrapolate(float *u, float *v, float *w, int32_t *tu, int32_t *tv, int32_t *tw, const float *phi, int nx,
                      int ny, int nz, int n_passes, void *stream);
 

@@ -112,3 +112,27 @@ def test_extrapolation_rejects_bad_arguments():
         _lib.call("flub_extrapolate_axis", None, None, 4, 4, 4, 1, None)
     with pytest.raises(FlubError):
         _lib.call("flub_extrapolate", *([None] * 7), 4, 4, 4, -1, None)
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1), (7, 8, 127), (8, 7, 128), (9, 9, 129), (16, 24, 256), (3, 20, 31)])
+@pytest.mark.parametrize("n_cells", [1, 3])
+def test_fused_extrapolation_tile_edges_bit_exact(shape, n_cells):
+    """Tile remainders along every axis, and a last face layer whose flags the
+    caller set (0 known, 1 to extrapolate, 2 neither): it keeps its flags, and
+    known faces there feed their neighbours."""
+    rng = np.random.default_rng(sum(shape) + n_cells)
+    phi = rng.standard_normal(shape).astype(np.float32)
+    phi[:, : shape[1] // 2] += 3.0  # a part without any known face
+    faces, flags = [], []
+    for d in range(3):
+        fs = tuple(n + (a == d) for a, n in enumerate(shape))
+        faces.append(rng.standard_normal(fs).astype(np.float32))
+        flags.append(rng.integers(0, 3, size=fs).astype(np.int32))
+    ref, rflags = [f.copy() for f in faces], [f.copy() for f in flags]
+    O.extrapolate(*ref, *rflags, phi, n_cells)
+    vel, tags = _mac(*faces), _macint(*flags)
+    extrapolate(vel, tags, Field(dev(phi)), n_cells)
+    for a, b in zip((vel.u.f, vel.v.f, vel.w.f), ref):
+        assert np.array_equal(host(a), b)
+    for a, b in zip((tags.u.f, tags.v.f, tags.w.f), rflags):
+        assert np.array_equal(host(a), b)
