@@ -21,19 +21,17 @@
 
 #include "mg_kernels.cuh"
 #include "cg8.cuh"
-#include "cluster.cuh"
+#include "coarse.cuh"
 #include "mixed.cuh"
 #include "persist.cuh"
 #include "restrict8.cuh"
 #include "smooth8.cuh"
 #include "smooth_split.cuh"
 #include "smooth_tile.cuh"
-#include "tail.cuh"
 
 namespace flub {
 
 constexpr int kMaxLevels = 12;
-constexpr size_t kTailMaxSmem = 200 * 1024;  // dynamic shared memory of the tail kernel
 
 // Per level: cell codes, residual r, and two correction buffers.  Pre-smoothing
 // and the restriction work on z2; the prolongation writes z2 + P z_coarse into
@@ -69,11 +67,9 @@ struct Level {
     unsigned char *tflags;
     int *tiles, *tiles_n;
     int n_tiles;
-    // levels small enough for the one-block tail (tail.cuh), nz even: the
-    // neighbour masks of each k-pair of cells the tail's sweeps use, built once
-    // by set_tags (the tail otherwise rebuilds them from the codes at every
-    // level entry of every V-cycle); NULL elsewhere
-    uint32_t *pmask;
+    // stencil words of every cell in natural order, on levels the coarse kernel
+    // (coarse.cuh) can run; NULL on larger ones
+    uint16_t *cw;
 };
 
 struct LaunchCtx {
@@ -109,12 +105,10 @@ struct flub_mg {
     bool split_ok;  // level 0 smooths on colour-split storage (smooth_split.cuh); FLUB_NO_SPLIT=1 turns it off
     bool iter_toggle[flub::kMaxLevels];  // flub_mg_smooth_iteration: direction of the next tiled call
     bool r_masked;  // r is 0 off the fluid (mask_interior since the last init)
-    int tail_start;  // first level run by the one-block tail kernel (== levels: none)
-    size_t tail_smem;
     int persist_blocks;  // blocks of the persistent V-cycle legs (persist.cuh); 0: launch per pass
-    int cl_start;    // first level run by the cluster kernel (== levels: none)
-    int cl_size;     // blocks per cluster
-    size_t cl_smem;
+    int co_start;    // first level run by the coarse kernel (coarse.cuh; == levels: none)
+    int co_blocks;   // its cluster size (1: one block without a cluster)
+    size_t co_smem;
     // V-cycle schedule (flub_mg_set_schedule); the reference's: -1, 3, 1
     int sched_nu;        // red-black iterations per side at every level (< 0: 6 << level)
     int sched_bottom;    // bottom: this many (0, 1) iterations, then as many (1, 0)
@@ -202,8 +196,7 @@ static size_t carve(flub_mg *mg, char *base) {
             L.tiles = (int *)take(sizeof(int) * (size_t)L.n_tiles);
             L.tiles_n = (int *)take(sizeof(int));
         }
-        L.pmask = nullptr;
-        if (nl <= kTailMaxCells && L.D.nz % 2 == 0) L.pmask = (uint32_t *)take(sizeof(uint32_t) * (size_t)(nl >> 1));
+        L.cw = nl <= kCoarseMaxCells ? (uint16_t *)take(sizeof(uint16_t) * (size_t)nl) : nullptr;
     }
     // per-block counts of the active-list build (level 0 has the most blocks)
     mg->act_scratch = (int *)take(sizeof(int) * (size_t)((n / 8 + kActPerBlock - 1) / kActPerBlock + 1));
@@ -211,193 +204,178 @@ static size_t carve(flub_mg *mg, char *base) {
     return off;
 }
 
-// Shared-memory layout of the tail kernel from level lt down; returns the
-// bytes needed (0 if the tail does not qualify).
-static size_t tail_layout(const flub_mg *mg, int lt, TailParams *P) {
-    if (lt >= mg->levels || mg->levels - lt > kTailMaxLevels) return 0;
-    size_t off = 0;
+static inline bool is_pow2(int v) { return v > 0 && (v & (v - 1)) == 0; }
+
+// Layout of the coarse kernel from level lc down on a cluster of C blocks;
+// returns the bytes of shared memory per block, 0 if the levels do not qualify.
+//
+// Levels of at most kBlockCells cells belong to block 0 alone.  Each larger
+// one is split into slabs of P i-planes, at most kBlockCells cells each; P
+// halves with the level, so that a block's coarse planes are the restriction
+// of its own, and is even on every split level that restricts further.  The
+// smallest P that works uses the most blocks.
+static size_t coarse_layout(const flub_mg *mg, int lc, int C, CoarseParams *P) {
+    if (lc >= mg->levels || mg->levels - lc > kCoarseMaxLevels) return 0;
+    auto dims = [&](int l) { return Dims{mg->nx >> l, mg->ny >> l, mg->nz >> l}; };
+    int nd = 0, p0 = 0;
+    if (dims(lc).n() > kBlockCells) {
+        const Dims T = dims(lc);
+        if (C < 2) return 0;
+        for (int p = (T.nx + C - 1) / C; p <= T.nx && (int64_t)p * T.ny * T.nz <= kBlockCells && nd == 0; p++) {
+            for (int l = lc, q = p;; l++, q >>= 1) {
+                if (l == mg->levels - 1) {
+                    nd = l - lc + 1;
+                    break;
+                }
+                if (q & 1) break;
+                if (dims(l + 1).n() <= kBlockCells) {
+                    nd = l - lc + 1;
+                    break;
+                }
+            }
+            p0 = p;
+        }
+        if (nd == 0) return 0;
+    }
+    size_t off = kCoarseFixed, scratch = 0;
     auto take = [&](size_t b) {
-        size_t o = off;
+        const size_t o = off;
         off += (b + 15) & ~(size_t)15;
         return (int)o;
     };
-    for (int l = lt; l < mg->levels; l++) {
-        const Dims D{mg->nx >> l, mg->ny >> l, mg->nz >> l};
-        const size_t n = (size_t)D.n();
-        TailLevel &T = P->lv[l - lt];
-        T.D = D;
-        T.code = mg->lv[l].code;
-        T.pmask = mg->lv[l].pmask;
-        T.abs_level = l;
-        T.off_z = take(sizeof(float) * n);
-        T.off_r = take(sizeof(float) * n);
-        T.off_c = take(n);
-        T.off_v = l + 1 < mg->levels ? take(sizeof(float) * n) : -1;
+    P->nl = mg->levels - lc;
+    P->nd = nd;
+    for (int t = 0; t < P->nl; t++) {
+        CoarseLevel &L = P->lv[t];
+        L.D = dims(lc + t);
+        L.abs_level = lc + t;
+        L.P = t < nd ? p0 >> t : L.D.nx;
+        const int hz = L.D.nz >> 1;
+        L.V = hz % 4 == 0 ? 4 : (hz % 2 == 0 ? 2 : 1);
+        const size_t cells = (size_t)L.P * L.D.ny * L.D.nz;
+        L.hn = (coarse_row(L.P + 1, 0, L.D.ny, hz) + 3) & ~3;  // planes -1 .. P
+        L.off_z = take(sizeof(float) * 2 * (size_t)L.hn);
+        L.off_r = take(sizeof(float) * cells);
+        L.off_w = take(sizeof(CoarseWeights) * cells);
+        L.div_seg = coarse_div_by(hz / L.V);
+        L.div_ny = coarse_div_by(L.D.ny);
+        L.div_nz = coarse_div_by(L.D.nz);
+        L.cw = mg->lv[lc + t].cw;
+        if (t + 1 < P->nl && cells > scratch) scratch = cells;
     }
-    P->nt = mg->levels - lt;
+    P->off_v = take(sizeof(float) * scratch);
     P->nu = mg->sched_nu;
     P->nbottom = mg->sched_bottom;
     P->rscale = mg->sched_rscale;
     P->bottom64 = mg->bottom64 ? 1 : 0;
-    P->off_zd = 0;
-    if (mg->bottom64) P->off_zd = take(sizeof(double) * (size_t)P->lv[P->nt - 1].D.n());
+    P->off_zd = mg->bottom64 ? take(sizeof(double) * (size_t)P->lv[P->nl - 1].D.n()) : 0;
     return off;
 }
 
-static int set_tail_smem_limit() {
-    FLUB_CHECK_CUDA(cudaFuncSetAttribute(k_tail_vcycle, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTailMaxSmem));
-    return FLUB_OK;
+// The kernel for this layout.
+static decltype(&k_coarse_vcycle<4>) coarse_kernel(const CoarseParams &P) {
+    for (int t = 0; t < P.nl; t++)
+        if (P.lv[t].V != 4) return k_coarse_vcycle<0>;
+    return k_coarse_vcycle<4>;
 }
 
-static int choose_tail(flub_mg *mg) {
-    mg->tail_start = mg->levels;
-    mg->tail_smem = 0;
-    for (int l = 0; l < mg->levels; l++) {
-        const Dims D{mg->nx >> l, mg->ny >> l, mg->nz >> l};
-        if (D.n() > kTailMaxCells) continue;
-        TailParams P;
-        const size_t b = tail_layout(mg, l, &P);
-        if (b > 0 && b <= kTailMaxSmem) {
-            mg->tail_start = l;
-            mg->tail_smem = b;
-        }
-        break;
-    }
-    return FLUB_OK;
-}
-
-static inline bool is_pow2(int v) { return v > 0 && (v & (v - 1)) == 0; }
-static inline int ilog2(int v) {
-    int l = 0;
-    while ((1 << l) < v) l++;
-    return l;
-}
-
-// Distributed-shared-memory layout of the cluster kernel from level lc down
-// with C blocks; returns the bytes per block (0 if the levels do not qualify:
-// every dimension a power of two, nx and nz at least 2 at every level).
-static size_t cluster_layout(const flub_mg *mg, int lc, int C, ClusterParams *P) {
-    if (lc >= mg->levels || mg->levels - lc > kClusterMaxLevels) return 0;
-    size_t off = 0;
-    auto take = [&](size_t b) {
-        size_t o = off;
-        off += (b + 15) & ~(size_t)15;
-        return (int)o;
-    };
-    P->tail = 0;
-    P->tail_off = 0;
-    // block 0 takes over the <= 16^3 levels: their sweeps then synchronise
-    // with block barriers instead of cluster barriers (measured at 256^3: the
-    // reference schedule's solve 30.0 -> 27.4 ms, V(2,2) 3.03 -> 2.96 ms).
-    // FLUB_CLUSTER_TAIL=0 keeps them in the cluster; both give the same bits.
-    const char *ct = getenv("FLUB_CLUSTER_TAIL");
-    const bool want_tail = !(ct && ct[0] == '0');
-    int lt = mg->levels;  // first level run by block 0 alone (== levels: none)
-    for (int l = lc; l < mg->levels; l++) {
-        const Dims D{mg->nx >> l, mg->ny >> l, mg->nz >> l};
-        if (want_tail && l > lc && D.n() <= kTailMaxCells && tail_layout(mg, l, &P->tp) > 0) {
-            lt = l;
-            break;
-        }
-        if (!is_pow2(D.nx) || !is_pow2(D.ny) || !is_pow2(D.nz) || D.nx < 2 || D.nz < 2) return 0;
-        ClusterLevel &L = P->lv[l - lc];
-        L.D = D;
-        L.abs_level = l;
-        L.ncta = D.nx / 2 < C ? D.nx / 2 : C;
-        L.P = D.nx / L.ncta;
-        L.lg_ny = ilog2(D.ny);
-        L.lg_nz = ilog2(D.nz);
-        L.code = mg->lv[l].code;
-        const size_t plane = (size_t)D.ny * D.nz;
-        L.off_z = take(sizeof(float) * (L.P + 2) * plane);
-        L.off_c = take((L.P + 2) * plane);
-        L.off_r = take(sizeof(float) * L.P * plane);
-    }
-    P->nl = lt - lc;
-    if (lt < mg->levels) {
-        // the coarsest levels in block 0: the tail layout after the distributed ones
-        const size_t tb = tail_layout(mg, lt, &P->tp);
-        P->tail = 1;
-        P->tail_off = take(tb);
-    }
-    P->nu = mg->sched_nu;
-    P->nbottom = mg->sched_bottom;
-    P->rscale = mg->sched_rscale;
-    return off;
-}
-
-static cudaError_t cluster_launch_config(int C, size_t smem, cudaStream_t s, cudaLaunchConfig_t *cfg,
-                                         cudaLaunchAttribute *attr) {
+static cudaError_t coarse_launch_config(int C, size_t smem, cudaStream_t s, cudaLaunchConfig_t *cfg,
+                                        cudaLaunchAttribute *attr) {
     memset(cfg, 0, sizeof(*cfg));
     cfg->gridDim = dim3(C);
-    cfg->blockDim = dim3(kClusterThreads);
+    cfg->blockDim = dim3(kCoarseThreads);
     cfg->dynamicSmemBytes = smem;
     cfg->stream = s;
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = C;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = C;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
     cfg->attrs = attr;
-    cfg->numAttrs = 2;
+    cfg->numAttrs = C > 1 ? 2 : 1;
     return cudaSuccess;
 }
 
-// Picks the first level of at most 32^3 cells whose coarse hierarchy fits one
-// cluster (16 blocks, else 8); none if the GPU cannot run it or
-// FLUB_NO_CLUSTER=1.
-static int choose_cluster(flub_mg *mg) {
-    mg->cl_start = mg->levels;
-    mg->cl_size = 0;
-    mg->cl_smem = 0;
+// Picks the finest level whose hierarchy fits the coarse kernel: on a cluster
+// of 16 blocks, else of 8, else (no clusters, or FLUB_NO_CLUSTER=1) the levels
+// one block holds.
+static int choose_coarse(flub_mg *mg) {
+    mg->co_start = mg->levels;
+    mg->co_blocks = 0;
+    mg->co_smem = 0;
     const char *off = getenv("FLUB_NO_CLUSTER");
-    if (off && off[0] == '1') return FLUB_OK;
+    const bool clusters = !(off && off[0] == '1');
     int dev = 0, max_smem = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) {
+        cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
+        cudaFuncSetAttribute(k_coarse_vcycle<4>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+        cudaFuncSetAttribute(k_coarse_vcycle<0>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
+            cudaSuccess ||
+        cudaFuncSetAttribute(k_coarse_vcycle<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem) !=
+            cudaSuccess ||
+        cudaFuncSetAttribute(k_coarse_vcycle<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem) !=
+            cudaSuccess) {
         cudaGetLastError();
         return FLUB_OK;
     }
-    // larger levels keep the 152-SM global sweeps: on 8-16 SMs a 64^3 half-sweep
-    // is bound by shared-memory bandwidth (FLUB_CLUSTER_MAX_CELLS overrides)
-    int64_t max_cells = 32768;
-    const char *mc = getenv("FLUB_CLUSTER_MAX_CELLS");
-    if (mc && atoll(mc) > 0) max_cells = atoll(mc);
-    for (int C : {16, 8}) {
+    for (int C : {16, 8, 1}) {
+        if (C > 1 && !clusters) continue;
         for (int l = 0; l < mg->levels; l++) {
-            const Dims D{mg->nx >> l, mg->ny >> l, mg->nz >> l};
-            if (D.n() > max_cells) continue;
-            ClusterParams P;
-            const size_t b = cluster_layout(mg, l, C, &P);
-            if (b == 0 || b > (size_t)max_smem) break;
-            if (cudaFuncSetAttribute(k_cluster_vcycle<false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
-                    cudaSuccess ||
-                cudaFuncSetAttribute(k_cluster_vcycle<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem) !=
-                    cudaSuccess ||
-                cudaFuncSetAttribute(k_cluster_vcycle<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
-                    cudaSuccess ||
-                cudaFuncSetAttribute(k_cluster_vcycle<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem) !=
-                    cudaSuccess) {
-                cudaGetLastError();
-                break;
+            CoarseParams P;
+            const size_t b = coarse_layout(mg, l, C, &P);
+            if (b == 0 || b > (size_t)max_smem) continue;
+            const int blocks = P.nd > 0 ? C : 1;
+            if (blocks > 1) {
+                cudaLaunchConfig_t cfg;
+                cudaLaunchAttribute attr[2];
+                coarse_launch_config(C, b, nullptr, &cfg, attr);
+                cfg.attrs = attr + 1;  // the cluster dimension only
+                cfg.numAttrs = 1;
+                int nclusters = 0;
+                if (cudaOccupancyMaxActiveClusters(&nclusters, coarse_kernel(P), &cfg) != cudaSuccess ||
+                    nclusters < 1) {
+                    cudaGetLastError();
+                    break;
+                }
             }
-            cudaLaunchConfig_t cfg;
-            cudaLaunchAttribute attr[2];
-            cluster_launch_config(C, b, nullptr, &cfg, attr);
-            cfg.numAttrs = 1;  // the cluster dimension only
-            int nclusters = 0;
-            if (cudaOccupancyMaxActiveClusters(&nclusters, k_cluster_vcycle<false>, &cfg) != cudaSuccess || nclusters < 1) {
-                cudaGetLastError();
-                break;
-            }
-            mg->cl_start = l;
-            mg->cl_size = C;
-            mg->cl_smem = b;
+            mg->co_start = l;
+            mg->co_blocks = blocks;
+            mg->co_smem = b;
             return FLUB_OK;
         }
     }
     return FLUB_OK;
+}
+
+// The level from which this library's mixed-precision handles leave the FP16
+// rows of 8 cells (smooth8.cuh), and with it where an FP64 bottom is offered:
+// both are part of the interface (a handle they exclude is refused), so they
+// follow the shapes alone -- the finest level of at most 32,768 cells with
+// power-of-two extents from there down to 4,096 cells, else the first level of
+// at most 4,096 -- and not what the coarse kernel happens to hold.
+static int small_levels_start(const flub_mg *mg, bool *bottom_small) {
+    const char *off = getenv("FLUB_NO_CLUSTER");
+    auto dims = [&](int l) { return Dims{mg->nx >> l, mg->ny >> l, mg->nz >> l}; };
+    const int b = mg->levels - 1;
+    if (!(off && off[0] == '1')) {
+        int l = 0;
+        while (l <= b && dims(l).n() > 32768) l++;
+        bool ok = l <= b;
+        int m = l;
+        for (; ok && m <= b && (m == l || dims(m).n() > kBlockCells); m++) {
+            const Dims D = dims(m);
+            ok = is_pow2(D.nx) && is_pow2(D.ny) && is_pow2(D.nz) && D.nx >= 2 && D.nz >= 2;
+        }
+        if (ok) {
+            *bottom_small = m <= b;
+            return l;
+        }
+    }
+    int l = 0;
+    while (l <= b && dims(l).n() > kBlockCells) l++;
+    *bottom_small = l <= b;
+    return l;
 }
 
 // The persistent cooperative V-cycle legs (persist.cuh), opt-in with
@@ -487,56 +465,14 @@ static int launch_leg(flub_mg *mg, const LaunchCtx &c, bool down, int l0, int l1
     return FLUB_OK;
 }
 
-// Opt-in (FLUB_CLUSTER_GLOBAL=1): the cluster kernel also runs the level just
-// above its distributed levels (cluster.cuh, ClusterGlobal) when that level is
-// below level 0, walks an active list with stencil words, the sweeps may skip
-// fluid-free groups, and neither the persistent legs nor tiled smoothing are
-// asked for there.  Measured on the 256^3 dam break it is slower than one
-// launch per pass on all SMs (V(2,2) solve 2.89 against 2.68 ms, the
-// reference schedule 25.5 against 23.3 ms): the 16 SMs of one cluster take
-// longer over a 64^3 level's sweep than the launch boundary costs.
-static bool use_cluster_global(const flub_mg *mg, int lt, int sk) {
-    if (!(mg->cl_start < mg->levels) || lt != mg->cl_start) return false;
-    const char *e = getenv("FLUB_CLUSTER_GLOBAL");
-    if (!(e && e[0] == '1')) return false;
-    const int G = lt - 1;
-    if (G < 1 || sk != 1 || !mg->skip_ok || mg->persist_blocks > 0) return false;
-    const Level &L = mg->lv[G];
-    if (L.D.nz % 8 != 0 || !L.act || !L.sw) return false;
-    return !(mg->tile_ok && L.n_tiles > 0);
-}
-
-static void fill_cluster_global(const flub_mg *mg, int G, bool half, ClusterGlobal *g) {
-    const Level &L = mg->lv[G], &C = mg->lv[G + 1];
-    g->on = 1;
-    g->half = half ? 1 : 0;
-    g->D = L.D;
-    g->code = L.code;
-    g->sw = L.sw;
-    g->act = L.act;
-    g->act_n = L.act_n;
-    g->r = half ? (void *)L.rh : (void *)L.r;
-    g->z = half ? (void *)L.zh : (void *)L.z;
-    g->z2 = half ? (void *)L.z2h : (void *)L.z2;
-    g->iters = level_iters(mg, G);
-    g->rscale = (half ? 0.125f : 1.0f) * mg->sched_rscale;
-    g->zc_scale = half ? 8.0f : 1.0f;
-    g->CD = C.D;
-    g->ccode = C.code;
-    g->cact = C.act;
-    g->cact_n = C.act_n;
-    g->cr = half ? (void *)C.rh : (void *)C.r;
-    g->cz = half ? (const void *)C.zh : (const void *)C.z;
-}
-
-// Whether the bottom level runs inside the one-block tail (tail.cuh), alone or
-// inside the cluster kernel: the only place with an FP64 bottom.
+// Whether the bottom level can be smoothed in FP64: it runs in one block of the
+// coarse kernel.
 static bool bottom_in_tail(flub_mg *mg) {
-    if (mg->cl_start < mg->levels) {
-        ClusterParams P;
-        return cluster_layout(mg, mg->cl_start, mg->cl_size, &P) > 0 && P.tail;
-    }
-    return mg->tail_start < mg->levels;
+    bool small = false;
+    small_levels_start(mg, &small);
+    if (!small || mg->co_start >= mg->levels) return false;
+    CoarseParams P;
+    return coarse_layout(mg, mg->co_start, mg->co_blocks, &P) > 0 && P.nd < P.nl;
 }
 
 static int validate_shape(int nx, int ny, int nz, int levels, int precision) {
@@ -799,6 +735,30 @@ static int tile_side(flub_mg *mg, const LaunchCtx &c, int l, bool post, int iter
     return FLUB_OK;
 }
 
+// The coarse kernel from level co_start down, with FP16 (mixed precision) or
+// FP32 residual and correction of its first level.
+static int launch_coarse(flub_mg *mg, const LaunchCtx &c, const float *r_top, float *z_top, const __half *r_top_h,
+                         __half *z_top_h) {
+    CoarseParams P = {};
+    coarse_layout(mg, mg->co_start, mg->co_blocks, &P);
+    P.r_top = r_top;
+    P.z_top = z_top;
+    P.r_top_h = r_top_h;
+    P.z_top_h = z_top_h;
+    P.status = mg->st ? reinterpret_cast<int *>(reinterpret_cast<char *>(mg->st) + offsetof(MgState, status)) : nullptr;
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr[2];
+    coarse_launch_config(mg->co_blocks, mg->co_smem, c.s, &cfg, attr);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, coarse_kernel(P), (const CoarseParams)P, c.kc);
+    if (e != cudaSuccess) {
+        set_last_error("coarse V-cycle launch: %s", cudaGetErrorString(e));
+        cudaGetLastError();
+        return FLUB_ERR_CUDA;
+    }
+    count_launches(1);
+    return FLUB_OK;
+}
+
 // multigrid/mgpcg.py:296-349 apply_preconditioner; level 0 uses (r0, z0).
 // z0_clean: z0 holds 0 on every non-fluid cell (true for the handle's own z).
 // dot_mode 1 / 2: the caller's next step is z.r (the prologue's p = z / the
@@ -807,8 +767,7 @@ static int tile_side(flub_mg *mg, const LaunchCtx &c, int l, bool post, int iter
 static int enqueue_vcycle(flub_mg *mg, const LaunchCtx &c, const float *r0, float *z0, bool z0_clean,
                           int dot_mode = 0, bool *dot_fused = nullptr) {
     if (dot_fused) *dot_fused = false;
-    const bool use_cl = mg->cl_start < mg->levels;
-    const int Lm = mg->levels, lt = use_cl ? mg->cl_start : mg->tail_start;
+    const int Lm = mg->levels, lt = mg->co_start;
     const int sk = mg->skip_ok ? 1 : 0;
     auto SK = [&](int l) { return (l == 0 && !z0_clean) ? 0 : sk; };
     auto R = [&](int l) -> const float * { return l == 0 ? r0 : mg->lv[l].r; };
@@ -822,13 +781,9 @@ static int enqueue_vcycle(flub_mg *mg, const LaunchCtx &c, const float *r0, floa
     auto TILED_POST = [&](int l) { return mg->tile_ok && mg->lv[l].n_tiles > 0 && SK(l) == 1; };
     // levels 1 .. lg-1 in the persistent cooperative kernels, or one launch per pass
     const bool pers = use_persist(mg, lg);
-    // the level above the cluster's in the cluster kernel: the launches per
-    // pass stop one level earlier
-    const bool clg = use_cl && use_cluster_global(mg, lt, sk);
-    const int lge = clg ? lt - 1 : lg;
     // level 0 on colour-split storage (smooth_split.cuh)
-    const bool split0 = use_split(mg, lge, sk, r0, z0);
-    for (int l = 0; l < (pers ? 1 : lge); l++) {
+    const bool split0 = use_split(mg, lg, sk, r0, z0);
+    for (int l = 0; l < (pers ? 1 : lg); l++) {
         const Level &L = mg->lv[l];
         const int iters = level_iters(mg, l);
         if (l == 0 && split0) {
@@ -873,29 +828,8 @@ static int enqueue_vcycle(flub_mg *mg, const LaunchCtx &c, const float *r0, floa
                                 L.code, C.r, C.code, C.D, mg->sched_rscale, c.kc));
     }
     if (pers) FLUB_TRY(launch_leg<float>(mg, c, true, 1, lg));
-    if (use_cl) {
-        ClusterParams P = {};
-        cluster_layout(mg, lt, mg->cl_size, &P);
-        P.r_top = R(lt);
-        P.z_top = ZF(lt);
-        if (clg) fill_cluster_global(mg, lt - 1, false, &P.g);
-        cudaLaunchConfig_t cfg;
-        cudaLaunchAttribute attr[2];
-        cluster_launch_config(mg->cl_size, mg->cl_smem, c.s, &cfg, attr);
-        const cudaError_t e = P.g.on ? cudaLaunchKernelEx(&cfg, k_cluster_vcycle<true>, (const ClusterParams)P, c.kc)
-                                     : cudaLaunchKernelEx(&cfg, k_cluster_vcycle<false>, (const ClusterParams)P, c.kc);
-        if (e != cudaSuccess) {
-            set_last_error("cluster V-cycle launch: %s", cudaGetErrorString(e));
-            cudaGetLastError();
-            return FLUB_ERR_CUDA;
-        }
-        count_launches(1);
-    } else if (lt < Lm) {
-        TailParams P = {};
-        tail_layout(mg, lt, &P);
-        P.r_top = R(lt);
-        P.z_top = ZF(lt);
-        FLUB_TRY(launch_pdl(k_tail_vcycle, dim3(1), dim3(kTailThreads), mg->tail_smem, c.s, P, c.kc));
+    if (lt < Lm) {
+        FLUB_TRY(launch_coarse(mg, c, R(lt), ZF(lt), nullptr, nullptr));
     } else {
         const int b = Lm - 1;
         const Level &L = mg->lv[b];
@@ -909,7 +843,7 @@ static int enqueue_vcycle(flub_mg *mg, const LaunchCtx &c, const float *r0, floa
         }
     }
     if (pers) FLUB_TRY(launch_leg<float>(mg, c, false, 1, lg));
-    for (int l = pers ? 0 : lge - 1; l >= 0; l--) {
+    for (int l = pers ? 0 : lg - 1; l >= 0; l--) {
         const Level &L = mg->lv[l];
         const int iters = level_iters(mg, l);
         if (l == 0 && split0) {
@@ -955,56 +889,19 @@ static int enqueue_vcycle(flub_mg *mg, const LaunchCtx &c, const float *r0, floa
     return FLUB_OK;
 }
 
-// Cluster or one-block kernel for the coarse levels from lt down, with FP16
-// (mixed precision) or FP32 top-level residual/correction.
-static int launch_coarse(flub_mg *mg, const LaunchCtx &c, int lt, const float *r_top, float *z_top,
-                         const __half *r_top_h, __half *z_top_h, bool global_half = false) {
-    if (mg->cl_start < mg->levels) {
-        ClusterParams P = {};
-        cluster_layout(mg, lt, mg->cl_size, &P);
-        P.r_top = r_top;
-        P.z_top = z_top;
-        P.r_top_h = r_top_h;
-        P.z_top_h = z_top_h;
-        if (global_half) fill_cluster_global(mg, lt - 1, true, &P.g);
-        cudaLaunchConfig_t cfg;
-        cudaLaunchAttribute attr[2];
-        cluster_launch_config(mg->cl_size, mg->cl_smem, c.s, &cfg, attr);
-        const cudaError_t e = P.g.on ? cudaLaunchKernelEx(&cfg, k_cluster_vcycle<true>, (const ClusterParams)P, c.kc)
-                                     : cudaLaunchKernelEx(&cfg, k_cluster_vcycle<false>, (const ClusterParams)P, c.kc);
-        if (e != cudaSuccess) {
-            set_last_error("cluster V-cycle launch: %s", cudaGetErrorString(e));
-            cudaGetLastError();
-            return FLUB_ERR_CUDA;
-        }
-        count_launches(1);
-        return FLUB_OK;
-    }
-    TailParams P = {};
-    tail_layout(mg, lt, &P);
-    P.r_top = r_top;
-    P.z_top = z_top;
-    P.r_top_h = r_top_h;
-    P.z_top_h = z_top_h;
-    return launch_pdl(k_tail_vcycle, dim3(1), dim3(kTailThreads), mg->tail_smem, c.s, P, c.kc);
-}
-
 // Mixed-precision V-cycle: the levels in global memory are FP16 at scale 8^-l
 // (mixed.cuh); the level-0 residual is read from its FP16 copy lv[0].rh, the
 // result z0 is FP32.  Same schedule as enqueue_vcycle.
 static int enqueue_vcycle_mixed(flub_mg *mg, const LaunchCtx &c, float *z0, bool z0_clean, int dot_mode = 0,
                                 bool *dot_fused = nullptr) {
     if (dot_fused) *dot_fused = false;
-    const bool use_cl = mg->cl_start < mg->levels;
-    const int Lm = mg->levels, lt = use_cl ? mg->cl_start : mg->tail_start;
+    const int Lm = mg->levels, lt = mg->co_start;
     const int sk = mg->skip_ok ? 1 : 0;
     const int sk0 = z0_clean ? sk : 0;
     const int lg = lt < Lm - 1 ? lt : Lm - 1;
     const bool pers = use_persist(mg, lg);
-    const bool clg = use_cl && use_cluster_global(mg, lt, sk);
-    const int lge = clg ? lt - 1 : lg;
-    const bool split0 = use_split(mg, lge, sk0, mg->lv[0].rh, z0);
-    for (int l = 0; l < (pers ? 1 : lge); l++) {
+    const bool split0 = use_split(mg, lg, sk0, mg->lv[0].rh, z0);
+    for (int l = 0; l < (pers ? 1 : lg); l++) {
         const Level &L = mg->lv[l];
         const int iters = level_iters(mg, l);
         if (l == 0 && split0) {
@@ -1044,9 +941,9 @@ static int enqueue_vcycle_mixed(flub_mg *mg, const LaunchCtx &c, float *z0, bool
     if (pers) FLUB_TRY(launch_leg<__half>(mg, c, true, 1, lg));
     if (lt < Lm) {
         if (lt == 0)
-            FLUB_TRY(launch_coarse(mg, c, 0, nullptr, z0, mg->lv[0].rh, nullptr));
+            FLUB_TRY(launch_coarse(mg, c, nullptr, z0, mg->lv[0].rh, nullptr));
         else
-            FLUB_TRY(launch_coarse(mg, c, lt, nullptr, nullptr, mg->lv[lt].rh, mg->lv[lt].zh, clg));
+            FLUB_TRY(launch_coarse(mg, c, nullptr, nullptr, mg->lv[lt].rh, mg->lv[lt].zh));
     } else {
         const int b = Lm - 1;
         const Level &L = mg->lv[b];
@@ -1066,7 +963,7 @@ static int enqueue_vcycle_mixed(flub_mg *mg, const LaunchCtx &c, float *z0, bool
         }
     }
     if (pers) FLUB_TRY(launch_leg<__half>(mg, c, false, 1, lg));
-    for (int l = pers ? 0 : lge - 1; l >= 0; l--) {
+    for (int l = pers ? 0 : lg - 1; l >= 0; l--) {
         const Level &L = mg->lv[l];
         const __half *zc = mg->lv[l + 1].zh;
         const int iters = level_iters(mg, l);
@@ -1377,6 +1274,16 @@ __global__ void __launch_bounds__(256) k_stencil_words(const uint8_t *__restrict
     }
 }
 
+// Stencil words of the levels the coarse kernel runs.
+static int enqueue_cell_words(flub_mg *mg, cudaStream_t s) {
+    for (int l = mg->co_start; l < mg->levels; l++) {
+        const Level &L = mg->lv[l];
+        k_cell_words<<<blocks_for(L.D.n(), 256), 256, 0, s>>>(L.code, L.cw, L.D);
+        FLUB_CHECK_LAUNCH();
+    }
+    return FLUB_OK;
+}
+
 // ---------------------------------------------------------------- warm-start support (no reference counterpart)
 
 // Stencil words in the colour-split order of smooth_split.cuh: natural cell
@@ -1607,25 +1514,24 @@ int flub_mg_create(int nx, int ny, int nz, int levels, int precision, void *work
     const char *hl = getenv("FLUB_SOLVE_HOST_LOOP");
     mg->host_loop = hl && hl[0] == '1';
     mg->skip_ok = true;  // the workspace is zeroed below and set_tags re-zeroes the z buffers
-    choose_tail(mg);
-    choose_cluster(mg);
+    choose_coarse(mg);
     choose_persist(mg);
     if (precision == FLUB_PRECISION_MIXED && bottom_in_tail(mg)) {
-        // mixed precision: FP64 at the coarsest level (the tail layouts grow by
-        // the bottom's doubles, so they are chosen again)
+        // mixed precision: FP64 at the coarsest level (the layout grows by the
+        // bottom's doubles, so it is chosen again)
         mg->bottom64 = true;
-        choose_tail(mg);
-        choose_cluster(mg);
+        choose_coarse(mg);
         if (!bottom_in_tail(mg)) {
             mg->bottom64 = false;
-            choose_tail(mg);
-            choose_cluster(mg);
+            choose_coarse(mg);
         }
     }
     if (precision == FLUB_PRECISION_MIXED) {
-        // the FP16 sweeps work on rows of 8 cells: every level left to the global
-        // kernels needs nz % 8 == 0
-        const int lt = mg->cl_start < mg->levels ? mg->cl_start : mg->tail_start;
+        // the FP16 sweeps work on rows of 8 cells: every level above the small
+        // ones needs nz % 8 == 0
+        bool small;
+        const int ls = small_levels_start(mg, &small);
+        const int lt = ls > mg->co_start ? ls : mg->co_start;
         const int last_global = lt < mg->levels ? lt - 1 : mg->levels - 1;
         for (int l = 0; l <= last_global; l++)
             if (mg->lv[l].D.nz % 8 != 0) {
@@ -1633,10 +1539,6 @@ int flub_mg_create(int nx, int ny, int nz, int levels, int precision, void *work
                 set_last_error("mixed precision needs nz %% 8 == 0 on level %d (nz = %d)", l, nz >> l);
                 return FLUB_ERR_UNSUPPORTED;
             }
-    }
-    if (set_tail_smem_limit() != FLUB_OK) {
-        flub_mg_destroy(mg);
-        return FLUB_ERR_CUDA;
     }
     // zero the state and all vectors once so that every buffer is defined
     if (cudaMemset(mg->ws, 0, need) != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) {
@@ -1674,12 +1576,7 @@ int flub_mg_set_tags(flub_mg *mg, const int32_t *tag, void *stream) {
         k_restrict_codes<<<blocks_for(C.D.n(), 256), 256, 0, s>>>(mg->lv[l].code, C.code, C.D);
         FLUB_CHECK_LAUNCH();
     }
-    for (int l = 0; l < mg->levels; l++) {
-        const Level &L = mg->lv[l];
-        if (!L.pmask) continue;
-        k_tail_masks<<<blocks_for(L.D.n() >> 1, 256), 256, 0, s>>>(L.code, L.D, L.pmask);
-        FLUB_CHECK_LAUNCH();
-    }
+    FLUB_TRY(enqueue_cell_words(mg, s));
     // stencil words and active 8-cell groups of every level that has them
     for (int l = 0; l < mg->levels; l++) {
         const Level &L = mg->lv[l];
@@ -1838,8 +1735,6 @@ int flub_mg_set_schedule(flub_mg *mg, int smooth_iters, int bottom_iters, float 
     mg->sched_nu = smooth_iters;
     mg->sched_bottom = bottom_iters;
     mg->sched_rscale = restrict_scale;
-    // the cluster kernel's layout depends on the schedule
-    FLUB_TRY(choose_cluster(mg));
     return FLUB_OK;
 }
 
@@ -1860,12 +1755,10 @@ int flub_mg_set_bottom_precision(flub_mg *mg, int bits) {
             mg->graph[g] = nullptr;
         }
     mg->bottom64 = want;
-    choose_tail(mg);
-    FLUB_TRY(choose_cluster(mg));
+    FLUB_TRY(choose_coarse(mg));
     if (want && !bottom_in_tail(mg)) {
         mg->bottom64 = false;
-        choose_tail(mg);
-        choose_cluster(mg);
+        choose_coarse(mg);
         set_last_error("flub_mg_set_bottom_precision: the FP64 bottom does not fit the coarse-level kernels");
         return FLUB_ERR_UNSUPPORTED;
     }
@@ -2054,7 +1947,7 @@ static size_t noalloc_layout(flub_mg *mg, char *base) {
         L.r = l ? (float *)take(sizeof(float) * L.D.n()) : nullptr;
         L.z = l ? (float *)take(sizeof(float) * L.D.n()) : nullptr;
         L.z2 = (float *)take(sizeof(float) * L.D.n());
-        L.pmask = nullptr;  // the tail builds its masks from the codes
+        L.cw = L.D.n() <= kCoarseMaxCells ? (uint16_t *)take(sizeof(uint16_t) * (size_t)L.D.n()) : nullptr;
     }
     return off;
 }
@@ -2104,9 +1997,7 @@ extern "C" int flub_vcycle_noalloc(const int32_t *tag, const float *r, float *z,
     void *base = nullptr;
     FLUB_TRY(noalloc_scratch_address(&base));
     noalloc_layout(&mg, (char *)base);
-    choose_tail(&mg);
-    choose_cluster(&mg);
-    FLUB_TRY(set_tail_smem_limit());
+    choose_coarse(&mg);
     cudaStream_t s = as_stream(stream);
     // every scratch element is written before it is read: the codes by these two
     // kernels, z_l by the first (from-zero) sweep of its level, r_l by the
@@ -2118,6 +2009,7 @@ extern "C" int flub_vcycle_noalloc(const int32_t *tag, const float *r, float *z,
         k_restrict_codes<<<blocks_for(C.D.n(), 256), 256, 0, s>>>(mg.lv[l].code, C.code, C.D);
         FLUB_CHECK_LAUNCH();
     }
+    FLUB_TRY(enqueue_cell_words(&mg, s));
     LaunchCtx c{s, nullptr, 0, 0};
     return enqueue_vcycle(&mg, c, r, z, false);  // mg.skip_ok is false: every sweep writes every cell
 }

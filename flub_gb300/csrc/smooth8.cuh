@@ -202,7 +202,7 @@ __device__ __forceinline__ float smooth_cell(uint32_t w, float xc, float xip, fl
 // spills.
 // kNC: r and zc may be read through the read-only (non-coherent) path, i.e.
 // nothing writes them while the kernel runs; false inside the persistent and
-// cluster V-cycle kernels (persist.cuh, cluster.cuh), where other blocks wrote
+// V-cycle kernels (persist.cuh), where other blocks wrote
 // them (and z) earlier in the same launch: then r, zc and z are read with
 // L2-only loads.  bid / nblk: this block's index and the number of blocks that
 // share the grid-stride loop.

@@ -40,7 +40,7 @@ struct St<float> {
         o[0] = a.x; o[1] = a.y;
     }
     // L2-only loads (ld.global.cg) of data other blocks wrote earlier in the
-    // same launch (persistent and cluster kernels)
+    // same launch (persistent kernels)
     static __device__ __forceinline__ float ld_cg(const float *p) { return __ldcg(p); }
     static __device__ __forceinline__ void ld2_cg(const float *p, float o[2]) {
         const float2 a = __ldcg(reinterpret_cast<const float2 *>(p));
