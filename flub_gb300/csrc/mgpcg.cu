@@ -26,6 +26,7 @@
 #include "persist.cuh"
 #include "restrict8.cuh"
 #include "smooth8.cuh"
+#include "smooth_block.cuh"
 #include "smooth_split.cuh"
 #include "smooth_tile.cuh"
 
@@ -68,8 +69,15 @@ struct Level {
     int *tiles, *tiles_n;
     int n_tiles;
     // stencil words of every cell in natural order, on levels the coarse kernel
-    // (coarse.cuh) can run; NULL on larger ones
+    // (coarse.cuh) can run or the blocked smoothing uses; NULL elsewhere
     uint16_t *cw;
+    // blocked smoothing (smooth_block.cuh): planes of a tile (0: not used on
+    // this level), the tiles with fluid and their number, and a third
+    // correction buffer (z3, or z3h in mixed precision) for the ping-pong
+    int b_ti, b_tiles;
+    uint32_t *b_list, *b_items;
+    int *b_n;
+    __half *z3h;
 };
 
 struct LaunchCtx {
@@ -134,6 +142,33 @@ static inline unsigned long long *kernel_counter(flub_mg *mg) {
     return reinterpret_cast<unsigned long long *>(reinterpret_cast<char *>(mg->st) + offsetof(MgState, kernels));
 }
 
+// Cells of one colour per thread item: rows are split into vectors of this many.
+static inline int row_vector(int nz) { return nz % 8 == 0 ? 4 : (nz % 4 == 0 ? 2 : 1); }
+
+static inline int block_row(const Dims D) { return (D.nz <= kKB + 2 * kKHalo ? D.nz : kKB + 2 * kKHalo) >> 1; }
+static inline int block_tiles_k(const Dims D) { return D.nz <= kKB + 2 * kKHalo ? 1 : (D.nz + kKB - 1) / kKB; }
+static inline int block_tiles(const Dims D, int ti) {
+    return ((D.nx + ti - 1) / ti) * ((D.ny + kTJb - 1) / kTJb) * block_tiles_k(D);
+}
+
+// Planes of a tile of the blocked smoothing on level l, or 0 where it is not
+// used: level 0 of a mixed-precision handle (its post-smoothing stores FP32),
+// levels one block of the coarse kernel holds, and rows of
+// odd pairs so long that a block has fewer threads than a tile has rows.
+// Not above 256 tiles either: a tile takes 6 us for four half-sweeps (13,000
+// cycles: 3,000 to load, 7,000 of sweeps bound by shared-memory bandwidth), so
+// on a larger level, full of fluid, waves of them take longer than four
+// launches over all of it (128^3, 1024 tiles: 13 us a half-sweep against 6.1).
+static int block_planes(const flub_mg *mg, int l) {
+    const Dims D{mg->nx >> l, mg->ny >> l, mg->nz >> l};
+    if (mg->tile_ok || D.n() <= kBlockCells || D.n() >= (int64_t)1 << 30 || D.nz % 2 != 0) return 0;
+    if (D.nx > 4 * 2047 || D.ny > kTJb * 2047 || D.nz > kKB * 1023) return 0;  // packed tile coordinates
+    if (l == 0 && (mg->precision == FLUB_PRECISION_MIXED || mg->levels < 2)) return 0;
+    const int V = row_vector(D.nz);
+    if (kBlockThreads / (block_row(D) / V) < kTJb + 6) return 0;
+    return block_tiles(D, 4) <= 256 ? 4 : 0;
+}
+
 // Workspace carve-up; with base == nullptr only the size is computed.
 static size_t carve(flub_mg *mg, char *base) {
     size_t off = 0;
@@ -196,7 +231,22 @@ static size_t carve(flub_mg *mg, char *base) {
             L.tiles = (int *)take(sizeof(int) * (size_t)L.n_tiles);
             L.tiles_n = (int *)take(sizeof(int));
         }
-        L.cw = nl <= kCoarseMaxCells ? (uint16_t *)take(sizeof(uint16_t) * (size_t)nl) : nullptr;
+        L.b_ti = block_planes(mg, l);
+        L.cw = nl <= kCoarseMaxCells || L.b_ti ? (uint16_t *)take(sizeof(uint16_t) * (size_t)nl) : nullptr;
+        L.b_tiles = 0;
+        L.b_list = L.b_items = nullptr;
+        L.b_n = nullptr;
+        L.z3h = nullptr;
+        if (L.b_ti) {
+            L.b_tiles = block_tiles(L.D, L.b_ti);
+            L.b_list = (uint32_t *)take(sizeof(uint32_t) * (size_t)L.b_tiles);
+            L.b_items = (uint32_t *)take(sizeof(uint32_t) * (size_t)(nl / row_vector(L.D.nz)));
+            L.b_n = (int *)take(sizeof(int));
+            if (mg->precision == FLUB_PRECISION_MIXED)
+                L.z3h = (__half *)take(sizeof(__half) * nl);
+            else if (!L.z3)
+                L.z3 = (float *)take(sizeof(float) * nl);
+        }
     }
     // per-block counts of the active-list build (level 0 has the most blocks)
     mg->act_scratch = (int *)take(sizeof(int) * (size_t)((n / 8 + kActPerBlock - 1) / kActPerBlock + 1));
@@ -251,7 +301,7 @@ static size_t coarse_layout(const flub_mg *mg, int lc, int C, CoarseParams *P) {
         L.abs_level = lc + t;
         L.P = t < nd ? p0 >> t : L.D.nx;
         const int hz = L.D.nz >> 1;
-        L.V = hz % 4 == 0 ? 4 : (hz % 2 == 0 ? 2 : 1);
+        L.V = row_vector(L.D.nz);
         const size_t cells = (size_t)L.P * L.D.ny * L.D.nz;
         L.hn = (coarse_row(L.P + 1, 0, L.D.ny, hz) + 3) & ~3;  // planes -1 .. P
         L.off_z = take(sizeof(float) * 2 * (size_t)L.hn);
@@ -735,6 +785,85 @@ static int tile_side(flub_mg *mg, const LaunchCtx &c, int l, bool post, int iter
     return FLUB_OK;
 }
 
+// ---------------------------------------------------------------- blocked smoothing (smooth_block.cuh)
+
+template <int V, typename T, int TI, int S>
+static int block_launch(const LaunchCtx &c, const Level &L, const BlockArgs &A) {
+    const size_t smem = block_smem(TI, S, A.ks, V);
+    if (!A.tiles) {  // block_prepare: the kernel's shared-memory limit on this device
+        FLUB_CHECK_CUDA(cudaFuncSetAttribute(k_smooth_block<V, T, TI, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)block_smem(TI, S, (kKB + 2 * kKHalo) / 2, V)));
+        return FLUB_OK;
+    }
+    const int blocks = L.b_tiles < kNumSMs ? L.b_tiles : kNumSMs;
+    return launch_pdl(k_smooth_block<V, T, TI, S>, dim3(blocks), dim3(kBlockThreads), smem, c.s, A, c.kc);
+}
+
+// One launch of `its` red-black iterations (1 or 2).
+template <typename T>
+static int block_iterations(const LaunchCtx &c, const Level &L, int its, int mode, bool post, const T *r, const T *zin,
+                            T *zout, const T *zc, float zc_scale, bool prepare = false) {
+    BlockArgs A = {};
+    A.D = L.D;
+    A.tiles = prepare ? nullptr : L.b_list;
+    A.tiles_n = L.b_n;
+    A.items = L.b_items;
+    A.cw = L.cw;
+    A.r = r;
+    A.zin = zin;
+    A.zout = zout;
+    A.zc = zc;
+    A.zc_scale = zc_scale;
+    A.mode = mode;
+    A.first_odd = post ? 0 : 1;
+    A.ks = block_row(L.D);
+    const int V = row_vector(L.D.nz);
+    if (V == 4) {
+        return its == 2 ? block_launch<4, T, 4, 4>(c, L, A) : block_launch<4, T, 4, 2>(c, L, A);
+    }
+    if constexpr (std::is_same<T, float>::value) {
+        if (V == 2) return its == 2 ? block_launch<2, T, 4, 4>(c, L, A) : block_launch<2, T, 4, 2>(c, L, A);
+        return its == 2 ? block_launch<1, T, 4, 4>(c, L, A) : block_launch<1, T, 4, 2>(c, L, A);
+    }
+    return FLUB_ERR_UNSUPPORTED;
+}
+
+// The shared-memory limits of a handle's blocked smoothing kernels.
+static int block_prepare(flub_mg *mg) {
+    const LaunchCtx c{nullptr, nullptr, 0, 0};
+    for (int l = 0; l < mg->levels; l++)
+        for (int its = 1; its <= 2 && mg->lv[l].b_ti; its++) {
+            if (mg->precision == FLUB_PRECISION_MIXED) {
+                if (mg->lv[l].D.nz % 8 == 0)
+                    FLUB_TRY(block_iterations<__half>(c, mg->lv[l], its, 0, false, nullptr, nullptr, nullptr, nullptr,
+                                                      1.0f, true));
+            } else {
+                FLUB_TRY(block_iterations<float>(c, mg->lv[l], its, 0, false, nullptr, nullptr, nullptr, nullptr, 1.0f,
+                                                 true));
+            }
+        }
+    return FLUB_OK;
+}
+
+// Pre-smoothing (iters iterations from z = 0, odd colour first) ending in
+// z_fin, or post-smoothing (from z_pre + P zc, even colour first) ending in
+// z_fin, two iterations a launch; the launches alternate between z_fin and z3
+// so that the last one writes z_fin.
+template <typename T>
+static int block_side(const LaunchCtx &c, const Level &L, bool post, int iters, const T *r, const T *z_pre, T *z_fin,
+                      T *z3, const T *zc, float zc_scale) {
+    const int launches = (iters + 1) / 2;
+    const T *prev = z_pre;
+    for (int t = 0; t < launches; t++) {
+        T *w = ((launches - 1 - t) % 2 == 0) ? z_fin : z3;
+        const int mode = t ? kBlockPlain : (post ? kBlockProlong : kBlockFromZero);
+        FLUB_TRY(block_iterations<T>(c, L, t + 1 == launches && iters % 2 ? 1 : 2, mode, post, r, prev, w, zc,
+                                     zc_scale));
+        prev = w;
+    }
+    return FLUB_OK;
+}
+
 // The coarse kernel from level co_start down, with FP16 (mixed precision) or
 // FP32 residual and correction of its first level.
 static int launch_coarse(flub_mg *mg, const LaunchCtx &c, const float *r_top, float *z_top, const __half *r_top_h,
@@ -781,8 +910,11 @@ static int enqueue_vcycle(flub_mg *mg, const LaunchCtx &c, const float *r0, floa
     auto TILED_POST = [&](int l) { return mg->tile_ok && mg->lv[l].n_tiles > 0 && SK(l) == 1; };
     // levels 1 .. lg-1 in the persistent cooperative kernels, or one launch per pass
     const bool pers = use_persist(mg, lg);
+    // blocked smoothing (smooth_block.cuh): neighbouring tiles read r and the
+    // input while others write the output
+    auto BLOCK = [&](int l) { return mg->lv[l].b_ti && sk == 1 && (l > 0 || r0 != z0); };
     // level 0 on colour-split storage (smooth_split.cuh)
-    const bool split0 = use_split(mg, lg, sk, r0, z0);
+    const bool split0 = !BLOCK(0) && use_split(mg, lg, sk, r0, z0);
     for (int l = 0; l < (pers ? 1 : lg); l++) {
         const Level &L = mg->lv[l];
         const int iters = level_iters(mg, l);
@@ -810,6 +942,8 @@ static int enqueue_vcycle(flub_mg *mg, const LaunchCtx &c, const float *r0, floa
         }
         if (TILED_PRE(l)) {
             FLUB_TRY(tile_side(mg, c, l, false, iters, R(l), nullptr, ZP(l), nullptr));
+        } else if (BLOCK(l)) {
+            FLUB_TRY(block_side<float>(c, L, false, iters, R(l), nullptr, ZP(l), L.z3, nullptr, 1.0f));
         } else {
             for (int it = 0; it < iters; it++) {
                 FLUB_TRY(sweep(c, L, 0, it == 0 ? kSweepFromZero : kSweepInPlace, sk, R(l), ZP(l), ZP(l), nullptr));
@@ -880,6 +1014,12 @@ static int enqueue_vcycle(flub_mg *mg, const LaunchCtx &c, const float *r0, floa
             FLUB_TRY(tile_side(mg, c, l, true, iters, R(l), ZP(l), ZF(l), mg->lv[l + 1].z));
             continue;
         }
+        if (BLOCK(l)) {
+            // only tiles with fluid are written: a caller's z0 gets 0 everywhere else first
+            if (l == 0 && !z0_clean) FLUB_CHECK_CUDA(cudaMemsetAsync(z0, 0, sizeof(float) * (size_t)mg->n, c.s));
+            FLUB_TRY(block_side<float>(c, L, true, iters, R(l), ZP(l), ZF(l), L.z3, mg->lv[l + 1].z, 1.0f));
+            continue;
+        }
         for (int it = 0; it < iters; it++) {
             FLUB_TRY(sweep(c, L, 1, it == 0 ? kSweepProlong : kSweepInPlace, SK(l), R(l), ZP(l), ZF(l),
                            mg->lv[l + 1].z));
@@ -926,7 +1066,9 @@ static int enqueue_vcycle_mixed(flub_mg *mg, const LaunchCtx &c, float *z0, bool
                                 0.125f * mg->sched_rscale, (const int *)C.act, (const int *)C.act_n, c.kc));
             continue;
         }
-        for (int it = 0; it < iters; it++) {
+        if (L.b_ti && sk == 1) {
+            FLUB_TRY(block_side<__half>(c, L, false, iters, L.rh, nullptr, L.z2h, L.z3h, nullptr, 1.0f));
+        } else for (int it = 0; it < iters; it++) {
             FLUB_TRY(sweep8<__half, __half, __half, __half>(c, L, 0, it == 0 ? kSweepFromZero : kSweepInPlace, sk,
                                                             L.rh, L.z2h, L.z2h, nullptr, 1.0f));
             FLUB_TRY(sweep8<__half, __half, __half, __half>(c, L, 1, kSweepInPlace, sk, L.rh, L.z2h, L.z2h, nullptr,
@@ -997,6 +1139,10 @@ static int enqueue_vcycle_mixed(flub_mg *mg, const LaunchCtx &c, float *z0, bool
                     FLUB_TRY((split_sweep<kInPlace, H, H, float, float, float>(c, L, 0, nullptr, L.rsh, nullptr,
                                                                                L.zs, nullptr, 1.0f, nullptr)));
             }
+            continue;
+        }
+        if (l > 0 && L.b_ti && sk == 1) {
+            FLUB_TRY(block_side<__half>(c, L, true, iters, L.rh, L.z2h, L.zh, L.z3h, zc, 8.0f));
             continue;
         }
         for (int it = 0; it < iters; it++) {
@@ -1274,10 +1420,11 @@ __global__ void __launch_bounds__(256) k_stencil_words(const uint8_t *__restrict
     }
 }
 
-// Stencil words of the levels the coarse kernel runs.
+// Stencil words of the levels the coarse kernel or the blocked smoothing runs.
 static int enqueue_cell_words(flub_mg *mg, cudaStream_t s) {
-    for (int l = mg->co_start; l < mg->levels; l++) {
+    for (int l = 0; l < mg->levels; l++) {
         const Level &L = mg->lv[l];
+        if (!L.cw || (l < mg->co_start && !L.b_ti)) continue;
         k_cell_words<<<blocks_for(L.D.n(), 256), 256, 0, s>>>(L.code, L.cw, L.D);
         FLUB_CHECK_LAUNCH();
     }
@@ -1540,6 +1687,10 @@ int flub_mg_create(int nx, int ny, int nz, int levels, int precision, void *work
                 return FLUB_ERR_UNSUPPORTED;
             }
     }
+    if (block_prepare(mg) != FLUB_OK) {
+        flub_mg_destroy(mg);
+        return FLUB_ERR_CUDA;
+    }
     // zero the state and all vectors once so that every buffer is defined
     if (cudaMemset(mg->ws, 0, need) != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) {
         flub_mg_destroy(mg);
@@ -1577,6 +1728,23 @@ int flub_mg_set_tags(flub_mg *mg, const int32_t *tag, void *stream) {
         FLUB_CHECK_LAUNCH();
     }
     FLUB_TRY(enqueue_cell_words(mg, s));
+    for (int l = 0; l < mg->co_start && l < mg->levels; l++) {
+        const Level &L = mg->lv[l];
+        if (!L.b_ti) continue;
+        FLUB_CHECK_CUDA(cudaMemsetAsync(L.b_n, 0, sizeof(int), s));
+        k_block_tiles<<<L.b_tiles, 128, 0, s>>>(L.code, L.D, L.b_ti, (L.D.ny + kTJb - 1) / kTJb, block_tiles_k(L.D),
+                                                L.b_list, L.b_n);
+        FLUB_CHECK_LAUNCH();
+        const int V = row_vector(L.D.nz);
+        const unsigned blocks = blocks_for(L.D.n() / (2 * V), 256);
+        if (V == 4)
+            k_block_items<4><<<blocks, 256, 0, s>>>(L.cw, L.D, L.b_items);
+        else if (V == 2)
+            k_block_items<2><<<blocks, 256, 0, s>>>(L.cw, L.D, L.b_items);
+        else
+            k_block_items<1><<<blocks, 256, 0, s>>>(L.cw, L.D, L.b_items);
+        FLUB_CHECK_LAUNCH();
+    }
     // stencil words and active 8-cell groups of every level that has them
     for (int l = 0; l < mg->levels; l++) {
         const Level &L = mg->lv[l];
@@ -1621,6 +1789,7 @@ int flub_mg_set_tags(flub_mg *mg, const int32_t *tag, void *stream) {
         char *last = L.z2h ? reinterpret_cast<char *>(L.z2h) + b / 2 : reinterpret_cast<char *>(L.z2) + b;
         FLUB_CHECK_CUDA(cudaMemsetAsync(first, 0, (size_t)(last - first), s));
         if (L.z3) FLUB_CHECK_CUDA(cudaMemsetAsync(L.z3, 0, b, s));
+        if (L.z3h) FLUB_CHECK_CUDA(cudaMemsetAsync(L.z3h, 0, b / 2, s));
     }
     FLUB_CHECK_CUDA(cudaMemsetAsync(mg->p, 0, sizeof(float) * (size_t)mg->n, s));
     FLUB_CHECK_CUDA(cudaMemsetAsync(mg->Ap, 0, sizeof(float) * (size_t)mg->n, s));

@@ -42,3 +42,28 @@ def test_coarse_levels_bit_exact(shape, levels, no_cluster, monkeypatch):
     z = mg.apply_preconditioner(rd).cpu().numpy()
     with O.schedule(2, 4, 0.5):
         assert np.array_equal(z, O.vcycle(r, tags, np.float32))
+
+
+# shape, levels, precision: rows of every item width with and without a halo
+# along k, tiles with remainders along every axis, levels just above the coarse
+# kernel's, and level 0 itself
+BLOCKED = [((48, 40, 44), 2), ((64, 64, 64), 2), ((41, 44, 42), 1), ((42, 44, 52), 2), ((128, 32, 64), 3),
+           ((50, 36, 88), 2), ((34, 30, 104), 2), ((128, 64, 128), 4), ((104, 72, 88), 3)]
+
+
+@pytest.mark.parametrize("nu", [1, 2, 3, 4])
+@pytest.mark.parametrize("shape,levels", BLOCKED)
+def test_blocked_smoothing_bit_exact(shape, levels, nu):
+    """smooth_block.cuh: one and two iterations a launch, odd and even numbers
+    of launches a side (the ping-pong of the buffers)."""
+    tag, r = _case(shape, sum(shape) + nu)
+    mg = MGPCG(3, shape, levels, float)
+    mg.set_tags(torch.from_numpy(tag).cuda())
+    mg.set_schedule(nu, 3, 0.5)
+    rd = torch.from_numpy(r).cuda()
+    tags = O.tag_levels(tag, levels)
+    with O.schedule(nu, 3, 0.5):
+        want = O.vcycle(r, tags, np.float32)
+    z = torch.full(shape, float("nan"), device="cuda")  # every cell is written
+    assert np.array_equal(mg.apply_preconditioner(rd, z).cpu().numpy(), want)
+    assert np.array_equal(mg.apply_preconditioner(rd, rd.clone()).cpu().numpy(), want)
