@@ -9,8 +9,12 @@
 // One thread per output element on a division-free row grid (k along
 // threadIdx.x, j = blockIdx.y, i = blockIdx.z): the 32 threads of a warp read
 // neighbouring k, so every gather instruction of the trace and the stencils
-// touches one or two cache lines.  The kernels are bound by L1 gather
-// throughput (about 280 loads per MacCormack element), not by HBM.
+// touches one or two cache lines.  The kernels are bound by instruction issue
+// and L1 gathers, not by HBM: a MacCormack element whose bounds leave no room
+// for the correction takes 144 loads (one trace and one tricubic), else 257.
+// Samples away from the array's ends address their rows from one base.
+// Measured on 256 x 64 x 256 (advect_phi and three face arrays): 1204 us with
+// both traces always taken and every index clamped on its own, 750 us now.
 #include <cmath>
 
 #include "common.cuh"
@@ -58,17 +62,32 @@ __device__ __forceinline__ float adv_lerp(float a, float b, float t) {
     return __fadd_rn(__fmul_rn(a, __fsub_rn(1.0f, t)), __fmul_rn(b, t));
 }
 
-// The eight corners (x.a|x.b, y.a|y.b, z.a|z.b) of q (plane stride sp, row
-// stride sr) blended as utils/util.py:55-88 and :106-120 write it:
+// The blend of eight corners (a..h = 000, 100, 010, 110, 001, 101, 011, 111)
+// as utils/util.py:55-88 and :106-120 write it:
 // lerp(lerp(lerp(a,b,fa), lerp(c,d,fa), fb), lerp(lerp(e,f,fa), lerp(g,h,fa), fb), fc).
+__device__ __forceinline__ float adv_blend8(float a, float b, float c, float d, float e, float f, float g, float h,
+                                            float fa, float fb, float fc) {
+    return adv_lerp(adv_lerp(adv_lerp(a, b, fa), adv_lerp(c, d, fa), fb),
+                    adv_lerp(adv_lerp(e, f, fa), adv_lerp(g, h, fa), fb), fc);
+}
+
+// The corners (x.a|x.b, y.a|y.b, z.a|z.b) of q (plane stride sp, row stride sr).
 __device__ __forceinline__ float adv_tri8(const float *__restrict__ q, int sp, int sr, AdvPair x, AdvPair y, AdvPair z,
                                           float fa, float fb, float fc) {
     const float *paa = q + (x.a * sp + y.a * sr), *pba = q + (x.b * sp + y.a * sr);
     const float *pab = q + (x.a * sp + y.b * sr), *pbb = q + (x.b * sp + y.b * sr);
-    const float a = __ldg(paa + z.a), b = __ldg(pba + z.a), c = __ldg(pab + z.a), d = __ldg(pbb + z.a);
-    const float e = __ldg(paa + z.b), f = __ldg(pba + z.b), g = __ldg(pab + z.b), h = __ldg(pbb + z.b);
-    return adv_lerp(adv_lerp(adv_lerp(a, b, fa), adv_lerp(c, d, fa), fb),
-                    adv_lerp(adv_lerp(e, f, fa), adv_lerp(g, h, fa), fb), fc);
+    return adv_blend8(__ldg(paa + z.a), __ldg(pba + z.a), __ldg(pab + z.a), __ldg(pbb + z.a), __ldg(paa + z.b),
+                      __ldg(pba + z.b), __ldg(pab + z.b), __ldg(pbb + z.b), fa, fb, fc);
+}
+
+// The same where no corner is clamped: (x, y, z) + {0, 1}^3 from one base, four
+// row addresses and immediate offsets instead of eight addresses.
+__device__ __forceinline__ float adv_tri8_in(const float *__restrict__ q, int sp, int sr, int x, int y, int z,
+                                             float fa, float fb, float fc) {
+    const float *p = q + (x * sp + y * sr + z);
+    const float *p10 = p + sp, *p01 = p + sr, *p11 = p10 + sr;
+    return adv_blend8(__ldg(p), __ldg(p10), __ldg(p01), __ldg(p11), __ldg(p + 1), __ldg(p10 + 1), __ldg(p01 + 1),
+                      __ldg(p11 + 1), fa, fb, fc);
 }
 
 // utils/util.py:34-88 sample_velocity_3d.  The three components share their
@@ -78,10 +97,19 @@ __device__ __forceinline__ AdvF3 adv_velocity(const AdvVel &M, AdvF3 p) {
     const float s = __fsub_rn(p.x, 0.5f), t = __fsub_rn(p.y, 0.5f), r = __fsub_rn(p.z, 0.5f);
     const float fu = adv_fract(p.x), fv = adv_fract(p.y), fw = adv_fract(p.z);
     const float fs = adv_fract(s), ft = adv_fract(t), fr = adv_fract(r);
-    const AdvPair xu = adv_pair(adv_floor(p.x), nx), xs = adv_pair(adv_floor(s), nx - 1);
-    const AdvPair yv = adv_pair(adv_floor(p.y), ny), yt = adv_pair(adv_floor(t), ny - 1);
-    const AdvPair zw = adv_pair(adv_floor(p.z), nz), zr = adv_pair(adv_floor(r), nz - 1);
+    const int iu = adv_floor(p.x), iv = adv_floor(p.y), iw = adv_floor(p.z);
+    const int is = adv_floor(s), it = adv_floor(t), ir = adv_floor(r);
     AdvF3 o;
+    // s = x - 1/2 rounded: is <= iu, so these bound all six indices
+    if (is >= 0 && iu < nx - 1 && it >= 0 && iv < ny - 1 && ir >= 0 && iw < nz - 1) {
+        o.x = adv_tri8_in(M.u, ny * nz, nz, iu, it, ir, fu, ft, fr);
+        o.y = adv_tri8_in(M.v, (ny + 1) * nz, nz, is, iv, ir, fs, fv, fr);
+        o.z = adv_tri8_in(M.w, ny * (nz + 1), nz + 1, is, it, iw, fs, ft, fw);
+        return o;
+    }
+    const AdvPair xu = adv_pair(iu, nx), xs = adv_pair(is, nx - 1);
+    const AdvPair yv = adv_pair(iv, ny), yt = adv_pair(it, ny - 1);
+    const AdvPair zw = adv_pair(iw, nz), zr = adv_pair(ir, nz - 1);
     o.x = adv_tri8(M.u, ny * nz, nz, xu, yt, zr, fu, ft, fr);
     o.y = adv_tri8(M.v, (ny + 1) * nz, nz, xs, yv, zr, fs, fv, fr);
     o.z = adv_tri8(M.w, ny * (nz + 1), nz + 1, xs, yt, zw, fs, ft, fw);
@@ -144,10 +172,28 @@ __device__ __forceinline__ void adv_quad(int i0, int hi, int stride, int o[4]) {
 // second, then the third.
 __device__ __forceinline__ float adv_tricubic(const AdvVol &Q, float s, float t, float r) {
     const AdvW4 wu = adv_cubic_w(adv_fract(s)), wv = adv_cubic_w(adv_fract(t)), ww = adv_cubic_w(adv_fract(r));
+    const int is = adv_floor(s), it = adv_floor(t), ir = adv_floor(r);
+    if (is >= 1 && is < Q.gx - 2 && it >= 1 && it < Q.gy - 2 && ir >= 1 && ir < Q.gz - 2) {
+        // no index is clamped: 16 row addresses, the third axis in immediate offsets
+        const int sr = Q.gz, sp = Q.gy * Q.gz;
+        const float *base = Q.q + (is * sp + it * sr + ir);
+        float qv[4][4];  // [third][second axis]
+#pragma unroll
+        for (int n = 0; n < 4; n++) {
+            const float *p0 = base + (n - 1) * sr - sp, *p1 = p0 + sp, *p2 = p1 + sp, *p3 = p2 + sp;
+#pragma unroll
+            for (int m = 0; m < 4; m++)
+                qv[m][n] = adv_dot4(__ldg(p0 + m - 1), __ldg(p1 + m - 1), __ldg(p2 + m - 1), __ldg(p3 + m - 1), wu);
+        }
+        float q4[4];
+#pragma unroll
+        for (int m = 0; m < 4; m++) q4[m] = adv_dot4(qv[m][0], qv[m][1], qv[m][2], qv[m][3], wv);
+        return adv_dot4(q4[0], q4[1], q4[2], q4[3], ww);
+    }
     int oi[4], oj[4], ok[4];
-    adv_quad(adv_floor(s), Q.gx - 1, Q.gy * Q.gz, oi);
-    adv_quad(adv_floor(t), Q.gy - 1, Q.gz, oj);
-    adv_quad(adv_floor(r), Q.gz - 1, 1, ok);
+    adv_quad(is, Q.gx - 1, Q.gy * Q.gz, oi);
+    adv_quad(it, Q.gy - 1, Q.gz, oj);
+    adv_quad(ir, Q.gz - 1, 1, ok);
     float qw[4];
 #pragma unroll
     for (int m = 0; m < 4; m++) {
@@ -218,23 +264,28 @@ __global__ void __launch_bounds__(kRowThreads) k_advect_mc(const AdvVel M, const
         (STAGE == 1 ? q_out : q_tmp)[f] = q;
         return;
     }
-    // foot over dt (pf) and over -dt (pb), and the tricubic samples there,
-    // as one loop of two so that the code is held once
-    AdvF3 pf = p, pb = p;
-    float q_sl = 0.0f, q_bk = 0.0f;
+    // foot over dt (pf) and over -dt, and the tricubic samples there, as one
+    // loop of two so that the code is held once.  Between them the bounds: the
+    // corrected value is kept where it lies strictly between them, so without
+    // mn < mx (a constant field, or the reference's minmax divisor, whose eight
+    // values are one corner of the array) it cannot be, whatever it is, and the
+    // second trace is not taken.
+    float q_sl = 0.0f, q_bk = 0.0f, mn = 0.0f, mx = 0.0f;
 #pragma unroll 1
     for (int s = 0; s < (STAGE == 0 ? 2 : 1); s++) {
         const AdvF3 e = adv_backtrace_v1(M, p, v1, s ? C.c1[1] : C.c1[0], s ? C.c2[1] : C.c2[0], s ? C.c3[1] : C.c3[0]);
         const float q = adv_sample_stagger(Q, e, st);
         if (s == 0) {
-            pf = e;
             q_sl = q;
+            adv_minmax(Q, e, mh, inv_mh, st, mn, mx);
+            if (!(mn < mx)) {
+                q_out[f] = q_sl;
+                return;
+            }
         } else {
-            pb = e;
             q_bk = q;
         }
     }
-    (void)pb;
     float qo, qt;
     if (STAGE == 3) {
         qo = q_out[f];
@@ -244,8 +295,6 @@ __global__ void __launch_bounds__(kRowThreads) k_advect_mc(const AdvVel M, const
         qt = q_bk;
     }
     const float q = __fadd_rn(qo, __fmul_rn(0.5f, __fsub_rn(__ldg(Q.q + f), qt)));
-    float mn, mx;
-    adv_minmax(Q, pf, mh, inv_mh, st, mn, mx);
     q_out[f] = (mn < q && q < mx) ? q : q_sl;
 }
 
