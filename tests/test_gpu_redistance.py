@@ -97,3 +97,31 @@ def test_redistance_rejects_bad_arguments():
         launch(_sweep, dim=(8, 8, 8), inputs=[g, 2, 1, 1, 0, 0.1])
     with pytest.raises(FlubError):
         init_distance(g, 0.1, 1, out=g)
+
+
+@pytest.mark.parametrize("n", [(6, 5, 255), (5, 9, 256), (4, 6, 257), (7, 4, 521), (3, 5, 2048), (3, 4, 2050)])
+@pytest.mark.parametrize("set_boundary", [0, 1])
+def test_redistance_row_lengths_bit_exact(n, set_boundary):
+    """Rows around a warp's 256 cells, odd ones, and the longest that is swept
+    with its even cells first (2048) against the next even length."""
+    phi, h = _field(n, 6)
+    phi[:, :, ::37] *= -1.0
+    ref = O.redistance(phi, h, set_boundary)
+    g = dev(phi)
+    redistance(g, h, set_boundary)
+    assert np.array_equal(host(g), ref)
+
+
+def test_redistance_values_beyond_the_initial_distance():
+    """Boundary values above 2 and non-finite ones (kept with set_boundary 0)
+    next to cells without a distance."""
+    phi, h = _field((20, 18, 40), 7)
+    rng = np.random.default_rng(8)
+    edge = np.ones(phi.shape, bool)
+    edge[1:-1, 1:-1, 1:-1] = False
+    vals = rng.choice([F(2.0), F(-2.0), F(7.5), F(-3.0), F(np.inf), F(0.1)], size=phi.shape)
+    phi = np.where(edge, vals, phi).astype(F)
+    ref = O.redistance(phi, h, 0)
+    g = dev(phi)
+    redistance(g, h, 0)
+    assert np.array_equal(host(g), ref, equal_nan=True)  # inf next to the surface makes NaN
