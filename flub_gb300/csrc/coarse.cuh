@@ -28,7 +28,11 @@
 // layout), against one cluster barrier per half-sweep on natural-order z with
 // six scalar neighbour loads a cell: 32^3 2.1 / 1.4 -> 0.47 / 0.41 us, 16^3 in
 // one block 0.40 -> 0.37 / 0.23 us, 64 x 16 x 64 in one launch each 2.6 -> 0.6
-// us.  At 32^3 the exchange of planes is 0.27 us of it.
+// us.  At 32^3 the exchange of planes is 0.27 us of it.  What a launch costs
+// beside its half-sweeps (reading words and residual, changing levels) is
+// latency as well, so its loads are issued in batches and the correction that
+// the whole cluster prolongates from block 0 is copied row by row first: 21.1
+// -> 19.2 us on three levels from 32^3.
 //
 // A block stores its first and last plane of each half-sweep into the
 // neighbouring blocks' ghost planes (distributed shared memory) and waits for
@@ -605,9 +609,23 @@ __device__ __noinline__ CoarseSync coarse_level(const CoarseParams &P, int t, in
         // others stay 0).  The parents of cell m of either colour are the same
         // coarse cell: (i / 2, j / 2, V kg + m).
         const CoarseLevel &C = P.lv[t + 1];
-        const bool remote = dist && t + 1 == P.nd;  // the coarse level is in block 0
         const float *zc = reinterpret_cast<const float *>(smem + C.off_z);
         const int chz = C.D.nz >> 1;
+        int chn = C.hn;  // floats per half of zc, whose first plane is this block's
+        if (dist && t + 1 == P.nd) {
+            // the coarse level is in block 0: a copy of this block's planes first,
+            // whole rows at a time (every block reads from the one)
+            const int first = coarse_row(i0 >> 1, 0, C.D.ny, chz);
+            const int len = ((np >> 1) * (C.D.ny + 1)) * chz;
+            float *v = reinterpret_cast<float *>(smem + P.off_v);
+            for (int q = threadIdx.x; q < 2 * len; q += kCoarseThreads) {
+                const int h = q >= len ? 1 : 0, x = q - h * len;
+                v[q] = remote_load(remote_addr(zc + h * C.hn + first + x, 0));
+            }
+            __syncthreads();
+            zc = v - coarse_row(0, 0, C.D.ny, chz);
+            chn = len;
+        }
 #pragma unroll
         for (int s = 0; s < Q; s++) {
             CoarseItem<V> &x = it[s];
@@ -615,13 +633,12 @@ __device__ __noinline__ CoarseSync coarse_level(const CoarseParams &P, int t, in
             const int e = threadIdx.x + s * kCoarseThreads;
             const int row = coarse_div(e, L.div_seg), kg = e - row * segs;
             const int il = coarse_div(row, L.div_ny), j = row - il * D.ny, I = (i0 + il) >> 1, J = j >> 1;
-            const float *pc = zc + coarse_row(remote ? I : il >> 1, J, C.D.ny, chz);
+            const float *pc = zc + coarse_row(il >> 1, J, C.D.ny, chz);
             float add[V];
 #pragma unroll
             for (int m = 0; m < V; m++) {
                 const int K = V * kg + m;
-                const float *q = pc + ((I + J + K) & 1) * C.hn + (K >> 1);
-                add[m] = remote ? remote_load(remote_addr(q, 0)) : *q;
+                add[m] = pc[((I + J + K) & 1) * chn + (K >> 1)];
             }
 #pragma unroll
             for (int c = 0; c < 2; c++) {
@@ -782,10 +799,20 @@ __global__ void __launch_bounds__(kCoarseThreads, 1) k_coarse_vcycle(const __gri
         const int pairs = (max(0, min(L.P, L.D.nx - first)) * yz) >> 1;
         const uint32_t *w2 = reinterpret_cast<const uint32_t *>(L.cw) + ((first * yz) >> 1);
         CoarseWeights *W = reinterpret_cast<CoarseWeights *>(smem + L.off_w);
-        for (int q = threadIdx.x; q < pairs; q += kCoarseThreads) {
-            const uint32_t w = __ldg(w2 + q);
-            W[2 * q] = coarse_weights(w & 0xffffu, 0);
-            W[2 * q + 1] = coarse_weights(w >> 16, 1);
+        // a block has at most 8 pairs a thread: all loads first
+        constexpr int U = kBlockCells / 2 / kCoarseThreads;
+        uint32_t w[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int q = threadIdx.x + u * kCoarseThreads;
+            w[u] = q < pairs ? __ldg(w2 + q) : 0u;
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int q = threadIdx.x + u * kCoarseThreads;
+            if (q >= pairs) break;
+            const CoarseWeights a = coarse_weights(w[u] & 0xffffu, 0), b = coarse_weights(w[u] >> 16, 1);
+            *reinterpret_cast<uint4 *>(W + 2 * q) = make_uint4(a.ml, a.k, b.ml, b.k);
         }
     }
     pdl_wait(kc);
@@ -794,10 +821,18 @@ __global__ void __launch_bounds__(kCoarseThreads, 1) k_coarse_vcycle(const __gri
     const int own = max(0, min(T.P, T.D.nx - i0)) * yz, base = i0 * yz;
     {
         float *R = reinterpret_cast<float *>(smem + T.off_r);
-        if (P.r_top_h)
-            for (int q = threadIdx.x; q < own; q += kCoarseThreads) R[q] = __half2float(P.r_top_h[base + q]);
-        else
-            for (int q = threadIdx.x; q < own; q += kCoarseThreads) R[q] = P.r_top[base + q];
+        constexpr int U = 8;
+        for (int q0 = threadIdx.x; q0 < own; q0 += U * kCoarseThreads) {
+            float v[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int q = q0 + u * kCoarseThreads;
+                v[u] = q >= own ? 0.0f : (P.r_top_h ? __half2float(P.r_top_h[base + q]) : P.r_top[base + q]);
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++)
+                if (q0 + u * kCoarseThreads < own) R[q0 + u * kCoarseThreads] = v[u];
+        }
     }
     if (P.nd > 0)
         cluster_barrier();  // the ghosts are zeroed before a neighbour stores into them

@@ -312,6 +312,11 @@ static size_t coarse_layout(const flub_mg *mg, int lc, int C, CoarseParams *P) {
         L.div_nz = coarse_div_by(L.D.nz);
         L.cw = mg->lv[lc + t].cw;
         if (t + 1 < P->nl && cells > scratch) scratch = cells;
+        // the copy of block 0's planes under a block's own
+        if (t + 1 == nd && t + 1 < P->nl) {
+            const size_t copy = (size_t)(L.P / 2) * (L.D.ny / 2 + 1) * (L.D.nz / 2);
+            if (copy > scratch) scratch = copy;
+        }
     }
     P->off_v = take(sizeof(float) * scratch);
     P->nu = mg->sched_nu;
