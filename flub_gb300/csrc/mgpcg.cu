@@ -237,10 +237,12 @@ static size_t carve(flub_mg *mg, char *base) {
         L.b_list = L.b_items = nullptr;
         L.b_n = nullptr;
         L.z3h = nullptr;
+        // (conditions on the shape, not on the pointers: those are NULL while sizing)
+        if (L.b_ti || (l == 0 && mg->split_ok && L.D.nz % 8 == 0))
+            L.b_items = (uint32_t *)take(sizeof(uint32_t) * (size_t)(nl / row_vector(L.D.nz)));
         if (L.b_ti) {
             L.b_tiles = block_tiles(L.D, L.b_ti);
             L.b_list = (uint32_t *)take(sizeof(uint32_t) * (size_t)L.b_tiles);
-            L.b_items = (uint32_t *)take(sizeof(uint32_t) * (size_t)(nl / row_vector(L.D.nz)));
             L.b_n = (int *)take(sizeof(int));
             if (mg->precision == FLUB_PRECISION_MIXED)
                 L.z3h = (__half *)take(sizeof(__half) * nl);
@@ -650,6 +652,7 @@ static int split_sweep(const LaunchCtx &c, const Level &L, int phase, const TRN 
     A.act = L.act;
     A.act_n = L.act_n;
     A.sws = L.sws;
+    A.items = L.b_items;
     A.rn = rn;
     A.rs = rs;
     A.zin = zin;
@@ -893,6 +896,14 @@ static int launch_coarse(flub_mg *mg, const LaunchCtx &c, const float *r_top, fl
     return FLUB_OK;
 }
 
+// Whether a V-cycle whose level 0 ran in natural order (a caller's z in mixed
+// precision, or z the same array as r) has to clear the pre-smoothing buffer
+// behind it: the colour-split sweeps read 0 there for cells that are never
+// updated, and their places hold other cells in natural order.
+static bool L0_natural_left_z2(const flub_mg *mg, int lg, bool other_layout) {
+    return mg->lv[0].sws && lg >= 1 && !other_layout && !(mg->tile_ok && mg->lv[0].n_tiles > 0);
+}
+
 // multigrid/mgpcg.py:296-349 apply_preconditioner; level 0 uses (r0, z0).
 // z0_clean: z0 holds 0 on every non-fluid cell (true for the handle's own z).
 // dot_mode 1 / 2: the caller's next step is z.r (the prologue's p = z / the
@@ -1031,6 +1042,8 @@ static int enqueue_vcycle(flub_mg *mg, const LaunchCtx &c, const float *r0, floa
             FLUB_TRY(sweep(c, L, 0, kSweepInPlace, SK(l), R(l), ZF(l), ZF(l), nullptr));
         }
     }
+    if (L0_natural_left_z2(mg, lg, split0 || BLOCK(0)))
+        FLUB_CHECK_CUDA(cudaMemsetAsync(ZP(0), 0, sizeof(float) * (size_t)mg->n, c.s));
     return FLUB_OK;
 }
 
@@ -1171,6 +1184,8 @@ static int enqueue_vcycle_mixed(flub_mg *mg, const LaunchCtx &c, float *z0, bool
             }
         }
     }
+    if (L0_natural_left_z2(mg, lg, split0))
+        FLUB_CHECK_CUDA(cudaMemsetAsync(mg->lv[0].z2h, 0, sizeof(__half) * (size_t)mg->n, c.s));
     return FLUB_OK;
 }
 
@@ -1759,6 +1774,8 @@ int flub_mg_set_tags(flub_mg *mg, const int32_t *tag, void *stream) {
         }
         if (L.sws) {
             k_split_words<<<blocks_for(L.D.n() >> 3, 256), 256, 0, s>>>(L.sw, L.sws, L.D);
+            FLUB_CHECK_LAUNCH();
+            k_block_items<4><<<blocks_for(L.D.n() >> 3, 256), 256, 0, s>>>(L.sw, L.D, L.b_items);
             FLUB_CHECK_LAUNCH();
             FLUB_CHECK_CUDA(cudaMemsetAsync(L.zs, 0, sizeof(float) * (size_t)L.D.n(), s));
         }

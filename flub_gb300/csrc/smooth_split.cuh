@@ -17,17 +17,32 @@
 // elements 4 kg .. 4 kg + 3 of the row in each half.
 //
 // One lane updates the 4 cells of the active colour in one active group: one
-// 8-byte load of their stencil words, 16-byte loads of their r and z and of
-// the other colour's four neighbour rows and own row, one 16-byte store -- all
-// of it data the update uses.  The arithmetic is smooth_cell (smooth8.cuh),
+// item word (smooth_block.cuh: the diagonal counts of the 4 cells, and whether
+// a solid is next to any), 16-byte loads of their r and z and of the other
+// colour's four neighbour rows and own row, one 16-byte store -- all of it data
+// the update uses.  The arithmetic is block_update: smooth_cell's operations,
 // cell by cell in the reference's order (multigrid/mgpcg.py:72-86), so results
 // are bit-identical to the natural-order kernels.
+//
+// z is 0 on every cell off the fluid, in both buffers, so an air neighbour
+// needs no test, and a solid or a wall is the cell itself (its term is 0).  What
+// bounds a half-sweep up to 256^3, where the buffers sit in L2, is issue: a
+// word per cell, decoded with a branch per cell wherever one of the 4 is not
+// interior, took ~400 instructions an item, and a warp of 32 rows nearly always
+// has such an item.  With the item word only items next to a solid load their
+// stencil words.  The first half of the prolongation still takes the stencil
+// words: it has the neighbours' corrections to add and no register to spare.
+// A half-sweep of 128^3 (FP32, dam break / full): 1.9 / 3.7 us, in natural order
+// 3.0 / 6.7.  Measured through a whole solve (before -> now): 128^3 sphere in mixed
+// precision 8536 -> 7859 us, 256^3 dam break 15880 -> 15310, 256 x 64 x 256
+// 3951 -> 3733, 104 x 72 x 88 2296 -> 2141.
 //
 // Modes of one half-sweep (phase 0 updates the odd cells, phase 1 the even):
 //   kFirst    first pre-smoothing half-sweep (phase 0, from zero): reads the
 //             natural residual rn, writes both halves of the split residual
-//             rs and z = r / d on the odd cells; the even cells are not
-//             touched (the next half-sweep runs kOwnZero).
+//             rs (0 on cells that are never updated) and z = r / d on the odd
+//             cells; the even cells are not touched (the next half-sweep runs
+//             kOwnZero).
 //   kOwnZero  second half-sweep of the first iteration: the updated cells'
 //             own z is 0 and is not read.
 //   kInPlace  z updated in place.
@@ -43,6 +58,7 @@
 #pragma once
 
 #include "smooth8.cuh"
+#include "smooth_block.cuh"
 
 namespace flub {
 
@@ -52,6 +68,7 @@ struct SplitArgs {
     Dims D;
     const int *act, *act_n;     // active 8-cell groups of level 0
     const uint16_t *sws;        // stencil words, colour-split
+    const uint32_t *items;      // item words (smooth_block.cuh) of every group: colour 0, then colour 1
     const void *rn;             // kFirst: natural residual (TRN)
     void *rs;                   // colour-split residual (TR): written by kFirst, read by the others
     const void *zin;            // kProlong: colour-split input z (TZI)
@@ -103,6 +120,7 @@ __device__ __forceinline__ uint32_t word_kcode(uint32_t w, bool kp) { return sw_
 template <int kMode, typename TRN, typename TR, typename TZI, typename TZ, typename TC>
 __global__ void __launch_bounds__(256, (kMode == kProlong || kMode == kLast) ? 4 : 3)
     k_smooth_split(const SplitArgs A, int phase, unsigned long long *kc) {
+    __shared__ float2 lut[8];  // -1/d and d
     pdl_open();
     const Dims D = A.D;
     const int hz = D.nz >> 1;             // split row length
@@ -116,12 +134,24 @@ __global__ void __launch_bounds__(256, (kMode == kProlong || kMode == kLast) ? 4
     const int stride = gridDim.x * blockDim.x;
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     int g_next = t < total ? __ldg(A.act + t) : 0;
-    // the list and the first stencil words do not depend on the previous kernel
+    // the list and the first words do not depend on the previous kernel
+    const uint32_t *items = A.items + (col ? (int)(D.n() >> 3) : 0), *other = A.items + (col ? 0 : (int)(D.n() >> 3));
+    uint32_t it_next = 0u;
     uint2 wd_next = make_uint2(0u, 0u);
     if (t < total) {
-        int i0, j0, kg0;
-        group_ijk(g_next, D, i0, j0, kg0);
-        wd_next = __ldg(reinterpret_cast<const uint2 *>(A.sws + uoff + (i0 * D.ny + j0) * hz + 4 * kg0));
+        if (kMode != kProlong) {
+            it_next = __ldg(items + g_next);
+        } else {
+            int i0, j0, kg0;
+            group_ijk(g_next, D, i0, j0, kg0);
+            wd_next = __ldg(reinterpret_cast<const uint2 *>(A.sws + uoff + (i0 * D.ny + j0) * hz + 4 * kg0));
+        }
+    }
+    if (kMode != kProlong) {
+        if (threadIdx.x < 8)
+            lut[threadIdx.x] =
+                make_float2(threadIdx.x ? __fdiv_rn(-1.0f, (float)threadIdx.x) : 0.0f, (float)threadIdx.x);
+        __syncthreads();
     }
     pdl_wait(kc);
     bool first = true;
@@ -135,7 +165,12 @@ __global__ void __launch_bounds__(256, (kMode == kProlong || kMode == kLast) ? 4
         group_ijk(g, D, i, j, kg);
         const int h = (i * D.ny + j) * hz + 4 * kg;  // split index of the group's first element
         const int q = (col + i + j) & 1;             // updated cell m sits at natural k = 8 kg + 2 m + q
-        const uint2 wd = first ? wd_next : __ldg(reinterpret_cast<const uint2 *>(A.sws + uoff + h));
+        uint2 wd = make_uint2(0u, 0u);
+        uint32_t item = 0u;
+        if (kMode == kProlong)
+            wd = first ? wd_next : __ldg(reinterpret_cast<const uint2 *>(A.sws + uoff + h));
+        else
+            item = first ? it_next : __ldg(items + g);
         first = false;
         float rr[4];
         if (kMode == kFirst) {
@@ -149,15 +184,23 @@ __global__ void __launch_bounds__(256, (kMode == kProlong || kMode == kLast) ? 4
                 if (((p + m) & 1) == 0) re[m >> 1] = rv[m];
                 else ro[m >> 1] = rv[m];
             }
+            // 0 where the smoothing never updates: the split residual is read
+            // for those cells as well
+            const uint32_t ov = __ldg(other + g);
+#pragma unroll
+            for (int m = 0; m < 4; m++) {
+                const uint32_t se = col ? ov : item, so = col ? item : ov;
+                if (!((se >> (4 * m)) & 7u)) re[m] = 0.0f;
+                if (!((so >> (4 * m)) & 7u)) ro[m] = 0.0f;
+            }
             TR *rsw = static_cast<TR *>(A.rs);
             St<TR>::st4(rsw + h, re);
             St<TR>::st4(rsw + hn + h, ro);
+            float out[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
             for (int m = 0; m < 4; m++) rr[m] = col ? ro[m] : re[m];
-            float out[4];
-#pragma unroll
-            for (int m = 0; m < 4; m++)
-                out[m] = smooth_cell<true>(word4_at(wd, m), 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, rr[m]);
+            const float zero[4] = {0.f, 0.f, 0.f, 0.f};
+            block_update<4>(item, out, zero, zero, zero, zero, zero, zero, rr, lut);
             St<TZ>::st4(z + uoff + h, out);
             continue;
         }
@@ -221,20 +264,53 @@ __global__ void __launch_bounds__(256, (kMode == kProlong || kMode == kLast) ? 4
             if (q == 1 && hkp)
                 w[4] = __fadd_rn(St<TZI>::ld(zi + voff + h + 4), __fmul_rn(St<TC>::ld_ro(zc + crow0 + 4 * kg + 4), s));
         } else {
+            // a neighbour row outside the domain is replaced by the cells
+            // themselves: their terms are then 0
             if (kMode != kOwnZero) St<TZ>::ld4(z + uoff + h, xc);
             St<TZ>::ld4(z + voff + h, vc);
-            if (hip) St<TZ>::ld4(z + voff + h + si, zip);
-            if (him) St<TZ>::ld4(z + voff + h - si, zim);
-            if (hjp) St<TZ>::ld4(z + voff + h + sj, zjp);
-            if (hjm) St<TZ>::ld4(z + voff + h - sj, zjm);
-            if (q == 0 && hkm) w[0] = St<TZ>::ld(z + voff + h - 1);
-            if (q == 1 && hkp) w[4] = St<TZ>::ld(z + voff + h + 4);
+            if (kMode != kOwnZero) {
+                St<TZ>::ld4(hip ? z + voff + h + si : z + uoff + h, zip);
+                St<TZ>::ld4(him ? z + voff + h - si : z + uoff + h, zim);
+                St<TZ>::ld4(hjp ? z + voff + h + sj : z + uoff + h, zjp);
+                St<TZ>::ld4(hjm ? z + voff + h - sj : z + uoff + h, zjm);
+            } else {  // own z is 0, whatever the buffer holds
+                if (hip) St<TZ>::ld4(z + voff + h + si, zip);
+                if (him) St<TZ>::ld4(z + voff + h - si, zim);
+                if (hjp) St<TZ>::ld4(z + voff + h + sj, zjp);
+                if (hjm) St<TZ>::ld4(z + voff + h - sj, zjm);
+            }
+            if (q == 0) w[0] = hkm ? St<TZ>::ld(z + voff + h - 1) : xc[0];
+            if (q == 1) w[4] = hkp ? St<TZ>::ld(z + voff + h + 4) : xc[3];
         }
         // w[t] is element h - 1 + q + t of the other colour's row
 #pragma unroll
         for (int m = 0; m < 4; m++) w[m + 1 - q] = vc[m];
         float out[4], vo[4];
-        if (wd.x == kInteriorWord2 && wd.y == kInteriorWord2) {
+        if (kMode != kProlong) {
+            float va[4], vb[4];  // the k neighbours inside the group's row, and the others
+#pragma unroll
+            for (int m = 0; m < 4; m++) {
+                va[m] = vc[m];
+                vb[m] = q ? w[m + 1] : w[m];
+                out[m] = xc[m];
+                vo[m] = vc[m];
+            }
+            if (item & kItemSolid) {
+                // solids next to it: the neighbours that do not count become the cell itself
+                const uint2 ws = __ldg(reinterpret_cast<const uint2 *>(A.sws + uoff + h));
+#pragma unroll
+                for (int m = 0; m < 4; m++) {
+                    const uint32_t ns = sw_ns(word4_at(ws, m));
+                    if (!(ns & 4u)) zip[m] = xc[m];
+                    if (!(ns & 16u)) zim[m] = xc[m];
+                    if (!(ns & 64u)) zjp[m] = xc[m];
+                    if (!(ns & 256u)) zjm[m] = xc[m];
+                    if (!(ns & (q ? 4096u : 1024u))) va[m] = xc[m];
+                    if (!(ns & (q ? 1024u : 4096u))) vb[m] = xc[m];
+                }
+            }
+            block_update<4>(item, out, zip, zim, zjp, zjm, va, vb, rr, lut);
+        } else if (wd.x == kInteriorWord2 && wd.y == kInteriorWord2) {
             // four interior cells (most of a water body): their k neighbours, the
             // other colour's elements of the group, are fluid too
 #pragma unroll
@@ -247,11 +323,10 @@ __global__ void __launch_bounds__(256, (kMode == kProlong || kMode == kLast) ? 4
             for (int m = 0; m < 4; m++)
                 out[m] = smooth_cell<false>(word4_at(wd, m), xc[m], zip[m], zim[m], zjp[m], zjm[m], w[m + 1], w[m],
                                             rr[m]);
-            // the other colour's cells of the group: element m is the k+ neighbour
-            // of updated cell m when q = 0, its k- neighbour when q = 1
+            // the other colour's cells of the group, 0 where they are never updated
+            const uint32_t ov = __ldg(other + g);
 #pragma unroll
-            for (int m = 0; m < 4; m++)
-                vo[m] = word_kcode(word4_at(wd, m), q == 0) == kCodeFluid ? vc[m] : 0.0f;
+            for (int m = 0; m < 4; m++) vo[m] = (ov >> (4 * m)) & 7u ? vc[m] : 0.0f;
         }
         if (kMode == kLast) {
             // natural row of the group: updated cell m at offset 2 m + q, the

@@ -1,0 +1,59 @@
+"""The colour-split half-sweeps (flub_gb300/csrc/smooth_split.cuh) against the
+oracle's V-cycle, bit for bit: solids, air and walls on every side of a group,
+1 to 3 iterations a side, a residual that holds anything off the fluid; and
+after a V-cycle that ran in natural order on the same handle."""
+import numpy as np
+import pytest
+import torch
+
+import oracle as O
+from flub_gb300 import MGPCG
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [((104, 72, 88), 3), ((66, 50, 80), 2), ((128, 128, 128), 4), ((34, 258, 16), 2), ((130, 66, 8), 2)]
+
+
+def _case(shape, seed, solids):
+    rng = np.random.default_rng(seed)
+    x = np.linspace(0, 1, shape[0])[:, None, None]
+    tag = np.where(x + 0.05 * rng.standard_normal(shape) < 0.8, 1, 0).astype(np.int32)
+    tag[rng.random(shape) < solids] = 2
+    r = np.where(tag == 1, rng.standard_normal(shape), 0).astype(np.float32)
+    return tag, r
+
+
+@pytest.mark.parametrize("solids", [0.0, 0.05])
+@pytest.mark.parametrize("nu", [1, 2, 3])
+@pytest.mark.parametrize("shape,levels", SHAPES)
+def test_split_bit_exact(shape, levels, nu, solids):
+    tag, r = _case(shape, sum(shape) + nu, solids)
+    mg = MGPCG(3, shape, levels, float)
+    mg.set_tags(torch.from_numpy(tag).cuda())
+    mg.set_schedule(nu, 3, 0.5)
+    rd = torch.from_numpy(r).cuda()
+    with O.schedule(nu, 3, 0.5):
+        want = O.vcycle(r, O.tag_levels(tag, levels), np.float32)
+    z = torch.full(shape, float("nan"), device="cuda")  # every cell is written
+    assert np.array_equal(mg.apply_preconditioner(rd, z).cpu().numpy(), want)
+    inplace = rd.clone()  # z the array of r: level 0 in natural order
+    mg.apply_preconditioner(inplace, inplace)
+    assert np.array_equal(mg.apply_preconditioner(rd).cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("shape,levels", [((64, 64, 64), 3), ((128, 32, 64), 3), ((128, 128, 128), 4)])
+def test_split_mixed_after_natural(shape, levels):
+    """A caller's z in mixed precision runs level 0 in natural order; the solve
+    after it is the one of a fresh handle."""
+    tag, r = _case(shape, sum(shape), 0.05)
+    rd = torch.from_numpy(r).cuda()
+    x = []
+    for natural in (False, True):
+        mg = MGPCG(3, shape, levels, float, precision="mixed")
+        mg.set_tags(torch.from_numpy(tag).cuda())
+        if natural:
+            mg.apply_preconditioner(rd)
+        mg.init(rd, 1.0)
+        mg.solve(max_iters=4, eps=1e-12, abs_tol=1e-12, rel_tol=1e-12, smoother="phases")
+        x.append(mg.x.cpu().numpy())
+    assert np.isfinite(x[0]).all() and np.array_equal(x[0], x[1])
