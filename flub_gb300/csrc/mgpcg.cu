@@ -53,13 +53,14 @@ struct Level {
     int *act, *act_n;
     // stencil words (smooth8.cuh), same condition
     uint16_t *sw;
-    // level 0 with nz % 8 == 0: the colour-split buffers of smooth_split.cuh --
-    // stencil words, the residual (FP32 rs, or FP16 rsh in mixed precision) and
-    // the post-smoothing correction zs; z2 / z2h hold the pre-smoothing
-    // correction split the same way
+    // levels that may smooth on colour-split storage (split_level): the buffers
+    // of smooth_split.cuh -- stencil words, the residual (FP32 rs, or FP16 rsh
+    // in mixed precision) and the post-smoothing correction (zs, or zsh below
+    // level 0 in mixed precision); z2 / z2h hold the pre-smoothing correction
+    // split the same way
     uint16_t *sws;
     float *rs, *zs;
-    __half *rsh;
+    __half *rsh, *zsh;
     // TMA-tiled smoothing (smooth_tile.cuh) on FP32 levels whose extents are
     // multiples of the tile: a third correction buffer for the ping-pong of
     // the out-of-place iterations, the tile flags, and the list of tiles that
@@ -169,6 +170,17 @@ static int block_planes(const flub_mg *mg, int l) {
     return block_tiles(D, 4) <= 256 ? 4 : 0;
 }
 
+// Whether level l has the buffers for smoothing on colour-split storage
+// (smooth_split.cuh): level 0, and the levels below it that are too large for
+// the coarse kernel and for tiles of one wave.  At 128^3 a half-sweep of the
+// dam break / a full grid takes 1.9 / 3.7 us on them, against 3.0 / 6.7 in
+// natural order; a level of 64^3 takes 1.25 / 1.2 in tiles.
+static bool split_level(const flub_mg *mg, int l) {
+    const Dims D{mg->nx >> l, mg->ny >> l, mg->nz >> l};
+    if (!mg->split_ok || D.nz % 8 != 0) return false;
+    return l == 0 || (l + 1 < mg->levels && D.n() > kCoarseMaxCells && !block_planes(mg, l));
+}
+
 // Workspace carve-up; with base == nullptr only the size is computed.
 static size_t carve(flub_mg *mg, char *base) {
     size_t off = 0;
@@ -202,14 +214,17 @@ static size_t carve(flub_mg *mg, char *base) {
         L.sw = nullptr;
         L.sws = nullptr;
         L.rs = L.zs = nullptr;
-        L.rsh = nullptr;
+        L.rsh = L.zsh = nullptr;
         if (L.D.nz % 8 == 0) {
             L.act = (int *)take(sizeof(int) * (size_t)(nl >> 3));
             L.act_n = (int *)take(sizeof(int));
             L.sw = (uint16_t *)take(sizeof(uint16_t) * (size_t)nl);
-            if (l == 0 && mg->split_ok) {
+            if (split_level(mg, l)) {
                 L.sws = (uint16_t *)take(sizeof(uint16_t) * (size_t)nl);
-                L.zs = (float *)take(sizeof(float) * nl);
+                if (l > 0 && mg->precision == FLUB_PRECISION_MIXED)
+                    L.zsh = (__half *)take(sizeof(__half) * nl);
+                else
+                    L.zs = (float *)take(sizeof(float) * nl);
                 if (mg->precision == FLUB_PRECISION_MIXED)
                     L.rsh = (__half *)take(sizeof(__half) * nl);
                 else
@@ -238,7 +253,7 @@ static size_t carve(flub_mg *mg, char *base) {
         L.b_n = nullptr;
         L.z3h = nullptr;
         // (conditions on the shape, not on the pointers: those are NULL while sizing)
-        if (L.b_ti || (l == 0 && mg->split_ok && L.D.nz % 8 == 0))
+        if (L.b_ti || split_level(mg, l))
             L.b_items = (uint32_t *)take(sizeof(uint32_t) * (size_t)(nl / row_vector(L.D.nz)));
         if (L.b_ti) {
             L.b_tiles = block_tiles(L.D, L.b_ti);
@@ -642,10 +657,11 @@ static int sweep(const LaunchCtx &c, const Level &L, int phase, int mode, int sk
 }
 
 
-// One level-0 half-sweep on colour-split storage (smooth_split.cuh).
+// One half-sweep on colour-split storage (smooth_split.cuh); kLast: zc's type
+// TC is the type of the natural-order output zn.
 template <int kMode, typename TRN, typename TR, typename TZI, typename TZ, typename TC>
 static int split_sweep(const LaunchCtx &c, const Level &L, int phase, const TRN *rn, TR *rs, const TZI *zin, TZ *z,
-                       const TC *zc, float zc_scale, float *zn, const SplitArgs *dot = nullptr) {
+                       const TC *zc, float zc_scale, TC *zn, const SplitArgs *dot = nullptr) {
     SplitArgs A = {};
     if (dot) A = *dot;  // kLast with z.r folded in: dot, rdot, pinit, st, partials
     A.D = L.D;
@@ -676,20 +692,57 @@ static int split_sweep(const LaunchCtx &c, const Level &L, int phase, const TRN 
                       c.kc);
 }
 
-// Colour-split level-0 smoothing unless FLUB_NO_SPLIT=1 (read when a handle is
-// created or sized).
+// A side of a level's smoothing on colour-split storage; T is the type of the
+// residual and of the pre-smoothing correction z2.  Before the restriction:
+// from zero, iterations of phases 0, 1 on z2.
+template <typename T>
+static int split_pre(const LaunchCtx &c, const Level &L, int iters, const T *r, T *rs, T *z2) {
+    const T *none = nullptr;
+    for (int it = 0; it < iters; it++) {
+        if (it == 0) {
+            FLUB_TRY((split_sweep<kFirst, T, T, T, T, T>(c, L, 0, r, rs, none, z2, none, 1.0f, nullptr)));
+            FLUB_TRY((split_sweep<kOwnZero, T, T, T, T, T>(c, L, 1, none, rs, none, z2, none, 1.0f, nullptr)));
+        } else {
+            FLUB_TRY((split_sweep<kInPlace, T, T, T, T, T>(c, L, 0, none, rs, none, z2, none, 1.0f, nullptr)));
+            FLUB_TRY((split_sweep<kInPlace, T, T, T, T, T>(c, L, 1, none, rs, none, z2, none, 1.0f, nullptr)));
+        }
+    }
+    return FLUB_OK;
+}
+
+// After the prolongation of zc: iterations of phases 1, 0 on zs from z2 + P zc,
+// the last half-sweep into the natural-order zn (TP: the type of both).
+template <typename T, typename TP>
+static int split_post(const LaunchCtx &c, const Level &L, int iters, T *rs, const T *z2, TP *zs, const T *zc,
+                      float zc_scale, TP *zn, const SplitArgs *dot) {
+    const T *none = nullptr;
+    const TP *nonep = nullptr;
+    for (int it = 0; it < iters; it++) {
+        if (it == 0)
+            FLUB_TRY((split_sweep<kProlong, T, T, T, TP, T>(c, L, 1, none, rs, z2, zs, zc, zc_scale, nullptr)));
+        else
+            FLUB_TRY((split_sweep<kInPlace, T, T, TP, TP, TP>(c, L, 1, none, rs, nonep, zs, nonep, 1.0f, nullptr)));
+        if (it + 1 == iters)
+            FLUB_TRY((split_sweep<kLast, T, T, TP, TP, TP>(c, L, 0, none, rs, nonep, zs, nonep, 1.0f, zn, dot)));
+        else
+            FLUB_TRY((split_sweep<kInPlace, T, T, TP, TP, TP>(c, L, 0, none, rs, nonep, zs, nonep, 1.0f, nullptr)));
+    }
+    return FLUB_OK;
+}
+
+// Colour-split smoothing unless FLUB_NO_SPLIT=1 (read when a handle is created
+// or sized).
 static bool split_requested() {
     const char *e = getenv("FLUB_NO_SPLIT");
     return !(e && e[0] == '1');
 }
 
-// Level 0 of the V-cycle on colour-split storage: the handle has the split
-// buffers, level 0 hands on to a coarser level (lg >= 1), the sweeps may skip
-// fluid-free groups, no tiled smoothing is asked for there, and the output z
-// is not the input r.
-static bool use_split(const flub_mg *mg, int lg, int sk, const void *r0, const void *z0) {
-    const Level &L = mg->lv[0];
-    return mg->split_ok && L.sws && lg >= 1 && sk == 1 && !(mg->tile_ok && L.n_tiles > 0) && r0 != z0;
+// Level l < lg of the V-cycle on colour-split storage: it has the split
+// buffers, the sweeps may skip fluid-free groups, neither tiled nor blocked
+// smoothing runs there, and at level 0 the output z is not the input r.
+static bool use_split(const flub_mg *mg, int l, int lg, int sk, const void *r0, const void *z0) {
+    const Level &L = mg->lv[l];
+    return L.sws && l < lg && sk == 1 && !(mg->tile_ok && L.n_tiles > 0) && !L.b_ti && (l > 0 || r0 != z0);
 }
 
 // ---------------------------------------------------------------- tiled smoothing (smooth_tile.cuh)
@@ -929,29 +982,16 @@ static int enqueue_vcycle(flub_mg *mg, const LaunchCtx &c, const float *r0, floa
     // blocked smoothing (smooth_block.cuh): neighbouring tiles read r and the
     // input while others write the output
     auto BLOCK = [&](int l) { return mg->lv[l].b_ti && sk == 1 && (l > 0 || r0 != z0); };
-    // level 0 on colour-split storage (smooth_split.cuh)
-    const bool split0 = !BLOCK(0) && use_split(mg, lg, sk, r0, z0);
+    // colour-split storage (smooth_split.cuh)
+    auto SPLIT = [&](int l) { return use_split(mg, l, lg, sk, r0, z0); };
     for (int l = 0; l < (pers ? 1 : lg); l++) {
         const Level &L = mg->lv[l];
         const int iters = level_iters(mg, l);
-        if (l == 0 && split0) {
-            float *z2 = ZP(0);
-            for (int it = 0; it < iters; it++) {
-                if (it == 0) {
-                    FLUB_TRY((split_sweep<kFirst, float, float, float, float, float>(c, L, 0, r0, L.rs, nullptr, z2,
-                                                                                   nullptr, 1.0f, nullptr)));
-                    FLUB_TRY((split_sweep<kOwnZero, float, float, float, float, float>(
-                        c, L, 1, nullptr, L.rs, nullptr, z2, nullptr, 1.0f, nullptr)));
-                } else {
-                    FLUB_TRY((split_sweep<kInPlace, float, float, float, float, float>(
-                        c, L, 0, nullptr, L.rs, nullptr, z2, nullptr, 1.0f, nullptr)));
-                    FLUB_TRY((split_sweep<kInPlace, float, float, float, float, float>(
-                        c, L, 1, nullptr, L.rs, nullptr, z2, nullptr, 1.0f, nullptr)));
-                }
-            }
-            const Level &C = mg->lv[1];
+        if (SPLIT(l)) {
+            FLUB_TRY(split_pre<float>(c, L, iters, R(l), L.rs, ZP(l)));
+            const Level &C = mg->lv[l + 1];
             FLUB_TRY(launch_pdl(k_restrict8_split<float, float, float>, dim3(blocks_for(C.D.n(), 256, kNumSMs * 4)),
-                                dim3(256), 0, c.s, r0, (const float *)z2, (const uint8_t *)L.code,
+                                dim3(256), 0, c.s, R(l), (const float *)ZP(l), (const uint8_t *)L.code,
                                 (const uint16_t *)L.sw, C.r, (const uint8_t *)C.code, C.D, mg->sched_rscale,
                                 (const int *)C.act, (const int *)C.act_n, c.kc));
             continue;
@@ -996,34 +1036,21 @@ static int enqueue_vcycle(flub_mg *mg, const LaunchCtx &c, const float *r0, floa
     for (int l = pers ? 0 : lg - 1; l >= 0; l--) {
         const Level &L = mg->lv[l];
         const int iters = level_iters(mg, l);
-        if (l == 0 && split0) {
-            // the last half-sweep writes the groups with fluid of the natural z0;
+        if (SPLIT(l)) {
+            // the last half-sweep writes the groups with fluid of the natural z;
             // a caller's z0 gets 0 everywhere else first
-            if (!z0_clean) FLUB_CHECK_CUDA(cudaMemsetAsync(z0, 0, sizeof(float) * (size_t)mg->n, c.s));
-            for (int it = 0; it < iters; it++) {
-                if (it == 0)
-                    FLUB_TRY((split_sweep<kProlong, float, float, float, float, float>(
-                        c, L, 1, nullptr, L.rs, ZP(0), L.zs, mg->lv[1].z, 1.0f, nullptr)));
-                else
-                    FLUB_TRY((split_sweep<kInPlace, float, float, float, float, float>(
-                        c, L, 1, nullptr, L.rs, nullptr, L.zs, nullptr, 1.0f, nullptr)));
-                if (it + 1 == iters) {
-                    SplitArgs D = {};
-                    if (dot_mode && dot_fused) {
-                        D.dot = dot_mode;
-                        D.rdot = r0;
-                        D.pinit = mg->p;
-                        D.st = mg->st;
-                        D.partials = mg->partials;
-                        *dot_fused = true;
-                    }
-                    FLUB_TRY((split_sweep<kLast, float, float, float, float, float>(
-                        c, L, 0, nullptr, L.rs, nullptr, L.zs, nullptr, 1.0f, z0, D.dot ? &D : nullptr)));
-                }
-                else
-                    FLUB_TRY((split_sweep<kInPlace, float, float, float, float, float>(
-                        c, L, 0, nullptr, L.rs, nullptr, L.zs, nullptr, 1.0f, nullptr)));
+            if (l == 0 && !z0_clean) FLUB_CHECK_CUDA(cudaMemsetAsync(z0, 0, sizeof(float) * (size_t)mg->n, c.s));
+            SplitArgs D = {};
+            if (l == 0 && dot_mode && dot_fused) {
+                D.dot = dot_mode;
+                D.rdot = r0;
+                D.pinit = mg->p;
+                D.st = mg->st;
+                D.partials = mg->partials;
+                *dot_fused = true;
             }
+            FLUB_TRY((split_post<float, float>(c, L, iters, L.rs, ZP(l), L.zs, mg->lv[l + 1].z, 1.0f, ZF(l),
+                                               D.dot ? &D : nullptr)));
             continue;
         }
         if (TILED_POST(l)) {
@@ -1042,7 +1069,7 @@ static int enqueue_vcycle(flub_mg *mg, const LaunchCtx &c, const float *r0, floa
             FLUB_TRY(sweep(c, L, 0, kSweepInPlace, SK(l), R(l), ZF(l), ZF(l), nullptr));
         }
     }
-    if (L0_natural_left_z2(mg, lg, split0 || BLOCK(0)))
+    if (L0_natural_left_z2(mg, lg, SPLIT(0) || mg->lv[0].b_ti))
         FLUB_CHECK_CUDA(cudaMemsetAsync(ZP(0), 0, sizeof(float) * (size_t)mg->n, c.s));
     return FLUB_OK;
 }
@@ -1058,26 +1085,14 @@ static int enqueue_vcycle_mixed(flub_mg *mg, const LaunchCtx &c, float *z0, bool
     const int sk0 = z0_clean ? sk : 0;
     const int lg = lt < Lm - 1 ? lt : Lm - 1;
     const bool pers = use_persist(mg, lg);
-    const bool split0 = use_split(mg, lg, sk0, mg->lv[0].rh, z0);
+    auto SPLIT = [&](int l) { return use_split(mg, l, lg, l == 0 ? sk0 : sk, mg->lv[0].rh, z0); };
     for (int l = 0; l < (pers ? 1 : lg); l++) {
         const Level &L = mg->lv[l];
         const int iters = level_iters(mg, l);
-        if (l == 0 && split0) {
+        if (SPLIT(l)) {
             using H = __half;
-            for (int it = 0; it < iters; it++) {
-                if (it == 0) {
-                    FLUB_TRY((split_sweep<kFirst, H, H, H, H, H>(c, L, 0, (const H *)L.rh, L.rsh, nullptr, L.z2h,
-                                                                 nullptr, 1.0f, nullptr)));
-                    FLUB_TRY((split_sweep<kOwnZero, H, H, H, H, H>(c, L, 1, nullptr, L.rsh, nullptr, L.z2h, nullptr,
-                                                                   1.0f, nullptr)));
-                } else {
-                    FLUB_TRY((split_sweep<kInPlace, H, H, H, H, H>(c, L, 0, nullptr, L.rsh, nullptr, L.z2h, nullptr,
-                                                                   1.0f, nullptr)));
-                    FLUB_TRY((split_sweep<kInPlace, H, H, H, H, H>(c, L, 1, nullptr, L.rsh, nullptr, L.z2h, nullptr,
-                                                                   1.0f, nullptr)));
-                }
-            }
-            const Level &C = mg->lv[1];
+            FLUB_TRY(split_pre<H>(c, L, iters, L.rh, L.rsh, L.z2h));
+            const Level &C = mg->lv[l + 1];
             FLUB_TRY(launch_pdl(k_restrict8_split<H, H, H>, dim3(blocks_for(C.D.n(), 256, kNumSMs * 4)), dim3(256),
                                 0, c.s, (const H *)L.rh, (const H *)L.z2h, (const uint8_t *)L.code,
                                 (const uint16_t *)L.sw, C.rh, (const uint8_t *)C.code, C.D,
@@ -1127,36 +1142,25 @@ static int enqueue_vcycle_mixed(flub_mg *mg, const LaunchCtx &c, float *z0, bool
         const Level &L = mg->lv[l];
         const __half *zc = mg->lv[l + 1].zh;
         const int iters = level_iters(mg, l);
-        if (l == 0 && split0) {
-            using H = __half;
+        if (SPLIT(l) && l > 0) {
+            FLUB_TRY((split_post<__half, __half>(c, L, iters, L.rsh, L.z2h, L.zsh, zc, 8.0f, L.zh, nullptr)));
+            continue;
+        }
+        if (SPLIT(l)) {
             if (!z0_clean) FLUB_CHECK_CUDA(cudaMemsetAsync(z0, 0, sizeof(float) * (size_t)mg->n, c.s));
-            for (int it = 0; it < iters; it++) {
-                if (it == 0)
-                    FLUB_TRY((split_sweep<kProlong, H, H, H, float, H>(c, L, 1, nullptr, L.rsh, L.z2h, L.zs, zc, 8.0f,
-                                                                       nullptr)));
-                else
-                    FLUB_TRY((split_sweep<kInPlace, H, H, float, float, float>(c, L, 1, nullptr, L.rsh, nullptr,
-                                                                               L.zs, nullptr, 1.0f, nullptr)));
-                if (it + 1 == iters) {
-                    SplitArgs D = {};
-                    if (dot_mode && dot_fused) {
-                        D.dot = dot_mode;  // 1: p = zscale z and zr_old, 3: flexible beta
-                        D.zscaled = 1;
-                        D.rdot = mg->lv[0].r;
-                        D.rold = mg->r_old;
-                        D.pinit = mg->p;
-                        D.st = mg->st;
-                        D.partials = mg->partials;
-                        *dot_fused = true;
-                    }
-                    FLUB_TRY((split_sweep<kLast, H, H, float, float, float>(c, L, 0, nullptr, L.rsh, nullptr, L.zs,
-                                                                            nullptr, 1.0f, z0,
-                                                                            D.dot ? &D : nullptr)));
-                }
-                else
-                    FLUB_TRY((split_sweep<kInPlace, H, H, float, float, float>(c, L, 0, nullptr, L.rsh, nullptr,
-                                                                               L.zs, nullptr, 1.0f, nullptr)));
+            SplitArgs D = {};
+            if (dot_mode && dot_fused) {
+                D.dot = dot_mode;  // 1: p = zscale z and zr_old, 3: flexible beta
+                D.zscaled = 1;
+                D.rdot = mg->lv[0].r;
+                D.rold = mg->r_old;
+                D.pinit = mg->p;
+                D.st = mg->st;
+                D.partials = mg->partials;
+                *dot_fused = true;
             }
+            FLUB_TRY((split_post<__half, float>(c, L, iters, L.rsh, L.z2h, L.zs, zc, 8.0f, z0,
+                                                D.dot ? &D : nullptr)));
             continue;
         }
         if (l > 0 && L.b_ti && sk == 1) {
@@ -1184,7 +1188,7 @@ static int enqueue_vcycle_mixed(flub_mg *mg, const LaunchCtx &c, float *z0, bool
             }
         }
     }
-    if (L0_natural_left_z2(mg, lg, split0))
+    if (L0_natural_left_z2(mg, lg, SPLIT(0)))
         FLUB_CHECK_CUDA(cudaMemsetAsync(mg->lv[0].z2h, 0, sizeof(__half) * (size_t)mg->n, c.s));
     return FLUB_OK;
 }
@@ -1777,7 +1781,10 @@ int flub_mg_set_tags(flub_mg *mg, const int32_t *tag, void *stream) {
             FLUB_CHECK_LAUNCH();
             k_block_items<4><<<blocks_for(L.D.n() >> 3, 256), 256, 0, s>>>(L.sw, L.D, L.b_items);
             FLUB_CHECK_LAUNCH();
-            FLUB_CHECK_CUDA(cudaMemsetAsync(L.zs, 0, sizeof(float) * (size_t)L.D.n(), s));
+            if (L.zsh)
+                FLUB_CHECK_CUDA(cudaMemsetAsync(L.zsh, 0, sizeof(__half) * (size_t)L.D.n(), s));
+            else
+                FLUB_CHECK_CUDA(cudaMemsetAsync(L.zs, 0, sizeof(float) * (size_t)L.D.n(), s));
         }
         if (!L.act) continue;
         const int ng = (int)(L.D.n() >> 3);

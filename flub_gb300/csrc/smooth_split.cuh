@@ -1,10 +1,10 @@
-// Level-0 red-black smoothing on colour-split storage.
+// Red-black smoothing of the large levels on colour-split storage.
 //
 // In natural order (k fastest) the cells of one colour alternate along k, so
 // a half-sweep that updates one colour still moves whole rows: half of every
 // neighbour row it loads and half of the row it stores belong to the colour it
-// does not update.  Inside the V-cycle the level-0 vectors are therefore kept
-// split by colour: a buffer of n values holds the even cells ((i + j + k) even)
+// does not update.  Inside the V-cycle the vectors of these levels are therefore
+// kept split by colour: a buffer of n values holds the even cells ((i + j + k) even)
 // in its first half and the odd cells in its second half, each half laid out
 // [i][j][k / 2].  Natural cell (i, j, k) is element k >> 1 of row (i, j) in the
 // half of parity (i + j + k) & 1, and
@@ -51,7 +51,7 @@
 //             the updated even cells and the odd cells of the group with the
 //             prolongation added (0 off the fluid).
 //   kLast     last post-smoothing half-sweep (phase 0): writes the group's 8
-//             cells to the natural-order output zn (float), the even cells
+//             cells to the natural-order output zn, the even cells
 //             passed through (0 off the fluid).
 // Only the groups of the active list are visited; the other groups of the
 // split buffers are never read for a value that enters a fluid cell's update.
@@ -66,7 +66,7 @@ enum SplitMode { kFirst = 0, kOwnZero = 1, kInPlace = 2, kProlong = 3, kLast = 4
 
 struct SplitArgs {
     Dims D;
-    const int *act, *act_n;     // active 8-cell groups of level 0
+    const int *act, *act_n;     // active 8-cell groups of the level
     const uint16_t *sws;        // stencil words, colour-split
     const uint32_t *items;      // item words (smooth_block.cuh) of every group: colour 0, then colour 1
     const void *rn;             // kFirst: natural residual (TRN)
@@ -75,7 +75,7 @@ struct SplitArgs {
     void *z;                    // colour-split z (TZ), in place / output
     const void *zc;             // kProlong: next level's correction, natural order (TC)
     float zc_scale;
-    float *zn;                  // kLast: natural-order output
+    void *zn;                   // kLast: natural-order output (TC)
     // kLast: z.r of the CG step folded in (mgpcg.py:401, 451): dot 1 --
     // zr_old = z.r and p = z (the solve's prologue), dot 2 -- beta = z.r /
     // zr_old, zr_old = z.r (each iteration), dot 3 -- the flexible beta =
@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(256, (kMode == kProlong || kMode == kLast) ? 4
                 o8[2 * m + q] = out[m];
                 o8[2 * m + 1 - q] = vo[m];
             }
-            St<float>::st8(A.zn + ((size_t)g << 3), o8);
+            St<TC>::st8(static_cast<TC *>(A.zn) + ((size_t)g << 3), o8);
             if (A.dot) {
                 float zv[8], rv[8];
 #pragma unroll

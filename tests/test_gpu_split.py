@@ -1,5 +1,5 @@
 """The colour-split half-sweeps (flub_gb300/csrc/smooth_split.cuh) against the
-oracle's V-cycle, bit for bit: solids, air and walls on every side of a group,
+oracle's V-cycle, bit for bit, at level 0 and below: solids, air and walls on every side of a group,
 1 to 3 iterations a side, a residual that holds anything off the fluid; and
 after a V-cycle that ran in natural order on the same handle."""
 import numpy as np
@@ -11,7 +11,8 @@ from flub_gb300 import MGPCG
 
 pytestmark = pytest.mark.gpu
 
-SHAPES = [((104, 72, 88), 3), ((66, 50, 80), 2), ((128, 128, 128), 4), ((34, 258, 16), 2), ((130, 66, 8), 2)]
+SHAPES = [((104, 72, 88), 3), ((66, 50, 80), 2), ((128, 128, 128), 4), ((34, 258, 16), 2), ((130, 66, 8), 2),
+          ((1028, 32, 16), 3), ((256, 192, 80), 3)]
 
 
 def _case(shape, seed, solids):
@@ -57,3 +58,22 @@ def test_split_mixed_after_natural(shape, levels):
         mg.solve(max_iters=4, eps=1e-12, abs_tol=1e-12, rel_tol=1e-12, smoother="phases")
         x.append(mg.x.cpu().numpy())
     assert np.isfinite(x[0]).all() and np.array_equal(x[0], x[1])
+
+
+@pytest.mark.parametrize("nu", [1, 3])
+@pytest.mark.parametrize("shape,levels", [((2048, 32, 16), 3), ((256, 256, 128), 4)])
+def test_split_mixed_lower_levels(shape, levels, nu, monkeypatch):
+    """FP16 levels below level 0: the values stored are those of the natural-order sweeps."""
+    tag, r = _case(shape, sum(shape), 0.05)
+    rd = torch.from_numpy(r).cuda()
+    z = []
+    for off in ("1", "0"):
+        monkeypatch.setenv("FLUB_NO_SPLIT", off)
+        mg = MGPCG(3, shape, levels, float, precision="mixed")
+        mg.set_tags(torch.from_numpy(tag).cuda())
+        mg.set_schedule(nu, 3, 0.5)
+        mg.init(rd, 1.0)
+        mg.solve(max_iters=3, eps=1e-12, abs_tol=1e-12, rel_tol=1e-12, smoother="phases")
+        z.append((mg.apply_preconditioner(rd).cpu().numpy(), mg.x.cpu().numpy()))
+    assert np.isfinite(z[0][1]).all()
+    assert np.array_equal(z[0][0], z[1][0]) and np.array_equal(z[0][1], z[1][1])
