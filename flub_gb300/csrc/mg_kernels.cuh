@@ -302,9 +302,10 @@ __global__ void __launch_bounds__(kActThreads) k_act_write(const uint8_t *__rest
 // Loop over the groups a kernel works on: the active list when act is not
 // NULL (its length read from *act_n on the device), else every group 0..ng-1.
 #define FLUB_ACT_LOOP(g, act, act_n, ng)                                                                   \
-    for (int _t = blockIdx.x * blockDim.x + threadIdx.x, _tot = (act) ? *(act_n) : (ng); _t < _tot;     \
-         _t += gridDim.x * blockDim.x)                                                                       \
-        if (const int g = (act) ? __ldg((act) + _t) : _t; true)
+    for (int _s = gridDim.x * blockDim.x, _t = blockIdx.x * blockDim.x + threadIdx.x,                       \
+             _tot = (act) ? *(act_n) : (ng), _n = _t < _tot ? ((act) ? __ldg((act) + _t) : _t) : 0;          \
+         _t < _tot; _t += _s)                                                                                \
+        if (const int g = _n; (_n = _t + _s < _tot ? ((act) ? __ldg((act) + _t + _s) : _t + _s) : 0, true))
 
 // multigrid/mgpcg.py:276-284 init: r = k * rhs, x = p = 0.
 __global__ void k_init(float *__restrict__ r, const float *__restrict__ rhs, float kk, float *__restrict__ x,

@@ -253,7 +253,7 @@ static size_t carve(flub_mg *mg, char *base) {
         L.b_n = nullptr;
         L.z3h = nullptr;
         // (conditions on the shape, not on the pointers: those are NULL while sizing)
-        if (L.b_ti || split_level(mg, l))
+        if (L.b_ti || (l == 0 && L.D.nz % 8 == 0) || split_level(mg, l))
             L.b_items = (uint32_t *)take(sizeof(uint32_t) * (size_t)(nl / row_vector(L.D.nz)));
         if (L.b_ti) {
             L.b_tiles = block_tiles(L.D, L.b_ti);
@@ -991,7 +991,7 @@ static int enqueue_vcycle(flub_mg *mg, const LaunchCtx &c, const float *r0, floa
             FLUB_TRY(split_pre<float>(c, L, iters, R(l), L.rs, ZP(l)));
             const Level &C = mg->lv[l + 1];
             FLUB_TRY(launch_pdl(k_restrict8_split<float, float, float>, dim3(blocks_for(C.D.n(), 256, kNumSMs * 4)),
-                                dim3(256), 0, c.s, R(l), (const float *)ZP(l), (const uint8_t *)L.code,
+                                dim3(256), 0, c.s, R(l), (const float *)ZP(l), (const uint32_t *)L.b_items,
                                 (const uint16_t *)L.sw, C.r, (const uint8_t *)C.code, C.D, mg->sched_rscale,
                                 (const int *)C.act, (const int *)C.act_n, c.kc));
             continue;
@@ -1094,7 +1094,7 @@ static int enqueue_vcycle_mixed(flub_mg *mg, const LaunchCtx &c, float *z0, bool
             FLUB_TRY(split_pre<H>(c, L, iters, L.rh, L.rsh, L.z2h));
             const Level &C = mg->lv[l + 1];
             FLUB_TRY(launch_pdl(k_restrict8_split<H, H, H>, dim3(blocks_for(C.D.n(), 256, kNumSMs * 4)), dim3(256),
-                                0, c.s, (const H *)L.rh, (const H *)L.z2h, (const uint8_t *)L.code,
+                                0, c.s, (const H *)L.rh, (const H *)L.z2h, (const uint32_t *)L.b_items,
                                 (const uint16_t *)L.sw, C.rh, (const uint8_t *)C.code, C.D,
                                 0.125f * mg->sched_rscale, (const int *)C.act, (const int *)C.act_n, c.kc));
             continue;
@@ -1225,8 +1225,8 @@ static int enqueue_first_half_mixed(flub_mg *mg, const LaunchCtx &c, int smoothe
     const Level &L0 = mg->lv[0];
     const unsigned b = red_blocks(mg->n), bg = red_blocks(mg->n / 8 + 1);
     FLUB_TRY(launch_pdl(k8_matvec_pap, dim3(matvec_blocks(mg->n / 8)), dim3(kRedThreads), 0, c.s, mg->st, mg->p,
-                        mg->Ap, L0.code, (const uint16_t *)L0.sw, L0.D, mg->partials, (const int *)L0.act,
-                        (const int *)L0.act_n, c.kc));
+                        mg->Ap, (const uint32_t *)L0.b_items, (const uint16_t *)L0.sw, L0.D, mg->partials,
+                        (const int *)L0.act, (const int *)L0.act_n, c.kc));
     if (smoother == FLUB_SMOOTHER_FRACTION) {
         FLUB_CHECK_CUDA(cudaMemcpyAsync(mg->r_old, L0.r, sizeof(float) * mg->n, cudaMemcpyDeviceToDevice, c.s));
         FLUB_TRY(launch_pdl(k_update_r, dim3(b), dim3(kRedThreads), 0, c.s, mg->st, L0.r, mg->Ap, mg->n, c.kc));
@@ -1250,7 +1250,7 @@ static int enqueue_second_half_mixed(flub_mg *mg, const LaunchCtx &c) {
     if (!fused)  // else the flexible beta came with the last level-0 half-sweep
         FLUB_TRY(launch_pdl(k8_dot_zr_flex, dim3(bg), dim3(kRedThreads), 0, c.s, mg->st, L0.z, L0.r, mg->r_old,
                             L0.code, mg->n, mg->partials, (const int *)L0.act, (const int *)L0.act_n, c.kc));
-    return launch_pdl(k8_update_xp<true>, dim3(blocks_for(mg->n / 8, 256, kNumSMs * 8)), dim3(256), 0, c.s, mg->st,
+    return launch_pdl(k8_update_xp<true>, dim3(blocks_for(mg->n / 8, 256, kNumSMs * 6)), dim3(256), 0, c.s, mg->st,
                       mg->x, mg->p, L0.z, L0.code, mg->n, (const int *)L0.act, (const int *)L0.act_n, c.kc);
 }
 
@@ -1294,8 +1294,8 @@ static int enqueue_first_half(flub_mg *mg, const LaunchCtx &c, int smoother) {
     const unsigned bg = red_blocks(mg->n / 8 + 1);
     if (v8)
         FLUB_TRY(launch_pdl(k8_matvec_pap, dim3(matvec_blocks(mg->n / 8)), dim3(kRedThreads), 0, c.s, mg->st,
-                            mg->p, mg->Ap, L0.code, (const uint16_t *)L0.sw, L0.D, mg->partials, (const int *)L0.act,
-                            (const int *)L0.act_n, c.kc));
+                            mg->p, mg->Ap, (const uint32_t *)L0.b_items, (const uint16_t *)L0.sw, L0.D, mg->partials,
+                            (const int *)L0.act, (const int *)L0.act_n, c.kc));
     else
         FLUB_TRY(launch_pdl(k_matvec_pap, dim3(b), dim3(kRedThreads), 0, c.s, mg->st, mg->p, mg->Ap, L0.code, L0.D,
                             mg->partials, c.kc));
@@ -1330,7 +1330,7 @@ static int enqueue_second_half(flub_mg *mg, const LaunchCtx &c) {
             FLUB_TRY(launch_pdl(k8_dot_zr<false>, dim3(bg), dim3(kRedThreads), 0, c.s, mg->st, L0.z, L0.r,
                                 (float *)nullptr, L0.code, mg->n, mg->partials, (const int *)L0.act,
                                 (const int *)L0.act_n, c.kc));
-        return launch_pdl(k8_update_xp<false>, dim3(blocks_for(mg->n / 8, 256, kNumSMs * 8)), dim3(256), 0, c.s,
+        return launch_pdl(k8_update_xp<false>, dim3(blocks_for(mg->n / 8, 256, kNumSMs * 6)), dim3(256), 0, c.s,
                           mg->st, mg->x, mg->p, L0.z, L0.code, mg->n, (const int *)L0.act, (const int *)L0.act_n,
                           c.kc);
     }
@@ -1761,6 +1761,7 @@ int flub_mg_set_tags(flub_mg *mg, const int32_t *tag, void *stream) {
         FLUB_CHECK_LAUNCH();
         const int V = row_vector(L.D.nz);
         const unsigned blocks = blocks_for(L.D.n() / (2 * V), 256);
+        if (L.sw) continue;  // its items follow its stencil words below
         if (V == 4)
             k_block_items<4><<<blocks, 256, 0, s>>>(L.cw, L.D, L.b_items);
         else if (V == 2)
@@ -1776,10 +1777,12 @@ int flub_mg_set_tags(flub_mg *mg, const int32_t *tag, void *stream) {
             k_stencil_words<<<blocks_for(L.D.n() >> 3, 256), 256, 0, s>>>(L.code, L.sw, L.D);
             FLUB_CHECK_LAUNCH();
         }
+        if (L.sw && L.b_items) {
+            k_block_items<4><<<blocks_for(L.D.n() >> 3, 256), 256, 0, s>>>(L.sw, L.D, L.b_items);
+            FLUB_CHECK_LAUNCH();
+        }
         if (L.sws) {
             k_split_words<<<blocks_for(L.D.n() >> 3, 256), 256, 0, s>>>(L.sw, L.sws, L.D);
-            FLUB_CHECK_LAUNCH();
-            k_block_items<4><<<blocks_for(L.D.n() >> 3, 256), 256, 0, s>>>(L.sw, L.D, L.b_items);
             FLUB_CHECK_LAUNCH();
             if (L.zsh)
                 FLUB_CHECK_CUDA(cudaMemsetAsync(L.zsh, 0, sizeof(__half) * (size_t)L.D.n(), s));

@@ -120,15 +120,15 @@ __global__ void __launch_bounds__(kRedThreads) k8_update_r_rr_mixed(MgState *st,
     FLUB_ACT_LOOP(g, ga, act_n, ng) {
         if (skip && !ga && !group_has_fluid(load_codes8(code + (g << 3)))) continue;
         float rv[8], av[8], hv[8];
-        St<float>::ld8(r + (g << 3), rv);
-        St<float>::ld8_ro(Ap + (g << 3), av);
-        St<float>::st8(r_old + (g << 3), rv);
+        St<float>::ld8_wide(r + (g << 3), rv);
+        St<float>::ld8_wide(Ap + (g << 3), av);
+        St<float>::st8_wide(r_old + (g << 3), rv);
 #pragma unroll
         for (int m = 0; m < 8; m++) {
             rv[m] = __fmaf_rn(-a, av[m], rv[m]);
             hv[m] = __fmul_rn(rv[m], hs);
         }
-        St<float>::st8(r + (g << 3), rv);
+        St<float>::st8_wide(r + (g << 3), rv);
         St<__half>::st8(rh + (g << 3), hv);
         s += dot8_ff(rv, rv);
     }
@@ -158,11 +158,11 @@ __global__ void __launch_bounds__(kRedThreads) k8_dot_zr_flex(MgState *st, const
     FLUB_ACT_LOOP(g, act, act_n, ng) {
         if (!act && !group_has_fluid(load_codes8(code + (g << 3)))) continue;  // z = 0 there
         float zv[8], rv[8], ov[8];
-        St<float>::ld8_ro(z + (g << 3), zv);
+        St<float>::ld8_wide(z + (g << 3), zv);
 #pragma unroll
         for (int m = 0; m < 8; m++) zv[m] = __fmul_rn(zv[m], zs);
-        St<float>::ld8_ro(r + (g << 3), rv);
-        St<float>::ld8_ro(r_old + (g << 3), ov);
+        St<float>::ld8_wide(r + (g << 3), rv);
+        St<float>::ld8_wide(r_old + (g << 3), ov);
         s += dot8_ff(zv, rv);
         so += dot8_ff(zv, ov);
     }

@@ -112,8 +112,10 @@ __global__ void __launch_bounds__(kPersistThreads, 2) k_vcycle_down(const LegPar
         }
         const LegLevel &C = P.lv[l + 1];
         if (l + 1 == P.l1) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-        restrict8_pass<false, false>(static_cast<const T *>(L.r), (const T *)z2, L.code, L.sw, static_cast<T *>(C.r),
-                                     C.code, C.D, P.rscale, C.act, C.act_n, blockIdx.x, gridDim.x);
+        restrict8_pass(static_cast<T *>(C.r), C.code, C.D, P.rscale, C.act, C.act_n, blockIdx.x, gridDim.x, false,
+                       nullptr, [&](int g, float *v) {
+                           residual_row8<false>(static_cast<const T *>(L.r), (const T *)z2, L.code, L.sw, L.D, g, v);
+                       });
         if (l + 1 < P.l1) grid_barrier(P.st);
     }
 }

@@ -35,12 +35,12 @@ enum BlockMode { kBlockFromZero = 0, kBlockPlain = 1, kBlockProlong = 2 };
 
 // What a half-sweep has to know of an item (V cells of one colour in a row),
 // in one word per colour: a nibble per cell with its diagonal count (0: never
-// updated), kItemAny when a count is not 0, and kItemSolid when a neighbour
-// does not count although it lies in the domain.  Built once by set_tags; an
+// updated), kItemAny when a count is not 0, kItemSolid when a neighbour does not
+// count although it lies in the domain, and kItemAir when one is air.  Built once by set_tags; an
 // item without kItemSolid needs no stencil words: a neighbour outside the
 // domain is replaced by the cell itself, whose term is then 0.
 constexpr uint32_t kAllCount = 0x1554u;  // sw_ns of a cell whose six neighbours all count
-constexpr uint32_t kItemAny = 1u << 16, kItemSolid = 1u << 17;
+constexpr uint32_t kItemAny = 1u << 16, kItemSolid = 1u << 17, kItemAir = 1u << 18;
 
 struct BlockArgs {
     Dims D;
@@ -324,9 +324,17 @@ __global__ void __launch_bounds__(256) k_block_items(const uint16_t *__restrict_
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
         const int seg = e % lsegs, row = e / lsegs, j = row % D.ny, i = row / D.ny, par = (i + j) & 1;
         uint32_t out[2] = {0u, 0u};
+        uint32_t wd[V];  // two words each
+        if constexpr (V == 4) {
+            const uint4 q = __ldg(reinterpret_cast<const uint4 *>(cw) + e);
+            wd[0] = q.x; wd[1] = q.y; wd[2] = q.z; wd[3] = q.w;
+        } else {
+#pragma unroll
+            for (int m = 0; m < V; m++) wd[m] = __ldg(reinterpret_cast<const uint32_t *>(cw) + (int64_t)e * V + m);
+        }
 #pragma unroll
         for (int m = 0; m < 2 * V; m++) {
-            const uint32_t w = __ldg(cw + (int64_t)e * (2 * V) + m);
+            const uint32_t w = (wd[m >> 1] >> (16 * (m & 1))) & 0xffffu;
             const int k = 2 * V * seg + m;
             if ((w & 3u) != kCodeFluid) continue;
             const uint32_t ns = sw_ns(w), d = __popc(ns);
@@ -341,6 +349,7 @@ __global__ void __launch_bounds__(256) k_block_items(const uint16_t *__restrict_
             o |= d << (4 * (m >> 1));
             if (d) o |= kItemAny;
             if (d && ns != inside) o |= kItemSolid;
+            if (d && (w & kAllCount)) o |= kItemAir;  // the low bit of a neighbour's code
         }
         items[e] = out[0];
         items[n + e] = out[1];

@@ -30,8 +30,8 @@
 // word per cell, decoded with a branch per cell wherever one of the 4 is not
 // interior, took ~400 instructions an item, and a warp of 32 rows nearly always
 // has such an item.  With the item word only items next to a solid load their
-// stencil words.  The first half of the prolongation still takes the stencil
-// words: it has the neighbours' corrections to add and no register to spare.
+// stencil words; the prolongation, which adds the correction to air as well, does
+// so next to air too.
 // A half-sweep of 128^3 (FP32, dam break / full): 1.9 / 3.7 us, in natural order
 // 3.0 / 6.7.  Measured through a whole solve (before -> now): 128^3 sphere in mixed
 // precision 8536 -> 7859 us, 256^3 dam break 15880 -> 15310, 256 x 64 x 256
@@ -90,35 +90,20 @@ struct SplitArgs {
     double *partials;
 };
 
-// Stencil word of a fluid cell whose six neighbours are all fluid (code 2 in
-// all seven 2-bit fields), twice: the 4 words of a lane are all interior when
-// both halves of its 8-byte word load equal this.
-constexpr uint32_t kInteriorWord2 = 0x2AAA2AAAu;
-
-// smooth_cell for an interior word (d = 6), without the per-cell word test.
-__device__ __forceinline__ float smooth_interior(float xc, float xip, float xim, float xjp, float xjm, float xkp,
-                                                 float xkm, float r) {
-    return __fadd_rn(xc, div6_rn(__fadd_rn(r, interior_nbsum(xc, xip, xim, xjp, xjm, xkp, xkm))));
-}
-
 __device__ __forceinline__ uint32_t word4_at(uint2 w, int m) {
     const uint32_t v = m < 2 ? w.x : w.y;
     return (m & 1) ? (v >> 16) : (v & 0xffffu);
 }
 
-// The code of the cell on the other side of word w's k+ (kp = true) or k-
-// neighbour bits.
-__device__ __forceinline__ uint32_t word_kcode(uint32_t w, bool kp) { return sw_code(w, kp ? 5 : 6); }
-
-// Register bound of 3 blocks of 256 threads per SM for the lean modes (the
-// in-place FP32 sweep then takes 64 registers and 4 blocks are resident), 4
-// for the prolongation and the natural-order output.  Measured on the 256^3
-// and 512^3 dam breaks: the lean modes at 5 blocks (48 registers) are as fast
-// at 256^3 and 10 % slower at 512^3 (fewer groups in flight at once stream
-// from DRAM more efficiently), 6 spills, and 2 blocks, or two groups per lane
-// with their loads issued together, are slower at both sizes.
+// Register bound of 4 blocks of 256 threads per SM: 55 to 64 registers.  No array
+// here is indexed by q, the parity of the updated cells' k: as an index it made
+// the compiler select among all elements for each (the last half-sweep took 600
+// instructions an item, now 310; 256^3-sized levels 17 -> 12 us, 512 x 256 x 256
+// with the dot product 123 -> 101 us and 54 -> 51 us in place, of DRAM traffic worth
+// 87 and 41).  More blocks, fewer, or two groups a lane with their loads issued
+// together measured no better.
 template <int kMode, typename TRN, typename TR, typename TZI, typename TZ, typename TC>
-__global__ void __launch_bounds__(256, (kMode == kProlong || kMode == kLast) ? 4 : 3)
+__global__ void __launch_bounds__(256, 4)
     k_smooth_split(const SplitArgs A, int phase, unsigned long long *kc) {
     __shared__ float2 lut[8];  // -1/d and d
     pdl_open();
@@ -136,25 +121,11 @@ __global__ void __launch_bounds__(256, (kMode == kProlong || kMode == kLast) ? 4
     int g_next = t < total ? __ldg(A.act + t) : 0;
     // the list and the first words do not depend on the previous kernel
     const uint32_t *items = A.items + (col ? (int)(D.n() >> 3) : 0), *other = A.items + (col ? 0 : (int)(D.n() >> 3));
-    uint32_t it_next = 0u;
-    uint2 wd_next = make_uint2(0u, 0u);
-    if (t < total) {
-        if (kMode != kProlong) {
-            it_next = __ldg(items + g_next);
-        } else {
-            int i0, j0, kg0;
-            group_ijk(g_next, D, i0, j0, kg0);
-            wd_next = __ldg(reinterpret_cast<const uint2 *>(A.sws + uoff + (i0 * D.ny + j0) * hz + 4 * kg0));
-        }
-    }
-    if (kMode != kProlong) {
-        if (threadIdx.x < 8)
-            lut[threadIdx.x] =
-                make_float2(threadIdx.x ? __fdiv_rn(-1.0f, (float)threadIdx.x) : 0.0f, (float)threadIdx.x);
-        __syncthreads();
-    }
+    uint32_t it_next = t < total ? __ldg(items + g_next) : 0u;
+    if (threadIdx.x < 8)
+        lut[threadIdx.x] = make_float2(threadIdx.x ? __fdiv_rn(-1.0f, (float)threadIdx.x) : 0.0f, (float)threadIdx.x);
+    __syncthreads();
     pdl_wait(kc);
-    bool first = true;
     double zr = 0.0, zro = 0.0;  // kLast with A.dot: this thread's parts of z.r and z.r_old
     const float zsc = (kMode == kLast && A.dot && A.zscaled) ? A.st->zscale : 1.0f;
     for (; t < total; t += stride) {
@@ -165,18 +136,13 @@ __global__ void __launch_bounds__(256, (kMode == kProlong || kMode == kLast) ? 4
         group_ijk(g, D, i, j, kg);
         const int h = (i * D.ny + j) * hz + 4 * kg;  // split index of the group's first element
         const int q = (col + i + j) & 1;             // updated cell m sits at natural k = 8 kg + 2 m + q
-        uint2 wd = make_uint2(0u, 0u);
-        uint32_t item = 0u;
-        if (kMode == kProlong)
-            wd = first ? wd_next : __ldg(reinterpret_cast<const uint2 *>(A.sws + uoff + h));
-        else
-            item = first ? it_next : __ldg(items + g);
-        first = false;
+        const uint32_t item = it_next;
+        it_next = tn < total ? __ldg(items + g_next) : 0u;
         float rr[4];
         if (kMode == kFirst) {
             // natural residual row -> both halves of the split residual
             float rv[8];
-            St<TRN>::ld8_ro(static_cast<const TRN *>(A.rn) + ((size_t)g << 3), rv);
+            St<TRN>::ld8_any(static_cast<const TRN *>(A.rn) + ((size_t)g << 3), rv);
             const int p = (i + j) & 1;  // natural cell m is even when (p + m) is even
             float re[4], ro[4];
 #pragma unroll
@@ -207,10 +173,9 @@ __global__ void __launch_bounds__(256, (kMode == kProlong || kMode == kLast) ? 4
         St<TR>::ld4_ro(rs + uoff + h, rr);
         const bool hip = i + 1 < D.nx, him = i > 0, hjp = j + 1 < D.ny, hjm = j > 0;
         const bool hkm = kg > 0, hkp = 4 * kg + 4 < hz;
-        // operands: own z, the other colour's row (i, j) as the window w[0..4]
-        // (w[m] is cell m's k- neighbour, w[m + 1] its k+ neighbour), and its
-        // four neighbour rows
-        float xc[4] = {0.f, 0.f, 0.f, 0.f}, w[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
+        // operands: own z, the other colour's row (i, j) with the element before
+        // (q = 0) or after it (q = 1), and its four neighbour rows
+        float xc[4] = {0.f, 0.f, 0.f, 0.f}, edge;
         float zip[4] = {0.f, 0.f, 0.f, 0.f}, zim[4] = {0.f, 0.f, 0.f, 0.f};
         float zjp[4] = {0.f, 0.f, 0.f, 0.f}, zjm[4] = {0.f, 0.f, 0.f, 0.f};
         float vc[4];
@@ -223,7 +188,7 @@ __global__ void __launch_bounds__(256, (kMode == kProlong || kMode == kLast) ? 4
             auto crow = [&](int ii, int jj, float o[4]) {
                 St<TC>::ld4_ro(zc + ((size_t)((ii >> 1) * cy + (jj >> 1)) * hz + 4 * kg), o);
             };
-            float cc[4], cn[4];
+            float cc[4], cn[4] = {0.f, 0.f, 0.f, 0.f};
             crow(i, j, cc);
             St<TZI>::ld4(zi + uoff + h, xc);
             St<TZI>::ld4(zi + voff + h, vc);
@@ -232,37 +197,24 @@ __global__ void __launch_bounds__(256, (kMode == kProlong || kMode == kLast) ? 4
                 xc[m] = __fadd_rn(xc[m], __fmul_rn(cc[m], s));
                 vc[m] = __fadd_rn(vc[m], __fmul_rn(cc[m], s));
             }
-            if (hip) {
-                St<TZI>::ld4(zi + voff + h + si, zip);
-                crow(i + 1, j, cn);
+            auto row = [&](bool in, int off, int ii, int jj, float o[4]) {
+                if (in) {
+                    St<TZI>::ld4(zi + voff + h + off, o);
+                    crow(ii, jj, cn);
+                }
 #pragma unroll
-                for (int m = 0; m < 4; m++) zip[m] = __fadd_rn(zip[m], __fmul_rn(cn[m], s));
-            }
-            if (him) {
-                St<TZI>::ld4(zi + voff + h - si, zim);
-                crow(i - 1, j, cn);
-#pragma unroll
-                for (int m = 0; m < 4; m++) zim[m] = __fadd_rn(zim[m], __fmul_rn(cn[m], s));
-            }
-            if (hjp) {
-                St<TZI>::ld4(zi + voff + h + sj, zjp);
-                crow(i, j + 1, cn);
-#pragma unroll
-                for (int m = 0; m < 4; m++) zjp[m] = __fadd_rn(zjp[m], __fmul_rn(cn[m], s));
-            }
-            if (hjm) {
-                St<TZI>::ld4(zi + voff + h - sj, zjm);
-                crow(i, j - 1, cn);
-#pragma unroll
-                for (int m = 0; m < 4; m++) zjm[m] = __fadd_rn(zjm[m], __fmul_rn(cn[m], s));
-            }
-            // the window's fifth value: element h - 1 (q = 0) or h + 4 (q = 1),
-            // whose parent is coarse K = 4 kg - 1 or 4 kg + 4
-            const size_t crow0 = (size_t)((i >> 1) * cy + (j >> 1)) * hz;
-            if (q == 0 && hkm)
-                w[0] = __fadd_rn(St<TZI>::ld(zi + voff + h - 1), __fmul_rn(St<TC>::ld_ro(zc + crow0 + 4 * kg - 1), s));
-            if (q == 1 && hkp)
-                w[4] = __fadd_rn(St<TZI>::ld(zi + voff + h + 4), __fmul_rn(St<TC>::ld_ro(zc + crow0 + 4 * kg + 4), s));
+                for (int m = 0; m < 4; m++) o[m] = in ? __fadd_rn(o[m], __fmul_rn(cn[m], s)) : xc[m];
+            };
+            row(hip, si, i + 1, j, zip);
+            row(him, -si, i - 1, j, zim);
+            row(hjp, sj, i, j + 1, zjp);
+            row(hjm, -sj, i, j - 1, zjm);
+            const int eo = q ? 4 : -1;
+            edge = q ? xc[3] : xc[0];
+            if (q ? hkp : hkm)
+                edge = __fadd_rn(
+                    St<TZI>::ld(zi + voff + h + eo),
+                    __fmul_rn(St<TC>::ld_ro(zc + (size_t)((i >> 1) * cy + (j >> 1)) * hz + 4 * kg + eo), s));
         } else {
             // a neighbour row outside the domain is replaced by the cells
             // themselves: their terms are then 0
@@ -279,54 +231,44 @@ __global__ void __launch_bounds__(256, (kMode == kProlong || kMode == kLast) ? 4
                 if (hjp) St<TZ>::ld4(z + voff + h + sj, zjp);
                 if (hjm) St<TZ>::ld4(z + voff + h - sj, zjm);
             }
-            if (q == 0) w[0] = hkm ? St<TZ>::ld(z + voff + h - 1) : xc[0];
-            if (q == 1) w[4] = hkp ? St<TZ>::ld(z + voff + h + 4) : xc[3];
+            edge = (q ? hkp : hkm) ? St<TZ>::ld(z + voff + h + (q ? 4 : -1)) : (q ? xc[3] : xc[0]);
         }
-        // w[t] is element h - 1 + q + t of the other colour's row
+        float out[4], vo[4], va[4], vb[4];  // va: the k neighbours inside the group's row, vb the others
 #pragma unroll
-        for (int m = 0; m < 4; m++) w[m + 1 - q] = vc[m];
-        float out[4], vo[4];
-        if (kMode != kProlong) {
-            float va[4], vb[4];  // the k neighbours inside the group's row, and the others
-#pragma unroll
-            for (int m = 0; m < 4; m++) {
-                va[m] = vc[m];
-                vb[m] = q ? w[m + 1] : w[m];
-                out[m] = xc[m];
-                vo[m] = vc[m];
-            }
-            if (item & kItemSolid) {
-                // solids next to it: the neighbours that do not count become the cell itself
-                const uint2 ws = __ldg(reinterpret_cast<const uint2 *>(A.sws + uoff + h));
-#pragma unroll
-                for (int m = 0; m < 4; m++) {
-                    const uint32_t ns = sw_ns(word4_at(ws, m));
-                    if (!(ns & 4u)) zip[m] = xc[m];
-                    if (!(ns & 16u)) zim[m] = xc[m];
-                    if (!(ns & 64u)) zjp[m] = xc[m];
-                    if (!(ns & 256u)) zjm[m] = xc[m];
-                    if (!(ns & (q ? 4096u : 1024u))) va[m] = xc[m];
-                    if (!(ns & (q ? 1024u : 4096u))) vb[m] = xc[m];
-                }
-            }
-            block_update<4>(item, out, zip, zim, zjp, zjm, va, vb, rr, lut);
-        } else if (wd.x == kInteriorWord2 && wd.y == kInteriorWord2) {
-            // four interior cells (most of a water body): their k neighbours, the
-            // other colour's elements of the group, are fluid too
+        for (int m = 0; m < 4; m++) {
+            va[m] = vc[m];
+            vb[m] = q ? (m < 3 ? vc[m < 3 ? m + 1 : m] : edge) : (m > 0 ? vc[m > 0 ? m - 1 : m] : edge);
+            out[m] = xc[m];
+            vo[m] = vc[m];
+        }
+        if (item & (kMode == kProlong ? kItemSolid | kItemAir : kItemSolid)) {
+            // solids next to it: the neighbours that do not count become the cell
+            // itself; air is 0 in z, but not after the prolongation's addition
+            const uint2 ws = __ldg(reinterpret_cast<const uint2 *>(A.sws + uoff + h));
 #pragma unroll
             for (int m = 0; m < 4; m++) {
-                out[m] = smooth_interior(xc[m], zip[m], zim[m], zjp[m], zjm[m], w[m + 1], w[m], rr[m]);
-                vo[m] = vc[m];
+                const uint32_t cw = word4_at(ws, m), ns = sw_ns(cw);
+                auto fix = [&](float &v, uint32_t bit) {
+                    if (!(ns & bit)) v = xc[m];
+                    else if (kMode == kProlong && (cw & bit)) v = 0.0f;
+                };
+                fix(zip[m], 4u);
+                fix(zim[m], 16u);
+                fix(zjp[m], 64u);
+                fix(zjm[m], 256u);
+                fix(va[m], q ? 4096u : 1024u);
+                fix(vb[m], q ? 1024u : 4096u);
             }
-        } else {
-#pragma unroll
-            for (int m = 0; m < 4; m++)
-                out[m] = smooth_cell<false>(word4_at(wd, m), xc[m], zip[m], zim[m], zjp[m], zjm[m], w[m + 1], w[m],
-                                            rr[m]);
-            // the other colour's cells of the group, 0 where they are never updated
+        }
+        block_update<4>(item, out, zip, zim, zjp, zjm, va, vb, rr, lut);
+        if (kMode == kProlong) {
+            // 0 where a cell is never updated: the addition left the correction there
             const uint32_t ov = __ldg(other + g);
 #pragma unroll
-            for (int m = 0; m < 4; m++) vo[m] = (ov >> (4 * m)) & 7u ? vc[m] : 0.0f;
+            for (int m = 0; m < 4; m++) {
+                if (!((item >> (4 * m)) & 7u)) out[m] = 0.0f;
+                if (!((ov >> (4 * m)) & 7u)) vo[m] = 0.0f;
+            }
         }
         if (kMode == kLast) {
             // natural row of the group: updated cell m at offset 2 m + q, the
@@ -334,22 +276,22 @@ __global__ void __launch_bounds__(256, (kMode == kProlong || kMode == kLast) ? 4
             float o8[8];
 #pragma unroll
             for (int m = 0; m < 4; m++) {
-                o8[2 * m + q] = out[m];
-                o8[2 * m + 1 - q] = vo[m];
+                o8[2 * m] = q ? vo[m] : out[m];
+                o8[2 * m + 1] = q ? out[m] : vo[m];
             }
-            St<TC>::st8(static_cast<TC *>(A.zn) + ((size_t)g << 3), o8);
+            St<TC>::st8_any(static_cast<TC *>(A.zn) + ((size_t)g << 3), o8);
             if (A.dot) {
                 float zv[8], rv[8];
+                St<float>::ld8_wide(A.rdot + ((size_t)g << 3), rv);
 #pragma unroll
                 for (int m = 0; m < 8; m++) zv[m] = A.zscaled ? __fmul_rn(o8[m], zsc) : o8[m];
-                St<float>::ld8_ro(A.rdot + ((size_t)g << 3), rv);
                 zr += dot8_ff(zv, rv);
                 if (A.dot == 3) {
                     float ov[8];
-                    St<float>::ld8_ro(A.rold + ((size_t)g << 3), ov);
+                    St<float>::ld8_wide(A.rold + ((size_t)g << 3), ov);
                     zro += dot8_ff(zv, ov);
                 }
-                if (A.dot == 1) St<float>::st8(A.pinit + ((size_t)g << 3), zv);
+                if (A.dot == 1) St<float>::st8_wide(A.pinit + ((size_t)g << 3), zv);
             }
         } else {
             St<TZ>::st4(z + uoff + h, out);

@@ -5,6 +5,8 @@
 
 #include <cuda_fp16.h>
 
+#include <cstdint>
+
 namespace flub {
 
 template <typename T>
@@ -61,6 +63,25 @@ struct St<float> {
     static __device__ __forceinline__ void st4(float *p, const float v[4]) {
         *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
     }
+    // 32 bytes in one access; p is 32-byte aligned.  A warp whose lanes hold
+    // consecutive groups then touches each 128-byte line once, not twice.
+    static __device__ __forceinline__ void ld8_wide(const float *p, float o[8]) {
+        asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=f"(o[0]), "=f"(o[1]), "=f"(o[2]), "=f"(o[3]), "=f"(o[4]), "=f"(o[5]), "=f"(o[6]), "=f"(o[7])
+                     : "l"(__cvta_generic_to_global(p)));
+    }
+    static __device__ __forceinline__ void st8_wide(float *p, const float v[8]) {
+        asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(__cvta_generic_to_global(p)),
+                     "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
+                     : "memory");
+    }
+    // the same where p may be a caller's array, 16-byte aligned only
+    static __device__ __forceinline__ void ld8_any(const float *p, float o[8]) {
+        if (reinterpret_cast<uintptr_t>(p) & 16) ld8(p, o); else ld8_wide(p, o);
+    }
+    static __device__ __forceinline__ void st8_any(float *p, const float v[8]) {
+        if (reinterpret_cast<uintptr_t>(p) & 16) st8(p, v); else st8_wide(p, v);
+    }
 };
 
 template <>
@@ -83,6 +104,7 @@ struct St<__half> {
     static __device__ __forceinline__ void ld8_ro(const __half *p, float o[8]) {
         unpack8(__ldg(reinterpret_cast<const uint4 *>(p)), o);
     }
+    static __device__ __forceinline__ void ld8_any(const __half *p, float o[8]) { ld8(p, o); }
     static __device__ __forceinline__ void ld4_ro(const __half *p, float o[4]) {
         const uint2 u = __ldg(reinterpret_cast<const uint2 *>(p));
         const __half2 *h = reinterpret_cast<const __half2 *>(&u);
@@ -128,6 +150,7 @@ struct St<__half> {
         for (int q = 0; q < 4; q++) h[q] = __floats2half2_rn(v[2 * q], v[2 * q + 1]);
         *reinterpret_cast<uint4 *>(p) = u;
     }
+    static __device__ __forceinline__ void st8_any(__half *p, const float v[8]) { st8(p, v); }
     static __device__ __forceinline__ void st4(__half *p, const float v[4]) {
         uint2 u;
         __half2 *h = reinterpret_cast<__half2 *>(&u);

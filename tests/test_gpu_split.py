@@ -77,3 +77,36 @@ def test_split_mixed_lower_levels(shape, levels, nu, monkeypatch):
         z.append((mg.apply_preconditioner(rd).cpu().numpy(), mg.x.cpu().numpy()))
     assert np.isfinite(z[0][1]).all()
     assert np.array_equal(z[0][0], z[1][0]) and np.array_equal(z[0][1], z[1][1])
+
+
+@pytest.mark.parametrize("solids", [0.0, 0.05])
+@pytest.mark.parametrize("shape,levels", [((32, 32, 32), 3), ((10, 6, 8), 1), ((66, 50, 80), 2), ((34, 258, 16), 2)])
+def test_solver_matvec_bit_exact(shape, levels, solids):
+    """A p of the solve's first iteration: rows read 32 bytes a lane, their ends
+    from the neighbouring lanes, a last warp that is not full."""
+    tag, r = _case(shape, sum(shape), solids)
+    mg = MGPCG(3, shape, levels, float)
+    mg.set_tags(torch.from_numpy(tag).cuda())
+    rd = torch.from_numpy(r).cuda()
+    mg.init(rd, 1.0)
+    mg.mask_interior()
+    mg.solve(max_iters=1, eps=1e-12, abs_tol=0.0, rel_tol=0.0, smoother="phases")
+    n = r.size
+    step = (4 * n + 255) // 256 * 256  # x, p, A p lie one after the other
+    Ap = mg._view(mg.x.data_ptr() + 2 * step, n)
+    assert torch.equal(Ap, mg.matvec(mg.apply_preconditioner(rd)))
+
+
+@pytest.mark.parametrize("precision", ["fp32", "mixed"])
+def test_split_arrays_16_byte_aligned(precision):
+    """A caller's r and z at an address that is a multiple of 16 but not of 32."""
+    shape, levels = (128, 128, 128), 4
+    tag, r = _case(shape, 5, 0.02)
+    mg = MGPCG(3, shape, levels, float, precision=precision)
+    mg.set_tags(torch.from_numpy(tag).cuda())
+    rd = torch.from_numpy(r).cuda()
+    ro = torch.empty(r.size + 4, device="cuda")[4:].view(shape)
+    zo = torch.empty(r.size + 4, device="cuda")[4:].view(shape)
+    ro.copy_(rd)
+    assert ro.data_ptr() % 32 == 16 and zo.data_ptr() % 32 == 16
+    assert torch.equal(mg.apply_preconditioner(ro, zo), mg.apply_preconditioner(rd))
