@@ -250,41 +250,49 @@ __global__ void __launch_bounds__(kConvThreads, 1)
 //
 // The same convolution for NZ % 8 == 0 and NY % 16 == 0 when the layer's
 // weights fit in shared memory, organised around input planes instead of
-// tap-shifted tiles, with no TMA and no waits between MMAs.
+// tap-shifted tiles, with no TMA.
 //
-// A CTA owns a 16 (y) x 8 (z) voxel tile at xr consecutive x planes x0 ..
-// x0 + xr - 1; GEMM row m is voxel (y0 + m / 8, z0 + m % 8).  First all 128
-// threads stage, with coalesced 16-byte loads:
-//   - input plane p (x = x0 - 1 + p, p = 0 .. xr + 1) of each source as the
-//     haloed 18 x 10 voxel region, zero outside the volume (the padding), in
-//     the no-swizzle K-major layout
-//         [chunk of 8 channels][y 0..17][z 0..9][8 channels]   (16-byte rows);
-//   - every tap's weights, [tap][chunk][Cout][8 channels], the same layout
-//     for the B operand (core matrix = 8 output channels x 16 bytes).
-// A proxy fence publishes them to the tensor core.  The A operand of tap
-// (dx, dy, dz) for output plane xi is plane xi + dx + 1 read from start
-// offset ((dy + 1) * 10 + dz + 1) * 16 bytes: a core matrix is the 8 z-voxels
-// of one y-row (128 contiguous bytes), core matrices adjacent in M are one
-// padded row apart (SBO = 160 bytes) and adjacent chunks one chunk region apart
-// (LBO = kHaloChunk).  So all 27 taps read one copy of the data, and one
-// thread then issues every MMA of the CTA back to back into xr FP32
-// accumulators side by side in TMEM (columns xi * Cout ...).
+// A CTA owns a 16 (y) x 8 (z) voxel tile at up to xr consecutive x planes x0 ..;
+// GEMM row m is voxel (y0 + m / 8, z0 + m % 8).  Input plane p (x = x0 - 1 + p)
+// of every source is staged once, in coalesced 16-byte pieces, as the haloed
+// 18 x 10 voxel region, zero outside the volume (the padding), in the
+// no-swizzle K-major layout
+//     [chunk of 8 channels][y 0..17][z 0..9][8 channels]   (16-byte rows).
+// The A operand of the nine taps (dy, dz) is that plane read from start offset
+// ((dy + 1) * 10 + dz + 1) * 16 bytes: a core matrix is the 8 z-voxels of one
+// y-row (128 contiguous bytes), core matrices adjacent in M are one padded row
+// apart (SBO = 160 bytes) and adjacent chunks one chunk region apart (LBO).
 //
-// Staging the weights with plain loads matters: per-tap TMA boxes of a few
-// hundred bytes, requested by many CTAs per SM, arrived about 0.4 us apart
-// and left the MMA thread waiting on every tap.
+// An MMA of N = 16 to 64 is bound by the SM reading its A operand (about 44
+// cycles for one 128 x 16 BF16 tile), so the three taps along x share it: input
+// plane p contributes to the output planes p - 2, p - 1 and p of the CTA, whose
+// accumulators lie side by side in TMEM (columns xi * Cout ...), and the weights
+// are staged as [dy, dz][chunk][dx = 1, 0, -1][Cout][8 channels], so that one MMA
+// of N = 3 Cout serves all three.  A plane is thus finished with after its own
+// MMAs, and planes pass through a ring of R buffers:
+//   - warps 4-7 stage planes with asynchronous copies, R - 1 planes ahead and,
+//     before they reuse a buffer, behind done[p - R]; when plane p has landed they
+//     publish it to the tensor core (a proxy fence) and arrive on full[p];
+//   - one thread of warp 8 issues its MMAs and commits them to done[p];
+//   - warps 0-3 write output plane o after done[o + 2].
+// Each role's chain of instructions for a plane is as long as its MMAs, so none
+// does another's work.
+// 4 x 64^3, 32 + 16 -> 16 channels: the tap tiles' 254 us -> 78 us; 16 -> 32
+// and 16 -> 16: 105 and 72 us with one MMA a tap and no overlap -> 56 and 40.
 constexpr int kHaloZ = 10, kHaloY = 18;
-constexpr int kHaloRows = kHaloZ * kHaloY;                      // 16-byte rows per chunk (180)
-constexpr int kHaloChunk = (kHaloRows * 16 + 127) / 128 * 128;  // chunk region, 128-byte aligned (2944)
+constexpr int kHaloRows = kHaloZ * kHaloY;  // 16-byte rows per chunk (180)
+constexpr int kHaloThreads = 2 * kConvThreads + 32;
+constexpr int kHaloMaxX = 16;               // output planes per CTA
+constexpr int kHaloBars = 8 * 2 * (kHaloMaxX + 2);
 
 struct HaloGeom {
     int B, NX, NY, NZ;
-    int xr;                 // output planes per CTA
+    int xr, ring;           // output planes per CTA, plane buffers
     int cin0, cin1, relu;   // cin1 = 0: one source
-    int plane0, plane1;     // bytes of one input plane per source (chunks x kHaloChunk)
-    int planes1_off;        // offset of source 1's planes
+    int chunk0, chunk1;     // bytes from one chunk region to the next, per source
+    int src1_off, slot;     // source 1's chunks within a plane buffer, bytes of one
     int w0_off, w1_off;     // weights of source 0 and 1 (27 taps each)
-    int bar_off;            // completion mbarrier and TMEM slot
+    int bar_off;            // mbarriers full[], done[], TMEM slot
     uint32_t tmem_cols;
 };
 
@@ -300,80 +308,61 @@ __device__ __forceinline__ uint64_t ns_desc(uint32_t saddr, uint32_t lbo, uint32
     return d;
 }
 
-// Stages the np haloed input planes of one source into dst (layout above).
-// Item q = ((p * 18 + yh) * 10 + zh) * C8 + c, chunks fastest, so that a
-// warp's loads cover whole voxel rows of the channels-last input.  Eight
-// loads are in flight per thread before their stores.
-__device__ __forceinline__ void halo_stage(const uint4 *__restrict__ x, unsigned char *dst, int c8_log2, int np,
-                                           int plane_bytes, int b, int x0, int y0, int z0, const HaloGeom &g) {
-    const int C8 = 1 << c8_log2;
-    const int total = np * kHaloRows * C8;
-    for (int base = 0; base < total; base += 8 * kConvThreads) {
-        uint4 v[8];
-        int off[8];
-#pragma unroll
-        for (int u = 0; u < 8; u++) {
-            const int q = base + u * kConvThreads + threadIdx.x;
-            off[u] = -1;
-            v[u] = make_uint4(0u, 0u, 0u, 0u);
-            if (q < total) {
-                const int c = q & (C8 - 1);
-                int r = q >> c8_log2;
-                const int zh = r % kHaloZ;
-                r /= kHaloZ;
-                const int yh = r % kHaloY, p = r / kHaloY;
-                const int xx = x0 - 1 + p, yy = y0 - 1 + yh, zz = z0 - 1 + zh;
-                off[u] = p * plane_bytes + c * kHaloChunk + (yh * kHaloZ + zh) * 16;
-                if ((unsigned)xx < (unsigned)g.NX && (unsigned)yy < (unsigned)g.NY && (unsigned)zz < (unsigned)g.NZ)
-                    v[u] = __ldg(x + ((((int64_t)b * g.NX + xx) * g.NY + yy) * g.NZ + zz) * C8 + c);
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < 8; u++)
-            if (off[u] >= 0) *reinterpret_cast<uint4 *>(dst + off[u]) = v[u];
-    }
+// 16 bytes to shared memory, or 16 zero bytes (src is not read then, but is a valid address).
+__device__ __forceinline__ void copy16_async(uint32_t dst, const void *src, bool in) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(__cvta_generic_to_global(src)),
+                 "r"(in ? 16 : 0)
+                 : "memory");
 }
 
-// Stages weights [27][COUT][Cin] (Cin = 8 << c8_log2) as [tap][chunk][COUT][8].
+// Stages weights [27][COUT][Cin] (Cin = 8 << c8_log2) as
+// [dy, dz][chunk][dx = 1, 0, -1][COUT][8].
 template <int COUT>
-__device__ __forceinline__ void halo_stage_weights(const uint4 *__restrict__ w, unsigned char *dst, int c8_log2) {
+__device__ __forceinline__ void halo_stage_weights(const uint4 *__restrict__ w, uint32_t dst, int c8_log2,
+                                                   int tid) {
     const int C8 = 1 << c8_log2;
     const int total = 27 * COUT * C8;
-    for (int q = threadIdx.x; q < total; q += kConvThreads) {
+    for (int q = tid; q < total; q += kConvThreads) {
         const int c = q & (C8 - 1);
         const int r = q >> c8_log2;  // tap * COUT + co
         const int tap = r / COUT, co = r - tap * COUT;
-        *reinterpret_cast<uint4 *>(dst + (((tap << c8_log2) + c) * COUT + co) * 16) = __ldg(w + q);
+        const int row = (2 - tap / 9) * COUT + co;
+        copy16_async(dst + ((((tap % 9) << c8_log2) + c) * 3 * COUT + row) * 16, w + q, true);
     }
 }
 
-template <int COUT>
-__global__ void __launch_bounds__(kConvThreads, 1)
+// ITEMS: 16-byte items of a plane per staging thread, (chunks of both sources) x 180 / 128 rounded up.
+template <int COUT, int ITEMS>
+__global__ void __launch_bounds__(kHaloThreads, COUT == 64 || ITEMS > 9 ? 2 : 3)
     k_conv3d_halo(const __nv_bfloat16 *__restrict__ x0p, const __nv_bfloat16 *__restrict__ w0p,
                   const __nv_bfloat16 *__restrict__ x1p, const __nv_bfloat16 *__restrict__ w1p, const HaloGeom g,
                   const float *__restrict__ bias, __nv_bfloat16 *__restrict__ y) {
     extern __shared__ unsigned char conv_smem_raw[];
     unsigned char *smem = reinterpret_cast<unsigned char *>(
         (reinterpret_cast<uintptr_t>(conv_smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-    unsigned char *planes1 = smem + g.planes1_off;
-    uint64_t *done = reinterpret_cast<uint64_t *>(smem + g.bar_off);
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(done + 1);
+    uint64_t *full = reinterpret_cast<uint64_t *>(smem + g.bar_off);
+    uint64_t *done = full + kHaloMaxX + 2;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(done + kHaloMaxX + 2);
     __shared__ int fail;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int t = blockIdx.x;
-    const int tz = g.NZ >> 3, ty = g.NY >> 4, tx = g.NX / g.xr;
+    const int tz = g.NZ >> 3, ty = g.NY >> 4, tx = (g.NX + g.xr - 1) / g.xr;
     const int z0 = (t % tz) * 8;
     t /= tz;
     const int y0 = (t % ty) * 16;
     t /= ty;
     const int x0 = (t % tx) * g.xr, b = t / tx;
+    const int xr = min(g.xr, g.NX - x0), np = xr + 2;
     const int nsrc = g.cin1 > 0 ? 2 : 1;
     const int lg0 = g.cin0 == 16 ? 1 : (g.cin0 == 32 ? 2 : 3), lg1 = g.cin1 == 16 ? 1 : (g.cin1 == 32 ? 2 : 3);
 
     if (threadIdx.x == 0) {
         fail = 0;
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(done)));
+        for (int p = 0; p < np; p++) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&full[p])), "r"(kConvThreads));
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&done[p])));
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
@@ -381,84 +370,150 @@ __global__ void __launch_bounds__(kConvThreads, 1)
                      "r"(g.tmem_cols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
-
-    // every input plane and every weight once, by all threads; then visible
-    // to the tensor core
-    halo_stage(reinterpret_cast<const uint4 *>(x0p), smem, lg0, g.xr + 2, g.plane0, b, x0, y0, z0, g);
-    halo_stage_weights<COUT>(reinterpret_cast<const uint4 *>(w0p), smem + g.w0_off, lg0);
-    if (nsrc > 1) {
-        halo_stage(reinterpret_cast<const uint4 *>(x1p), planes1, lg1, g.xr + 2, g.plane1, b, x0, y0, z0, g);
-        halo_stage_weights<COUT>(reinterpret_cast<const uint4 *>(w1p), smem + g.w1_off, lg1);
-    }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tmem_slot;
 
-    if (threadIdx.x == 32) {
-        // MMA issuer: 27 taps x sources x planes x (Cin / 16), then one commit
-        const uint32_t idesc = mma_idesc(COUT);
-        for (int src = 0; src < nsrc; src++) {
-            const int lg = src ? lg1 : lg0, ksteps = 1 << (lg - 1);
-            const int pl = src ? g.plane1 : g.plane0;
-            const uint32_t pbase = smem_u32(src ? planes1 : smem);
-            const uint32_t wbase = smem_u32(smem + (src ? g.w1_off : g.w0_off));
-            const uint64_t pstep = (uint64_t)(pl >> 4);
-            for (int tap = 0; tap < 27; tap++) {
-                const int dx = tap / 9 - 1, dy = (tap / 3) % 3 - 1, dz = tap % 3 - 1;
-                const uint32_t off = (uint32_t)(((dy + 1) * kHaloZ + dz + 1) * 16);
-                // descriptors of (xi = 0, kk = 0); the start address field
-                // (16-byte units) advances by one plane per xi and by two
-                // chunks per kk
-                const uint64_t a0 = ns_desc(pbase + (uint32_t)((dx + 1) * pl) + off, kHaloChunk, kHaloZ * 16);
-                const uint64_t b0 = ns_desc(wbase + (uint32_t)(tap << lg) * (COUT * 16), COUT * 16, 128);
-                const uint32_t acc = (tap > 0 || src > 0) ? 1u : 0u;
-                uint64_t ax = a0;
-                uint32_t d = tmem;
-                for (int xi = 0; xi < g.xr; xi++, ax += pstep, d += COUT) {
-#pragma unroll 1
-                    for (int kk = 0; kk < ksteps; kk++) {
-                        const uint64_t ad = ax + (uint64_t)(kk * (2 * kHaloChunk >> 4));
-                        const uint64_t bd = b0 + (uint64_t)(kk * (2 * COUT * 16 >> 4));
-                        asm volatile(
-                            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
-                            "l"(ad), "l"(bd), "r"(idesc), "r"(acc | (uint32_t)kk));
-                    }
-                }
-            }
+    if (warp >= 4 && warp < 8) {
+        const int tid = threadIdx.x - kConvThreads;
+        // this thread's items of a plane, the same for every plane: where they
+        // come from (in 16-byte units of their source's plane; -1 outside the
+        // volume) and where they go
+        int from[ITEMS], to[ITEMS];
+        const int n0 = kHaloRows << lg0, n1 = nsrc > 1 ? kHaloRows << lg1 : 0;
+#pragma unroll
+        for (int u = 0; u < ITEMS; u++) {
+            int q = u * kConvThreads + tid;
+            from[u] = -1;
+            to[u] = -1;
+            if (q >= n0 + n1) continue;
+            const bool second = q >= n0;
+            if (second) q -= n0;
+            const int lg = second ? lg1 : lg0, c = q & ((1 << lg) - 1);
+            const int r = q >> lg, zh = r % kHaloZ, yh = r / kHaloZ;
+            const int yy = y0 - 1 + yh, zz = z0 - 1 + zh;
+            to[u] = (second ? g.src1_off + c * g.chunk1 : c * g.chunk0) + r * 16;
+            if ((unsigned)yy < (unsigned)g.NY && (unsigned)zz < (unsigned)g.NZ)
+                from[u] = ((yy * g.NZ + zz) << lg) + c;
         }
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-            smem_u32(done))
-                     : "memory");
-    }
-    __syncwarp();
-    // epilogue: row m of each accumulator is TMEM lane m, owned by warp m / 32
-    const bool got = __all_sync(0xffffffffu, mbar_wait(smem_u32(done), 0) ? 1 : 0) != 0;
-    if (!got) fail = 1;
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const int m = warp * 32 + lane;
-    const int yy = y0 + (m >> 3), zz = z0 + (m & 7);
-    if (got) {
-        for (int xi = 0; xi < g.xr; xi++) {
+        const uint4 *g0 = reinterpret_cast<const uint4 *>(x0p), *g1 = reinterpret_cast<const uint4 *>(x1p);
+        const int64_t plane = (int64_t)g.NY * g.NZ;
+        auto stage = [&](int p) {
+            const int xx = x0 - 1 + p;
+            const bool in = (unsigned)xx < (unsigned)g.NX;
+            const int64_t at = in ? ((int64_t)b * g.NX + xx) * plane : 0;
+            const uint4 *s0 = g0 + (at << lg0), *s1 = g1 + (at << lg1);
+            const uint32_t dst = smem_u32(smem) + (uint32_t)((p % g.ring) * g.slot);
+#pragma unroll
+            for (int u = 0; u < ITEMS; u++) {
+                const bool first = u * kConvThreads + tid < n0, any = in && from[u] >= 0;
+                if (to[u] >= 0) copy16_async(dst + (uint32_t)to[u], (first ? s0 : s1) + (any ? from[u] : 0), any);
+            }
+        };
+        const int ahead = g.ring - 1;
+        for (int p = 0; p < ahead; p++) {
+            if (p == 0) {
+                halo_stage_weights<COUT>(reinterpret_cast<const uint4 *>(w0p), smem_u32(smem + g.w0_off), lg0, tid);
+                if (nsrc > 1)
+                    halo_stage_weights<COUT>(reinterpret_cast<const uint4 *>(w1p), smem_u32(smem + g.w1_off), lg1, tid);
+            }
+            if (p < np) stage(p);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        }
+        for (int p = 0; p < np; p++) {
+            // plane p has landed when at most the ahead - 1 groups after its own are in flight
+            if (ahead == 3) asm volatile("cp.async.wait_group 2;" ::: "memory");
+            else asm volatile("cp.async.wait_group 1;" ::: "memory");
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&full[p])) : "memory");
+            if (p + ahead < np) {
+                if (p >= 1 && !mbar_wait(smem_u32(&done[p - 1]), 0)) {
+                    fail = 1;
+                    break;
+                }
+                stage(p + ahead);
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    } else if (warp < 4) {
+        // output plane o, complete with input plane o + 2: row m of its accumulator is TMEM lane m
+        const int m = threadIdx.x;
+        float bs[COUT <= 32 ? COUT : 1];
+        if (COUT <= 32)
+#pragma unroll
+            for (int c = 0; c < (COUT <= 32 ? COUT : 1); c++) bs[c] = bias ? __ldg(bias + c) : 0.0f;
+        __nv_bfloat16 *yo = y + ((((int64_t)b * g.NX + x0) * g.NY + y0 + (m >> 3)) * g.NZ + z0 + (m & 7)) * COUT;
+        for (int o = 0; o < xr; o++, yo += (int64_t)g.NY * g.NZ * COUT) {
+            // warp-uniform outcome: tcgen05.ld is a .sync.aligned warp instruction
+            if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&done[o + 2]), 0) ? 1 : 0)) {
+                fail = 1;
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             float acc[COUT];
 #pragma unroll
             for (int c = 0; c < COUT; c += 16)
-                tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(xi * COUT + c), acc + c);
+                tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(o * COUT + c), acc + c);
             __align__(16) __nv_bfloat16 out[COUT];
 #pragma unroll
             for (int c = 0; c < COUT; c++) {
-                float v = acc[c] + (bias ? __ldg(bias + c) : 0.0f);
+                float v = acc[c] + (COUT <= 32 ? bs[COUT <= 32 ? c : 0] : (bias ? __ldg(bias + c) : 0.0f));
                 if (g.relu) v = fmaxf(v, 0.0f);
                 out[c] = __float2bfloat16_rn(v);
             }
-            const int64_t vox = (((int64_t)b * g.NX + x0 + xi) * g.NY + yy) * g.NZ + zz;
-            uint4 *dst = reinterpret_cast<uint4 *>(y + vox * COUT);
+            uint4 *dst = reinterpret_cast<uint4 *>(yo);
 #pragma unroll
             for (int q = 0; q < COUT / 8; q++) dst[q] = reinterpret_cast<const uint4 *>(out)[q];
         }
+    } else if (lane == 0) {
+        // MMA issuer: per plane 9 x sources x (Cin / 16) steps of N = 3 Cout, then one commit
+        for (int p = 0; p < np; p++) {
+            if (!mbar_wait(smem_u32(&full[p]), 0)) {
+                fail = 1;
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t slot = smem_u32(smem) + (uint32_t)((p % g.ring) * g.slot);
+            const int lo = max(0, p - 2), hi = min(p, xr - 1);  // the output planes it contributes to
+            const uint32_t d = tmem + (uint32_t)(lo * COUT), idesc = mma_idesc((hi - lo + 1) * COUT);
+            const uint32_t wrow = (uint32_t)((lo - (p - 2)) * COUT * 16);
+            auto mma = [&](uint32_t dd, uint64_t aa, uint64_t bb, uint32_t id, uint32_t acc) {
+                asm volatile(
+                    "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(dd),
+                    "l"(aa), "l"(bb), "r"(id), "r"(acc));
+            };
+            for (int src = 0; src < nsrc; src++) {
+                const int lg = src ? lg1 : lg0, ksteps = 1 << (lg - 1);
+                const uint32_t chunk = (uint32_t)(src ? g.chunk1 : g.chunk0);
+                const uint32_t wbase = smem_u32(smem + (src ? g.w1_off : g.w0_off));
+                uint64_t a0 = ns_desc(slot + (src ? (uint32_t)g.src1_off : 0u), chunk, kHaloZ * 16);
+                uint64_t b0 = ns_desc(wbase + wrow, 3 * COUT * 16, 128);
+                const uint64_t bstep = (uint64_t)((3 * COUT) << lg);  // in 16-byte units, as the address field
+                for (int kk = 0; kk < ksteps; kk++) {
+#pragma unroll
+                    for (int sft = 0; sft < 9; sft++) {
+                        const uint64_t ad = a0 + (uint64_t)((sft / 3) * kHaloZ + sft % 3), bd = b0 + sft * bstep;
+                        if (sft == 0 && src == 0 && kk == 0 && p < xr) {
+                            // the planes begun before, then the new one from zero
+                            if (hi > lo) mma(d, ad, bd, mma_idesc((hi - lo) * COUT), 1u);
+                            mma(tmem + (uint32_t)(p * COUT), ad, bd + (uint64_t)((hi - lo) * COUT), mma_idesc(COUT), 0u);
+                        } else {
+                            mma(d, ad, bd, idesc, 1u);
+                        }
+                    }
+                    a0 += (uint64_t)((2 * chunk) >> 4);
+                    b0 += (uint64_t)(2 * 3 * COUT);
+                }
+            }
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                smem_u32(&done[p]))
+                         : "memory");
+        }
     }
+    __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (fail && threadIdx.x == 0) atomicExch(&g_conv_error, 1);
@@ -726,20 +781,23 @@ constexpr int kHaloSmemMax = 227 * 1024 - 128;
 
 static inline int align_up(int v, int a) { return (v + a - 1) / a * a; }
 
-// Shared-memory layout of k_conv3d_halo for xr planes; returns the dynamic
-// shared memory size (including the 1 KB alignment slack).
+// Shared-memory layout of k_conv3d_halo; returns the dynamic shared memory size
+// (including the 1 KB alignment slack).
 static size_t halo_layout(HaloGeom &h, int cout) {
-    h.plane0 = (h.cin0 >> 3) * kHaloChunk;
-    h.plane1 = (h.cin1 >> 3) * kHaloChunk;
-    const int np = h.xr + 2;
-    h.planes1_off = np * h.plane0;
-    h.w0_off = h.planes1_off + np * h.plane1;
+    // chunk regions start at different 16-byte columns of the banks, so that the
+    // lanes that stage one voxel's chunks do not collide
+    auto chunk = [](int cin) { return kHaloRows * 16 + (cin == 32 ? 32 : (cin == 64 ? 16 : 0)); };
+    h.chunk0 = chunk(h.cin0);
+    h.chunk1 = chunk(h.cin1);
+    h.src1_off = (h.cin0 >> 3) * h.chunk0;
+    h.slot = align_up(h.src1_off + (h.cin1 >> 3) * h.chunk1, 128);
+    h.w0_off = h.ring * h.slot;
     h.w1_off = h.w0_off + 27 * cout * h.cin0 * 2;
     h.bar_off = align_up(h.w1_off + 27 * cout * h.cin1 * 2, 16);
     uint32_t cols = 32;
     while (cols < (uint32_t)(h.xr * cout)) cols <<= 1;
     h.tmem_cols = cols;
-    return (size_t)h.bar_off + 16 /* mbarrier, TMEM slot */ + 1024;
+    return (size_t)h.bar_off + kHaloBars + 16 /* TMEM slot */ + 1024;
 }
 
 static bool halo_enabled() {
@@ -747,60 +805,82 @@ static bool halo_enabled() {
     return !(e && e[0] == '0');
 }
 
-// FLUB_CONV_XR=n forces n planes per CTA (1, 2, 4 or 8) where it fits.
+// FLUB_CONV_XR=n forces n planes per CTA (1 to 16, at most NX) where it fits.
 static int forced_xr() {
     const char *e = getenv("FLUB_CONV_XR");
     return e ? atoi(e) : 0;
 }
 
-// Chooses the planes per CTA for k_conv3d_halo: the largest xr in {8, 4, 2, 1}
-// that divides NX, keeps the accumulators within 256 TMEM columns and the
-// planes and weights within shared memory, and still gives at least three
-// CTAs per SM (xr = 1 when none does).  Returns 0 when the layer goes to
-// k_conv3d_tc instead: its weights do not fit beside three planes, or
-// k_conv3d_tc takes its shape and it has two sources or fewer tiles than SMs.
-// Both kernels run the same count of M = 128, N = Cout, K = 16 MMAs, which at
-// N = 16 to 64 are bound by the SM reading their A operand (about 44 cycles
-// for one 128 x 16 BF16 tile); the halo kernel saves the tap-shifted tile
-// loads, and wins where its planes and weights leave room for several CTAs
-// per SM.  For the two-source decoder layers they do not, and on grids of
-// fewer tiles than SMs (16^3) its staging is not hidden: the tap-tile kernel
-// measured faster in both cases.  FLUB_CONV_XR forces the halo kernel
-// wherever it fits.
+// Chooses the planes per CTA and the ring of k_conv3d_halo; returns 0 when the
+// layer goes to k_conv3d_tc instead: its weights do not fit beside the planes,
+// or k_conv3d_tc takes its shape and there are fewer tiles than SMs (16^3),
+// where the staging is not hidden and the tap-tile kernel measured faster.
+// The CTAs on an SM share its tensor core, and each has its xr + 2 planes and
+// about one more for its start; one that has no other beside it waits for its
+// loads in half of that again.  So the shortest is the least CTAs per SM x
+// (xr + 3), half as much again without overlap.
 static size_t halo_plan(HaloGeom &h, int cout) {
     if (h.NZ % 8 || h.NY % 16 || !halo_enabled()) return 0;
     const int64_t tiles = (int64_t)h.B * (h.NY / 16) * (h.NZ / 8);
-    const int fx = forced_xr();
+    const int fx = forced_xr() < h.NX ? forced_xr() : h.NX;
     const int nzb = h.NZ < 128 ? h.NZ : 128;
     const bool tap_ok = 128 % nzb == 0 && h.NZ % nzb == 0 && h.NY % (128 / nzb) == 0;
-    if (!fx && tap_ok && (h.cin1 > 0 || tiles * h.NX < kNumSMs)) return 0;
-    for (int xr = 8; xr >= 1; xr >>= 1) {
-        if (fx && xr != fx) continue;
-        if (h.NX % xr || xr * cout > 256) continue;
-        if (!fx && xr > 1 && tiles * (h.NX / xr) < 3 * kNumSMs) continue;
-        h.xr = xr;
-        const size_t smem = halo_layout(h, cout);
-        if (smem <= (size_t)kHaloSmemMax) return smem;
+    if (!fx && tap_ok && tiles * h.NX < kNumSMs) return 0;
+    if (h.cin0 + h.cin1 > 96) return 0;
+    HaloGeom best = h;
+    size_t best_smem = 0;
+    int64_t best_cost = 0;
+    for (int xr = kHaloMaxX < h.NX ? kHaloMaxX : h.NX; xr >= 1; xr--) {
+        if ((fx && xr != fx) || xr * cout > 256) continue;
+        for (int ring = 4; ring >= 3; ring--) {
+            h.xr = xr;
+            h.ring = ring;
+            const size_t smem = halo_layout(h, cout);
+            if (smem > (size_t)kHaloSmemMax) continue;
+            int occ = (int)((size_t)(228 * 1024) / (smem + 1024));
+            const int regs = cout == 64 || h.cin0 + h.cin1 > 48 ? 2 : 3;  // as the kernel's launch bounds
+            occ = occ < regs ? occ : regs;
+            occ = occ < (int)(512 / h.tmem_cols) ? occ : (int)(512 / h.tmem_cols);
+            const int64_t ctas = tiles * ((h.NX + xr - 1) / xr), per_sm = (ctas + kNumSMs - 1) / kNumSMs;
+            const int64_t cost = per_sm * (xr + 3) * (occ == 1 || per_sm == 1 ? 3 : 2);
+            if (!best_smem || cost < best_cost) {
+                best = h;
+                best_smem = smem;
+                best_cost = cost;
+            }
+        }
     }
-    return 0;
+    h = best;
+    return best_smem;
 }
 
-template <int COUT>
+template <int COUT, int ITEMS>
 static int launch_halo(const void *x0, const void *w0, const void *x1, const void *w1, const HaloGeom &h, size_t smem,
                        const float *bias, __nv_bfloat16 *y, cudaStream_t s) {
     static size_t attr_smem = 0;  // largest dynamic shared memory enabled so far
     if (smem > attr_smem) {
         FLUB_CHECK_CUDA(
-            cudaFuncSetAttribute(k_conv3d_halo<COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            cudaFuncSetAttribute(k_conv3d_halo<COUT, ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         attr_smem = smem;
     }
-    const unsigned ctas = (unsigned)((int64_t)h.B * (h.NX / h.xr) * (h.NY / 16) * (h.NZ / 8));
-    k_conv3d_halo<COUT><<<ctas, kConvThreads, smem, s>>>(
+    const unsigned ctas = (unsigned)((int64_t)h.B * ((h.NX + h.xr - 1) / h.xr) * (h.NY / 16) * (h.NZ / 8));
+    k_conv3d_halo<COUT, ITEMS><<<ctas, kHaloThreads, smem, s>>>(
         static_cast<const __nv_bfloat16 *>(x0), static_cast<const __nv_bfloat16 *>(w0),
         static_cast<const __nv_bfloat16 *>(x1 ? x1 : x0), static_cast<const __nv_bfloat16 *>(w1 ? w1 : w0), h, bias,
         y);
     FLUB_CHECK_LAUNCH();
     return FLUB_OK;
+}
+
+template <int COUT>
+static int launch_halo_items(const void *x0, const void *w0, const void *x1, const void *w1, const HaloGeom &h,
+                             size_t smem, const float *bias, __nv_bfloat16 *y, cudaStream_t s) {
+    const int items = ((h.cin0 + h.cin1) / 8 * kHaloRows + kConvThreads - 1) / kConvThreads;
+    if (items <= 3) return launch_halo<COUT, 3>(x0, w0, x1, w1, h, smem, bias, y, s);
+    if (items <= 6) return launch_halo<COUT, 6>(x0, w0, x1, w1, h, smem, bias, y, s);
+    if (items <= 9) return launch_halo<COUT, 9>(x0, w0, x1, w1, h, smem, bias, y, s);
+    if (items <= 12) return launch_halo<COUT, 12>(x0, w0, x1, w1, h, smem, bias, y, s);
+    return launch_halo<COUT, 17>(x0, w0, x1, w1, h, smem, bias, y, s);
 }
 
 }  // namespace flub
@@ -831,9 +911,9 @@ extern "C" int flub_conv3d_bf16(const void *x0, int cin0, const void *w0, const 
             cudaStream_t s = as_stream(stream);
             __nv_bfloat16 *yo = static_cast<__nv_bfloat16 *>(y);
             switch (cout) {
-            case 16: return launch_halo<16>(x0, w0, x1, w1, h, smem, bias, yo, s);
-            case 32: return launch_halo<32>(x0, w0, x1, w1, h, smem, bias, yo, s);
-            default: return launch_halo<64>(x0, w0, x1, w1, h, smem, bias, yo, s);
+            case 16: return launch_halo_items<16>(x0, w0, x1, w1, h, smem, bias, yo, s);
+            case 32: return launch_halo_items<32>(x0, w0, x1, w1, h, smem, bias, yo, s);
+            default: return launch_halo_items<64>(x0, w0, x1, w1, h, smem, bias, yo, s);
             }
         }
     }
