@@ -297,38 +297,55 @@ __global__ void __launch_bounds__(256) k_unet_output(const float *__restrict__ o
 }
 
 // Bias gradient db[co] += sum_v dy[v][co]: each thread owns one 8-channel
-// chunk (16 bytes) of the voxel rows it visits; per-block sums in shared
-// memory, one global atomic per channel and block.
+// chunk (16 bytes) of the voxel rows it visits, four loads in flight; the lanes
+// of a warp with the same chunk are summed by shuffles, the warps in shared
+// memory, then one global atomic per channel and block.  (Shared-memory atomics
+// by every thread on 16 to 64 addresses took 36 us, whatever the size; 64^3 x 16
+// channels x 4 now 9 us.)
 __global__ void __launch_bounds__(256) k_bias_grad(const uint4 *__restrict__ dy, int nch, int64_t nq,
                                                    float *__restrict__ db) {
-    __shared__ float sb[64];
-    if (threadIdx.x < 64) sb[threadIdx.x] = 0.0f;
-    __syncthreads();
+    __shared__ float sb[8][64];
+    constexpr int U = 4;
     float acc[8];
 #pragma unroll
     for (int e = 0; e < 8; e++) acc[e] = 0.0f;
-    // blockDim and the grid stride are multiples of nch: q % nch is fixed per thread
-    GRID_LOOP(q, nq) {
-        const uint4 u = dy[q];
-        const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&u);
+    // nch is 2, 4 or 8, so blockDim and the grid stride are multiples of it: q % nch is fixed per thread
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < nq; q += U * stride) {
+        uint4 u[U];
 #pragma unroll
-        for (int e = 0; e < 4; e++) {
-            const float2 f = __bfloat1622float2(h[e]);
-            acc[2 * e] += f.x;
-            acc[2 * e + 1] += f.y;
+        for (int k = 0; k < U; k++) u[k] = q + k * stride < nq ? __ldg(dy + q + k * stride) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (int k = 0; k < U; k++) {
+            const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&u[k]);
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                const float2 f = __bfloat1622float2(h[e]);
+                acc[2 * e] += f.x;
+                acc[2 * e + 1] += f.y;
+            }
         }
     }
-    const int j = threadIdx.x % nch;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int o = 16; o >= nch; o >>= 1)
 #pragma unroll
-    for (int e = 0; e < 8; e++) atomicAdd(&sb[j * 8 + e], acc[e]);
+        for (int e = 0; e < 8; e++) acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], o);
+    if (lane < nch)
+#pragma unroll
+        for (int e = 0; e < 8; e++) sb[warp][lane * 8 + e] = acc[e];
     __syncthreads();
-    if (threadIdx.x < nch * 8) atomicAdd(&db[threadIdx.x], sb[threadIdx.x]);
+    if (threadIdx.x < nch * 8) {
+        float v = 0.0f;
+#pragma unroll
+        for (int w = 0; w < 8; w++) v += sb[w][threadIdx.x];
+        atomicAdd(&db[threadIdx.x], v);
+    }
 }
 
 int launch_bias_grad(const void *dy, int cout, int64_t nvox, float *db, cudaStream_t s) {
     const int nch = cout / 8;
     const int64_t nq = nvox * nch;
-    k_bias_grad<<<blocks_for(nq, 256, 152 * 8), 256, 0, s>>>(static_cast<const uint4 *>(dy), nch, nq, db);
+    k_bias_grad<<<blocks_for(nq, 1024, 152 * 2), 256, 0, s>>>(static_cast<const uint4 *>(dy), nch, nq, db);
     FLUB_CHECK_LAUNCH();
     return FLUB_OK;
 }
