@@ -20,7 +20,8 @@
 //
 // k_conv3d_halo (below) computes the same convolution from input planes
 // staged once per CTA; halo_plan chooses between the two kernels per layer.
-// The weight gradient (k_conv3d_wgrad_tc) is a third tcgen05 kernel.
+// The weight gradient has two more, k_conv3d_wgrad_tc from tap tiles and
+// k_conv3d_wgrad_halo from staged planes.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cudaTypedefs.h>
@@ -283,6 +284,8 @@ constexpr int kHaloZ = 10, kHaloY = 18;
 constexpr int kHaloRows = kHaloZ * kHaloY;  // 16-byte rows per chunk (180)
 constexpr int kHaloThreads = 2 * kConvThreads + 32;
 constexpr int kHaloMaxX = 16;               // output planes per CTA
+// opt-in shared memory per block less an allowance for the kernel's static shared variables
+constexpr int kHaloSmemMax = 227 * 1024 - 128;
 constexpr int kHaloBars = 8 * 2 * (kHaloMaxX + 2);
 
 struct HaloGeom {
@@ -313,6 +316,31 @@ __device__ __forceinline__ void copy16_async(uint32_t dst, const void *src, bool
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(__cvta_generic_to_global(src)),
                  "r"(in ? 16 : 0)
                  : "memory");
+}
+
+// One lane of a converged warp.  The MMA warps run their loops with all lanes and
+// predicate only the instruction: in a branch of one lane the descriptors, which
+// the instruction takes from uniform registers, were moved there one by one.
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t lead;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(lead));
+    return lead;
+}
+
+__device__ __forceinline__ void mma_if(uint32_t lead, uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
+        "l"(a), "l"(b), "r"(idesc), "r"(acc), "r"(lead));
+}
+
+__device__ __forceinline__ void commit_if(uint32_t lead, uint32_t bar) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar),
+        "r"(lead)
+        : "memory");
 }
 
 // Stages weights [27][COUT][Cin] (Cin = 8 << c8_log2) as
@@ -467,7 +495,8 @@ __global__ void __launch_bounds__(kHaloThreads, COUT == 64 || ITEMS > 9 ? 2 : 3)
 #pragma unroll
             for (int q = 0; q < COUT / 8; q++) dst[q] = reinterpret_cast<const uint4 *>(out)[q];
         }
-    } else if (lane == 0) {
+    } else {
+        const uint32_t lead = elect_one();
         // MMA issuer: per plane 9 x sources x (Cin / 16) steps of N = 3 Cout, then one commit
         for (int p = 0; p < np; p++) {
             if (!mbar_wait(smem_u32(&full[p]), 0)) {
@@ -480,10 +509,7 @@ __global__ void __launch_bounds__(kHaloThreads, COUT == 64 || ITEMS > 9 ? 2 : 3)
             const uint32_t d = tmem + (uint32_t)(lo * COUT), idesc = mma_idesc((hi - lo + 1) * COUT);
             const uint32_t wrow = (uint32_t)((lo - (p - 2)) * COUT * 16);
             auto mma = [&](uint32_t dd, uint64_t aa, uint64_t bb, uint32_t id, uint32_t acc) {
-                asm volatile(
-                    "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(dd),
-                    "l"(aa), "l"(bb), "r"(id), "r"(acc));
+                mma_if(lead, dd, aa, bb, id, acc);
             };
             for (int src = 0; src < nsrc; src++) {
                 const int lg = src ? lg1 : lg0, ksteps = 1 << (lg - 1);
@@ -508,9 +534,7 @@ __global__ void __launch_bounds__(kHaloThreads, COUT == 64 || ITEMS > 9 ? 2 : 3)
                     b0 += (uint64_t)(2 * 3 * COUT);
                 }
             }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                smem_u32(&done[p]))
-                         : "memory");
+            commit_if(lead, smem_u32(&done[p]));
         }
     }
     __syncwarp();
@@ -698,6 +722,256 @@ __global__ void __launch_bounds__(kConvThreads, 1)
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tmem_cols));
 }
 
+// ---------------------------------------------------------------- halo-plane weight gradient
+//
+// The same sums for NZ % 8 == 0, NY % 16 == 0, Cin <= 32 and Cout <= 32 from
+// haloed input planes staged once, as k_conv3d_halo stages them, instead of 27
+// tap-shifted tiles (216 KB of shared memory filled per 128 voxels and 32
+// channels: the copies bound k_conv3d_wgrad_tc).
+//
+// A segment is a 16 (y) x 8 (z) voxel tile at NQ consecutive x planes x0 ..: the
+// NQ tiles of dY and the NQ + 2 haloed planes of X, x = x0 - 1 .., side by side in
+// shared memory, so that one MMA of M = 128 rows (plane, ci) and N = NQ Cout
+// columns (q, co) multiplies 128 / Cin planes with all NQ tiles: of these
+// products those with dx = plane - 1 - q in -1 .. 1 are kept, 3 of 4 with Cin = 32
+// and NQ = 2, and the others cost nothing that the A operand's reads do not.  Both
+// operands are MN-major without swizzle: a core matrix is 8 channels x 8 voxels of
+// a z row (128 contiguous bytes), the next along M or N one chunk region on (SBO),
+// the next along K one row of voxels on (LBO; padded for X).  The nine shifts (dy,
+// dz) are start offsets into the planes, each with its own accumulator in TMEM for
+// the CTA's whole life (S of them; blockIdx.y takes the next S).  At the end the
+// CTA sums its NQ parts of every tap in shared memory and adds them to dW with one
+// atomic per entry.
+// Warps 0-7 stage segments through a ring with asynchronous copies, one thread of
+// warp 8 issues the MMAs.  4 x 64^3: Cin 32, Cout 16 232 -> 76 us, Cin 16
+// 156 -> 61 us; an MMA here takes about 45 cycles, 32 of them the A operand.
+constexpr int kWhStagers = 256;
+constexpr int kWhThreads = kWhStagers + 32;
+constexpr int kWhMaxRing = 4;
+
+template <int CIN, int COUT>
+struct WhShape {
+    static constexpr int NQ = CIN == 16 ? 3 : 2;               // dY planes of a segment
+    static constexpr int S = COUT == 16 ? 9 : 5;               // shifts per CTA: S * NQ * COUT <= 512 columns
+    static constexpr int CHUNK = kHaloRows * 16 + (CIN == 32 ? 32 : 0);
+    static constexpr int PLANE = CIN / 8 * CHUNK;
+    static constexpr int DCHUNK = 128 * 16 + (COUT == 32 ? 32 : 64);
+    static constexpr int DPLANE = COUT / 8 * DCHUNK;
+    static constexpr int XBYTES = (NQ + 2) * PLANE;
+    static constexpr int SEG = (XBYTES + NQ * DPLANE + 127) / 128 * 128;
+    // rows beyond the segment's planes are read and never used: room for them after the last buffer
+    static constexpr int OVER = 128 / CIN * PLANE > SEG ? 128 / CIN * PLANE - SEG : 0;
+    static constexpr int RING = (kHaloSmemMax - 1024 - 256 - OVER) / SEG < kWhMaxRing
+                                    ? (kHaloSmemMax - 1024 - 256 - OVER) / SEG : kWhMaxRing;
+    static constexpr int BARS = (RING * SEG + OVER + 15) / 16 * 16;
+    static constexpr int SMEM = BARS + 128 + 1024;
+    static_assert(27 * CIN * COUT * 4 <= RING * SEG, "the sums reuse the ring");
+    static_assert(S * NQ * COUT <= 512 && RING >= 2, "");
+};
+
+template <int CIN, int COUT>
+__global__ void __launch_bounds__(kWhThreads, 1)
+    k_conv3d_wgrad_halo(const __nv_bfloat16 *__restrict__ xp, const __nv_bfloat16 *__restrict__ dyp, int B, int NX,
+                        int NY, int NZ, float *__restrict__ dw) {
+    using W = WhShape<CIN, COUT>;
+    constexpr int NQ = W::NQ, C8 = CIN / 8, D8 = COUT / 8;
+    extern __shared__ unsigned char conv_smem_raw[];
+    unsigned char *smem = reinterpret_cast<unsigned char *>(
+        (reinterpret_cast<uintptr_t>(conv_smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+    uint64_t *full = reinterpret_cast<uint64_t *>(smem + W::BARS);
+    uint64_t *empty = full + kWhMaxRing;
+    uint64_t *done = empty + kWhMaxRing;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(done + 1);
+    __shared__ int fail;
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int tz = NZ >> 3, ty = NY >> 4, tx = (NX + NQ - 1) / NQ;
+    const int nseg = B * tx * ty * tz;
+    const int mine = blockIdx.x < (unsigned)nseg ? (nseg - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+    const int s0 = blockIdx.y * W::S, ns = min(9 - s0, W::S);
+    // segment i of this CTA
+    auto where = [&](int i, int &b, int &x0, int &y0, int &z0) {
+        int t = (int)blockIdx.x + i * (int)gridDim.x;
+        z0 = (t % tz) * 8;
+        t /= tz;
+        y0 = (t % ty) * 16;
+        t /= ty;
+        x0 = (t % tx) * NQ;
+        b = t / tx;
+    };
+    if (threadIdx.x == 0) {
+        fail = 0;
+        for (int r = 0; r < W::RING; r++) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&full[r])), "r"(kWhStagers));
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&empty[r])));
+        }
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(done)));
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tmem_slot)));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = *tmem_slot;
+
+    if (warp < 8) {
+        constexpr int IX = (kHaloRows * C8 + kWhStagers - 1) / kWhStagers;  // items of an X plane per thread
+        constexpr int ID = 128 * D8 / kWhStagers > 0 ? 128 * D8 / kWhStagers : 1;
+        const uint4 *gx = reinterpret_cast<const uint4 *>(xp), *gd = reinterpret_cast<const uint4 *>(dyp);
+        const int64_t plane = (int64_t)NY * NZ;
+        const uint32_t base = smem_u32(smem);
+        auto stage = [&](int i) {
+            int b, x0, y0, z0;
+            where(i, b, x0, y0, z0);
+            const int nq = min(NQ, NX - x0);
+            const uint32_t buf = base + (uint32_t)((i % W::RING) * W::SEG);
+#pragma unroll
+            for (int u = 0; u < IX; u++) {
+                const int q = u * kWhStagers + threadIdx.x;
+                if (q >= kHaloRows * C8) break;
+                const int c = q % C8, r = q / C8, zh = r % kHaloZ, yh = r / kHaloZ;
+                const int yy = y0 - 1 + yh, zz = z0 - 1 + zh;
+                const bool in = (unsigned)yy < (unsigned)NY && (unsigned)zz < (unsigned)NZ;
+                const int from = in ? (yy * NZ + zz) * C8 + c : 0;
+                const uint32_t to = buf + (uint32_t)(c * W::CHUNK + r * 16);
+#pragma unroll
+                for (int pl = 0; pl < NQ + 2; pl++) {
+                    const int xx = x0 - 1 + pl;
+                    if (pl >= nq + 2) break;
+                    const bool ok = in && (unsigned)xx < (unsigned)NX;
+                    copy16_async(to + (uint32_t)(pl * W::PLANE), gx + (ok ? ((int64_t)b * NX + xx) * plane * C8 + from : 0),
+                                 ok);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < ID; u++) {
+                const int q = u * kWhStagers + threadIdx.x;
+                if (q >= 128 * D8) break;
+                const int c = q % D8, v = q / D8;
+                const int from = ((y0 + (v >> 3)) * NZ + z0 + (v & 7)) * D8 + c;
+                const uint32_t to = buf + (uint32_t)(W::XBYTES + c * W::DCHUNK + v * 16);
+#pragma unroll
+                for (int t = 0; t < NQ; t++) {
+                    if (t >= nq) break;
+                    copy16_async(to + (uint32_t)(t * W::DPLANE),
+                                 gd + ((int64_t)b * NX + x0 + t) * plane * D8 + from, true);
+                }
+            }
+        };
+        constexpr int ahead = W::RING - 1;
+        for (int i = 0; i < ahead; i++) {
+            if (i < mine) stage(i);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        }
+        for (int i = 0; i < mine; i++) {
+            // segment i has landed when at most the ahead - 1 groups after its own are in flight
+            asm volatile("cp.async.wait_group %0;" ::"n"(ahead - 1) : "memory");
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&full[i % W::RING])) : "memory");
+            const int n = i + ahead;
+            if (n < mine) {
+                // its buffer was segment n - RING's
+                if (n >= W::RING &&
+                    !mbar_wait(smem_u32(&empty[n % W::RING]), (uint32_t)((n / W::RING - 1) & 1))) {
+                    fail = 1;
+                    break;
+                }
+                stage(n);
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    } else {
+        const uint32_t lead = elect_one();
+        const uint32_t mn = (1u << 15) | (1u << 16);  // A and B MN-major
+        int init = 0;                                  // dY planes whose accumulators hold something
+        for (int i = 0; i < mine; i++) {
+            if (!mbar_wait(smem_u32(&full[i % W::RING]), (uint32_t)((i / W::RING) & 1))) {
+                fail = 1;
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            int b, x0, y0, z0;
+            where(i, b, x0, y0, z0);
+            const int nq = min(NQ, NX - x0);
+            const uint32_t buf = smem_u32(smem) + (uint32_t)((i % W::RING) * W::SEG);
+            const uint64_t a0 = ns_desc(buf, kHaloZ * 16, W::CHUNK), b0 = ns_desc(buf + W::XBYTES, 128, W::DCHUNK);
+            auto mma = [&](uint32_t d, uint64_t aa, uint64_t bb, int n, uint32_t acc) {
+                mma_if(lead, d, aa, bb, mma_idesc(n) | mn, acc);
+            };
+            // shifts inside: successive MMAs add to different accumulators
+            for (int kk = 0; kk < 8; kk++) {  // two rows of 8 voxels per MMA
+                const uint64_t ak = a0 + (uint64_t)(kk * 2 * kHaloZ), bd = b0 + (uint64_t)(kk * 16);
+#pragma unroll
+                for (int sl = 0; sl < W::S; sl++) {
+                    if (sl >= ns) break;
+                    const int sft = s0 + sl;
+                    const uint32_t d = tmem + (uint32_t)(sl * NQ * COUT);
+                    const uint64_t ad = ak + (uint64_t)((sft / 3) * kHaloZ + sft % 3);
+                    if (kk == 0 && nq > init) {
+                        if (init > 0) mma(d, ad, bd, init * COUT, 1u);
+                        mma(d + (uint32_t)(init * COUT), ad, bd + (uint64_t)(init * (W::DPLANE >> 4)), (nq - init) * COUT,
+                            0u);
+                    } else {
+                        mma(d, ad, bd, nq * COUT, 1u);
+                    }
+                }
+            }
+            init = max(init, nq);
+            commit_if(lead, smem_u32(&empty[i % W::RING]));
+        }
+        commit_if(lead, smem_u32(done));
+    }
+    __syncwarp();
+    const bool got = __all_sync(0xffffffffu, mbar_wait_long(smem_u32(done), 0) ? 1 : 0) != 0;
+    if (!got) fail = 1;
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    __syncthreads();  // every thread sees a failure; nothing reads the ring any more
+    if (!fail && mine > 0) {
+        // the dY planes that this CTA had at all
+        int init = 0;
+        for (int i = 0; i < mine && init < NQ; i++) {
+            int b, x0, y0, z0;
+            where(i, b, x0, y0, z0);
+            init = max(init, min(NQ, NX - x0));
+        }
+        constexpr int entries = 27 * COUT * CIN;
+        float *sum = reinterpret_cast<float *>(smem);
+        for (int q = threadIdx.x; q < entries; q += kWhThreads) sum[q] = 0.0f;
+        __syncthreads();
+        for (int t = 0; t < init; t++) {
+            if (warp < 4) {
+                const int m = threadIdx.x, ci = m % CIN, dx = m / CIN - 1 - t;
+                const bool use = dx >= -1 && dx <= 1;
+                if (__any_sync(0xffffffffu, use))
+                    for (int sl = 0; sl < ns; sl++)
+#pragma unroll
+                        for (int c = 0; c < COUT; c += 16) {
+                            float v[16];
+                            tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)((sl * NQ + t) * COUT + c), v);
+                            if (use) {
+                                float *at = sum + (((dx + 1) * 9 + s0 + sl) * COUT + c) * CIN + ci;
+#pragma unroll
+                                for (int e = 0; e < 16; e++) at[e * CIN] += v[e];
+                            }
+                        }
+            }
+            __syncthreads();  // the next plane's parts go to the same taps from other threads
+        }
+        for (int q = threadIdx.x; q < entries; q += kWhThreads) {
+            const int sft = (q / (COUT * CIN)) % 9;
+            if (sft >= s0 && sft < s0 + ns) atomicAdd(dw + q, sum[q]);
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (fail && threadIdx.x == 0) atomicExch(&g_conv_error, 1);
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem));
+}
+
 // ---------------------------------------------------------------- host side
 
 static PFN_cuTensorMapEncodeTiled_v12000 g_encode = nullptr;
@@ -775,9 +1049,6 @@ static int launch_conv(const CUtensorMap &mx0, const CUtensorMap &mw0, const CUt
 }
 
 static bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
-
-// opt-in shared memory per block less an allowance for the kernel's static shared variables
-constexpr int kHaloSmemMax = 227 * 1024 - 128;
 
 static inline int align_up(int v, int a) { return (v + a - 1) / a * a; }
 
@@ -975,6 +1246,25 @@ static int launch_wgrad(const CUtensorMap &mx, const CUtensorMap &mdy, const Con
     FLUB_CHECK_LAUNCH();
     return FLUB_OK;
 }
+
+// k_conv3d_wgrad_halo where it takes the shape and its channels.
+template <int CIN, int COUT>
+static int launch_wgrad_halo(const void *x, const void *dy, int B, int NX, int NY, int NZ, float *dw, cudaStream_t s) {
+    using W = WhShape<CIN, COUT>;
+    static bool attr_set = false;
+    if (!attr_set) {
+        FLUB_CHECK_CUDA(
+            cudaFuncSetAttribute(k_conv3d_wgrad_halo<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, W::SMEM));
+        attr_set = true;
+    }
+    const int64_t nseg = (int64_t)B * ((NX + W::NQ - 1) / W::NQ) * (NY / 16) * (NZ / 8);
+    const int slices = (9 + W::S - 1) / W::S, sms = kNumSMs / slices;
+    const unsigned gx = (unsigned)(nseg < sms ? nseg : sms);
+    k_conv3d_wgrad_halo<CIN, COUT><<<dim3(gx, slices), kWhThreads, W::SMEM, s>>>(
+        static_cast<const __nv_bfloat16 *>(x), static_cast<const __nv_bfloat16 *>(dy), B, NX, NY, NZ, dw);
+    FLUB_CHECK_LAUNCH();
+    return FLUB_OK;
+}
 }  // namespace flub
 
 extern "C" int flub_conv3d_wgrad(const void *x, int cin, const void *dy, int cout, float *dw, float *db, int B, int NX,
@@ -996,11 +1286,25 @@ extern "C" int flub_conv3d_wgrad(const void *x, int cin, const void *dy, int cou
     g.cin0 = cin;
     g.cin1 = 0;
     g.relu = 0;
+    cudaStream_t s = as_stream(stream);
+    // from two waves of tiles: below, at 32^3, the sums at the end weigh more than
+    // the tap tiles' copies (1 x 32^3, 16 -> 32: 19 us against 15; 4 x: 27 and 29).
+    // FLUB_CONV_XR forces the halo kernel wherever it fits.
+    if (cin <= 32 && cout <= 32 && NZ % 8 == 0 && NY % 16 == 0 && halo_enabled() &&
+        (forced_xr() || (int64_t)B * NX * (NY / 16) * (NZ / 8) >= 4 * kNumSMs)) {
+        int st = FLUB_OK;
+#define FLUB_WGH(CI, CO) \
+    if (cin == CI && cout == CO) st = launch_wgrad_halo<CI, CO>(x, dy, B, NX, NY, NZ, dw, s);
+        FLUB_WGH(16, 16) FLUB_WGH(16, 32) FLUB_WGH(32, 16) FLUB_WGH(32, 32)
+#undef FLUB_WGH
+        if (st) return st;
+        if (db) return launch_bias_grad(dy, cout, (int64_t)B * NX * NY * NZ, db, s);
+        return FLUB_OK;
+    }
     int st = get_encode();
     if (st) return st;
     CUtensorMap mx, mdy;
     if ((st = make_act_map(&mx, x, cin, g)) || (st = make_act_map(&mdy, dy, cout, g))) return st;
-    cudaStream_t s = as_stream(stream);
 #define FLUB_WG(CI, CO) \
     if (cin == CI && cout == CO) st = launch_wgrad<CI, CO>(mx, mdy, g, dw, s);
     FLUB_WG(16, 16) FLUB_WG(16, 32) FLUB_WG(16, 64)

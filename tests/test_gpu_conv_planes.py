@@ -48,3 +48,26 @@ def test_bias_gradient_matches_float64(grid, co):
     n = dy.numel() // co
     # FP32 partial sums: n rounding errors of 2^-24 of sums below sum |dy|
     assert float((db.double().cpu() - want).abs().max()) <= 2.0 ** -20 * n
+
+
+@pytest.mark.parametrize("grid", [(1, 1, 16, 8), (1, 2, 16, 16), (2, 3, 32, 8), (1, 7, 16, 16), (1, 20, 48, 64)])
+@pytest.mark.parametrize("ci,co", [(16, 16), (16, 32), (32, 16), (32, 32)])
+def test_wgrad_planes_match_float64(grid, ci, co, monkeypatch):
+    """The halo-plane weight gradient: fewer x planes than a segment, rests of
+    one and two, more segments than buffers; added to what dW holds."""
+    from flub_gb300 import unet as U
+    from oracle import unet_ref as R
+    monkeypatch.setenv("FLUB_CONV_XR", "1")  # forces the kernel on small grids
+    g = torch.Generator().manual_seed(sum(grid) + ci + co)
+    x = torch.randn(grid + (ci,), generator=g).to(torch.bfloat16)
+    dy = torch.randn(grid + (co,), generator=g).to(torch.bfloat16)
+    dw = torch.full((27, co, ci), 0.25, device="cuda")
+    U.conv_error(reset=True)
+    U.conv3d_wgrad(x.cuda(), dy.cuda(), dw)
+    assert U.conv_error() == 0
+    w = torch.zeros((27, co, ci), dtype=torch.float64, requires_grad=True)
+    (R.conv3d(x.double(), w, bias=torch.zeros(co, dtype=torch.float64), relu=False) * dy.double()).sum().backward()
+    want = 0.25 + w.grad
+    # exact products of BF16 values, FP32 sums of n of them: n roundings of 2^-24 of sums below n
+    n = grid[0] * grid[1] * grid[2] * grid[3]
+    assert float((dw.double().cpu() - want).abs().max()) <= 2.0 ** -22 * n + 2.0 ** -20
