@@ -67,7 +67,6 @@ __global__ void __launch_bounds__(kRedThreads, 4) k8_matvec_pap(MgState *st, con
                                                              const uint16_t *__restrict__ sw, Dims D, double *partials,
                                                              const int *__restrict__ act,
                                                              const int *__restrict__ act_n, unsigned long long *kc) {
-    __shared__ double red[32];
     pdl_open();
     const int ng = (int)(D.n() >> 3);
     const int tot = *act_n;
@@ -82,7 +81,8 @@ __global__ void __launch_bounds__(kRedThreads, 4) k8_matvec_pap(MgState *st, con
         o_next = __ldg(items + ng + g_next);
     }
     pdl_wait(kc);
-    if (st->it >= st->max_iters || st->converged || st->status) return;
+    const unsigned nb = working_blocks(tot);
+    if (blockIdx.x >= nb || st->it >= st->max_iters || st->converged || st->status) return;
     const int sj = D.nz, si = D.ny * D.nz;
     double s = 0.0;
     for (; base < tot; base += stride) {
@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(kRedThreads, 4) k8_matvec_pap(MgState *st, con
         }
     }
     double total;
-    if (finish_partials(s, partials, &st->ticket, red, &total) && threadIdx.x == 0) {
+    if (finish_partials(s, partials, &st->ticket, &total, nb) && threadIdx.x == 0) {
         st->pap = total;
         const double alpha = st->zr_old / (total + st->eps);
         st->alpha = alpha;
@@ -163,7 +163,6 @@ __global__ void __launch_bounds__(kRedThreads) k8_update_r_rr(MgState *st, float
                                                               cudaGraphConditionalHandle h, int set_cond,
                                                               const int *__restrict__ act,
                                                               const int *__restrict__ act_n, unsigned long long *kc) {
-    __shared__ double red[32];
     count_kernel(kc);
     if (st->it >= st->max_iters || st->converged || st->status) {
         if ((blockIdx.x | threadIdx.x) == 0) publish_cond(st, 0, h, set_cond);
@@ -173,6 +172,8 @@ __global__ void __launch_bounds__(kRedThreads) k8_update_r_rr(MgState *st, float
     const int skip = st->skip_r;
     const int *ga = skip ? act : nullptr;
     const int ng = (int)(n >> 3);
+    const unsigned nb = working_blocks(ga ? *act_n : ng);
+    if (blockIdx.x >= nb) return;
     double s = 0.0;
     FLUB_ACT_LOOP(g, ga, act_n, ng) {
         if (skip && !ga && !group_has_fluid(load_codes8(code + (g << 3)))) continue;
@@ -188,7 +189,7 @@ __global__ void __launch_bounds__(kRedThreads) k8_update_r_rr(MgState *st, float
         s += dot8_ff(rv.v, rv.v);
     }
     double total;
-    if (finish_partials(s, partials, &st->ticket, red, &total) && threadIdx.x == 0) {
+    if (finish_partials(s, partials, &st->ticket, &total, nb) && threadIdx.x == 0) {
         st->rtr = total;
         if (st->it < kHistory) hist[st->it] = total;
         if (!isfinite(total)) st->status = FLUB_ERR_BREAKDOWN;
@@ -203,7 +204,6 @@ __global__ void __launch_bounds__(kRedThreads) k8_dot_rr0(MgState *st, const flo
                                                           const uint8_t *__restrict__ code, int64_t n,
                                                           double *partials, const int *__restrict__ act,
                                                           const int *__restrict__ act_n, unsigned long long *kc) {
-    __shared__ double red[32];
     count_kernel(kc);
     const int skip = st->skip_r;
     const int *ga = skip ? act : nullptr;
@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(kRedThreads) k8_dot_rr0(MgState *st, const flo
         s += dot8_ff(rv.v, rv.v);
     }
     double total;
-    if (finish_partials(s, partials, &st->ticket, red, &total) && threadIdx.x == 0) {
+    if (finish_partials(s, partials, &st->ticket, &total) && threadIdx.x == 0) {
         st->rtr0 = total;
         st->rtr = total;
         const double rel = total * st->rel_tol;
@@ -232,10 +232,11 @@ __global__ void __launch_bounds__(kRedThreads) k8_dot_zr(MgState *st, const floa
                                                          const uint8_t *__restrict__ code, int64_t n,
                                                          double *partials, const int *__restrict__ act,
                                                          const int *__restrict__ act_n, unsigned long long *kc) {
-    __shared__ double red[32];
     count_kernel(kc);
     const int ng = (int)(n >> 3);
     const float zs = kScaleZ ? st->zscale : 1.0f;
+    const unsigned nb = working_blocks(act ? *act_n : ng);
+    if (blockIdx.x >= nb) return;
     double s = 0.0;
     FLUB_ACT_LOOP(g, act, act_n, ng) {
         if (!act && !group_has_fluid(load_codes8(code + (g << 3)))) continue;  // z = 0 (and p = 0) there
@@ -250,7 +251,7 @@ __global__ void __launch_bounds__(kRedThreads) k8_dot_zr(MgState *st, const floa
         if (kInit) St<float>::st8_wide(p + (g << 3), zv.v);
     }
     double total;
-    if (finish_partials(s, partials, &st->ticket, red, &total) && threadIdx.x == 0) {
+    if (finish_partials(s, partials, &st->ticket, &total, nb) && threadIdx.x == 0) {
         if (kInit) {
             st->zr_old = total;
         } else {
@@ -327,7 +328,6 @@ __global__ void __launch_bounds__(kRedThreads) k8_x0_gamma(MgState *st, const fl
                                                            const uint16_t *__restrict__ sw, Dims D, double *partials,
                                                            const int *__restrict__ act,
                                                            const int *__restrict__ act_n) {
-    __shared__ double red[32];
     const int ng = (int)(D.n() >> 3);
     double s_ld = 0.0, s_b = 0.0;
     FLUB_ACT_LOOP(g, act, act_n, ng) {
@@ -343,15 +343,15 @@ __global__ void __launch_bounds__(kRedThreads) k8_x0_gamma(MgState *st, const fl
         s_ld += dot8_ff(dm, ld);
         s_b += dot8_ff(dm, bv.v);
     }
-    const double bb = block_sum(s_b, red);
+    const double bb = block_sum_red(s_b);
     __syncthreads();
     if (threadIdx.x == 0) partials[kMaxRedBlocks + blockIdx.x] = bb;
     double total;
-    if (finish_partials(s_ld, partials, &st->ticket, red, &total)) {
+    if (finish_partials(s_ld, partials, &st->ticket, &total)) {
         __syncthreads();
         double t2 = 0.0;
         for (unsigned q = threadIdx.x; q < gridDim.x; q += blockDim.x) t2 += __ldcg(&partials[kMaxRedBlocks + q]);
-        t2 = block_sum(t2, red);
+        t2 = block_sum_red(t2);
         if (threadIdx.x == 0) {
             const double gm = t2 / total;
             st->x0_scale = (total != 0.0 && isfinite(gm)) ? gm : 0.0;

@@ -34,11 +34,16 @@ struct MgState {
 // Power of two near 1 / RMS of a vector with squared norm rtr over n entries:
 // the FP16 residual copy is stored at this scale so that it neither overflows
 // nor underflows as CG drives the residual down by orders of magnitude.
+// The exponent of the RMS is half that of rtr / n, which the exponents and
+// mantissas of both give by comparison: no FP64 division and square root.
 __device__ __forceinline__ float fp16_residual_scale(double rtr, int64_t n) {
     if (!(rtr > 0.0) || !isfinite(rtr)) return 1.0f;
-    int e = ilogb(sqrt(rtr / (double)n));
+    const long long a = __double_as_longlong(rtr), b = __double_as_longlong((double)n);
+    constexpr long long mant = (1ll << 52) - 1;
+    const int q = (int)(a >> 52) - (int)(b >> 52) - ((a & mant) < (b & mant) ? 1 : 0);  // floor(log2(rtr / n))
+    int e = q >> 1;
     e = e < -100 ? -100 : (e > 100 ? 100 : e);
-    return ldexpf(1.0f, -e);
+    return __int_as_float((127 - e) << 23);
 }
 
 // fp16_residual_scale evaluated once per block by thread 0 and shared: the
@@ -148,24 +153,50 @@ __device__ __forceinline__ void unflatten(int64_t c, const Dims D, int &i, int &
 }
 
 // ---------------------------------------------------------------- last-block reductions
-// Each block stores its partial, the last block to finish combines all
-// partials in index order (deterministic for a fixed grid size).
-__device__ __forceinline__ bool finish_partials(double v, double *partials, unsigned int *ticket, double *red,
-                                                double *total) {
+// Sum over a block of kRedThreads threads in a fixed tree order, valid in thread
+// 0: through shared memory, so that one warp does the additions.  An FP64 addition
+// occupies this GPU's FP64 pipe for 16 cycles a warp whatever its lanes hold: by
+// shuffles in every warp a block took 45 of them, here 12.
+__device__ __forceinline__ double block_sum_red(double v) {
+    __shared__ double part[kRedThreads];
+    __syncthreads();
+    part[threadIdx.x] = v;
+    __syncthreads();
+    double t = 0.0;
+    if (threadIdx.x < 32) {
+        const double *p = part + threadIdx.x;
+        t = ((p[0] + p[32]) + (p[64] + p[96])) + ((p[128] + p[160]) + (p[192] + p[224]));
+        t = warp_sum(t);
+    }
+    return t;
+}
+
+// Blocks of a grid-stride loop over tot items that have any (at least one): the
+// others of a reduction's grid, which is sized for a full level, leave at once.
+__device__ __forceinline__ unsigned working_blocks(int tot) {
+    const unsigned b = ((unsigned)tot + blockDim.x - 1) / blockDim.x;
+    return b < 1 ? 1 : (b < gridDim.x ? b : gridDim.x);
+}
+
+// Each of the first nb blocks stores its partial, the last of them to finish
+// combines all partials in index order (deterministic for a fixed grid size).
+// Blocks of kRedThreads threads.
+__device__ __forceinline__ bool finish_partials(double v, double *partials, unsigned int *ticket, double *total,
+                                                unsigned nb = gridDim.x) {
     __shared__ bool am_last;
-    double b = block_sum(v, red);
+    double b = block_sum_red(v);
     if (threadIdx.x == 0) {
         partials[blockIdx.x] = b;
         __threadfence();
         const unsigned t = atomicAdd(ticket, 1u);
-        am_last = (t == gridDim.x - 1);
+        am_last = (t == nb - 1);
     }
     __syncthreads();
     if (!am_last) return false;
     __threadfence();
     double s = 0.0;
-    for (unsigned q = threadIdx.x; q < gridDim.x; q += blockDim.x) s += __ldcg(&partials[q]);
-    s = block_sum(s, red);
+    for (unsigned q = threadIdx.x; q < nb; q += blockDim.x) s += __ldcg(&partials[q]);
+    s = block_sum_red(s);
     if (threadIdx.x == 0) {
         *total = s;
         *ticket = 0u;
@@ -492,7 +523,6 @@ __global__ void __launch_bounds__(256) k_residual_x0(MgState *st, float *__restr
 __global__ void __launch_bounds__(kRedThreads) k_fluid_mean(MgState *st, const float *__restrict__ r,
                                                             const uint8_t *__restrict__ code, int64_t n,
                                                             double *partials, int guard, unsigned long long *kc) {
-    __shared__ double red[32];
     count_kernel(kc);
     if (guard == 1 && (st->it >= st->max_iters || st->converged || st->status)) return;
     if (guard == 2 && !st->use_x0) return;
@@ -504,14 +534,14 @@ __global__ void __launch_bounds__(kRedThreads) k_fluid_mean(MgState *st, const f
         }
     double total;
     // two reductions share one ticket: pack the count into the second half of partials
-    double bc = block_sum(cnt, red);
+    double bc = block_sum_red(cnt);
     __syncthreads();
     if (threadIdx.x == 0) partials[kMaxRedBlocks + blockIdx.x] = bc;
-    if (finish_partials(s, partials, &st->ticket, red, &total)) {
+    if (finish_partials(s, partials, &st->ticket, &total)) {
         __syncthreads();
         double c2 = 0.0;
         for (unsigned q = threadIdx.x; q < gridDim.x; q += blockDim.x) c2 += __ldcg(&partials[kMaxRedBlocks + q]);
-        c2 = block_sum(c2, red);
+        c2 = block_sum_red(c2);
         if (threadIdx.x == 0) st->mean = c2 > 0.0 ? total / c2 : 0.0;
     }
 }
@@ -531,7 +561,6 @@ __global__ void __launch_bounds__(kRedThreads) k_sub_mean(MgState *st, float *__
 // rTr0 and the tolerance (multigrid/mgpcg.py:391-393).
 __global__ void __launch_bounds__(kRedThreads) k_dot_rr0(MgState *st, const float *__restrict__ r, int64_t n,
                                                          double *partials, unsigned long long *kc) {
-    __shared__ double red[32];
     count_kernel(kc);
     double s = 0.0;
     for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x) {
@@ -539,7 +568,7 @@ __global__ void __launch_bounds__(kRedThreads) k_dot_rr0(MgState *st, const floa
         s = fma(v, v, s);
     }
     double total;
-    if (finish_partials(s, partials, &st->ticket, red, &total) && threadIdx.x == 0) {
+    if (finish_partials(s, partials, &st->ticket, &total) && threadIdx.x == 0) {
         st->rtr0 = total;
         st->rtr = total;
         const double rel = total * st->rel_tol;
@@ -551,7 +580,6 @@ __global__ void __launch_bounds__(kRedThreads) k_dot_rr0(MgState *st, const floa
 __global__ void __launch_bounds__(kRedThreads) k_dot_zr_init(MgState *st, const float *__restrict__ z,
                                                              const float *__restrict__ r, float *__restrict__ p,
                                                              int64_t n, double *partials, unsigned long long *kc) {
-    __shared__ double red[32];
     count_kernel(kc);
     double s = 0.0;
     for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x) {
@@ -560,7 +588,7 @@ __global__ void __launch_bounds__(kRedThreads) k_dot_zr_init(MgState *st, const 
         p[c] = zc;
     }
     double total;
-    if (finish_partials(s, partials, &st->ticket, red, &total) && threadIdx.x == 0) st->zr_old = total;
+    if (finish_partials(s, partials, &st->ticket, &total) && threadIdx.x == 0) st->zr_old = total;
 }
 
 // Ap = L p and p.Ap -> alpha (mgpcg.py:410-419).  Guarded: a no-op once the
@@ -568,7 +596,6 @@ __global__ void __launch_bounds__(kRedThreads) k_dot_zr_init(MgState *st, const 
 __global__ void __launch_bounds__(kRedThreads) k_matvec_pap(MgState *st, const float *__restrict__ p,
                                                             float *__restrict__ Ap, const uint8_t *__restrict__ code,
                                                             Dims D, double *partials, unsigned long long *kc) {
-    __shared__ double red[32];
     count_kernel(kc);
     if (st->it >= st->max_iters || st->converged || st->status) return;
     const int64_t n = D.n();
@@ -585,7 +612,7 @@ __global__ void __launch_bounds__(kRedThreads) k_matvec_pap(MgState *st, const f
         s = fma((double)pc, (double)a, s);
     }
     double total;
-    if (finish_partials(s, partials, &st->ticket, red, &total) && threadIdx.x == 0) {
+    if (finish_partials(s, partials, &st->ticket, &total) && threadIdx.x == 0) {
         st->pap = total;
         const double alpha = st->zr_old / (total + st->eps);
         st->alpha = alpha;
@@ -607,7 +634,6 @@ __global__ void __launch_bounds__(kRedThreads) k_update_r_rr(MgState *st, float 
                                                              double *partials, double *hist,
                                                              cudaGraphConditionalHandle h, int set_cond,
                                                              unsigned long long *kc) {
-    __shared__ double red[32];
     count_kernel(kc);
     if (st->it >= st->max_iters || st->converged || st->status) {
         if (blockIdx.x == 0 && threadIdx.x == 0) publish_cond(st, 0, h, set_cond);
@@ -624,7 +650,7 @@ __global__ void __launch_bounds__(kRedThreads) k_update_r_rr(MgState *st, float 
         s = fma((double)rv, (double)rv, s);
     }
     double total;
-    if (finish_partials(s, partials, &st->ticket, red, &total) && threadIdx.x == 0) {
+    if (finish_partials(s, partials, &st->ticket, &total) && threadIdx.x == 0) {
         st->rtr = total;
         if (st->it < kHistory) hist[st->it] = total;
         if (!isfinite(total)) st->status = FLUB_ERR_BREAKDOWN;
@@ -649,13 +675,12 @@ __global__ void __launch_bounds__(kRedThreads) k_update_r(MgState *st, float *__
 __global__ void __launch_bounds__(kRedThreads) k_dot_zr_beta(MgState *st, const float *__restrict__ z,
                                                              const float *__restrict__ r, int64_t n,
                                                              double *partials, unsigned long long *kc) {
-    __shared__ double red[32];
     count_kernel(kc);
     double s = 0.0;
     for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x)
         s = fma((double)z[c], (double)r[c], s);
     double total;
-    if (finish_partials(s, partials, &st->ticket, red, &total) && threadIdx.x == 0) {
+    if (finish_partials(s, partials, &st->ticket, &total) && threadIdx.x == 0) {
         const double beta = total / (st->zr_old + st->eps);
         st->beta = beta;
         st->zr_old = total;

@@ -1489,7 +1489,6 @@ __global__ void __launch_bounds__(kRedThreads) k_x0_gamma(MgState *st, const flo
                                                           const float *__restrict__ b,
                                                           const uint8_t *__restrict__ code, Dims D,
                                                           double *partials) {
-    __shared__ double red[32];
     const int64_t n = D.n();
     double s_ld = 0.0, s_b = 0.0;
     for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x) {
@@ -1501,15 +1500,15 @@ __global__ void __launch_bounds__(kRedThreads) k_x0_gamma(MgState *st, const flo
         s_ld = fma((double)dc, (double)ld, s_ld);
         s_b = fma((double)dc, (double)b[c], s_b);
     }
-    const double bb = block_sum(s_b, red);
+    const double bb = block_sum_red(s_b);
     __syncthreads();
     if (threadIdx.x == 0) partials[kMaxRedBlocks + blockIdx.x] = bb;
     double total;
-    if (finish_partials(s_ld, partials, &st->ticket, red, &total)) {
+    if (finish_partials(s_ld, partials, &st->ticket, &total)) {
         __syncthreads();
         double t2 = 0.0;
         for (unsigned q = threadIdx.x; q < gridDim.x; q += blockDim.x) t2 += __ldcg(&partials[kMaxRedBlocks + q]);
-        t2 = block_sum(t2, red);
+        t2 = block_sum_red(t2);
         if (threadIdx.x == 0) {
             const double g = t2 / total;
             st->x0_scale = (total != 0.0 && isfinite(g)) ? g : 0.0;

@@ -100,7 +100,6 @@ __global__ void __launch_bounds__(kRedThreads) k8_update_r_rr_mixed(MgState *st,
                                                                     const int *__restrict__ act,
                                                                     const int *__restrict__ act_n,
                                                                     unsigned long long *kc) {
-    __shared__ double red[32];
     count_kernel(kc);
     if (st->it >= st->max_iters || st->converged || st->status) {
         if ((blockIdx.x | threadIdx.x) == 0) publish_cond(st, 0, h, set_cond);
@@ -113,6 +112,8 @@ __global__ void __launch_bounds__(kRedThreads) k8_update_r_rr_mixed(MgState *st,
     const int *ga = skip ? act : nullptr;
     // scale of the FP16 copy from the previous residual norm (st->rtr is only
     // overwritten by the last block, after every block has read it)
+    const unsigned nb = working_blocks(ga ? *act_n : (int)(n >> 3));
+    if (blockIdx.x >= nb) return;
     const float hs = block_fp16_residual_scale(threadIdx.x == 0 ? st->rtr : 0.0, n);
     if ((blockIdx.x | threadIdx.x) == 0) st->zscale = 1.0f / hs;
     const int ng = (int)(n >> 3);
@@ -133,7 +134,7 @@ __global__ void __launch_bounds__(kRedThreads) k8_update_r_rr_mixed(MgState *st,
         s += dot8_ff(rv, rv);
     }
     double total;
-    if (finish_partials(s, partials, &st->ticket, red, &total) && threadIdx.x == 0) {
+    if (finish_partials(s, partials, &st->ticket, &total, nb) && threadIdx.x == 0) {
         st->rtr = total;
         if (st->it < kHistory) hist[st->it] = total;
         if (!isfinite(total)) st->status = FLUB_ERR_BREAKDOWN;
@@ -150,10 +151,11 @@ __global__ void __launch_bounds__(kRedThreads) k8_dot_zr_flex(MgState *st, const
                                                               const uint8_t *__restrict__ code, int64_t n,
                                                               double *partials, const int *__restrict__ act,
                                                               const int *__restrict__ act_n, unsigned long long *kc) {
-    __shared__ double red[32];
     count_kernel(kc);
     const int ng = (int)(n >> 3);
     const float zs = st->zscale;
+    const unsigned nb = working_blocks(act ? *act_n : ng);
+    if (blockIdx.x >= nb) return;
     double s = 0.0, so = 0.0;
     FLUB_ACT_LOOP(g, act, act_n, ng) {
         if (!act && !group_has_fluid(load_codes8(code + (g << 3)))) continue;  // z = 0 there
@@ -166,15 +168,15 @@ __global__ void __launch_bounds__(kRedThreads) k8_dot_zr_flex(MgState *st, const
         s += dot8_ff(zv, rv);
         so += dot8_ff(zv, ov);
     }
-    const double bo = block_sum(so, red);
+    const double bo = block_sum_red(so);
     __syncthreads();
     if (threadIdx.x == 0) partials[kMaxRedBlocks + blockIdx.x] = bo;
     double total;
-    if (finish_partials(s, partials, &st->ticket, red, &total)) {
+    if (finish_partials(s, partials, &st->ticket, &total, nb)) {
         __syncthreads();
         double t2 = 0.0;
-        for (unsigned q = threadIdx.x; q < gridDim.x; q += blockDim.x) t2 += __ldcg(&partials[kMaxRedBlocks + q]);
-        t2 = block_sum(t2, red);
+        for (unsigned q = threadIdx.x; q < nb; q += blockDim.x) t2 += __ldcg(&partials[kMaxRedBlocks + q]);
+        t2 = block_sum_red(t2);
         if (threadIdx.x == 0) {
             const double beta = (total - t2) / (st->zr_old + st->eps);
             st->beta = beta;

@@ -126,6 +126,8 @@ __global__ void __launch_bounds__(256, 4)
         lut[threadIdx.x] = make_float2(threadIdx.x ? __fdiv_rn(-1.0f, (float)threadIdx.x) : 0.0f, (float)threadIdx.x);
     __syncthreads();
     pdl_wait(kc);
+    const unsigned nb = working_blocks(total);
+    if (kMode == kLast && A.dot && blockIdx.x >= nb) return;
     double zr = 0.0, zro = 0.0;  // kLast with A.dot: this thread's parts of z.r and z.r_old
     const float zsc = (kMode == kLast && A.dot && A.zscaled) ? A.st->zscale : 1.0f;
     for (; t < total; t += stride) {
@@ -301,20 +303,19 @@ __global__ void __launch_bounds__(256, 4)
     if (kMode == kLast && A.dot) {
         // the grid's z.r in FP64 (deterministic two-level reduction) and the
         // CG scalars, as k8_dot_zr sets them
-        __shared__ double red[32];
-        if (A.dot == 3) {
-            const double bo = block_sum(zro, red);
+            if (A.dot == 3) {
+            const double bo = block_sum_red(zro);
             __syncthreads();
             if (threadIdx.x == 0) A.partials[kMaxRedBlocks + blockIdx.x] = bo;
         }
         double tot;
-        if (finish_partials(zr, A.partials, &A.st->ticket, red, &tot)) {
+        if (finish_partials(zr, A.partials, &A.st->ticket, &tot, nb)) {
             double t2 = 0.0;
             if (A.dot == 3) {
                 __syncthreads();
-                for (unsigned q = threadIdx.x; q < gridDim.x; q += blockDim.x)
+                for (unsigned q = threadIdx.x; q < nb; q += blockDim.x)
                     t2 += __ldcg(&A.partials[kMaxRedBlocks + q]);
-                t2 = block_sum(t2, red);
+                t2 = block_sum_red(t2);
             }
             if (threadIdx.x == 0) {
                 if (A.dot == 1) {
