@@ -260,74 +260,11 @@ __device__ __forceinline__ void group_ijk(int g, const Dims D, int &i, int &j, i
 // of 8 consecutive cells along k that contains a fluid cell.  Kernels that
 // only have work on fluid cells walk the list instead of the whole grid
 // (in the 256^3 dam break 20 % of the groups are active).  Built once per
-// set_tags in three deterministic passes: per-block counts, one-block scan,
-// ordered write.
-constexpr int kActThreads = 256;
-constexpr int kActRounds = 4;
-constexpr int kActPerBlock = kActThreads * kActRounds;
-
+// set_tags in three deterministic passes (setup_levels.cuh): per-block counts,
+// one-block scan, ordered write.
 __device__ __forceinline__ bool group_active(const uint8_t *__restrict__ code, int g) {
     const uint2 c = __ldg(reinterpret_cast<const uint2 *>(code + ((int64_t)g << 3)));
     return ((c.x | c.y) & 0x02020202u) != 0u;  // a fluid byte (code 2) among the 8
-}
-
-__global__ void __launch_bounds__(kActThreads) k_act_count(const uint8_t *__restrict__ code, int ng,
-                                                           int *__restrict__ bcount) {
-    int total = 0;
-    for (int q = 0; q < kActRounds; q++) {
-        const int g = blockIdx.x * kActPerBlock + q * kActThreads + threadIdx.x;
-        total += __syncthreads_count(g < ng && group_active(code, g));
-    }
-    if (threadIdx.x == 0) bcount[blockIdx.x] = total;
-}
-
-// Exclusive scan of nb block counts in place (one block of kActThreads), total to *act_n.
-__global__ void __launch_bounds__(kActThreads) k_act_scan(int *__restrict__ bcount, int nb, int *__restrict__ act_n) {
-    __shared__ int part[kActThreads];
-    const int per = (nb + kActThreads - 1) / kActThreads;
-    const int b0 = threadIdx.x * per, b1 = min(nb, b0 + per);
-    int s = 0;
-    for (int b = b0; b < b1; b++) s += bcount[b];
-    part[threadIdx.x] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int run = 0;
-        for (int t = 0; t < kActThreads; t++) {
-            const int v = part[t];
-            part[t] = run;
-            run += v;
-        }
-        *act_n = run;
-    }
-    __syncthreads();
-    int run = part[threadIdx.x];
-    for (int b = b0; b < b1; b++) {
-        const int v = bcount[b];
-        bcount[b] = run;
-        run += v;
-    }
-}
-
-__global__ void __launch_bounds__(kActThreads) k_act_write(const uint8_t *__restrict__ code, int ng,
-                                                           const int *__restrict__ boff, int *__restrict__ act) {
-    __shared__ int wcount[kActThreads / 32];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    int base = boff[blockIdx.x];
-    for (int q = 0; q < kActRounds; q++) {
-        const int g = blockIdx.x * kActPerBlock + q * kActThreads + threadIdx.x;
-        const bool f = g < ng && group_active(code, g);
-        const unsigned m = __ballot_sync(0xffffffffu, f);
-        if (lane == 0) wcount[wid] = __popc(m);
-        __syncthreads();
-        int before = 0, round = 0;
-        for (int w = 0; w < kActThreads / 32; w++) {
-            before += w < wid ? wcount[w] : 0;
-            round += wcount[w];
-        }
-        if (f) act[base + before + __popc(m & ((1u << lane) - 1u))] = g;
-        base += round;
-        __syncthreads();
-    }
 }
 
 // Loop over the groups a kernel works on: the active list when act is not

@@ -25,6 +25,7 @@
 #include "mixed.cuh"
 #include "persist.cuh"
 #include "restrict8.cuh"
+#include "setup_levels.cuh"
 #include "smooth8.cuh"
 #include "smooth_block.cuh"
 #include "smooth_split.cuh"
@@ -247,7 +248,9 @@ static size_t carve(flub_mg *mg, char *base) {
             L.tiles_n = (int *)take(sizeof(int));
         }
         L.b_ti = block_planes(mg, l);
-        L.cw = nl <= kCoarseMaxCells || L.b_ti ? (uint16_t *)take(sizeof(uint16_t) * (size_t)nl) : nullptr;
+        L.cw = nullptr;  // the coarse kernel's and the blocked smoothing's words are sw where that is kept
+        if (nl <= kCoarseMaxCells || L.b_ti)
+            L.cw = L.D.nz % 8 == 0 ? L.sw : (uint16_t *)take(sizeof(uint16_t) * (size_t)nl);
         L.b_tiles = 0;
         L.b_list = L.b_items = nullptr;
         L.b_n = nullptr;
@@ -265,8 +268,10 @@ static size_t carve(flub_mg *mg, char *base) {
                 L.z3 = (float *)take(sizeof(float) * nl);
         }
     }
-    // per-block counts of the active-list build (level 0 has the most blocks)
-    mg->act_scratch = (int *)take(sizeof(int) * (size_t)((n / 8 + kActPerBlock - 1) / kActPerBlock + 1));
+    // per-block counts of the active-list build of all levels
+    int64_t setup_blocks = 0;
+    for (int l = 0; l < mg->levels; l++) setup_blocks += (mg->lv[l].D.n() / 8 + kSetupThreads - 1) / kSetupThreads;
+    mg->act_scratch = (int *)take(sizeof(int) * (size_t)setup_blocks);
     mg->r_old = mg->precision == FLUB_PRECISION_MIXED ? (float *)take(sizeof(float) * n) : nullptr;
     return off;
 }
@@ -1433,22 +1438,12 @@ static int read_info(flub_mg *mg, cudaStream_t s, flub_solve_info *info) {
     return FLUB_OK;
 }
 
-// Stencil words of every group of a level (nz % 8 == 0).
-__global__ void __launch_bounds__(256) k_stencil_words(const uint8_t *__restrict__ code, uint16_t *__restrict__ sw,
-                                                       Dims D) {
-    const int ng = (int)(D.n() >> 3);
-    for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < ng; g += gridDim.x * blockDim.x) {
-        int i, j, kg;
-        group_ijk(g, D, i, j, kg);
-        *reinterpret_cast<uint4 *>(sw + ((int64_t)g << 3)) = words8_from_codes(code, D, i, j, kg << 3, g << 3);
-    }
-}
-
-// Stencil words of the levels the coarse kernel or the blocked smoothing runs.
+// Stencil words of the levels the coarse kernel or the blocked smoothing runs
+// whose rows are not whole 8-cell groups (the others' are Level::sw).
 static int enqueue_cell_words(flub_mg *mg, cudaStream_t s) {
     for (int l = 0; l < mg->levels; l++) {
         const Level &L = mg->lv[l];
-        if (!L.cw || (l < mg->co_start && !L.b_ti)) continue;
+        if (!L.cw || L.sw || (l < mg->co_start && !L.b_ti)) continue;
         k_cell_words<<<blocks_for(L.D.n(), 256), 256, 0, s>>>(L.code, L.cw, L.D);
         FLUB_CHECK_LAUNCH();
     }
@@ -1456,29 +1451,6 @@ static int enqueue_cell_words(flub_mg *mg, cudaStream_t s) {
 }
 
 // ---------------------------------------------------------------- warm-start support (no reference counterpart)
-
-// Stencil words in the colour-split order of smooth_split.cuh: natural cell
-// (i, j, k) -> element k >> 1 of row (i, j) in half (i + j + k) & 1.  One
-// thread per natural 8-cell group.
-__global__ void __launch_bounds__(256) k_split_words(const uint16_t *__restrict__ sw, uint16_t *__restrict__ sws,
-                                                     Dims D) {
-    const int ng = (int)(D.n() >> 3), hz = D.nz >> 1, hn = (int)(D.n() >> 1);
-    for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < ng; g += gridDim.x * blockDim.x) {
-        int i, j, kg;
-        group_ijk(g, D, i, j, kg);
-        const uint4 u = __ldg(reinterpret_cast<const uint4 *>(sw + ((size_t)g << 3)));
-        const int h = (i * D.ny + j) * hz + 4 * kg, p = (i + j) & 1;
-        uint32_t e[4], o[4];
-#pragma unroll
-        for (int m = 0; m < 8; m++) {
-            const uint32_t w = word_at(u, m);
-            if (((p + m) & 1) == 0) e[m >> 1] = w;
-            else o[m >> 1] = w;
-        }
-        *reinterpret_cast<uint2 *>(sws + h) = make_uint2(e[0] | (e[1] << 16), e[2] | (e[3] << 16));
-        *reinterpret_cast<uint2 *>(sws + hn + h) = make_uint2(o[0] | (o[1] << 16), o[2] | (o[3] << 16));
-    }
-}
 
 __global__ void k_set_x0_scale(MgState *st, double v) { st->x0_scale = v; }
 
@@ -1747,67 +1719,26 @@ int flub_mg_set_tags(flub_mg *mg, const int32_t *tag, void *stream) {
     FLUB_CHECK_LAUNCH();
     for (int l = 0; l + 1 < mg->levels; l++) {
         const Level &C = mg->lv[l + 1];
+        if (mg->lv[l].D.nz % 8 == 0) {
+            FLUB_TRY(launch_pdl(k_restrict_codes8, dim3(blocks_for(C.D.n() / 4, 256)), dim3(256), 0, s,
+                                (const uint8_t *)mg->lv[l].code, C.code, C.D));
+            continue;
+        }
         k_restrict_codes<<<blocks_for(C.D.n(), 256), 256, 0, s>>>(mg->lv[l].code, C.code, C.D);
         FLUB_CHECK_LAUNCH();
     }
     FLUB_TRY(enqueue_cell_words(mg, s));
-    for (int l = 0; l < mg->co_start && l < mg->levels; l++) {
-        const Level &L = mg->lv[l];
-        if (!L.b_ti) continue;
-        FLUB_CHECK_CUDA(cudaMemsetAsync(L.b_n, 0, sizeof(int), s));
-        k_block_tiles<<<L.b_tiles, 128, 0, s>>>(L.code, L.D, L.b_ti, (L.D.ny + kTJb - 1) / kTJb, block_tiles_k(L.D),
-                                                L.b_list, L.b_n);
-        FLUB_CHECK_LAUNCH();
-        const int V = row_vector(L.D.nz);
-        const unsigned blocks = blocks_for(L.D.n() / (2 * V), 256);
-        if (L.sw) continue;  // its items follow its stencil words below
-        if (V == 4)
-            k_block_items<4><<<blocks, 256, 0, s>>>(L.cw, L.D, L.b_items);
-        else if (V == 2)
-            k_block_items<2><<<blocks, 256, 0, s>>>(L.cw, L.D, L.b_items);
-        else
-            k_block_items<1><<<blocks, 256, 0, s>>>(L.cw, L.D, L.b_items);
-        FLUB_CHECK_LAUNCH();
-    }
-    // stencil words and active 8-cell groups of every level that has them
-    for (int l = 0; l < mg->levels; l++) {
-        const Level &L = mg->lv[l];
-        if (L.sw) {
-            k_stencil_words<<<blocks_for(L.D.n() >> 3, 256), 256, 0, s>>>(L.code, L.sw, L.D);
-            FLUB_CHECK_LAUNCH();
-        }
-        if (L.sw && L.b_items) {
-            k_block_items<4><<<blocks_for(L.D.n() >> 3, 256), 256, 0, s>>>(L.sw, L.D, L.b_items);
-            FLUB_CHECK_LAUNCH();
-        }
-        if (L.sws) {
-            k_split_words<<<blocks_for(L.D.n() >> 3, 256), 256, 0, s>>>(L.sw, L.sws, L.D);
-            FLUB_CHECK_LAUNCH();
-            if (L.zsh)
-                FLUB_CHECK_CUDA(cudaMemsetAsync(L.zsh, 0, sizeof(__half) * (size_t)L.D.n(), s));
-            else
-                FLUB_CHECK_CUDA(cudaMemsetAsync(L.zs, 0, sizeof(float) * (size_t)L.D.n(), s));
-        }
-        if (!L.act) continue;
-        const int ng = (int)(L.D.n() >> 3);
-        const int nb = (ng + kActPerBlock - 1) / kActPerBlock;
-        k_act_count<<<nb, kActThreads, 0, s>>>(L.code, ng, mg->act_scratch);
-        FLUB_CHECK_LAUNCH();
-        k_act_scan<<<1, kActThreads, 0, s>>>(mg->act_scratch, nb, L.act_n);
-        FLUB_CHECK_LAUNCH();
-        k_act_write<<<nb, kActThreads, 0, s>>>(L.code, ng, mg->act_scratch, L.act);
-        FLUB_CHECK_LAUNCH();
-        if (L.n_tiles) {
-            FLUB_CHECK_CUDA(cudaMemsetAsync(L.tflags, 0, (size_t)L.n_tiles, s));
-            FLUB_CHECK_CUDA(cudaMemsetAsync(L.tiles_n, 0, sizeof(int), s));
-            k_tile_flags<<<blocks_for(ng, 256, kNumSMs * 8), 256, 0, s>>>(L.act, L.act_n, L.D, L.tflags);
-            FLUB_CHECK_LAUNCH();
-            k_tile_list<<<blocks_for(L.n_tiles, 256), 256, 0, s>>>(L.tflags, L.n_tiles, L.tiles, L.tiles_n);
-            FLUB_CHECK_LAUNCH();
-        }
-    }
     // new tags: re-establish z = p = Ap = 0 off the fluid (the kernels skip
-    // 8-cell groups without fluid and rely on it)
+    // 8-cell groups without fluid and rely on it), and the tiles' count
+    ClearParams clear = {};
+    int64_t clear_blocks = 0;
+    auto zero = [&](void *p, size_t bytes) {
+        ClearRange &r = clear.lv[clear.n++];
+        r.p = (uint4 *)p;
+        r.n = (unsigned)((bytes + 15) / 16);  // every buffer is padded to 256 bytes
+        r.first = (int)clear_blocks;
+        clear_blocks += (r.n + kClearChunk - 1) / kClearChunk;
+    };
     for (int l = 0; l < mg->levels; l++) {
         const Level &L = mg->lv[l];
         const size_t b = sizeof(float) * (size_t)L.D.n();
@@ -1818,12 +1749,72 @@ int flub_mg_set_tags(flub_mg *mg, const int32_t *tag, void *stream) {
         // residual) and its FP16 copy is rewritten before each use
         char *first = l > 0 ? reinterpret_cast<char *>(L.r) : reinterpret_cast<char *>(L.z);
         char *last = L.z2h ? reinterpret_cast<char *>(L.z2h) + b / 2 : reinterpret_cast<char *>(L.z2) + b;
-        FLUB_CHECK_CUDA(cudaMemsetAsync(first, 0, (size_t)(last - first), s));
-        if (L.z3) FLUB_CHECK_CUDA(cudaMemsetAsync(L.z3, 0, b, s));
-        if (L.z3h) FLUB_CHECK_CUDA(cudaMemsetAsync(L.z3h, 0, b / 2, s));
+        zero(first, (size_t)(last - first));
+        if (L.z3) zero(L.z3, b);
+        if (L.z3h) zero(L.z3h, b / 2);
+        if (L.sws) zero(L.zsh ? (void *)L.zsh : (void *)L.zs, L.zsh ? b / 2 : b);
+        if (L.b_n) zero(L.b_n, sizeof(int));
     }
-    FLUB_CHECK_CUDA(cudaMemsetAsync(mg->p, 0, sizeof(float) * (size_t)mg->n, s));
-    FLUB_CHECK_CUDA(cudaMemsetAsync(mg->Ap, 0, sizeof(float) * (size_t)mg->n, s));
+    zero(mg->p, (size_t)(reinterpret_cast<char *>(mg->Ap) - reinterpret_cast<char *>(mg->p)) +
+                    sizeof(float) * (size_t)mg->n);
+    FLUB_TRY(launch_pdl(k_setup_clear, dim3((unsigned)clear_blocks), dim3(kSetupThreads), 0, s, clear));
+    // words and active groups of every level that has them
+    SetupParams P = {};
+    P.bcount = mg->act_scratch;
+    for (int l = 0; l < mg->levels; l++) {
+        const Level &L = mg->lv[l];
+        if (!L.act) continue;
+        SetupLevel &q = P.lv[P.n++];
+        q.D = L.D;
+        q.code = L.code;
+        q.sw = L.sw;
+        q.sws = L.sws;
+        q.items = L.b_items;
+        q.act = L.act;
+        q.act_n = L.act_n;
+        q.first = P.blocks;
+        P.blocks += (int)((L.D.n() / 8 + kSetupThreads - 1) / kSetupThreads);
+    }
+    if (P.n) {
+        FLUB_TRY(launch_pdl(k_setup_words, dim3(P.blocks), dim3(kSetupThreads), 0, s, P));
+        FLUB_TRY(launch_pdl(k_setup_scan, dim3(P.n), dim3(1024), 0, s, P));
+        FLUB_TRY(launch_pdl(k_setup_write, dim3(P.blocks), dim3(kSetupThreads), 0, s, P));
+    }
+    TileParams T = {};
+    int tile_blocks = 0;
+    for (int l = 0; l < mg->co_start && l < mg->levels; l++) {
+        const Level &L = mg->lv[l];
+        if (!L.b_ti) continue;
+        TileLevel &q = T.lv[T.n++];
+        q.D = L.D;
+        q.code = L.code;
+        q.ti = L.b_ti;
+        q.ntj = (L.D.ny + kTJb - 1) / kTJb;
+        q.ntk = block_tiles_k(L.D);
+        q.first = tile_blocks;
+        q.tiles = L.b_list;
+        q.count = L.b_n;
+        tile_blocks += L.b_tiles;
+        if (L.sw) continue;  // its items came with its words
+        const int V = row_vector(L.D.nz);
+        const unsigned blocks = blocks_for(L.D.n() / (2 * V), 256);
+        if (V == 2)
+            k_block_items<2><<<blocks, 256, 0, s>>>(L.cw, L.D, L.b_items);
+        else
+            k_block_items<1><<<blocks, 256, 0, s>>>(L.cw, L.D, L.b_items);
+        FLUB_CHECK_LAUNCH();
+    }
+    if (T.n) FLUB_TRY(launch_pdl(k_setup_tiles, dim3(tile_blocks), dim3(128), 0, s, T));
+    for (int l = 0; l < mg->levels; l++) {
+        const Level &L = mg->lv[l];
+        if (!L.act || !L.n_tiles) continue;
+        FLUB_CHECK_CUDA(cudaMemsetAsync(L.tflags, 0, (size_t)L.n_tiles, s));
+        FLUB_CHECK_CUDA(cudaMemsetAsync(L.tiles_n, 0, sizeof(int), s));
+        k_tile_flags<<<blocks_for(L.D.n() >> 3, 256, kNumSMs * 8), 256, 0, s>>>(L.act, L.act_n, L.D, L.tflags);
+        FLUB_CHECK_LAUNCH();
+        k_tile_list<<<blocks_for(L.n_tiles, 256), 256, 0, s>>>(L.tflags, L.n_tiles, L.tiles, L.tiles_n);
+        FLUB_CHECK_LAUNCH();
+    }
     return FLUB_OK;
 }
 

@@ -317,59 +317,49 @@ __global__ void __launch_bounds__(kBlockThreads, 1) k_smooth_block(const BlockAr
     if (!waited) pdl_wait(kc);
 }
 
-// The item words of a level from its stencil words.
+// The item words of the 2 V cells of a row from k0 on, from their stencil words
+// (two in each element of wd).
+template <int V>
+__device__ __forceinline__ void item_words(const uint32_t (&wd)[V], const Dims D, int i, int j, int k0,
+                                           uint32_t (&out)[2]) {
+    const int par = (i + j) & 1;
+    uint32_t ab[2] = {0u, 0u};  // of the cells k0 + 0, 2, .. and k0 + 1, 3, ..
+#pragma unroll
+    for (int m = 0; m < 2 * V; m++) {
+        const uint32_t w = (wd[m >> 1] >> (16 * (m & 1))) & 0xffffu;
+        const int k = k0 + m;
+        if ((w & 3u) != kCodeFluid) continue;
+        const uint32_t ns = sw_ns(w), d = __popc(ns);
+        uint32_t inside = kAllCount;  // the neighbours that lie in the domain
+        if (i + 1 >= D.nx) inside &= ~4u;
+        if (i == 0) inside &= ~16u;
+        if (j + 1 >= D.ny) inside &= ~64u;
+        if (j == 0) inside &= ~256u;
+        if (k + 1 >= D.nz) inside &= ~1024u;
+        if (k == 0) inside &= ~4096u;
+        uint32_t &o = ab[m & 1];
+        o |= d << (4 * (m >> 1));
+        if (d) o |= kItemAny;
+        if (d && ns != inside) o |= kItemSolid;
+        if (d && (w & kAllCount)) o |= kItemAir;  // the low bit of a neighbour's code
+    }
+    out[0] = par ? ab[1] : ab[0];
+    out[1] = par ? ab[0] : ab[1];
+}
+
+// The item words of a level whose rows are not whole 8-cell groups (V = 2 or 1).
 template <int V>
 __global__ void __launch_bounds__(256) k_block_items(const uint16_t *__restrict__ cw, Dims D, uint32_t *__restrict__ items) {
     const int lsegs = D.nz / (2 * V), n = D.nx * D.ny * lsegs;
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
-        const int seg = e % lsegs, row = e / lsegs, j = row % D.ny, i = row / D.ny, par = (i + j) & 1;
-        uint32_t out[2] = {0u, 0u};
-        uint32_t wd[V];  // two words each
-        if constexpr (V == 4) {
-            const uint4 q = __ldg(reinterpret_cast<const uint4 *>(cw) + e);
-            wd[0] = q.x; wd[1] = q.y; wd[2] = q.z; wd[3] = q.w;
-        } else {
+        const int seg = e % lsegs, row = e / lsegs, j = row % D.ny, i = row / D.ny;
+        uint32_t wd[V], out[2];
 #pragma unroll
-            for (int m = 0; m < V; m++) wd[m] = __ldg(reinterpret_cast<const uint32_t *>(cw) + (int64_t)e * V + m);
-        }
-#pragma unroll
-        for (int m = 0; m < 2 * V; m++) {
-            const uint32_t w = (wd[m >> 1] >> (16 * (m & 1))) & 0xffffu;
-            const int k = 2 * V * seg + m;
-            if ((w & 3u) != kCodeFluid) continue;
-            const uint32_t ns = sw_ns(w), d = __popc(ns);
-            uint32_t inside = kAllCount;  // the neighbours that lie in the domain
-            if (i + 1 >= D.nx) inside &= ~4u;
-            if (i == 0) inside &= ~16u;
-            if (j + 1 >= D.ny) inside &= ~64u;
-            if (j == 0) inside &= ~256u;
-            if (k + 1 >= D.nz) inside &= ~1024u;
-            if (k == 0) inside &= ~4096u;
-            uint32_t &o = out[(par + m) & 1];
-            o |= d << (4 * (m >> 1));
-            if (d) o |= kItemAny;
-            if (d && ns != inside) o |= kItemSolid;
-            if (d && (w & kAllCount)) o |= kItemAir;  // the low bit of a neighbour's code
-        }
+        for (int m = 0; m < V; m++) wd[m] = __ldg(reinterpret_cast<const uint32_t *>(cw) + (int64_t)e * V + m);
+        item_words<V>(wd, D, i, j, 2 * V * seg, out);
         items[e] = out[0];
         items[n + e] = out[1];
     }
-}
-
-// The tiles that hold a fluid cell, in any order (they do not depend on each
-// other).  One block per tile; *n is 0 before.
-__global__ void __launch_bounds__(128) k_block_tiles(const uint8_t *__restrict__ code, Dims D, int ti, int ntj, int ntk,
-                                                     uint32_t *__restrict__ tiles, int *n) {
-    const int tile = blockIdx.x, tk = tile % ntk, tq = tile / ntk;
-    const int ib = (tq / ntj) * ti, jb = (tq % ntj) * kTJb, kb = ntk > 1 ? tk * kKB : 0;
-    const int kn = ntk > 1 ? min(kKB, D.nz - kb) : D.nz;
-    bool any = false;
-    for (int e = threadIdx.x; e < ti * kTJb * kn; e += blockDim.x) {
-        const int k = e % kn, row = e / kn, i = ib + row / kTJb, j = jb + row % kTJb;
-        if (i < D.nx && j < D.ny) any |= code[((int64_t)i * D.ny + j) * D.nz + kb + k] == kCodeFluid;
-    }
-    if (__syncthreads_or(any) && threadIdx.x == 0)
-        tiles[atomicAdd(n, 1)] = (uint32_t)(tq / ntj) | (uint32_t)(tq % ntj) << 11 | (uint32_t)tk << 22;
 }
 
 }  // namespace flub
