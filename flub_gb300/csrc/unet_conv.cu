@@ -270,7 +270,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
 // accumulators lie side by side in TMEM (columns xi * Cout ...), and the weights
 // are staged as [dy, dz][chunk][dx = 1, 0, -1][Cout][8 channels], so that one MMA
 // of N = 3 Cout serves all three.  A plane is thus finished with after its own
-// MMAs, and planes pass through a ring of R buffers:
+// MMAs, and planes pass through a ring of R buffers, source 0's, then source 1's:
 //   - warps 4-7 stage planes with asynchronous copies, R - 1 planes ahead and,
 //     before they reuse a buffer, behind done[p - R]; when plane p has landed they
 //     publish it to the tensor core (a proxy fence) and arrive on full[p];
@@ -278,22 +278,23 @@ __global__ void __launch_bounds__(kConvThreads, 1)
 //   - warps 0-3 write output plane o after done[o + 2].
 // Each role's chain of instructions for a plane is as long as its MMAs, so none
 // does another's work.
-// 4 x 64^3, 32 + 16 -> 16 channels: the tap tiles' 254 us -> 78 us; 16 -> 32
-// and 16 -> 16: 105 and 72 us with one MMA a tap and no overlap -> 56 and 40.
+// 4 x 64^3, 32 + 16 -> 16 channels: the tap tiles' 254 us -> 77 us; 16 -> 32
+// and 16 -> 16: 105 and 72 us with one MMA a tap and no overlap -> 54 and 38.
 constexpr int kHaloZ = 10, kHaloY = 18;
 constexpr int kHaloRows = kHaloZ * kHaloY;  // 16-byte rows per chunk (180)
 constexpr int kHaloThreads = 2 * kConvThreads + 32;
 constexpr int kHaloMaxX = 16;               // output planes per CTA
 // opt-in shared memory per block less an allowance for the kernel's static shared variables
 constexpr int kHaloSmemMax = 227 * 1024 - 128;
-constexpr int kHaloBars = 8 * 2 * (kHaloMaxX + 2);
+constexpr int kHaloSteps = 2 * (kHaloMaxX + 2);  // planes of both sources
+constexpr int kHaloBars = 8 * 2 * kHaloSteps;
 
 struct HaloGeom {
     int B, NX, NY, NZ;
     int xr, ring;           // output planes per CTA, plane buffers
     int cin0, cin1, relu;   // cin1 = 0: one source
     int chunk0, chunk1;     // bytes from one chunk region to the next, per source
-    int src1_off, slot;     // source 1's chunks within a plane buffer, bytes of one
+    int slot;               // bytes of a plane buffer
     int w0_off, w1_off;     // weights of source 0 and 1 (27 taps each)
     int bar_off;            // mbarriers full[], done[], TMEM slot
     uint32_t tmem_cols;
@@ -359,9 +360,9 @@ __device__ __forceinline__ void halo_stage_weights(const uint4 *__restrict__ w, 
     }
 }
 
-// ITEMS: 16-byte items of a plane per staging thread, (chunks of both sources) x 180 / 128 rounded up.
+// ITEMS: 16-byte items of a plane per staging thread, chunks x 180 / 128 rounded up.
 template <int COUT, int ITEMS>
-__global__ void __launch_bounds__(kHaloThreads, COUT == 64 || ITEMS > 9 ? 2 : 3)
+__global__ void __launch_bounds__(kHaloThreads, COUT == 64 || ITEMS > 6 ? 2 : 3)
     k_conv3d_halo(const __nv_bfloat16 *__restrict__ x0p, const __nv_bfloat16 *__restrict__ w0p,
                   const __nv_bfloat16 *__restrict__ x1p, const __nv_bfloat16 *__restrict__ w1p, const HaloGeom g,
                   const float *__restrict__ bias, __nv_bfloat16 *__restrict__ y) {
@@ -369,8 +370,8 @@ __global__ void __launch_bounds__(kHaloThreads, COUT == 64 || ITEMS > 9 ? 2 : 3)
     unsigned char *smem = reinterpret_cast<unsigned char *>(
         (reinterpret_cast<uintptr_t>(conv_smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + g.bar_off);
-    uint64_t *done = full + kHaloMaxX + 2;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(done + kHaloMaxX + 2);
+    uint64_t *done = full + kHaloSteps;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(done + kHaloSteps);
     __shared__ int fail;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -382,12 +383,12 @@ __global__ void __launch_bounds__(kHaloThreads, COUT == 64 || ITEMS > 9 ? 2 : 3)
     t /= ty;
     const int x0 = (t % tx) * g.xr, b = t / tx;
     const int xr = min(g.xr, g.NX - x0), np = xr + 2;
-    const int nsrc = g.cin1 > 0 ? 2 : 1;
+    const int nsrc = g.cin1 > 0 ? 2 : 1, steps = nsrc * np;  // step i: plane i % np of source i / np
     const int lg0 = g.cin0 == 16 ? 1 : (g.cin0 == 32 ? 2 : 3), lg1 = g.cin1 == 16 ? 1 : (g.cin1 == 32 ? 2 : 3);
 
     if (threadIdx.x == 0) {
         fail = 0;
-        for (int p = 0; p < np; p++) {
+        for (int p = 0; p < steps; p++) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&full[p])), "r"(kConvThreads));
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&done[p])));
         }
@@ -405,38 +406,37 @@ __global__ void __launch_bounds__(kHaloThreads, COUT == 64 || ITEMS > 9 ? 2 : 3)
 
     if (warp >= 4 && warp < 8) {
         const int tid = threadIdx.x - kConvThreads;
-        // this thread's items of a plane, the same for every plane: where they
-        // come from (in 16-byte units of their source's plane; -1 outside the
-        // volume) and where they go
+        // this thread's items of a plane, the same for every plane of a source: where
+        // they come from (in 16-byte units of the plane; -1 outside the volume) and
+        // where they go
         int from[ITEMS], to[ITEMS];
-        const int n0 = kHaloRows << lg0, n1 = nsrc > 1 ? kHaloRows << lg1 : 0;
-#pragma unroll
-        for (int u = 0; u < ITEMS; u++) {
-            int q = u * kConvThreads + tid;
-            from[u] = -1;
-            to[u] = -1;
-            if (q >= n0 + n1) continue;
-            const bool second = q >= n0;
-            if (second) q -= n0;
-            const int lg = second ? lg1 : lg0, c = q & ((1 << lg) - 1);
-            const int r = q >> lg, zh = r % kHaloZ, yh = r / kHaloZ;
-            const int yy = y0 - 1 + yh, zz = z0 - 1 + zh;
-            to[u] = (second ? g.src1_off + c * g.chunk1 : c * g.chunk0) + r * 16;
-            if ((unsigned)yy < (unsigned)g.NY && (unsigned)zz < (unsigned)g.NZ)
-                from[u] = ((yy * g.NZ + zz) << lg) + c;
-        }
-        const uint4 *g0 = reinterpret_cast<const uint4 *>(x0p), *g1 = reinterpret_cast<const uint4 *>(x1p);
-        const int64_t plane = (int64_t)g.NY * g.NZ;
-        auto stage = [&](int p) {
-            const int xx = x0 - 1 + p;
-            const bool in = (unsigned)xx < (unsigned)g.NX;
-            const int64_t at = in ? ((int64_t)b * g.NX + xx) * plane : 0;
-            const uint4 *s0 = g0 + (at << lg0), *s1 = g1 + (at << lg1);
-            const uint32_t dst = smem_u32(smem) + (uint32_t)((p % g.ring) * g.slot);
+        auto map = [&](int src) {
+            const int lg = src ? lg1 : lg0, chunk = src ? g.chunk1 : g.chunk0, n = kHaloRows << lg;
 #pragma unroll
             for (int u = 0; u < ITEMS; u++) {
-                const bool first = u * kConvThreads + tid < n0, any = in && from[u] >= 0;
-                if (to[u] >= 0) copy16_async(dst + (uint32_t)to[u], (first ? s0 : s1) + (any ? from[u] : 0), any);
+                const int q = u * kConvThreads + tid;
+                from[u] = -1;
+                to[u] = -1;
+                if (q >= n) continue;
+                const int c = q & ((1 << lg) - 1), r = q >> lg, zh = r % kHaloZ, yh = r / kHaloZ;
+                const int yy = y0 - 1 + yh, zz = z0 - 1 + zh;
+                to[u] = c * chunk + r * 16;
+                if ((unsigned)yy < (unsigned)g.NY && (unsigned)zz < (unsigned)g.NZ)
+                    from[u] = ((yy * g.NZ + zz) << lg) + c;
+            }
+        };
+        const int64_t plane = (int64_t)g.NY * g.NZ;
+        auto stage = [&](int i) {
+            const int src = i >= np ? 1 : 0, xx = x0 - 1 + i - src * np;
+            if (i == 0 || i == np) map(src);
+            const bool in = (unsigned)xx < (unsigned)g.NX;
+            const int64_t at = in ? ((int64_t)b * g.NX + xx) * plane : 0;
+            const uint4 *sp = reinterpret_cast<const uint4 *>(src ? x1p : x0p) + (at << (src ? lg1 : lg0));
+            const uint32_t dst = smem_u32(smem) + (uint32_t)((i % g.ring) * g.slot);
+#pragma unroll
+            for (int u = 0; u < ITEMS; u++) {
+                const bool any = in && from[u] >= 0;
+                if (to[u] >= 0) copy16_async(dst + (uint32_t)to[u], sp + (any ? from[u] : 0), any);
             }
         };
         const int ahead = g.ring - 1;
@@ -446,16 +446,16 @@ __global__ void __launch_bounds__(kHaloThreads, COUT == 64 || ITEMS > 9 ? 2 : 3)
                 if (nsrc > 1)
                     halo_stage_weights<COUT>(reinterpret_cast<const uint4 *>(w1p), smem_u32(smem + g.w1_off), lg1, tid);
             }
-            if (p < np) stage(p);
+            if (p < steps) stage(p);
             asm volatile("cp.async.commit_group;" ::: "memory");
         }
-        for (int p = 0; p < np; p++) {
-            // plane p has landed when at most the ahead - 1 groups after its own are in flight
+        for (int p = 0; p < steps; p++) {
+            // step p has landed when at most the ahead - 1 groups after its own are in flight
             if (ahead == 3) asm volatile("cp.async.wait_group 2;" ::: "memory");
             else asm volatile("cp.async.wait_group 1;" ::: "memory");
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&full[p])) : "memory");
-            if (p + ahead < np) {
+            if (p + ahead < steps) {
                 if (p >= 1 && !mbar_wait(smem_u32(&done[p - 1]), 0)) {
                     fail = 1;
                     break;
@@ -466,7 +466,7 @@ __global__ void __launch_bounds__(kHaloThreads, COUT == 64 || ITEMS > 9 ? 2 : 3)
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
     } else if (warp < 4) {
-        // output plane o, complete with input plane o + 2: row m of its accumulator is TMEM lane m
+        // output plane o, complete with the last source's input plane o + 2: row m of its accumulator is TMEM lane m
         const int m = threadIdx.x;
         float bs[COUT <= 32 ? COUT : 1];
         if (COUT <= 32)
@@ -475,7 +475,7 @@ __global__ void __launch_bounds__(kHaloThreads, COUT == 64 || ITEMS > 9 ? 2 : 3)
         __nv_bfloat16 *yo = y + ((((int64_t)b * g.NX + x0) * g.NY + y0 + (m >> 3)) * g.NZ + z0 + (m & 7)) * COUT;
         for (int o = 0; o < xr; o++, yo += (int64_t)g.NY * g.NZ * COUT) {
             // warp-uniform outcome: tcgen05.ld is a .sync.aligned warp instruction
-            if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&done[o + 2]), 0) ? 1 : 0)) {
+            if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&done[steps - np + o + 2]), 0) ? 1 : 0)) {
                 fail = 1;
                 break;
             }
@@ -497,44 +497,40 @@ __global__ void __launch_bounds__(kHaloThreads, COUT == 64 || ITEMS > 9 ? 2 : 3)
         }
     } else {
         const uint32_t lead = elect_one();
-        // MMA issuer: per plane 9 x sources x (Cin / 16) steps of N = 3 Cout, then one commit
-        for (int p = 0; p < np; p++) {
-            if (!mbar_wait(smem_u32(&full[p]), 0)) {
+        // MMA issuer: per step 9 x (Cin / 16) MMAs of N = 3 Cout, then one commit.  For
+        // an output their order is source, dx, (dy, dz), channels, as in the tap-tile
+        // kernel, so the two round alike.
+        for (int i = 0; i < steps; i++) {
+            if (!mbar_wait(smem_u32(&full[i]), 0)) {
                 fail = 1;
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t slot = smem_u32(smem) + (uint32_t)((p % g.ring) * g.slot);
+            const int src = i >= np ? 1 : 0, p = i - src * np;
+            const uint32_t slot = smem_u32(smem) + (uint32_t)((i % g.ring) * g.slot);
             const int lo = max(0, p - 2), hi = min(p, xr - 1);  // the output planes it contributes to
             const uint32_t d = tmem + (uint32_t)(lo * COUT), idesc = mma_idesc((hi - lo + 1) * COUT);
             const uint32_t wrow = (uint32_t)((lo - (p - 2)) * COUT * 16);
-            auto mma = [&](uint32_t dd, uint64_t aa, uint64_t bb, uint32_t id, uint32_t acc) {
-                mma_if(lead, dd, aa, bb, id, acc);
-            };
-            for (int src = 0; src < nsrc; src++) {
-                const int lg = src ? lg1 : lg0, ksteps = 1 << (lg - 1);
-                const uint32_t chunk = (uint32_t)(src ? g.chunk1 : g.chunk0);
-                const uint32_t wbase = smem_u32(smem + (src ? g.w1_off : g.w0_off));
-                uint64_t a0 = ns_desc(slot + (src ? (uint32_t)g.src1_off : 0u), chunk, kHaloZ * 16);
-                uint64_t b0 = ns_desc(wbase + wrow, 3 * COUT * 16, 128);
-                const uint64_t bstep = (uint64_t)((3 * COUT) << lg);  // in 16-byte units, as the address field
-                for (int kk = 0; kk < ksteps; kk++) {
+            const int lg = src ? lg1 : lg0, ksteps = 1 << (lg - 1);
+            const uint32_t chunk = (uint32_t)(src ? g.chunk1 : g.chunk0);
+            const uint64_t a0 = ns_desc(slot, chunk, kHaloZ * 16);
+            uint64_t bd = ns_desc(smem_u32(smem + (src ? g.w1_off : g.w0_off)) + wrow, 3 * COUT * 16, 128);
+            const uint64_t astep = (uint64_t)((2 * chunk) >> 4);  // in 16-byte units, as the address field
 #pragma unroll
-                    for (int sft = 0; sft < 9; sft++) {
-                        const uint64_t ad = a0 + (uint64_t)((sft / 3) * kHaloZ + sft % 3), bd = b0 + sft * bstep;
-                        if (sft == 0 && src == 0 && kk == 0 && p < xr) {
-                            // the planes begun before, then the new one from zero
-                            if (hi > lo) mma(d, ad, bd, mma_idesc((hi - lo) * COUT), 1u);
-                            mma(tmem + (uint32_t)(p * COUT), ad, bd + (uint64_t)((hi - lo) * COUT), mma_idesc(COUT), 0u);
-                        } else {
-                            mma(d, ad, bd, idesc, 1u);
-                        }
+            for (int sft = 0; sft < 9; sft++) {
+                uint64_t ad = a0 + (uint64_t)((sft / 3) * kHaloZ + sft % 3);
+                for (int kk = 0; kk < ksteps; kk++, ad += astep, bd += (uint64_t)(2 * 3 * COUT)) {
+                    if (sft == 0 && src == 0 && kk == 0 && p < xr) {
+                        // the planes begun before, then the new one from zero
+                        if (hi > lo) mma_if(lead, d, ad, bd, mma_idesc((hi - lo) * COUT), 1u);
+                        mma_if(lead, tmem + (uint32_t)(p * COUT), ad, bd + (uint64_t)((hi - lo) * COUT),
+                               mma_idesc(COUT), 0u);
+                    } else {
+                        mma_if(lead, d, ad, bd, idesc, 1u);
                     }
-                    a0 += (uint64_t)((2 * chunk) >> 4);
-                    b0 += (uint64_t)(2 * 3 * COUT);
                 }
             }
-            commit_if(lead, smem_u32(&done[p]));
+            commit_if(lead, smem_u32(&done[i]));
         }
     }
     __syncwarp();
@@ -1060,8 +1056,8 @@ static size_t halo_layout(HaloGeom &h, int cout) {
     auto chunk = [](int cin) { return kHaloRows * 16 + (cin == 32 ? 32 : (cin == 64 ? 16 : 0)); };
     h.chunk0 = chunk(h.cin0);
     h.chunk1 = chunk(h.cin1);
-    h.src1_off = (h.cin0 >> 3) * h.chunk0;
-    h.slot = align_up(h.src1_off + (h.cin1 >> 3) * h.chunk1, 128);
+    const int plane0 = (h.cin0 >> 3) * h.chunk0, plane1 = (h.cin1 >> 3) * h.chunk1;
+    h.slot = align_up(plane0 > plane1 ? plane0 : plane1, 128);
     h.w0_off = h.ring * h.slot;
     h.w1_off = h.w0_off + 27 * cout * h.cin0 * 2;
     h.bar_off = align_up(h.w1_off + 27 * cout * h.cin1 * 2, 16);
@@ -1097,7 +1093,6 @@ static size_t halo_plan(HaloGeom &h, int cout) {
     const int nzb = h.NZ < 128 ? h.NZ : 128;
     const bool tap_ok = 128 % nzb == 0 && h.NZ % nzb == 0 && h.NY % (128 / nzb) == 0;
     if (!fx && tap_ok && tiles * h.NX < kNumSMs) return 0;
-    if (h.cin0 + h.cin1 > 96) return 0;
     HaloGeom best = h;
     size_t best_smem = 0;
     int64_t best_cost = 0;
@@ -1109,7 +1104,7 @@ static size_t halo_plan(HaloGeom &h, int cout) {
             const size_t smem = halo_layout(h, cout);
             if (smem > (size_t)kHaloSmemMax) continue;
             int occ = (int)((size_t)(228 * 1024) / (smem + 1024));
-            const int regs = cout == 64 || h.cin0 + h.cin1 > 48 ? 2 : 3;  // as the kernel's launch bounds
+            const int regs = cout == 64 || h.cin0 == 64 || h.cin1 == 64 ? 2 : 3;  // as the kernel's launch bounds
             occ = occ < regs ? occ : regs;
             occ = occ < (int)(512 / h.tmem_cols) ? occ : (int)(512 / h.tmem_cols);
             const int64_t ctas = tiles * ((h.NX + xr - 1) / xr), per_sm = (ctas + kNumSMs - 1) / kNumSMs;
@@ -1146,12 +1141,10 @@ static int launch_halo(const void *x0, const void *w0, const void *x1, const voi
 template <int COUT>
 static int launch_halo_items(const void *x0, const void *w0, const void *x1, const void *w1, const HaloGeom &h,
                              size_t smem, const float *bias, __nv_bfloat16 *y, cudaStream_t s) {
-    const int items = ((h.cin0 + h.cin1) / 8 * kHaloRows + kConvThreads - 1) / kConvThreads;
-    if (items <= 3) return launch_halo<COUT, 3>(x0, w0, x1, w1, h, smem, bias, y, s);
-    if (items <= 6) return launch_halo<COUT, 6>(x0, w0, x1, w1, h, smem, bias, y, s);
-    if (items <= 9) return launch_halo<COUT, 9>(x0, w0, x1, w1, h, smem, bias, y, s);
-    if (items <= 12) return launch_halo<COUT, 12>(x0, w0, x1, w1, h, smem, bias, y, s);
-    return launch_halo<COUT, 17>(x0, w0, x1, w1, h, smem, bias, y, s);
+    const int cin = h.cin0 > h.cin1 ? h.cin0 : h.cin1;
+    if (cin == 16) return launch_halo<COUT, 3>(x0, w0, x1, w1, h, smem, bias, y, s);
+    if (cin == 32) return launch_halo<COUT, 6>(x0, w0, x1, w1, h, smem, bias, y, s);
+    return launch_halo<COUT, 12>(x0, w0, x1, w1, h, smem, bias, y, s);
 }
 
 }  // namespace flub

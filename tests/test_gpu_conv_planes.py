@@ -35,6 +35,20 @@ def test_conv3d_planes_match_float64(case, planes, monkeypatch):
     assert float(((y - ref).abs() - 2.0 ** -8 * ref.abs()).max()) <= 2.0 ** -10 * float(ref.abs().max())
 
 
+@pytest.mark.parametrize("case", [(2, 64, 64, 64, 32, 16, 16), (1, 23, 64, 64, 16, 0, 16), (2, 32, 32, 32, 32, 0, 32)])
+def test_conv3d_planes_round_as_the_tap_tiles(case, monkeypatch):
+    """The same products in the same order per output: not a bit apart."""
+    from flub_gb300 import unet as U
+    B, X, Y, Z, c0, c1, co = case
+    g = torch.Generator(device="cuda").manual_seed(X)
+    rand = lambda *s: torch.randn(s, generator=g, device="cuda").to(torch.bfloat16)
+    args = (rand(B, X, Y, Z, c0), rand(27, co, c0), rand(B, X, Y, Z, c1) if c1 else None,
+            rand(27, co, c1) if c1 else None, torch.randn(co, generator=g, device="cuda"))
+    y = U.conv3d(*args, relu=False)
+    monkeypatch.setenv("FLUB_CONV_HALO", "0")
+    assert torch.equal(y, U.conv3d(*args, relu=False))
+
+
 @pytest.mark.parametrize("co", [16, 32, 64])
 @pytest.mark.parametrize("grid", [(1, 1, 2, 64), (1, 3, 8, 16), (2, 33, 32, 32)])
 def test_bias_gradient_matches_float64(grid, co):
