@@ -374,6 +374,8 @@ static cudaError_t coarse_launch_config(int C, size_t smem, cudaStream_t s, cuda
     return cudaSuccess;
 }
 
+static int small_levels_start(const flub_mg *mg, bool *bottom_small);
+
 // Picks the finest level whose hierarchy fits the coarse kernel: on a cluster
 // of 16 blocks, else of 8, else (no clusters, or FLUB_NO_CLUSTER=1) the levels
 // one block holds.
@@ -383,6 +385,10 @@ static int choose_coarse(flub_mg *mg) {
     mg->co_smem = 0;
     const char *off = getenv("FLUB_NO_CLUSTER");
     const bool clusters = !(off && off[0] == '1');
+    // in mixed precision not above the levels that leave FP16: this kernel's are
+    // FP32, and the V-cycle is the one that the storage types define
+    bool small;
+    const int first = mg->precision == FLUB_PRECISION_MIXED ? small_levels_start(mg, &small) : 0;
     int dev = 0, max_smem = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
@@ -398,7 +404,7 @@ static int choose_coarse(flub_mg *mg) {
     }
     for (int C : {16, 8, 1}) {
         if (C > 1 && !clusters) continue;
-        for (int l = 0; l < mg->levels; l++) {
+        for (int l = first; l < mg->levels; l++) {
             CoarseParams P;
             const size_t b = coarse_layout(mg, l, C, &P);
             if (b == 0 || b > (size_t)max_smem) continue;
