@@ -22,6 +22,7 @@
 #include "mg_kernels.cuh"
 #include "cg8.cuh"
 #include "coarse.cuh"
+#include "cg_small.cuh"
 #include "mixed.cuh"
 #include "persist.cuh"
 #include "restrict8.cuh"
@@ -110,6 +111,7 @@ struct flub_mg {
     int graph_nodes[3];
     cudaStream_t cap_stream, cap_stream2;
     bool host_loop;
+    int cg_blocks;  // blocks of the CG step in one cluster (cg_small.cuh), 0: the four kernels
     bool skip_ok;   // internal z buffers keep z = 0 off the fluid (see k_smooth8)
     bool tile_ok;   // the TMA-tiled smoother runs where a level has tiles (FLUB_TILE=1)
     bool split_ok;  // level 0 smooths on colour-split storage (smooth_split.cuh); FLUB_NO_SPLIT=1 turns it off
@@ -1351,6 +1353,71 @@ static int enqueue_second_half(flub_mg *mg, const LaunchCtx &c) {
                       c.kc);
 }
 
+// Blocks of the small CG kernels for the handle: a power of two that holds the groups with
+// one a thread, or 16 with two; 0 where it does not apply.
+static int choose_cg_small(const flub_mg *mg) {
+    const char *off = getenv("FLUB_NO_CLUSTER");
+    const bool clusters = !(off && off[0] == '1');
+    if (mg->precision != FLUB_PRECISION_FP32 || mg->nz % 8 != 0 || mg->n > kCgSmallMaxCells) return 0;
+    const int need = (int)((mg->n / 8 + kRedThreads - 1) / kRedThreads);
+    int C = 1;
+    while (C < need && C < kCgSmallMaxBlocks) C <<= 1;
+    if (C == 1) return 1;
+    if (!clusters) return 0;
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr[2];
+    coarse_launch_config(C, 0, nullptr, &cfg, attr);
+    cfg.attrs = attr + 1;  // the cluster dimension only
+    cfg.numAttrs = 1;
+    for (const void *k : {need > C ? (const void *)k_cg_small_dir<2> : (const void *)k_cg_small_dir<1>,
+                          need > C ? (const void *)k_cg_small_res<2> : (const void *)k_cg_small_res<1>}) {
+        int n = 0;
+        if (cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess || n < 1) {
+            cudaGetLastError();
+            return 0;
+        }
+    }
+    return C;
+}
+
+// The loop's body: z = M r, then the CG step up to the next loop condition.
+static int enqueue_iteration(flub_mg *mg, const LaunchCtx &c, int smoother) {
+    if (!mg->cg_blocks || smoother == FLUB_SMOOTHER_FRACTION) {
+        FLUB_TRY(enqueue_second_half(mg, c));
+        return enqueue_first_half(mg, c, smoother);
+    }
+    const Level &L0 = mg->lv[0];
+    FLUB_TRY(enqueue_vcycle(mg, c, L0.r, L0.z, true));
+    CgSmallArgs A = {};
+    A.D = L0.D;
+    A.st = mg->st;
+    A.x = mg->x;
+    A.p = mg->p;
+    A.r = L0.r;
+    A.z = L0.z;
+    A.code = L0.code;
+    A.items = L0.b_items;
+    A.sw = L0.sw;
+    A.hist = mg->hist;
+    A.h = c.h;
+    A.set_cond = c.set_cond;
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr[2];
+    coarse_launch_config(mg->cg_blocks, 0, c.s, &cfg, attr);
+    const bool two = (int64_t)mg->cg_blocks * kRedThreads * 8 < mg->n;
+    for (auto k : {two ? k_cg_small_dir<2> : k_cg_small_dir<1>, two ? k_cg_small_res<2> : k_cg_small_res<1>}) {
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, k, (const CgSmallArgs)A, c.kc);
+        if (e != cudaSuccess) {
+            set_last_error("CG step launch: %s", cudaGetErrorString(e));
+            cudaGetLastError();
+            return FLUB_ERR_CUDA;
+        }
+        count_launches(1);
+    }
+    return FLUB_OK;
+}
+
 static int enqueue_epilogue(flub_mg *mg, const LaunchCtx &c) {
     const Level &L0 = mg->lv[0];
     if ((L0.D.nz % 8) == 0)
@@ -1408,8 +1475,7 @@ static int build_graph(flub_mg *mg, int smoother, cudaGraphExec_t *out) {
         return abort_capture((set_last_error("cudaStreamBeginCaptureToGraph: %s", cudaGetErrorString(e)),
                               FLUB_ERR_CUDA));
     LaunchCtx c2{s2, kernel_counter(mg), h, 1};
-    rc = enqueue_second_half(mg, c2);
-    if (!rc) rc = enqueue_first_half(mg, c2, smoother);
+    rc = enqueue_iteration(mg, c2, smoother);
     cudaGraph_t body_out = nullptr;
     e = cudaStreamEndCapture(s2, &body_out);
     if (rc || e != cudaSuccess) {
@@ -1664,6 +1730,7 @@ int flub_mg_create(int nx, int ny, int nz, int levels, int precision, void *work
     mg->skip_ok = true;  // the workspace is zeroed below and set_tags re-zeroes the z buffers
     choose_coarse(mg);
     choose_persist(mg);
+    mg->cg_blocks = choose_cg_small(mg);
     if (precision == FLUB_PRECISION_MIXED && bottom_in_tail(mg)) {
         // mixed precision: FP64 at the coarsest level (the layout grows by the
         // bottom's doubles, so it is chosen again)
@@ -1879,8 +1946,7 @@ int flub_mg_solve(flub_mg *mg, int max_iters, double eps, double abs_tol, double
             FLUB_CHECK_CUDA(cudaMemcpyAsync(&h, mg->st, sizeof(MgState), cudaMemcpyDeviceToHost, s));
             FLUB_CHECK_CUDA(cudaStreamSynchronize(s));
             if (!h.cond) break;
-            FLUB_TRY(enqueue_second_half(mg, c));
-            FLUB_TRY(enqueue_first_half(mg, c, smoother));
+            FLUB_TRY(enqueue_iteration(mg, c, smoother));
         }
         FLUB_TRY(enqueue_epilogue(mg, c));
     } else {
