@@ -75,6 +75,7 @@ struct CoarseLevel {
     int off_w;           // and: the cells' weights (natural order)
     int hn;              // floats per half of z
     uint32_t div_seg, div_ny, div_nz;  // for coarse_div by nz / 2 / V, ny and nz
+    int half;            // a level that the storage types define as FP16 (see coarse_level)
     const uint16_t *cw;  // stencil words of the level, natural order
 };
 
@@ -329,13 +330,16 @@ __device__ __forceinline__ void coarse_residual(const CoarseItem<V> &t, const fl
     }
 }
 
+// A value as FP16 storage holds it.
+__device__ __forceinline__ float half_stored(float v) { return __half2float(__float2half_rn(v)); }
+
 // z += (r + L z) / d on the item's cells of colour COL, the quotient by
 // Markstein's FMA correction with y = -1/d: q0 = a y, -q = q0 + (a + d q0) y.
 // For d = 1..6 that is IEEE a / d for every finite a but ties between two
 // denormals at d = 6 (tests/test_coarse_div.py checks all 2^32 values), so it
 // needs no guard; a branch here cost 100 ns of a 350 ns half-sweep.  A cell
 // that is never updated has y = d = 0: its z stays 0.
-template <int V, int COL, bool kKeep>
+template <int V, int COL, bool kKeep, bool kHalf>
 __device__ __forceinline__ void coarse_half(CoarseItem<V> &t, float *zs, int hn, int ps, int rs) {
     constexpr int h = V > 1 ? 1 : 0;
     float a[V];
@@ -347,6 +351,9 @@ __device__ __forceinline__ void coarse_half(CoarseItem<V> &t, float *zs, int hn,
         f2_get(f2_sub(f2(t.z[COL][m], t.z[COL][m + h]), f2_fma(f2_fma(q0, d, aa), y, q0)), t.z[COL][m],
                t.z[COL][m + h]);
     }
+    if (kHalf)
+#pragma unroll
+        for (int m = 0; m < V; m++) t.z[COL][m] = half_stored(t.z[COL][m]);
     st_vec<V>(zs + COL * hn + t.o, t.z[COL]);
 }
 
@@ -530,7 +537,13 @@ __device__ __forceinline__ CoarseWeights coarse_weights(uint32_t w, int odd_k) {
 // sweeps; 512 threads of 128 hold the same cells and were slower (16^3 full of
 // fluid in one block 0.41 against 0.36 us a half-sweep, 8^3 0.19 against 0.12,
 // 32^3 on 16 blocks 0.54 against 0.41).
-template <int V, bool kWide>
+//
+// kHalf: a level of a mixed-precision V-cycle that is FP16 at scale 8^-l
+// (mixed.cuh).  Its values are held as floats, rounded where the level-by-level
+// sweeps store them -- every update, the colour that the first half-sweep after
+// the prolongation read unrounded, the coarse residual -- with the same scales
+// between levels, so the V-cycle is bit-identical.
+template <int V, bool kWide, bool kHalf = false>
 __device__ __noinline__ CoarseSync coarse_level(const CoarseParams &P, int t, int mode, unsigned char *smem,
                                                 unsigned rank, CoarseSync S) {
     constexpr int Q = (kWide ? 8 : 4) / V;  // items per thread
@@ -639,6 +652,7 @@ __device__ __noinline__ CoarseSync coarse_level(const CoarseParams &P, int t, in
             for (int m = 0; m < V; m++) {
                 const int K = V * kg + m;
                 add[m] = pc[((I + J + K) & 1) * chn + (K >> 1)];
+                if (kHalf) add[m] = __fmul_rn(half_stored(add[m]), 8.0f);
             }
 #pragma unroll
             for (int c = 0; c < 2; c++) {
@@ -660,7 +674,7 @@ __device__ __noinline__ CoarseSync coarse_level(const CoarseParams &P, int t, in
         constexpr int COL = decltype(col)::value;
 #pragma unroll
         for (int s = 0; s < Q; s++)
-            if (it[s].on) coarse_half<V, COL, kKeep>(it[s], zs, hn, ps, hz);
+            if (it[s].on) coarse_half<V, COL, kKeep, kHalf>(it[s], zs, hn, ps, hz);
         if (dist) {
             exchange_open(S, ghost);
 #pragma unroll
@@ -679,8 +693,13 @@ __device__ __noinline__ CoarseSync coarse_level(const CoarseParams &P, int t, in
             bool skip = even_first;
             for (int n = mode == kCoarseBottom ? P.nbottom : iters; n > 0; n--) {
                 if (!skip) half(std::integral_constant<int, 1>{});
-                skip = false;
                 half(std::integral_constant<int, 0>{});
+                if (kHalf && skip && mode == kCoarseUp)
+#pragma unroll
+                    for (int s = 0; s < Q; s++)
+#pragma unroll
+                        for (int m = 0; m < V; m++) it[s].z[1][m] = half_stored(it[s].z[1][m]);
+                skip = false;
             }
             if (even_first) half(std::integral_constant<int, 1>{});
         }
@@ -729,7 +748,7 @@ __device__ __noinline__ CoarseSync coarse_level(const CoarseParams &P, int t, in
                 s = __fadd_rn(s, vc[si + 1]);
                 s = __fadd_rn(s, vc[si + sj]);
                 s = __fadd_rn(s, vc[si + sj + 1]);
-                s = __fmul_rn(s, P.rscale);
+                s = kHalf ? half_stored(__fmul_rn(s, 0.125f * P.rscale)) : __fmul_rn(s, P.rscale);
             }
             if (remote)
                 remote_store(remote_addr(Rc + g, 0), s);
@@ -744,10 +763,11 @@ __device__ __noinline__ CoarseSync coarse_level(const CoarseParams &P, int t, in
     return S;
 }
 
-template <int kV>
+template <int kV, bool kMixed>
 __device__ __forceinline__ CoarseSync coarse_dispatch(const CoarseParams &P, int t, int mode, unsigned char *smem,
                                                       unsigned rank, CoarseSync S) {
     const int V = kV ? kV : P.lv[t].V;
+    if (kMixed && P.lv[t].half) return coarse_level<4, true, true>(P, t, mode, smem, rank, S);  // rows of 8 cells
     if (V == 4) {
         if (P.lv[t].P * P.lv[t].D.ny * P.lv[t].D.nz > 8 * kCoarseThreads)
             return coarse_level<kV ? kV : 4, true>(P, t, mode, smem, rank, S);
@@ -759,8 +779,8 @@ __device__ __forceinline__ CoarseSync coarse_dispatch(const CoarseParams &P, int
 
 // Grid: one cluster (P.nd > 0), or one block.  kV = 4: every level has V = 4 (nz a
 // multiple of 8 down to the bottom); the general kernel also holds the code
-// for shorter items, which costs it registers.
-template <int kV>
+// for shorter items, which costs it registers.  kMixed: there are levels of kind half.
+template <int kV, bool kMixed>
 __global__ void __launch_bounds__(kCoarseThreads, 1) k_coarse_vcycle(const __grid_constant__ CoarseParams P,
                                                                      unsigned long long *kc) {
     extern __shared__ __align__(16) unsigned char coarse_smem[];
@@ -847,7 +867,7 @@ __global__ void __launch_bounds__(kCoarseThreads, 1) k_coarse_vcycle(const __gri
         if (t < P.nd) {
             // block 0 has finished the levels below
             if (mode == kCoarseUp && t == P.nd - 1 && P.nd < P.nl) cluster_barrier();
-            S = coarse_dispatch<kV>(P, t, mode, smem, rank, S);
+            S = coarse_dispatch<kV, kMixed>(P, t, mode, smem, rank, S);
         } else if (rank == 0) {
             if (mode == kCoarseBottom && P.bottom64)
                 coarse_bottom64(reinterpret_cast<double *>(smem + P.off_zd),
@@ -855,7 +875,7 @@ __global__ void __launch_bounds__(kCoarseThreads, 1) k_coarse_vcycle(const __gri
                                 reinterpret_cast<const float *>(smem + P.lv[t].off_r), P.lv[t].hn, P.lv[t].cw,
                                 P.lv[t].D, P.nbottom);
             else
-                S = coarse_dispatch<kV>(P, t, mode, smem, 0u, S);
+                S = coarse_dispatch<kV, kMixed>(P, t, mode, smem, 0u, S);
         }
     }
     // the first level's correction in natural order

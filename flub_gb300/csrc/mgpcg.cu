@@ -280,6 +280,8 @@ static size_t carve(flub_mg *mg, char *base) {
 
 static inline bool is_pow2(int v) { return v > 0 && (v & (v - 1)) == 0; }
 
+static int small_levels_start(const flub_mg *mg, bool *bottom_small);
+
 // Layout of the coarse kernel from level lc down on a cluster of C blocks;
 // returns the bytes of shared memory per block, 0 if the levels do not qualify.
 //
@@ -319,10 +321,16 @@ static size_t coarse_layout(const flub_mg *mg, int lc, int C, CoarseParams *P) {
     };
     P->nl = mg->levels - lc;
     P->nd = nd;
+    // the levels that the storage types define as FP16 are rows of 8 cells
+    bool small;
+    const int fp16_end = mg->precision == FLUB_PRECISION_MIXED ? small_levels_start(mg, &small) : 0;
+    for (int l = lc; l < fp16_end; l++)
+        if (l >= mg->levels || dims(l).nz % 8 != 0) return 0;
     for (int t = 0; t < P->nl; t++) {
         CoarseLevel &L = P->lv[t];
         L.D = dims(lc + t);
         L.abs_level = lc + t;
+        L.half = lc + t < fp16_end ? 1 : 0;
         L.P = t < nd ? p0 >> t : L.D.nx;
         const int hz = L.D.nz >> 1;
         L.V = row_vector(L.D.nz);
@@ -352,10 +360,11 @@ static size_t coarse_layout(const flub_mg *mg, int lc, int C, CoarseParams *P) {
 }
 
 // The kernel for this layout.
-static decltype(&k_coarse_vcycle<4>) coarse_kernel(const CoarseParams &P) {
+static decltype(&k_coarse_vcycle<4, false>) coarse_kernel(const CoarseParams &P) {
+    const bool mixed = P.lv[0].half != 0;
     for (int t = 0; t < P.nl; t++)
-        if (P.lv[t].V != 4) return k_coarse_vcycle<0>;
-    return k_coarse_vcycle<4>;
+        if (P.lv[t].V != 4) return mixed ? k_coarse_vcycle<0, true> : k_coarse_vcycle<0, false>;
+    return mixed ? k_coarse_vcycle<4, true> : k_coarse_vcycle<4, false>;
 }
 
 static cudaError_t coarse_launch_config(int C, size_t smem, cudaStream_t s, cudaLaunchConfig_t *cfg,
@@ -376,8 +385,6 @@ static cudaError_t coarse_launch_config(int C, size_t smem, cudaStream_t s, cuda
     return cudaSuccess;
 }
 
-static int small_levels_start(const flub_mg *mg, bool *bottom_small);
-
 // Picks the finest level whose hierarchy fits the coarse kernel: on a cluster
 // of 16 blocks, else of 8, else (no clusters, or FLUB_NO_CLUSTER=1) the levels
 // one block holds.
@@ -387,23 +394,28 @@ static int choose_coarse(flub_mg *mg) {
     mg->co_smem = 0;
     const char *off = getenv("FLUB_NO_CLUSTER");
     const bool clusters = !(off && off[0] == '1');
-    // in mixed precision not above the levels that leave FP16: this kernel's are
-    // FP32, and the V-cycle is the one that the storage types define
-    bool small;
-    const int first = mg->precision == FLUB_PRECISION_MIXED ? small_levels_start(mg, &small) : 0;
+    // in mixed precision level 0 has other storage before and after the coarse
+    // correction: below it at the earliest, unless all levels have left FP16.
+    // FLUB_COARSE_FP16=0 leaves every FP16 level to the level-by-level sweeps.
+    int first = 0;
+    if (mg->precision == FLUB_PRECISION_MIXED) {
+        bool small;
+        const char *fp16 = getenv("FLUB_COARSE_FP16");
+        const int end = small_levels_start(mg, &small);
+        first = end > 0 && !(fp16 && fp16[0] == '0') ? 1 : end;
+    }
     int dev = 0, max_smem = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
-        cudaFuncSetAttribute(k_coarse_vcycle<4>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
-        cudaFuncSetAttribute(k_coarse_vcycle<0>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
-            cudaSuccess ||
-        cudaFuncSetAttribute(k_coarse_vcycle<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem) !=
-            cudaSuccess ||
-        cudaFuncSetAttribute(k_coarse_vcycle<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem) !=
-            cudaSuccess) {
+        cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) {
         cudaGetLastError();
         return FLUB_OK;
     }
+    for (auto k : {k_coarse_vcycle<4, false>, k_coarse_vcycle<0, false>, k_coarse_vcycle<4, true>, k_coarse_vcycle<0, true>})
+        if (cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+            cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem) != cudaSuccess) {
+            cudaGetLastError();
+            return FLUB_OK;
+        }
     for (int C : {16, 8, 1}) {
         if (C > 1 && !clusters) continue;
         for (int l = first; l < mg->levels; l++) {

@@ -110,3 +110,24 @@ def test_split_arrays_16_byte_aligned(precision):
     ro.copy_(rd)
     assert ro.data_ptr() % 32 == 16 and zo.data_ptr() % 32 == 16
     assert torch.equal(mg.apply_preconditioner(ro, zo), mg.apply_preconditioner(rd))
+
+
+@pytest.mark.parametrize("nu", [1, 2, 5])
+@pytest.mark.parametrize("shape,levels", [((88, 64, 64), 4), ((176, 128, 128), 5), ((48, 48, 64), 3), ((64, 64, 32), 2),
+                                          ((40, 64, 128), 3)])
+def test_fp16_levels_in_the_coarse_kernel(shape, levels, nu, monkeypatch):
+    """Small FP16 levels run in the coarse kernel with every value rounded where
+    the level-by-level sweeps store it: the same bits."""
+    tag, r = _case(shape, sum(shape), 0.05)
+    rd = torch.from_numpy(r).cuda()
+    z = []
+    for on in ("0", "1"):
+        monkeypatch.setenv("FLUB_COARSE_FP16", on)
+        mg = MGPCG(3, shape, levels, float, precision="mixed")
+        mg.set_tags(torch.from_numpy(tag).cuda())
+        mg.set_schedule(nu, 3, 0.5)
+        mg.init(rd, 1.0)
+        mg.solve(max_iters=3, eps=1e-12, abs_tol=1e-12, rel_tol=1e-12, smoother="phases")
+        z.append((mg.apply_preconditioner(rd).cpu().numpy(), mg.x.cpu().numpy()))
+    assert np.isfinite(z[0][1]).all()
+    assert np.array_equal(z[0][0], z[1][0]) and np.array_equal(z[0][1], z[1][1])
