@@ -162,7 +162,8 @@ static inline int block_tiles(const Dims D, int ti) {
 // Not above 256 tiles either: a tile takes 6 us for four half-sweeps (13,000
 // cycles: 3,000 to load, 7,000 of sweeps bound by shared-memory bandwidth), so
 // on a larger level, full of fluid, waves of them take longer than four
-// launches over all of it (128^3, 1024 tiles: 13 us a half-sweep against 6.1).
+// launches over all of it (128^3, 1024 tiles: 13 us a half-sweep against 3.3 on
+// colour-split storage).
 static int block_planes(const flub_mg *mg, int l) {
     const Dims D{mg->nx >> l, mg->ny >> l, mg->nz >> l};
     if (mg->tile_ok || D.n() <= kBlockCells || D.n() >= (int64_t)1 << 30 || D.nz % 2 != 0) return 0;
@@ -176,7 +177,7 @@ static int block_planes(const flub_mg *mg, int l) {
 // Whether level l has the buffers for smoothing on colour-split storage
 // (smooth_split.cuh): level 0, and the levels below it that are too large for
 // the coarse kernel and for tiles of one wave.  At 128^3 a half-sweep of the
-// dam break / a full grid takes 1.9 / 3.7 us on them, against 3.0 / 6.7 in
+// dam break / a full grid takes 1.9 / 3.3 us on them, against 3.0 / 6.7 in
 // natural order; a level of 64^3 takes 1.25 / 1.2 in tiles.
 static bool split_level(const flub_mg *mg, int l) {
     const Dims D{mg->nx >> l, mg->ny >> l, mg->nz >> l};

@@ -10,7 +10,7 @@
 //   k_vcycle_down  pre-smoothing of each level (the first half-sweep from
 //                  zero), then its residual + restriction into the next level
 //                  (the restriction out of l1-1 writes the first coarse level,
-//                  which the cluster / tail kernel takes over);
+//                  which the coarse kernel takes over);
 //   k_vcycle_up    from level l1-1 up to l0: the first post-smoothing half-sweep
 //                  fused with the prolongation of the coarser correction, then
 //                  the remaining half-sweeps.

@@ -32,7 +32,7 @@
 // has such an item.  With the item word only items next to a solid load their
 // stencil words; the prolongation, which adds the correction to air as well, does
 // so next to air too.
-// A half-sweep of 128^3 (FP32, dam break / full): 1.9 / 3.7 us, in natural order
+// A half-sweep of 128^3 (FP32, dam break / full): 1.9 / 3.3 us, in natural order
 // 3.0 / 6.7.  Measured through a whole solve (before -> now): 128^3 sphere in mixed
 // precision 8536 -> 7859 us, 256^3 dam break 15880 -> 15310, 256 x 64 x 256
 // 3951 -> 3733, 104 x 72 x 88 2296 -> 2141.

@@ -368,7 +368,7 @@ int flub_mg_set_schedule(flub_mg *mg, int smooth_iters, int bottom_iters, float 
  * reference smooths its coarsest level in FP32, multigrid/mgpcg.py:319-336):
  * bits = 32, or 64 -- the bottom's red-black sweeps in FP64 on the FP32
  * restricted residual, the result rounded to FP32 once for the prolongation.
- * FP64 needs the bottom inside the one-block tail of the coarse-level kernels
+ * FP64 needs the bottom in the one block of the coarse-level kernel
  * (FLUB_ERR_UNSUPPORTED otherwise).  Handles created with
  * FLUB_PRECISION_MIXED start at 64, FP32 handles at 32 (the reference's
  * arithmetic).  Synchronises the device when the setting changes (the
