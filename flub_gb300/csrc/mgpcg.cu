@@ -322,11 +322,12 @@ static size_t coarse_layout(const flub_mg *mg, int lc, int C, CoarseParams *P) {
     };
     P->nl = mg->levels - lc;
     P->nd = nd;
-    // the levels that the storage types define as FP16 are rows of 8 cells
+    // with levels that the storage types define as FP16 every level has rows of 8
+    // cells (one more kernel for other bottoms would be a quarter of this file's code)
     bool small;
     const int fp16_end = mg->precision == FLUB_PRECISION_MIXED ? small_levels_start(mg, &small) : 0;
-    for (int l = lc; l < fp16_end; l++)
-        if (l >= mg->levels || dims(l).nz % 8 != 0) return 0;
+    for (int l = lc; lc < fp16_end && l < mg->levels; l++)
+        if (dims(l).nz % 8 != 0) return 0;
     for (int t = 0; t < P->nl; t++) {
         CoarseLevel &L = P->lv[t];
         L.D = dims(lc + t);
@@ -364,7 +365,7 @@ static size_t coarse_layout(const flub_mg *mg, int lc, int C, CoarseParams *P) {
 static decltype(&k_coarse_vcycle<4, false>) coarse_kernel(const CoarseParams &P) {
     const bool mixed = P.lv[0].half != 0;
     for (int t = 0; t < P.nl; t++)
-        if (P.lv[t].V != 4) return mixed ? k_coarse_vcycle<0, true> : k_coarse_vcycle<0, false>;
+        if (P.lv[t].V != 4) return k_coarse_vcycle<0, false>;
     return mixed ? k_coarse_vcycle<4, true> : k_coarse_vcycle<4, false>;
 }
 
@@ -411,7 +412,7 @@ static int choose_coarse(flub_mg *mg) {
         cudaGetLastError();
         return FLUB_OK;
     }
-    for (auto k : {k_coarse_vcycle<4, false>, k_coarse_vcycle<0, false>, k_coarse_vcycle<4, true>, k_coarse_vcycle<0, true>})
+    for (auto k : {k_coarse_vcycle<4, false>, k_coarse_vcycle<0, false>, k_coarse_vcycle<4, true>})
         if (cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
             cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem) != cudaSuccess) {
             cudaGetLastError();
