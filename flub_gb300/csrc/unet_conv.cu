@@ -1087,37 +1087,43 @@ static int forced_xr() {
 // loads in half of that again.  So the shortest is the least CTAs per SM x
 // (xr + 3), half as much again without overlap.
 static size_t halo_plan(HaloGeom &h, int cout) {
-    if (h.NZ % 8 || h.NY % 16 || !halo_enabled()) return 0;
+    if (h.NZ % 8 || h.NY % 16) return 0;
     const int64_t tiles = (int64_t)h.B * (h.NY / 16) * (h.NZ / 8);
-    const int fx = forced_xr() < h.NX ? forced_xr() : h.NX;
+    // before anything else what rules the layer out: this runs on every call
+    h.xr = 1;
+    h.ring = 3;
+    if (halo_layout(h, cout) > (size_t)kHaloSmemMax || !halo_enabled()) return 0;
+    const int forced = forced_xr(), fx = forced < h.NX ? forced : h.NX;
     const int nzb = h.NZ < 128 ? h.NZ : 128;
     const bool tap_ok = 128 % nzb == 0 && h.NZ % nzb == 0 && h.NY % (128 / nzb) == 0;
     if (!fx && tap_ok && tiles * h.NX < kNumSMs) return 0;
-    HaloGeom best = h;
-    size_t best_smem = 0;
+    h.ring = 4;
+    size_t smem = halo_layout(h, cout);  // of any xr
+    if (smem > (size_t)kHaloSmemMax) {
+        h.ring = 3;
+        smem = halo_layout(h, cout);
+    }
+    const int fit = (int)((size_t)(228 * 1024) / (smem + 1024));
+    const int regs = cout == 64 || h.cin0 == 64 || h.cin1 == 64 ? 2 : 3;  // as the kernel's launch bounds
+    int best = 0;
     int64_t best_cost = 0;
-    for (int xr = kHaloMaxX < h.NX ? kHaloMaxX : h.NX; xr >= 1; xr--) {
-        if ((fx && xr != fx) || xr * cout > 256) continue;
-        for (int ring = 4; ring >= 3; ring--) {
-            h.xr = xr;
-            h.ring = ring;
-            const size_t smem = halo_layout(h, cout);
-            if (smem > (size_t)kHaloSmemMax) continue;
-            int occ = (int)((size_t)(228 * 1024) / (smem + 1024));
-            const int regs = cout == 64 || h.cin0 == 64 || h.cin1 == 64 ? 2 : 3;  // as the kernel's launch bounds
-            occ = occ < regs ? occ : regs;
-            occ = occ < (int)(512 / h.tmem_cols) ? occ : (int)(512 / h.tmem_cols);
-            const int64_t ctas = tiles * ((h.NX + xr - 1) / xr), per_sm = (ctas + kNumSMs - 1) / kNumSMs;
-            const int64_t cost = per_sm * (xr + 3) * (occ == 1 || per_sm == 1 ? 3 : 2);
-            if (!best_smem || cost < best_cost) {
-                best = h;
-                best_smem = smem;
-                best_cost = cost;
-            }
+    const int top = 256 / cout < kHaloMaxX ? 256 / cout : kHaloMaxX;
+    for (int xr = top < h.NX ? top : h.NX; xr >= 1; xr--) {
+        if (fx && xr != fx) continue;
+        int cols = 32;
+        while (cols < xr * cout) cols <<= 1;
+        int occ = fit < regs ? fit : regs;
+        occ = occ < 512 / cols ? occ : 512 / cols;
+        const int64_t ctas = tiles * ((h.NX + xr - 1) / xr), per_sm = (ctas + kNumSMs - 1) / kNumSMs;
+        const int64_t cost = per_sm * (xr + 3) * (occ == 1 || per_sm == 1 ? 3 : 2);
+        if (!best || cost < best_cost) {
+            best = xr;
+            best_cost = cost;
         }
     }
-    h = best;
-    return best_smem;
+    if (!best) return 0;
+    h.xr = best;
+    return halo_layout(h, cout);
 }
 
 template <int COUT, int ITEMS>
