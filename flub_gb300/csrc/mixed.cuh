@@ -16,59 +16,6 @@
 
 namespace flub {
 
-// Residual + restriction (mgpcg.py:94-101, gather form) between stored levels:
-// r_c = out_scale * sum over children of (r_f + L z_f).
-template <typename TRI, typename TZI, typename TRO>
-__global__ void __launch_bounds__(256) k_restrict_t(const TRI *__restrict__ rf, const TZI *__restrict__ zf,
-                                                    const uint8_t *__restrict__ cf, TRO *__restrict__ rc,
-                                                    const uint8_t *__restrict__ cc, Dims C, float out_scale,
-                                                    unsigned long long *kc) {
-    count_kernel(kc);
-    const Dims F{2 * C.nx, 2 * C.ny, 2 * C.nz};
-    const int n = (int)C.n();
-    const int si = F.ny * F.nz, sj = F.nz;
-    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
-        if (cc[q] != kCodeFluid) {
-            St<TRO>::st(rc + q, 0.0f);
-            continue;
-        }
-        const int K = q % C.nz, J = (q / C.nz) % C.ny, I = q / (C.nz * C.ny);
-        float s = 0.0f;
-        bool first = true;
-#pragma unroll
-        for (int ii = 0; ii < 2; ii++)
-#pragma unroll
-            for (int jj = 0; jj < 2; jj++)
-#pragma unroll
-                for (int kk = 0; kk < 2; kk++) {
-                    const int i = 2 * I + ii, j = 2 * J + jj, k = 2 * K + kk;
-                    const int c = (i * F.ny + j) * F.nz + k;
-                    float lz = 0.0f;
-                    if (cf[c] == kCodeFluid) {
-                        const float xc = St<TZI>::ld_ro(zf + c);
-                        float tp, tm;
-                        uint8_t cn;
-                        tp = 0.0f; tm = 0.0f;
-                        if (i + 1 < F.nx) { cn = cf[c + si]; if (cn != kCodeSolid) tp = __fsub_rn(cn == kCodeAir ? 0.0f : St<TZI>::ld_ro(zf + c + si), xc); }
-                        if (i > 0)        { cn = cf[c - si]; if (cn != kCodeSolid) tm = __fsub_rn(cn == kCodeAir ? 0.0f : St<TZI>::ld_ro(zf + c - si), xc); }
-                        lz = __fadd_rn(lz, __fadd_rn(tp, tm));
-                        tp = 0.0f; tm = 0.0f;
-                        if (j + 1 < F.ny) { cn = cf[c + sj]; if (cn != kCodeSolid) tp = __fsub_rn(cn == kCodeAir ? 0.0f : St<TZI>::ld_ro(zf + c + sj), xc); }
-                        if (j > 0)        { cn = cf[c - sj]; if (cn != kCodeSolid) tm = __fsub_rn(cn == kCodeAir ? 0.0f : St<TZI>::ld_ro(zf + c - sj), xc); }
-                        lz = __fadd_rn(lz, __fadd_rn(tp, tm));
-                        tp = 0.0f; tm = 0.0f;
-                        if (k + 1 < F.nz) { cn = cf[c + 1]; if (cn != kCodeSolid) tp = __fsub_rn(cn == kCodeAir ? 0.0f : St<TZI>::ld_ro(zf + c + 1), xc); }
-                        if (k > 0)        { cn = cf[c - 1]; if (cn != kCodeSolid) tm = __fsub_rn(cn == kCodeAir ? 0.0f : St<TZI>::ld_ro(zf + c - 1), xc); }
-                        lz = __fadd_rn(lz, __fadd_rn(tp, tm));
-                    }
-                    const float v = __fadd_rn(St<TRI>::ld_ro(rf + c), lz);
-                    s = first ? v : __fadd_rn(s, v);
-                    first = false;
-                }
-        St<TRO>::st(rc + q, __fmul_rn(s, out_scale));
-    }
-}
-
 // FP16 copy of the level-0 residual for the V-cycle (every group).  With a
 // solver state, the copy is r / zscale with zscale a power of two near the
 // RMS of r (fp16_residual_scale), recorded in st->zscale; without one
