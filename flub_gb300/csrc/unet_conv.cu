@@ -13,7 +13,7 @@
 // A second source (the skip connection of a U-Net decoder) is accumulated
 // into the same tile, so a concatenation is never materialised.
 //
-// Roles (128 threads): thread 0 issues TMA loads into a 4-stage ring, thread 32
+// Roles (128 threads): thread 0 issues TMA loads into a 4-stage ring, warp 1
 // issues the MMAs (one per 16 input channels), all four warps run the
 // epilogue (TMEM -> registers, bias, ReLU, BF16 store).  Every mbarrier wait
 // is bounded; a timeout sets the error word and the CTA still frees its TMEM.
@@ -122,6 +122,40 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float v[16]) {
     for (int q = 0; q < 16; q++) v[q] = __uint_as_float(r[q]);
 }
 
+// One lane of a converged warp.  The MMA warps run their loops with all lanes and
+// predicate only the instruction: in a branch of one lane the descriptors, which
+// the instruction takes from uniform registers, were moved there one by one.
+// k_conv3d_tc, 4 x 32^3, 64 + 32 -> 32 channels: 86.7 us -> 72.4; 16^3, 32 -> 64:
+// 17 -> 15.  k_conv3d_wgrad_tc, bound by its copies, is as fast as before.
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t lead;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(lead));
+    return lead;
+}
+
+// The wait of such a warp: no lane goes on, and so no slot is handed back and
+// refilled, before every lane has seen the phase; one left behind could find the
+// barrier's parity come round again.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity) ? 1 : 0) != 0;
+}
+
+__device__ __forceinline__ void mma_if(uint32_t lead, uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
+        "l"(a), "l"(b), "r"(idesc), "r"(acc), "r"(lead));
+}
+
+__device__ __forceinline__ void commit_if(uint32_t lead, uint32_t bar) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar),
+        "r"(lead)
+        : "memory");
+}
+
 template <int COUT>
 __global__ void __launch_bounds__(kConvThreads, 1)
     k_conv3d_tc(const __grid_constant__ CUtensorMap mx0, const __grid_constant__ CUtensorMap mw0,
@@ -187,13 +221,13 @@ __global__ void __launch_bounds__(kConvThreads, 1)
             tma_load_5d(a, src ? &mx1 : &mx0, 0, z0 + dz, y0 + dy, x + dx, b, fb);
             tma_load_2d(w, src ? &mw1 : &mw0, 0, tap * COUT, fb);
         }
-    } else if (threadIdx.x == 32) {
+    } else if (warp == 1) {
         // MMA issuer
-        const uint32_t idesc = mma_idesc(COUT);
+        const uint32_t lead = elect_one(), idesc = mma_idesc(COUT);
         bool ok = true;
         for (int it = 0; it < T && ok; it++) {
             const int s = it % kConvStages, u = it / kConvStages;
-            if (!mbar_wait(smem_u32(&full[s]), u & 1)) {
+            if (!mbar_wait_warp(smem_u32(&full[s]), u & 1)) {
                 ok = false;
                 fail = 1;
                 break;
@@ -204,18 +238,11 @@ __global__ void __launch_bounds__(kConvThreads, 1)
             for (int kk = 0; kk < cin / 16; kk++) {
                 const uint64_t ad = sw_desc(a + kk * 32, cin * 2), bd = sw_desc(w + kk * 32, cin * 2);
                 const uint32_t acc = (it > 0 || kk > 0) ? 1u : 0u;
-                asm volatile(
-                    "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
-                    "l"(ad), "l"(bd), "r"(idesc), "r"(acc));
+                mma_if(lead, tmem, ad, bd, idesc, acc);
             }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                smem_u32(&empty[s]))
-                         : "memory");
+            commit_if(lead, smem_u32(&empty[s]));
         }
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-            smem_u32(done))
-                     : "memory");
+        commit_if(lead, smem_u32(done));
     }
     __syncwarp();
     // epilogue: row m of the accumulator is TMEM lane m, owned by warp m / 32
@@ -317,31 +344,6 @@ __device__ __forceinline__ void copy16_async(uint32_t dst, const void *src, bool
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(__cvta_generic_to_global(src)),
                  "r"(in ? 16 : 0)
                  : "memory");
-}
-
-// One lane of a converged warp.  The MMA warps run their loops with all lanes and
-// predicate only the instruction: in a branch of one lane the descriptors, which
-// the instruction takes from uniform registers, were moved there one by one.
-__device__ __forceinline__ uint32_t elect_one() {
-    uint32_t lead;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(lead));
-    return lead;
-}
-
-__device__ __forceinline__ void mma_if(uint32_t lead, uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
-        "l"(a), "l"(b), "r"(idesc), "r"(acc), "r"(lead));
-}
-
-__device__ __forceinline__ void commit_if(uint32_t lead, uint32_t bar) {
-    asm volatile(
-        "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
-        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar),
-        "r"(lead)
-        : "memory");
 }
 
 // Stages weights [27][COUT][Cin] (Cin = 8 << c8_log2) as
@@ -501,7 +503,7 @@ __global__ void __launch_bounds__(kHaloThreads, COUT == 64 || ITEMS > 6 ? 2 : 3)
         // an output their order is source, dx, (dy, dz), channels, as in the tap-tile
         // kernel, so the two round alike.
         for (int i = 0; i < steps; i++) {
-            if (!mbar_wait(smem_u32(&full[i]), 0)) {
+            if (!mbar_wait_warp(smem_u32(&full[i]), 0)) {
                 fail = 1;
                 break;
             }
@@ -662,11 +664,12 @@ __global__ void __launch_bounds__(kConvThreads, 1)
             }
             tma_load_5d(a + kWgA, &mdy, 0, z0, y0, x, b, fb);
         }
-    } else if (threadIdx.x == 32) {
+    } else if (warp == 1) {
+        const uint32_t lead = elect_one();
         const uint32_t idesc = mma_idesc(COUT) | (1u << 15) | (1u << 16);  // A and B MN-major
         for (int it = 0; it < T; it++) {
             const int s = it % kWgStages, u = it / kWgStages;
-            if (!mbar_wait(smem_u32(&full[s]), u & 1)) {
+            if (!mbar_wait_warp(smem_u32(&full[s]), u & 1)) {
                 fail = 1;
                 break;
             }
@@ -678,18 +681,11 @@ __global__ void __launch_bounds__(kConvThreads, 1)
                 const uint64_t ad = sw_desc_mn(a + kk * 16 * CIN * 2, CIN * 2, TILE_A);
                 const uint64_t bd = sw_desc_mn(bb + kk * 16 * COUT * 2, COUT * 2, TILE_B);
                 const uint32_t acc = (it >= ng || kk > 0) ? 1u : 0u;
-                asm volatile(
-                    "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem + (uint32_t)(j * COUT)),
-                    "l"(ad), "l"(bd), "r"(idesc), "r"(acc));
+                mma_if(lead, tmem + (uint32_t)(j * COUT), ad, bd, idesc, acc);
             }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                smem_u32(&empty[s]))
-                         : "memory");
+            commit_if(lead, smem_u32(&empty[s]));
         }
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-            smem_u32(done))
-                     : "memory");
+        commit_if(lead, smem_u32(done));
     }
     __syncwarp();
     const bool got = __all_sync(0xffffffffu, mbar_wait_long(smem_u32(done), 0) ? 1 : 0) != 0;
@@ -885,7 +881,7 @@ __global__ void __launch_bounds__(kWhThreads, 1)
         const uint32_t mn = (1u << 15) | (1u << 16);  // A and B MN-major
         int init = 0;                                  // dY planes whose accumulators hold something
         for (int i = 0; i < mine; i++) {
-            if (!mbar_wait(smem_u32(&full[i % W::RING]), (uint32_t)((i / W::RING) & 1))) {
+            if (!mbar_wait_warp(smem_u32(&full[i % W::RING]), (uint32_t)((i / W::RING) & 1))) {
                 fail = 1;
                 break;
             }
