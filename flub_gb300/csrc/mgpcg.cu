@@ -88,6 +88,13 @@ struct LaunchCtx {
     unsigned long long *kc;  // device kernel counter when captured into a graph, else nullptr
     cudaGraphConditionalHandle h;
     int set_cond;
+    // The next launch is an ordinary one, which starts when everything before it
+    // on the stream has finished, and clears this.  The solver's kernels read what
+    // new tags set up (lists, words, codes) before they wait for the kernel in
+    // front of them; a call that may follow flub_mg_set_tags with no ordinary launch
+    // between would otherwise start while the set-up kernels, which let their
+    // dependents in at once, still write it.
+    mutable bool ordinary = false;
 };
 
 }  // namespace flub
@@ -614,19 +621,21 @@ static unsigned matvec_blocks(int64_t groups) {
     } while (0)
 
 // Kernel launch with programmatic stream serialisation (the kernel's entry
-// waits on griddepcontrol.wait, see count_kernel), counted like the others.
+// waits on griddepcontrol.wait, see count_kernel; LaunchCtx::ordinary: without
+// it), counted like the others.
 template <typename... KArgs, typename... Args>
-static int launch_pdl(void (*kern)(KArgs...), dim3 g, dim3 b, size_t smem, cudaStream_t s, Args... args) {
+static int launch_pdl(void (*kern)(KArgs...), dim3 g, dim3 b, size_t smem, const LaunchCtx &c, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = g;
     cfg.blockDim = b;
     cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
+    cfg.stream = c.s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = c.ordinary ? 0 : 1;
+    c.ordinary = false;
     cudaError_t e = cudaLaunchKernelEx(&cfg, kern, ((KArgs)args)...);
     if (e != cudaSuccess) {
         set_last_error("cudaLaunchKernelEx: %s", cudaGetErrorString(e));
@@ -656,13 +665,13 @@ static int sweep8(const LaunchCtx &c, const Level &L, int phase, int mode, int s
     const int *act_n = skip ? L.act_n : nullptr;
     const dim3 blk(256), grd(blocks_for(D.n() >> 2, 256, kNumSMs * 6));  // two lanes per group, 6 resident blocks per SM
     if (mode == kSweepFromZero)
-        return launch_pdl(k_smooth8<true, false, TO, TO, TR, TC>, grd, blk, 0, c.s, zout, (const TO *)zout,
+        return launch_pdl(k_smooth8<true, false, TO, TO, TR, TC>, grd, blk, 0, c, zout, (const TO *)zout,
                           (const TC *)nullptr, 1.0f, r, (const uint8_t *)L.code, (const uint16_t *)L.sw, D, phase,
                           act, act_n, c.kc);
     if (mode == kSweepProlong)
-        return launch_pdl(k_smooth8<false, true, TO, TI, TR, TC>, grd, blk, 0, c.s, zout, zin, zc, zc_scale, r,
+        return launch_pdl(k_smooth8<false, true, TO, TI, TR, TC>, grd, blk, 0, c, zout, zin, zc, zc_scale, r,
                           (const uint8_t *)L.code, (const uint16_t *)L.sw, D, phase, act, act_n, c.kc);
-    return launch_pdl(k_smooth8<false, false, TO, TO, TR, TC>, grd, blk, 0, c.s, zout, (const TO *)zout,
+    return launch_pdl(k_smooth8<false, false, TO, TO, TR, TC>, grd, blk, 0, c, zout, (const TO *)zout,
                       (const TC *)nullptr, 1.0f, r, (const uint8_t *)L.code, (const uint16_t *)L.sw, D, phase, act,
                       act_n, c.kc);
 }
@@ -673,13 +682,13 @@ static int sweep(const LaunchCtx &c, const Level &L, int phase, int mode, int sk
     if (D.nz % 8 == 0) return sweep8<float, float, float, float>(c, L, phase, mode, skip, r, zin, zout, zc, 1.0f);
     // scalar path for levels whose nz is not a multiple of 8
     if (mode == kSweepProlong)
-        FLUB_TRY(launch_pdl(k_prolong, dim3(blocks_for(D.n(), 256, 1 << 20)), dim3(256), 0, c.s, zout, zin, zc, D,
+        FLUB_TRY(launch_pdl(k_prolong, dim3(blocks_for(D.n(), 256, 1 << 20)), dim3(256), 0, c, zout, zin, zc, D,
                             c.kc));
     const unsigned b = blocks_for(D.n() / 2, 256, 1 << 20);
     if (mode == kSweepFromZero)
-        return launch_pdl(k_smooth_half<true>, dim3(b), dim3(256), 0, c.s, zout, r, (const uint8_t *)L.code, D, phase,
+        return launch_pdl(k_smooth_half<true>, dim3(b), dim3(256), 0, c, zout, r, (const uint8_t *)L.code, D, phase,
                           c.kc);
-    return launch_pdl(k_smooth_half<false>, dim3(b), dim3(256), 0, c.s, zout, r, (const uint8_t *)L.code, D, phase,
+    return launch_pdl(k_smooth_half<false>, dim3(b), dim3(256), 0, c, zout, r, (const uint8_t *)L.code, D, phase,
                       c.kc);
 }
 
@@ -715,7 +724,7 @@ static int split_sweep(const LaunchCtx &c, const Level &L, int phase, const TRN 
         resident = b;
     }
     const dim3 grd(blocks_for(L.D.n() >> 3, 256, (int64_t)kNumSMs * resident));
-    return launch_pdl(k_smooth_split<kMode, TRN, TR, TZI, TZ, TC>, grd, dim3(256), 0, c.s, (const SplitArgs)A, phase,
+    return launch_pdl(k_smooth_split<kMode, TRN, TR, TZI, TZ, TC>, grd, dim3(256), 0, c, (const SplitArgs)A, phase,
                       c.kc);
 }
 
@@ -847,12 +856,12 @@ static int tile_iteration(flub_mg *mg, const LaunchCtx &c, int l, int first_phas
     int *status = &mg->st->status;
     const int *tl = L.tiles, *tn = L.tiles_n;
     if (mode == kTileFromZero)
-        return launch_pdl(k_smooth_tile<kTileFromZero>, grd, dim3(kTileThreads), kTileSmem, c.s, mz, mr, mw, mc, zout,
+        return launch_pdl(k_smooth_tile<kTileFromZero>, grd, dim3(kTileThreads), kTileSmem, c, mz, mr, mw, mc, zout,
                           L.D, first_phase, tl, tn, status, c.kc);
     if (mode == kTileProlong)
-        return launch_pdl(k_smooth_tile<kTileProlong>, grd, dim3(kTileThreads), kTileSmem, c.s, mz, mr, mw, mc, zout,
+        return launch_pdl(k_smooth_tile<kTileProlong>, grd, dim3(kTileThreads), kTileSmem, c, mz, mr, mw, mc, zout,
                           L.D, first_phase, tl, tn, status, c.kc);
-    return launch_pdl(k_smooth_tile<kTileInPlaceInput>, grd, dim3(kTileThreads), kTileSmem, c.s, mz, mr, mw, mc,
+    return launch_pdl(k_smooth_tile<kTileInPlaceInput>, grd, dim3(kTileThreads), kTileSmem, c, mz, mr, mw, mc,
                       zout, L.D, first_phase, tl, tn, status, c.kc);
 }
 
@@ -884,7 +893,7 @@ static int block_launch(const LaunchCtx &c, const Level &L, const BlockArgs &A) 
         return FLUB_OK;
     }
     const int blocks = L.b_tiles < kNumSMs ? L.b_tiles : kNumSMs;
-    return launch_pdl(k_smooth_block<V, T, TI, S>, dim3(blocks), dim3(kBlockThreads), smem, c.s, A, c.kc);
+    return launch_pdl(k_smooth_block<V, T, TI, S>, dim3(blocks), dim3(kBlockThreads), smem, c, A, c.kc);
 }
 
 // One launch of `its` red-black iterations (1 or 2).
@@ -966,6 +975,11 @@ static int launch_coarse(flub_mg *mg, const LaunchCtx &c, const float *r_top, fl
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[2];
     coarse_launch_config(mg->co_blocks, mg->co_smem, c.s, &cfg, attr);
+    if (c.ordinary) {  // without the first attribute
+        cfg.attrs = attr + 1;
+        cfg.numAttrs--;
+        c.ordinary = false;
+    }
     const cudaError_t e = cudaLaunchKernelEx(&cfg, coarse_kernel(P), (const CoarseParams)P, c.kc);
     if (e != cudaSuccess) {
         set_last_error("coarse V-cycle launch: %s", cudaGetErrorString(e));
@@ -1018,7 +1032,7 @@ static int enqueue_vcycle(flub_mg *mg, const LaunchCtx &c, const float *r0, floa
             FLUB_TRY(split_pre<float>(c, L, iters, R(l), L.rs, ZP(l)));
             const Level &C = mg->lv[l + 1];
             FLUB_TRY(launch_pdl(k_restrict8_split<float, float, float>, dim3(blocks_for(C.D.n(), 256, kNumSMs * 4)),
-                                dim3(256), 0, c.s, R(l), (const float *)ZP(l), (const uint32_t *)L.b_items,
+                                dim3(256), 0, c, R(l), (const float *)ZP(l), (const uint32_t *)L.b_items,
                                 (const uint16_t *)L.sw, C.r, (const uint8_t *)C.code, C.D, mg->sched_rscale,
                                 (const int *)C.act, (const int *)C.act_n, c.kc));
             continue;
@@ -1036,12 +1050,12 @@ static int enqueue_vcycle(flub_mg *mg, const LaunchCtx &c, const float *r0, floa
         const Level &C = mg->lv[l + 1];
         if (L.D.nz % 8 == 0)
             FLUB_TRY(launch_pdl(k_restrict8<float, float, float>, dim3(blocks_for(C.D.n(), 256, kNumSMs * 4)),
-                                dim3(256), 0, c.s, R(l), (const float *)ZP(l), (const uint8_t *)L.code,
+                                dim3(256), 0, c, R(l), (const float *)ZP(l), (const uint8_t *)L.code,
                                 (const uint16_t *)L.sw, C.r,
                                 (const uint8_t *)C.code, C.D, mg->sched_rscale, (const int *)C.act,
                                 (const int *)C.act_n, c.kc));
         else
-            FLUB_TRY(launch_pdl(k_restrict, dim3(blocks_for(C.D.n(), 256, 1 << 20)), dim3(256), 0, c.s, R(l), ZP(l),
+            FLUB_TRY(launch_pdl(k_restrict, dim3(blocks_for(C.D.n(), 256, 1 << 20)), dim3(256), 0, c, R(l), ZP(l),
                                 L.code, C.r, C.code, C.D, mg->sched_rscale, c.kc));
     }
     if (pers) FLUB_TRY(launch_leg<float>(mg, c, true, 1, lg));
@@ -1121,7 +1135,7 @@ static int enqueue_vcycle_mixed(flub_mg *mg, const LaunchCtx &c, float *z0, bool
             FLUB_TRY(split_pre<H>(c, L, iters, L.rh, L.rsh, L.z2h));
             const Level &C = mg->lv[l + 1];
             FLUB_TRY(launch_pdl(k_restrict8_split<H, H, H>, dim3(blocks_for(C.D.n(), 256, kNumSMs * 4)), dim3(256),
-                                0, c.s, (const H *)L.rh, (const H *)L.z2h, (const uint32_t *)L.b_items,
+                                0, c, (const H *)L.rh, (const H *)L.z2h, (const uint32_t *)L.b_items,
                                 (const uint16_t *)L.sw, C.rh, (const uint8_t *)C.code, C.D,
                                 0.125f * mg->sched_rscale, (const int *)C.act, (const int *)C.act_n, c.kc));
             continue;
@@ -1136,7 +1150,7 @@ static int enqueue_vcycle_mixed(flub_mg *mg, const LaunchCtx &c, float *z0, bool
         }
         const Level &C = mg->lv[l + 1];
         FLUB_TRY(launch_pdl(k_restrict8<__half, __half, __half>, dim3(blocks_for(C.D.n(), 256, kNumSMs * 4)),
-                            dim3(256), 0, c.s, (const __half *)L.rh, (const __half *)L.z2h, (const uint8_t *)L.code,
+                            dim3(256), 0, c, (const __half *)L.rh, (const __half *)L.z2h, (const uint8_t *)L.code,
                             (const uint16_t *)L.sw, C.rh, (const uint8_t *)C.code, C.D, 0.125f * mg->sched_rscale, (const int *)C.act,
                             (const int *)C.act_n, c.kc));
     }
@@ -1222,8 +1236,8 @@ static int enqueue_vcycle_mixed(flub_mg *mg, const LaunchCtx &c, float *z0, bool
 
 static int enqueue_mean_removal(flub_mg *mg, const LaunchCtx &c, int guard) {
     const unsigned b = red_blocks(mg->n);
-    FLUB_TRY(launch_pdl(k_fluid_mean, dim3(b), dim3(kRedThreads), 0, c.s, mg->st, mg->lv[0].r, mg->lv[0].code, mg->n, mg->partials, guard, c.kc));
-    FLUB_TRY(launch_pdl(k_sub_mean, dim3(b), dim3(kRedThreads), 0, c.s, mg->st, mg->lv[0].r, mg->lv[0].code, mg->n, guard, c.kc));
+    FLUB_TRY(launch_pdl(k_fluid_mean, dim3(b), dim3(kRedThreads), 0, c, mg->st, mg->lv[0].r, mg->lv[0].code, mg->n, mg->partials, guard, c.kc));
+    FLUB_TRY(launch_pdl(k_sub_mean, dim3(b), dim3(kRedThreads), 0, c, mg->st, mg->lv[0].r, mg->lv[0].code, mg->n, guard, c.kc));
     return FLUB_OK;
 }
 
@@ -1232,39 +1246,39 @@ static int enqueue_prologue_mixed(flub_mg *mg, const LaunchCtx &c, int smoother)
     const Level &L0 = mg->lv[0];
     const unsigned bg = red_blocks(mg->n / 8 + 1);
     if (smoother == FLUB_SMOOTHER_FRACTION) FLUB_TRY(enqueue_mean_removal(mg, c, 0));
-    FLUB_TRY(launch_pdl(k8_dot_rr0, dim3(bg), dim3(kRedThreads), 0, c.s, mg->st, L0.r, L0.code, mg->n, mg->partials,
+    FLUB_TRY(launch_pdl(k8_dot_rr0, dim3(bg), dim3(kRedThreads), 0, c, mg->st, L0.r, L0.code, mg->n, mg->partials,
                         (const int *)L0.act, (const int *)L0.act_n, c.kc));
-    FLUB_TRY(launch_pdl(k8_residual_x0, dim3(blocks_for(mg->n / 8, 256, kNumSMs * 8)), dim3(256), 0, c.s, mg->st,
+    FLUB_TRY(launch_pdl(k8_residual_x0, dim3(blocks_for(mg->n / 8, 256, kNumSMs * 8)), dim3(256), 0, c, mg->st,
                         L0.r, (const float *)mg->x, (const uint8_t *)L0.code, (const uint16_t *)L0.sw, L0.D,
                         (const int *)L0.act,
                         (const int *)L0.act_n, c.kc));
     if (smoother == FLUB_SMOOTHER_FRACTION) FLUB_TRY(enqueue_mean_removal(mg, c, 2));
-    FLUB_TRY(launch_pdl(k8_to_half, dim3(blocks_for(mg->n / 8, 256)), dim3(256), 0, c.s, mg->st, (const float *)L0.r, L0.rh,
+    FLUB_TRY(launch_pdl(k8_to_half, dim3(blocks_for(mg->n / 8, 256)), dim3(256), 0, c, mg->st, (const float *)L0.r, L0.rh,
                         mg->n, c.kc));
     bool fused = false;
     FLUB_TRY(enqueue_vcycle_mixed(mg, c, L0.z, true, 1, &fused));
     if (fused) return FLUB_OK;  // p = zscale z and z.r in the last level-0 half-sweep
-    return launch_pdl(k8_dot_zr<true, true>, dim3(bg), dim3(kRedThreads), 0, c.s, mg->st, L0.z, L0.r, mg->p, L0.code,
+    return launch_pdl(k8_dot_zr<true, true>, dim3(bg), dim3(kRedThreads), 0, c, mg->st, L0.z, L0.r, mg->p, L0.code,
                       mg->n, mg->partials, (const int *)L0.act, (const int *)L0.act_n, c.kc);
 }
 
 static int enqueue_first_half_mixed(flub_mg *mg, const LaunchCtx &c, int smoother) {
     const Level &L0 = mg->lv[0];
     const unsigned b = red_blocks(mg->n), bg = red_blocks(mg->n / 8 + 1);
-    FLUB_TRY(launch_pdl(k8_matvec_pap, dim3(matvec_blocks(mg->n / 8)), dim3(kRedThreads), 0, c.s, mg->st, mg->p,
+    FLUB_TRY(launch_pdl(k8_matvec_pap, dim3(matvec_blocks(mg->n / 8)), dim3(kRedThreads), 0, c, mg->st, mg->p,
                         mg->Ap, (const uint32_t *)L0.b_items, (const uint16_t *)L0.sw, L0.D, mg->partials,
                         (const int *)L0.act, (const int *)L0.act_n, c.kc));
     if (smoother == FLUB_SMOOTHER_FRACTION) {
         FLUB_CHECK_CUDA(cudaMemcpyAsync(mg->r_old, L0.r, sizeof(float) * mg->n, cudaMemcpyDeviceToDevice, c.s));
-        FLUB_TRY(launch_pdl(k_update_r, dim3(b), dim3(kRedThreads), 0, c.s, mg->st, L0.r, mg->Ap, mg->n, c.kc));
+        FLUB_TRY(launch_pdl(k_update_r, dim3(b), dim3(kRedThreads), 0, c, mg->st, L0.r, mg->Ap, mg->n, c.kc));
         FLUB_TRY(enqueue_mean_removal(mg, c, 1));
-        FLUB_TRY(launch_pdl(k8_to_half, dim3(blocks_for(mg->n / 8, 256)), dim3(256), 0, c.s, mg->st, (const float *)L0.r,
+        FLUB_TRY(launch_pdl(k8_to_half, dim3(blocks_for(mg->n / 8, 256)), dim3(256), 0, c, mg->st, (const float *)L0.r,
                             L0.rh, mg->n, c.kc));
-        return launch_pdl(k8_update_r_rr<false>, dim3(bg), dim3(kRedThreads), 0, c.s, mg->st, L0.r, mg->Ap, L0.code,
+        return launch_pdl(k8_update_r_rr<false>, dim3(bg), dim3(kRedThreads), 0, c, mg->st, L0.r, mg->Ap, L0.code,
                           mg->n, mg->partials, mg->hist, c.h, c.set_cond, (const int *)L0.act, (const int *)L0.act_n,
                           c.kc);
     }
-    return launch_pdl(k8_update_r_rr_mixed, dim3(bg), dim3(kRedThreads), 0, c.s, mg->st, L0.r, mg->r_old, L0.rh,
+    return launch_pdl(k8_update_r_rr_mixed, dim3(bg), dim3(kRedThreads), 0, c, mg->st, L0.r, mg->r_old, L0.rh,
                       mg->Ap, L0.code, mg->n, mg->partials, mg->hist, c.h, c.set_cond, (const int *)L0.act,
                       (const int *)L0.act_n, c.kc);
 }
@@ -1275,9 +1289,9 @@ static int enqueue_second_half_mixed(flub_mg *mg, const LaunchCtx &c) {
     bool fused = false;
     FLUB_TRY(enqueue_vcycle_mixed(mg, c, L0.z, true, 3, &fused));
     if (!fused)  // else the flexible beta came with the last level-0 half-sweep
-        FLUB_TRY(launch_pdl(k8_dot_zr_flex, dim3(bg), dim3(kRedThreads), 0, c.s, mg->st, L0.z, L0.r, mg->r_old,
+        FLUB_TRY(launch_pdl(k8_dot_zr_flex, dim3(bg), dim3(kRedThreads), 0, c, mg->st, L0.z, L0.r, mg->r_old,
                             L0.code, mg->n, mg->partials, (const int *)L0.act, (const int *)L0.act_n, c.kc));
-    return launch_pdl(k8_update_xp<true>, dim3(blocks_for(mg->n / 8, 256, kNumSMs * 6)), dim3(256), 0, c.s, mg->st,
+    return launch_pdl(k8_update_xp<true>, dim3(blocks_for(mg->n / 8, 256, kNumSMs * 6)), dim3(256), 0, c, mg->st,
                       mg->x, mg->p, L0.z, L0.code, mg->n, (const int *)L0.act, (const int *)L0.act_n, c.kc);
 }
 
@@ -1289,26 +1303,26 @@ static int enqueue_prologue(flub_mg *mg, const LaunchCtx &c, int smoother) {
     const unsigned bg = red_blocks(mg->n / 8 + 1);
     if (smoother == FLUB_SMOOTHER_FRACTION) FLUB_TRY(enqueue_mean_removal(mg, c, 0));
     if (v8)
-        FLUB_TRY(launch_pdl(k8_dot_rr0, dim3(bg), dim3(kRedThreads), 0, c.s, mg->st, L0.r, L0.code, mg->n,
+        FLUB_TRY(launch_pdl(k8_dot_rr0, dim3(bg), dim3(kRedThreads), 0, c, mg->st, L0.r, L0.code, mg->n,
                             mg->partials, (const int *)L0.act, (const int *)L0.act_n, c.kc));
     else
-        FLUB_TRY(launch_pdl(k_dot_rr0, dim3(b), dim3(kRedThreads), 0, c.s, mg->st, L0.r, mg->n, mg->partials, c.kc));
+        FLUB_TRY(launch_pdl(k_dot_rr0, dim3(b), dim3(kRedThreads), 0, c, mg->st, L0.r, mg->n, mg->partials, c.kc));
     if (v8)
-        FLUB_TRY(launch_pdl(k8_residual_x0, dim3(blocks_for(mg->n / 8, 256, kNumSMs * 8)), dim3(256), 0, c.s,
+        FLUB_TRY(launch_pdl(k8_residual_x0, dim3(blocks_for(mg->n / 8, 256, kNumSMs * 8)), dim3(256), 0, c,
                             mg->st, L0.r, (const float *)mg->x, (const uint8_t *)L0.code, (const uint16_t *)L0.sw, L0.D,
                         (const int *)L0.act,
                             (const int *)L0.act_n, c.kc));
     else
-        FLUB_TRY(launch_pdl(k_residual_x0, dim3(blocks_for(mg->n, 256)), dim3(256), 0, c.s, mg->st, L0.r, mg->x,
+        FLUB_TRY(launch_pdl(k_residual_x0, dim3(blocks_for(mg->n, 256)), dim3(256), 0, c, mg->st, L0.r, mg->x,
                             L0.code, L0.D, c.kc));
     if (smoother == FLUB_SMOOTHER_FRACTION) FLUB_TRY(enqueue_mean_removal(mg, c, 2));
     bool fused = false;
     FLUB_TRY(enqueue_vcycle(mg, c, L0.r, L0.z, true, 1, &fused));
     if (fused) return FLUB_OK;  // p = z and z.r in the last level-0 half-sweep
     if (v8)
-        return launch_pdl(k8_dot_zr<true, false>, dim3(bg), dim3(kRedThreads), 0, c.s, mg->st, L0.z, L0.r, mg->p, L0.code,
+        return launch_pdl(k8_dot_zr<true, false>, dim3(bg), dim3(kRedThreads), 0, c, mg->st, L0.z, L0.r, mg->p, L0.code,
                           mg->n, mg->partials, (const int *)L0.act, (const int *)L0.act_n, c.kc);
-    return launch_pdl(k_dot_zr_init, dim3(b), dim3(kRedThreads), 0, c.s, mg->st, L0.z, L0.r, mg->p, mg->n,
+    return launch_pdl(k_dot_zr_init, dim3(b), dim3(kRedThreads), 0, c, mg->st, L0.z, L0.r, mg->p, mg->n,
                       mg->partials, c.kc);
 }
 
@@ -1320,27 +1334,27 @@ static int enqueue_first_half(flub_mg *mg, const LaunchCtx &c, int smoother) {
     const bool v8 = (L0.D.nz % 8) == 0;
     const unsigned bg = red_blocks(mg->n / 8 + 1);
     if (v8)
-        FLUB_TRY(launch_pdl(k8_matvec_pap, dim3(matvec_blocks(mg->n / 8)), dim3(kRedThreads), 0, c.s, mg->st,
+        FLUB_TRY(launch_pdl(k8_matvec_pap, dim3(matvec_blocks(mg->n / 8)), dim3(kRedThreads), 0, c, mg->st,
                             mg->p, mg->Ap, (const uint32_t *)L0.b_items, (const uint16_t *)L0.sw, L0.D, mg->partials,
                             (const int *)L0.act, (const int *)L0.act_n, c.kc));
     else
-        FLUB_TRY(launch_pdl(k_matvec_pap, dim3(b), dim3(kRedThreads), 0, c.s, mg->st, mg->p, mg->Ap, L0.code, L0.D,
+        FLUB_TRY(launch_pdl(k_matvec_pap, dim3(b), dim3(kRedThreads), 0, c, mg->st, mg->p, mg->Ap, L0.code, L0.D,
                             mg->partials, c.kc));
     if (smoother == FLUB_SMOOTHER_FRACTION) {
-        FLUB_TRY(launch_pdl(k_update_r, dim3(b), dim3(kRedThreads), 0, c.s, mg->st, L0.r, mg->Ap, mg->n, c.kc));
+        FLUB_TRY(launch_pdl(k_update_r, dim3(b), dim3(kRedThreads), 0, c, mg->st, L0.r, mg->Ap, mg->n, c.kc));
         FLUB_TRY(enqueue_mean_removal(mg, c, 1));
         if (v8)
-            return launch_pdl(k8_update_r_rr<false>, dim3(bg), dim3(kRedThreads), 0, c.s, mg->st, L0.r, mg->Ap,
+            return launch_pdl(k8_update_r_rr<false>, dim3(bg), dim3(kRedThreads), 0, c, mg->st, L0.r, mg->Ap,
                               L0.code, mg->n, mg->partials, mg->hist, c.h, c.set_cond, (const int *)L0.act,
                               (const int *)L0.act_n, c.kc);
-        return launch_pdl(k_update_r_rr<false>, dim3(b), dim3(kRedThreads), 0, c.s, mg->st, L0.r, mg->Ap, mg->n,
+        return launch_pdl(k_update_r_rr<false>, dim3(b), dim3(kRedThreads), 0, c, mg->st, L0.r, mg->Ap, mg->n,
                           mg->partials, mg->hist, c.h, c.set_cond, c.kc);
     }
     if (v8)
-        return launch_pdl(k8_update_r_rr<true>, dim3(bg), dim3(kRedThreads), 0, c.s, mg->st, L0.r, mg->Ap, L0.code,
+        return launch_pdl(k8_update_r_rr<true>, dim3(bg), dim3(kRedThreads), 0, c, mg->st, L0.r, mg->Ap, L0.code,
                           mg->n, mg->partials, mg->hist, c.h, c.set_cond, (const int *)L0.act,
                           (const int *)L0.act_n, c.kc);
-    return launch_pdl(k_update_r_rr<true>, dim3(b), dim3(kRedThreads), 0, c.s, mg->st, L0.r, mg->Ap, mg->n,
+    return launch_pdl(k_update_r_rr<true>, dim3(b), dim3(kRedThreads), 0, c, mg->st, L0.r, mg->Ap, mg->n,
                       mg->partials, mg->hist, c.h, c.set_cond, c.kc);
 }
 
@@ -1354,16 +1368,16 @@ static int enqueue_second_half(flub_mg *mg, const LaunchCtx &c) {
     if ((L0.D.nz % 8) == 0) {
         const unsigned bg = red_blocks(mg->n / 8 + 1);
         if (!fused)  // else beta came with the last level-0 half-sweep
-            FLUB_TRY(launch_pdl(k8_dot_zr<false>, dim3(bg), dim3(kRedThreads), 0, c.s, mg->st, L0.z, L0.r,
+            FLUB_TRY(launch_pdl(k8_dot_zr<false>, dim3(bg), dim3(kRedThreads), 0, c, mg->st, L0.z, L0.r,
                                 (float *)nullptr, L0.code, mg->n, mg->partials, (const int *)L0.act,
                                 (const int *)L0.act_n, c.kc));
-        return launch_pdl(k8_update_xp<false>, dim3(blocks_for(mg->n / 8, 256, kNumSMs * 6)), dim3(256), 0, c.s,
+        return launch_pdl(k8_update_xp<false>, dim3(blocks_for(mg->n / 8, 256, kNumSMs * 6)), dim3(256), 0, c,
                           mg->st, mg->x, mg->p, L0.z, L0.code, mg->n, (const int *)L0.act, (const int *)L0.act_n,
                           c.kc);
     }
-    FLUB_TRY(launch_pdl(k_dot_zr_beta, dim3(b), dim3(kRedThreads), 0, c.s, mg->st, L0.z, L0.r, mg->n, mg->partials,
+    FLUB_TRY(launch_pdl(k_dot_zr_beta, dim3(b), dim3(kRedThreads), 0, c, mg->st, L0.z, L0.r, mg->n, mg->partials,
                         c.kc));
-    return launch_pdl(k_update_xp, dim3(blocks_for(mg->n, 256)), dim3(256), 0, c.s, mg->st, mg->x, mg->p, L0.z, mg->n,
+    return launch_pdl(k_update_xp, dim3(blocks_for(mg->n, 256)), dim3(256), 0, c, mg->st, mg->x, mg->p, L0.z, mg->n,
                       c.kc);
 }
 
@@ -1435,9 +1449,9 @@ static int enqueue_iteration(flub_mg *mg, const LaunchCtx &c, int smoother) {
 static int enqueue_epilogue(flub_mg *mg, const LaunchCtx &c) {
     const Level &L0 = mg->lv[0];
     if ((L0.D.nz % 8) == 0)
-        return launch_pdl(k8_solve_end, dim3(blocks_for(mg->n / 8, 256, kNumSMs * 8)), dim3(256), 0, c.s, mg->st,
+        return launch_pdl(k8_solve_end, dim3(blocks_for(mg->n / 8, 256, kNumSMs * 8)), dim3(256), 0, c, mg->st,
                           mg->x, mg->p, L0.code, mg->n, (const int *)L0.act, (const int *)L0.act_n, c.kc);
-    return launch_pdl(k_solve_end, dim3(blocks_for(mg->n, 256)), dim3(256), 0, c.s, mg->st, mg->x, mg->p, mg->n,
+    return launch_pdl(k_solve_end, dim3(blocks_for(mg->n, 256)), dim3(256), 0, c, mg->st, mg->x, mg->p, mg->n,
                       c.kc);
 }
 
@@ -1797,6 +1811,7 @@ int flub_mg_destroy(flub_mg *mg) {
 int flub_mg_set_tags(flub_mg *mg, const int32_t *tag, void *stream) {
     FLUB_REQUIRE(mg && tag, "flub_mg_set_tags: NULL argument");
     cudaStream_t s = as_stream(stream);
+    const LaunchCtx c{s, nullptr, 0, 0};
     if (mg->n % 4 == 0 && (uintptr_t)tag % 16 == 0)
         k_encode_tags4<<<blocks_for(mg->n / 4, 256), 256, 0, s>>>(reinterpret_cast<const int4 *>(tag),
                                                                   reinterpret_cast<uint32_t *>(mg->lv[0].code),
@@ -1807,7 +1822,7 @@ int flub_mg_set_tags(flub_mg *mg, const int32_t *tag, void *stream) {
     for (int l = 0; l + 1 < mg->levels; l++) {
         const Level &C = mg->lv[l + 1];
         if (mg->lv[l].D.nz % 8 == 0) {
-            FLUB_TRY(launch_pdl(k_restrict_codes8, dim3(blocks_for(C.D.n() / 4, 256)), dim3(256), 0, s,
+            FLUB_TRY(launch_pdl(k_restrict_codes8, dim3(blocks_for(C.D.n() / 4, 256)), dim3(256), 0, c,
                                 (const uint8_t *)mg->lv[l].code, C.code, C.D));
             continue;
         }
@@ -1844,7 +1859,7 @@ int flub_mg_set_tags(flub_mg *mg, const int32_t *tag, void *stream) {
     }
     zero(mg->p, (size_t)(reinterpret_cast<char *>(mg->Ap) - reinterpret_cast<char *>(mg->p)) +
                     sizeof(float) * (size_t)mg->n);
-    FLUB_TRY(launch_pdl(k_setup_clear, dim3((unsigned)clear_blocks), dim3(kSetupThreads), 0, s, clear));
+    FLUB_TRY(launch_pdl(k_setup_clear, dim3((unsigned)clear_blocks), dim3(kSetupThreads), 0, c, clear));
     // words and active groups of every level that has them
     SetupParams P = {};
     P.bcount = mg->act_scratch;
@@ -1863,9 +1878,9 @@ int flub_mg_set_tags(flub_mg *mg, const int32_t *tag, void *stream) {
         P.blocks += (int)((L.D.n() / 8 + kSetupThreads - 1) / kSetupThreads);
     }
     if (P.n) {
-        FLUB_TRY(launch_pdl(k_setup_words, dim3(P.blocks), dim3(kSetupThreads), 0, s, P));
-        FLUB_TRY(launch_pdl(k_setup_scan, dim3(P.n), dim3(1024), 0, s, P));
-        FLUB_TRY(launch_pdl(k_setup_write, dim3(P.blocks), dim3(kSetupThreads), 0, s, P));
+        FLUB_TRY(launch_pdl(k_setup_words, dim3(P.blocks), dim3(kSetupThreads), 0, c, P));
+        FLUB_TRY(launch_pdl(k_setup_scan, dim3(P.n), dim3(1024), 0, c, P));
+        FLUB_TRY(launch_pdl(k_setup_write, dim3(P.blocks), dim3(kSetupThreads), 0, c, P));
     }
     TileParams T = {};
     int tile_blocks = 0;
@@ -1891,7 +1906,7 @@ int flub_mg_set_tags(flub_mg *mg, const int32_t *tag, void *stream) {
             k_block_items<1><<<blocks, 256, 0, s>>>(L.cw, L.D, L.b_items);
         FLUB_CHECK_LAUNCH();
     }
-    if (T.n) FLUB_TRY(launch_pdl(k_setup_tiles, dim3(tile_blocks), dim3(128), 0, s, T));
+    if (T.n) FLUB_TRY(launch_pdl(k_setup_tiles, dim3(tile_blocks), dim3(128), 0, c, T));
     for (int l = 0; l < mg->levels; l++) {
         const Level &L = mg->lv[l];
         if (!L.act || !L.n_tiles) continue;
@@ -2117,9 +2132,9 @@ int flub_mg_get_x(flub_mg *mg, float *out, float scale, void *stream) {
 
 int flub_mg_apply_preconditioner(flub_mg *mg, const float *r, float *z, void *stream) {
     FLUB_REQUIRE(mg && r && z, "flub_mg_apply_preconditioner: NULL argument");
-    LaunchCtx c{as_stream(stream), nullptr, 0, 0};
+    LaunchCtx c{as_stream(stream), nullptr, 0, 0, true};  // may follow set_tags directly
     if (mg->precision == FLUB_PRECISION_MIXED) {
-        FLUB_TRY(launch_pdl(k8_to_half, dim3(blocks_for(mg->n / 8, 256)), dim3(256), 0, c.s, (MgState *)nullptr, r, mg->lv[0].rh, mg->n,
+        FLUB_TRY(launch_pdl(k8_to_half, dim3(blocks_for(mg->n / 8, 256)), dim3(256), 0, c, (MgState *)nullptr, r, mg->lv[0].rh, mg->n,
                             c.kc));
         return enqueue_vcycle_mixed(mg, c, z, false);
     }
@@ -2138,7 +2153,7 @@ int flub_mg_smooth(flub_mg *mg, int level, int phase, void *stream) {
     FLUB_REQUIRE(mg, "flub_mg_smooth: NULL handle");
     FLUB_REQUIRE(level >= 0 && level < mg->levels, "flub_mg_smooth: level %d outside [0, %d)", level, mg->levels);
     FLUB_REQUIRE(phase == 0 || phase == 1, "flub_mg_smooth: phase must be 0 or 1");
-    LaunchCtx c{as_stream(stream), nullptr, 0, 0};
+    LaunchCtx c{as_stream(stream), nullptr, 0, 0, true};  // may follow set_tags directly
     const Level &L = mg->lv[level];
     return sweep(c, L, phase, kSweepInPlace, mg->skip_ok ? 1 : 0, L.r, L.z, L.z, nullptr);
 }
@@ -2148,7 +2163,7 @@ int flub_mg_smooth_iteration(flub_mg *mg, int level, int phase, int *tiled, void
     FLUB_REQUIRE(level >= 0 && level < mg->levels, "flub_mg_smooth_iteration: level %d outside [0, %d)", level,
                  mg->levels);
     FLUB_REQUIRE(phase == 0 || phase == 1, "flub_mg_smooth_iteration: phase must be 0 or 1");
-    LaunchCtx c{as_stream(stream), nullptr, 0, 0};
+    LaunchCtx c{as_stream(stream), nullptr, 0, 0, true};  // may follow set_tags directly
     const Level &L = mg->lv[level];
     const bool t = mg->tile_ok && L.n_tiles > 0 && mg->skip_ok;
     if (tiled) *tiled = t ? 1 : 0;
@@ -2287,6 +2302,6 @@ extern "C" int flub_vcycle_noalloc(const int32_t *tag, const float *r, float *z,
         FLUB_CHECK_LAUNCH();
     }
     FLUB_TRY(enqueue_cell_words(&mg, s));
-    LaunchCtx c{s, nullptr, 0, 0};
+    LaunchCtx c{s, nullptr, 0, 0, true};  // follows the words directly
     return enqueue_vcycle(&mg, c, r, z, false);  // mg.skip_ok is false: every sweep writes every cell
 }
