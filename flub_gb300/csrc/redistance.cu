@@ -162,13 +162,15 @@ __global__ void __launch_bounds__(32 * kRdRows) k_redistance_sweep_rows(float *p
         const int t = t0 + 32 * u, k = 2 * t + q;
         pc[u] = 0.0f;
         if (k < 1 || k >= nz - 1) continue;
+        // not the read-only path: the sweep in front of this one may have been
+        // writing these cells while this block was already resident
         pc[u] = own[t];
-        xm[u] = __ldg(own + t - dx);
-        xp[u] = __ldg(own + t + dx);
-        ym[u] = __ldg(own + t - dy);
-        yp[u] = __ldg(own + t + dy);
-        zm[u] = __ldg(oth + t + (incz < 0 ? 1 : 0));
-        zp[u] = __ldg(oth + t + (incz < 0 ? 0 : 1));
+        xm[u] = own[t - dx];
+        xp[u] = own[t + dx];
+        ym[u] = own[t - dy];
+        yp[u] = own[t + dy];
+        zm[u] = oth[t + (incz < 0 ? 1 : 0)];
+        zp[u] = oth[t + (incz < 0 ? 0 : 1)];
     }
 #pragma unroll
     for (int u = 0; u < kRdCells; u++) {
