@@ -182,8 +182,10 @@ __global__ void __launch_bounds__(kBlockThreads, 1) k_smooth_block(const BlockAr
                 for (int m = 0; m < V; m++) {
                     ze[m] = par ? zn[u][2 * m + 1] : zn[u][2 * m];
                     zo[m] = par ? zn[u][2 * m] : zn[u][2 * m + 1];
-                    re[m] = par ? rn[u][2 * m + 1] : rn[u][2 * m];
-                    ro[m] = par ? rn[u][2 * m] : rn[u][2 * m + 1];
+                    // 0 on the cells that are never updated: their factor 0 would turn a
+                    // caller's infinity there into NaN, and an air cell's z is read
+                    re[m] = (we[u] >> (4 * m)) & 7u ? (par ? rn[u][2 * m + 1] : rn[u][2 * m]) : 0.0f;
+                    ro[m] = (wo[u] >> (4 * m)) & 7u ? (par ? rn[u][2 * m] : rn[u][2 * m + 1]) : 0.0f;
                 }
                 if (A.mode == kBlockProlong && in) {
                     // z stays 0 on the cells that are never updated
