@@ -1021,8 +1021,12 @@ static int enqueue_vcycle(flub_mg *mg, const LaunchCtx &c, const float *r0, floa
     // levels 1 .. lg-1 in the persistent cooperative kernels, or one launch per pass
     const bool pers = use_persist(mg, lg);
     // blocked smoothing (smooth_block.cuh): neighbouring tiles read r and the
-    // input while others write the output
-    auto BLOCK = [&](int l) { return mg->lv[l].b_ti && sk == 1 && (l > 0 || r0 != z0); };
+    // input while others write the output; a caller's arrays are read in vectors
+    // of an item's cells (the scalar sweeps of rows of 4 k cells take any address)
+    auto BLOCK = [&](int l) {
+        return mg->lv[l].b_ti && sk == 1 &&
+               (l > 0 || (r0 != z0 && ((uintptr_t)r0 | (uintptr_t)z0) % (4 * row_vector(mg->lv[0].D.nz)) == 0));
+    };
     // colour-split storage (smooth_split.cuh)
     auto SPLIT = [&](int l) { return use_split(mg, l, lg, sk, r0, z0); };
     for (int l = 0; l < (pers ? 1 : lg); l++) {
