@@ -1554,6 +1554,38 @@ static int enqueue_cell_words(flub_mg *mg, cudaStream_t s) {
     return FLUB_OK;
 }
 
+// The tiles with fluid of the levels that are smoothed in them (those above the
+// coarse kernel's), and their item words where those do not come with the stencil
+// words.  Their counts are 0 before.
+static int enqueue_tile_lists(flub_mg *mg, const LaunchCtx &c) {
+    TileParams T = {};
+    int tile_blocks = 0;
+    for (int l = 0; l < mg->co_start && l < mg->levels; l++) {
+        const Level &L = mg->lv[l];
+        if (!L.b_ti) continue;
+        TileLevel &q = T.lv[T.n++];
+        q.D = L.D;
+        q.code = L.code;
+        q.ti = L.b_ti;
+        q.ntj = (L.D.ny + kTJb - 1) / kTJb;
+        q.ntk = block_tiles_k(L.D);
+        q.first = tile_blocks;
+        q.tiles = L.b_list;
+        q.count = L.b_n;
+        tile_blocks += L.b_tiles;
+        if (L.sw) continue;  // its items came with its words
+        const int V = row_vector(L.D.nz);
+        const unsigned blocks = blocks_for(L.D.n() / (2 * V), 256);
+        if (V == 2)
+            k_block_items<2><<<blocks, 256, 0, c.s>>>(L.cw, L.D, L.b_items);
+        else
+            k_block_items<1><<<blocks, 256, 0, c.s>>>(L.cw, L.D, L.b_items);
+        FLUB_CHECK_LAUNCH();
+    }
+    if (T.n) FLUB_TRY(launch_pdl(k_setup_tiles, dim3(tile_blocks), dim3(128), 0, c, T));
+    return FLUB_OK;
+}
+
 // ---------------------------------------------------------------- warm-start support (no reference counterpart)
 
 __global__ void k_set_x0_scale(MgState *st, double v) { st->x0_scale = v; }
@@ -1886,31 +1918,7 @@ int flub_mg_set_tags(flub_mg *mg, const int32_t *tag, void *stream) {
         FLUB_TRY(launch_pdl(k_setup_scan, dim3(P.n), dim3(1024), 0, c, P));
         FLUB_TRY(launch_pdl(k_setup_write, dim3(P.blocks), dim3(kSetupThreads), 0, c, P));
     }
-    TileParams T = {};
-    int tile_blocks = 0;
-    for (int l = 0; l < mg->co_start && l < mg->levels; l++) {
-        const Level &L = mg->lv[l];
-        if (!L.b_ti) continue;
-        TileLevel &q = T.lv[T.n++];
-        q.D = L.D;
-        q.code = L.code;
-        q.ti = L.b_ti;
-        q.ntj = (L.D.ny + kTJb - 1) / kTJb;
-        q.ntk = block_tiles_k(L.D);
-        q.first = tile_blocks;
-        q.tiles = L.b_list;
-        q.count = L.b_n;
-        tile_blocks += L.b_tiles;
-        if (L.sw) continue;  // its items came with its words
-        const int V = row_vector(L.D.nz);
-        const unsigned blocks = blocks_for(L.D.n() / (2 * V), 256);
-        if (V == 2)
-            k_block_items<2><<<blocks, 256, 0, s>>>(L.cw, L.D, L.b_items);
-        else
-            k_block_items<1><<<blocks, 256, 0, s>>>(L.cw, L.D, L.b_items);
-        FLUB_CHECK_LAUNCH();
-    }
-    if (T.n) FLUB_TRY(launch_pdl(k_setup_tiles, dim3(tile_blocks), dim3(128), 0, c, T));
+    FLUB_TRY(enqueue_tile_lists(mg, c));
     for (int l = 0; l < mg->levels; l++) {
         const Level &L = mg->lv[l];
         if (!L.act || !L.n_tiles) continue;
@@ -2050,6 +2058,7 @@ int flub_mg_set_bottom_precision(flub_mg *mg, int bits) {
             cudaGraphExecDestroy(mg->graph[g]);
             mg->graph[g] = nullptr;
         }
+    const int start = mg->co_start;
     mg->bottom64 = want;
     FLUB_TRY(choose_coarse(mg));
     if (want && !bottom_in_tail(mg)) {
@@ -2057,6 +2066,17 @@ int flub_mg_set_bottom_precision(flub_mg *mg, int bits) {
         choose_coarse(mg);
         set_last_error("flub_mg_set_bottom_precision: the FP64 bottom does not fit the coarse-level kernels");
         return FLUB_ERR_UNSUPPORTED;
+    }
+    if (mg->co_start != start) {
+        // levels changed hands: the words and tile lists of the present tags for those
+        // that have them now (the bottom's doubles can push a level out of the
+        // coarse kernel)
+        const LaunchCtx c{nullptr, nullptr, 0, 0};
+        for (int l = 0; l < mg->levels; l++)
+            if (mg->lv[l].b_n) FLUB_CHECK_CUDA(cudaMemsetAsync(mg->lv[l].b_n, 0, sizeof(int), c.s));
+        FLUB_TRY(enqueue_cell_words(mg, c.s));
+        FLUB_TRY(enqueue_tile_lists(mg, c));
+        FLUB_CHECK_CUDA(cudaDeviceSynchronize());
     }
     return FLUB_OK;
 }
