@@ -118,6 +118,9 @@ struct flub_mg {
     int graph_nodes[3];
     cudaStream_t cap_stream, cap_stream2;
     bool host_loop;
+    // FLUB_NO_CLUSTER=1 and FLUB_COARSE_FP16=0 when the handle was created: what
+    // they decide is looked at again whenever a graph is captured
+    bool no_cluster, no_coarse_fp16;
     int cg_blocks;  // blocks of the CG step in one cluster (cg_small.cuh), 0: the four kernels
     bool skip_ok;   // internal z buffers keep z = 0 off the fluid (see k_smooth8)
     bool tile_ok;   // the TMA-tiled smoother runs where a level has tiles (FLUB_TILE=1)
@@ -286,6 +289,12 @@ static size_t carve(flub_mg *mg, char *base) {
     return off;
 }
 
+static void read_cluster_options(flub_mg *mg) {
+    const char *nc = getenv("FLUB_NO_CLUSTER"), *fp16 = getenv("FLUB_COARSE_FP16");
+    mg->no_cluster = nc && nc[0] == '1';
+    mg->no_coarse_fp16 = fp16 && fp16[0] == '0';
+}
+
 static inline bool is_pow2(int v) { return v > 0 && (v & (v - 1)) == 0; }
 
 static int small_levels_start(const flub_mg *mg, bool *bottom_small);
@@ -401,17 +410,14 @@ static int choose_coarse(flub_mg *mg) {
     mg->co_start = mg->levels;
     mg->co_blocks = 0;
     mg->co_smem = 0;
-    const char *off = getenv("FLUB_NO_CLUSTER");
-    const bool clusters = !(off && off[0] == '1');
     // in mixed precision level 0 has other storage before and after the coarse
     // correction: below it at the earliest, unless all levels have left FP16.
     // FLUB_COARSE_FP16=0 leaves every FP16 level to the level-by-level sweeps.
     int first = 0;
     if (mg->precision == FLUB_PRECISION_MIXED) {
         bool small;
-        const char *fp16 = getenv("FLUB_COARSE_FP16");
         const int end = small_levels_start(mg, &small);
-        first = end > 0 && !(fp16 && fp16[0] == '0') ? 1 : end;
+        first = end > 0 && !mg->no_coarse_fp16 ? 1 : end;
     }
     int dev = 0, max_smem = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -426,7 +432,7 @@ static int choose_coarse(flub_mg *mg) {
             return FLUB_OK;
         }
     for (int C : {16, 8, 1}) {
-        if (C > 1 && !clusters) continue;
+        if (C > 1 && mg->no_cluster) continue;
         for (int l = first; l < mg->levels; l++) {
             CoarseParams P;
             const size_t b = coarse_layout(mg, l, C, &P);
@@ -461,10 +467,9 @@ static int choose_coarse(flub_mg *mg) {
 // power-of-two extents from there down to 4,096 cells, else the first level of
 // at most 4,096 -- and not what the coarse kernel happens to hold.
 static int small_levels_start(const flub_mg *mg, bool *bottom_small) {
-    const char *off = getenv("FLUB_NO_CLUSTER");
     auto dims = [&](int l) { return Dims{mg->nx >> l, mg->ny >> l, mg->nz >> l}; };
     const int b = mg->levels - 1;
-    if (!(off && off[0] == '1')) {
+    if (!mg->no_cluster) {
         int l = 0;
         while (l <= b && dims(l).n() > 32768) l++;
         bool ok = l <= b;
@@ -966,7 +971,10 @@ static int block_side(const LaunchCtx &c, const Level &L, bool post, int iters, 
 static int launch_coarse(flub_mg *mg, const LaunchCtx &c, const float *r_top, float *z_top, const __half *r_top_h,
                          __half *z_top_h) {
     CoarseParams P = {};
-    coarse_layout(mg, mg->co_start, mg->co_blocks, &P);
+    if (coarse_layout(mg, mg->co_start, mg->co_blocks, &P) != mg->co_smem) {
+        set_last_error("coarse V-cycle launch: the layout is not the one chosen for the handle");
+        return FLUB_ERR_CUDA;
+    }
     P.r_top = r_top;
     P.z_top = z_top;
     P.r_top_h = r_top_h;
@@ -1388,14 +1396,12 @@ static int enqueue_second_half(flub_mg *mg, const LaunchCtx &c) {
 // Blocks of the small CG kernels for the handle: a power of two that holds the groups with
 // one a thread, or 16 with two; 0 where it does not apply.
 static int choose_cg_small(const flub_mg *mg) {
-    const char *off = getenv("FLUB_NO_CLUSTER");
-    const bool clusters = !(off && off[0] == '1');
     if (mg->precision != FLUB_PRECISION_FP32 || mg->nz % 8 != 0 || mg->n > kCgSmallMaxCells) return 0;
     const int need = (int)((mg->n / 8 + kRedThreads - 1) / kRedThreads);
     int C = 1;
     while (C < need && C < kCgSmallMaxBlocks) C <<= 1;
     if (C == 1) return 1;
-    if (!clusters) return 0;
+    if (mg->no_cluster) return 0;
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[2];
     coarse_launch_config(C, 0, nullptr, &cfg, attr);
@@ -1760,6 +1766,7 @@ int flub_mg_create(int nx, int ny, int nz, int levels, int precision, void *work
     mg->n = (int64_t)nx * ny * nz;
     mg->tile_ok = tile_requested();    // decides the tile buffers carved below
     mg->split_ok = split_requested();  // and the colour-split ones
+    read_cluster_options(mg);
     const size_t need = carve(mg, nullptr);
     if (workspace) {
         if (workspace_bytes < need || ((uintptr_t)workspace & 255)) {
@@ -2313,6 +2320,7 @@ extern "C" int flub_vcycle_noalloc(const int32_t *tag, const float *r, float *z,
     void *base = nullptr;
     FLUB_TRY(noalloc_scratch_address(&base));
     noalloc_layout(&mg, (char *)base);
+    read_cluster_options(&mg);
     choose_coarse(&mg);
     cudaStream_t s = as_stream(stream);
     // every scratch element is written before it is read: the codes by these two
