@@ -87,12 +87,12 @@ __device__ __forceinline__ float rd_update(float pc, float phii, float phiii, fl
     }
     const float phi0 = rd_min(rd_min(phii, phij), phik);
     const float phi2 = rd_max(rd_max(phii, phij), phik);
-    // Where no neighbour has a distance yet (all at the 2 of the initialisation
-    // or more) none of the solutions below 2 exists: each is at least
-    // the smallest neighbour there (the sums of values >= 2 round to no less
-    // than 4 and 6, and 6 times the rounded 1/3 rounds to 2), or NaN, which
-    // loses against |pc| as well.  Most warps far from the interface leave here.
-    if (phi0 >= 2.0f && fabsf(pc) <= 2.0f) return __fmul_rn(sgn, fabsf(pc));
+    // Where no neighbour has a distance yet (all three at the 2 of the
+    // initialisation) no solution below 2 exists: phi1 is exactly 2, the sums 4 and
+    // 6 are exact, each square root is at least 0, and 6 times the rounded 1/3 rounds
+    // to 2.  (A larger phi2, a boundary value that was kept, could round phi1 below
+    // phi0.)  Most warps far from the interface leave here.
+    if (phi0 >= 2.0f && phi2 <= 2.0f && fabsf(pc) <= 2.0f && h >= 0.0f) return __fmul_rn(sgn, fabsf(pc));
     const float phi1 = __fsub_rn(__fsub_rn(__fadd_rn(__fadd_rn(phii, phij), phik), phi0), phi2);
     float d = __fadd_rn(phi0, h);
     if (d > phi1) {
