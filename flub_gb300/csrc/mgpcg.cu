@@ -1394,14 +1394,15 @@ static int enqueue_second_half(flub_mg *mg, const LaunchCtx &c) {
 }
 
 // Blocks of the small CG kernels for the handle: a power of two that holds the groups with
-// one a thread, or 16 with two; 0 where it does not apply.
+// one a thread, or 16 with two; 0 where it does not apply, and with FLUB_NO_CLUSTER=1
+// also where one block would do, so that the separate kernels can be run at every size.
 static int choose_cg_small(const flub_mg *mg) {
-    if (mg->precision != FLUB_PRECISION_FP32 || mg->nz % 8 != 0 || mg->n > kCgSmallMaxCells) return 0;
+    if (mg->precision != FLUB_PRECISION_FP32 || mg->nz % 8 != 0 || mg->n > kCgSmallMaxCells || mg->no_cluster)
+        return 0;
     const int need = (int)((mg->n / 8 + kRedThreads - 1) / kRedThreads);
     int C = 1;
     while (C < need && C < kCgSmallMaxBlocks) C <<= 1;
     if (C == 1) return 1;
-    if (mg->no_cluster) return 0;
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[2];
     coarse_launch_config(C, 0, nullptr, &cfg, attr);
