@@ -101,8 +101,8 @@ __global__ void __launch_bounds__(kRedThreads, 4) k8_matvec_pap(MgState *st, con
         const bool own_m = lane == 0 || gm != g - 1, own_p = lane == 31 || gp != g + 1;
         const bool in_m = kg > 0, in_p = 8 * kg + 8 < D.nz;
         float em = 0.0f, ep = 0.0f;
-        if (own_m && in_m) em = __ldg(c - 1);
-        if (own_p && in_p) ep = __ldg(c + 8);
+        if (own_m && in_m) em = St<float>::ld_in(c - 1);
+        if (own_p && in_p) ep = St<float>::ld_in(c + 8);
         float x[8], n[4][8];
         St<float>::ld8_wide(c, x);
         St<float>::ld8_wide(i + 1 < D.nx ? c + si : c, n[0]);

@@ -331,7 +331,7 @@ __global__ void k_matvec(const float *__restrict__ p, float *__restrict__ Ap, co
 // parity.  kFromZero: z is implicitly 0 before the sweep (first sweep of a
 // level in the V-cycle), the thread then writes both members of its pair.
 template <bool kFromZero>
-__global__ void __launch_bounds__(256) k_smooth_half(float *__restrict__ z, const float *__restrict__ r,
+__global__ void __launch_bounds__(256) k_smooth_half(float *__restrict__ z, const float *r,
                                                      const uint8_t *__restrict__ code, Dims D, int phase,
                                                      unsigned long long *kc) {
     count_kernel(kc);
@@ -366,7 +366,7 @@ __global__ void __launch_bounds__(256) k_smooth_half(float *__restrict__ z, cons
 
 // multigrid/mgpcg.py:94-101 _restrict_mcadams as a gather: the coarse cell
 // sums r + L z of its 8 children in (ii, jj, kk) order; 0 unless coarse fluid.
-__global__ void __launch_bounds__(256) k_restrict(const float *__restrict__ rf, const float *__restrict__ zf,
+__global__ void __launch_bounds__(256) k_restrict(const float *rf, const float *zf,
                                                   const uint8_t *__restrict__ cf, float *__restrict__ rc,
                                                   const uint8_t *__restrict__ cc, Dims C, float scale,
                                                   unsigned long long *kc) {
@@ -405,7 +405,7 @@ __global__ void __launch_bounds__(256) k_restrict(const float *__restrict__ rf, 
 
 // multigrid/mgpcg.py:113-116 _prolongate: z_h += z_2h[I/2], written to zout
 // (zout may equal zin).
-__global__ void __launch_bounds__(256) k_prolong(float *zout, const float *zin, const float *__restrict__ zc, Dims F,
+__global__ void __launch_bounds__(256) k_prolong(float *zout, const float *zin, const float *zc, Dims F,
                                                  unsigned long long *kc) {
     count_kernel(kc);
     const int64_t n = F.n();
@@ -457,7 +457,7 @@ __global__ void __launch_bounds__(256) k_residual_x0(MgState *st, float *__restr
 // guard: 0 always run, 1 skip once the CG loop is finished, 2 run only when
 // an initial guess was given.
 // The count of fluid cells is accumulated as a double (exact below 2^53).
-__global__ void __launch_bounds__(kRedThreads) k_fluid_mean(MgState *st, const float *__restrict__ r,
+__global__ void __launch_bounds__(kRedThreads) k_fluid_mean(MgState *st, const float *r,
                                                             const uint8_t *__restrict__ code, int64_t n,
                                                             double *partials, int guard, unsigned long long *kc) {
     count_kernel(kc);
@@ -496,7 +496,7 @@ __global__ void __launch_bounds__(kRedThreads) k_sub_mean(MgState *st, float *__
 }
 
 // rTr0 and the tolerance (multigrid/mgpcg.py:391-393).
-__global__ void __launch_bounds__(kRedThreads) k_dot_rr0(MgState *st, const float *__restrict__ r, int64_t n,
+__global__ void __launch_bounds__(kRedThreads) k_dot_rr0(MgState *st, const float *r, int64_t n,
                                                          double *partials, unsigned long long *kc) {
     count_kernel(kc);
     double s = 0.0;
@@ -514,8 +514,8 @@ __global__ void __launch_bounds__(kRedThreads) k_dot_rr0(MgState *st, const floa
 }
 
 // z.r after the first preconditioner application; p = z (mgpcg.py:396-401).
-__global__ void __launch_bounds__(kRedThreads) k_dot_zr_init(MgState *st, const float *__restrict__ z,
-                                                             const float *__restrict__ r, float *__restrict__ p,
+__global__ void __launch_bounds__(kRedThreads) k_dot_zr_init(MgState *st, const float *z,
+                                                             const float *r, float *__restrict__ p,
                                                              int64_t n, double *partials, unsigned long long *kc) {
     count_kernel(kc);
     double s = 0.0;
@@ -530,7 +530,7 @@ __global__ void __launch_bounds__(kRedThreads) k_dot_zr_init(MgState *st, const 
 
 // Ap = L p and p.Ap -> alpha (mgpcg.py:410-419).  Guarded: a no-op once the
 // iteration budget is spent or the solve has converged / broken down.
-__global__ void __launch_bounds__(kRedThreads) k_matvec_pap(MgState *st, const float *__restrict__ p,
+__global__ void __launch_bounds__(kRedThreads) k_matvec_pap(MgState *st, const float *p,
                                                             float *__restrict__ Ap, const uint8_t *__restrict__ code,
                                                             Dims D, double *partials, unsigned long long *kc) {
     count_kernel(kc);
@@ -567,7 +567,7 @@ __device__ __forceinline__ void publish_cond(MgState *st, int cond, cudaGraphCon
 // and removed the mean), r.r, convergence test (mgpcg.py:421-446).
 template <bool kUpdate>
 __global__ void __launch_bounds__(kRedThreads) k_update_r_rr(MgState *st, float *__restrict__ r,
-                                                             const float *__restrict__ Ap, int64_t n,
+                                                             const float *Ap, int64_t n,
                                                              double *partials, double *hist,
                                                              cudaGraphConditionalHandle h, int set_cond,
                                                              unsigned long long *kc) {
@@ -599,7 +599,7 @@ __global__ void __launch_bounds__(kRedThreads) k_update_r_rr(MgState *st, float 
 
 // Fraction smoother: r -= alpha Ap only (mean removal and r.r follow).
 __global__ void __launch_bounds__(kRedThreads) k_update_r(MgState *st, float *__restrict__ r,
-                                                          const float *__restrict__ Ap, int64_t n,
+                                                          const float *Ap, int64_t n,
                                                           unsigned long long *kc) {
     count_kernel(kc);
     if (st->it >= st->max_iters || st->converged || st->status) return;
@@ -609,8 +609,8 @@ __global__ void __launch_bounds__(kRedThreads) k_update_r(MgState *st, float *__
 }
 
 // z.r -> beta (mgpcg.py:451-455).
-__global__ void __launch_bounds__(kRedThreads) k_dot_zr_beta(MgState *st, const float *__restrict__ z,
-                                                             const float *__restrict__ r, int64_t n,
+__global__ void __launch_bounds__(kRedThreads) k_dot_zr_beta(MgState *st, const float *z,
+                                                             const float *r, int64_t n,
                                                              double *partials, unsigned long long *kc) {
     count_kernel(kc);
     double s = 0.0;
@@ -627,7 +627,7 @@ __global__ void __launch_bounds__(kRedThreads) k_dot_zr_beta(MgState *st, const 
 
 // x += alpha p; p = z + beta p; it += 1 (mgpcg.py:457-461).
 __global__ void __launch_bounds__(256) k_update_xp(MgState *st, float *__restrict__ x, float *__restrict__ p,
-                                                   const float *__restrict__ z, int64_t n, unsigned long long *kc) {
+                                                   const float *z, int64_t n, unsigned long long *kc) {
     count_kernel(kc);
     const float a = (float)st->alpha, b = (float)st->beta;
     for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x) {
@@ -639,7 +639,7 @@ __global__ void __launch_bounds__(256) k_update_xp(MgState *st, float *__restric
 }
 
 // On convergence: x += alpha p (mgpcg.py:444-446).
-__global__ void __launch_bounds__(256) k_solve_end(MgState *st, float *__restrict__ x, const float *__restrict__ p,
+__global__ void __launch_bounds__(256) k_solve_end(MgState *st, float *__restrict__ x, const float *p,
                                                    int64_t n, unsigned long long *kc) {
     count_kernel(kc);
     if (!st->converged) return;

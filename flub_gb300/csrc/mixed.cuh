@@ -29,7 +29,7 @@ __global__ void __launch_bounds__(256) k8_to_half(MgState *st, const float *__re
     // every group: afterwards rh = r / zscale everywhere (0 off the fluid when r is masked)
     FLUB_ACT_LOOP(g, (const int *)nullptr, (const int *)nullptr, ng) {
         float v[8];
-        St<float>::ld8_ro(r + (g << 3), v);
+        St<float>::ld8_in(r + (g << 3), v);
 #pragma unroll
         for (int m = 0; m < 8; m++) v[m] = __fmul_rn(v[m], hs);
         St<__half>::st8(rh + (g << 3), v);

@@ -26,7 +26,7 @@ __device__ __forceinline__ void residual_row8(const TR *__restrict__ r, const TZ
     const int sj = D.nz, si = D.ny * D.nz;
     const int c0 = g << 3;
     float rv[8];
-    if (kNC) St<TR>::ld8_ro(r + c0, rv); else St<TR>::ld8_cg(r + c0, rv);
+    if (kNC) St<TR>::ld8_in(r + c0, rv); else St<TR>::ld8_cg(r + c0, rv);
     const uint4 wd = load_words8(sw, code, D, i, j, k0, c0);
     if (!words_have_fluid(wd)) {
 #pragma unroll
@@ -37,9 +37,9 @@ __device__ __forceinline__ void residual_row8(const TR *__restrict__ r, const TZ
     const bool hkp = k0 + 8 < D.nz, hkm = k0 > 0;
     float xc[8], xip[8], xim[8], xjp[8], xjm[8];
     auto ld8 = [&](const TZ *p, float o[8]) {
-        if (kNC) St<TZ>::ld8_ro(p, o); else St<TZ>::ld8_cg(p, o);
+        if (kNC) St<TZ>::ld8_in(p, o); else St<TZ>::ld8_cg(p, o);
     };
-    auto ld1 = [&](const TZ *p) { return kNC ? St<TZ>::ld_ro(p) : St<TZ>::ld_cg(p); };
+    auto ld1 = [&](const TZ *p) { return kNC ? St<TZ>::ld_in(p) : St<TZ>::ld_cg(p); };
 #pragma unroll
     for (int m = 0; m < 8; m++) xip[m] = xim[m] = xjp[m] = xjm[m] = 0.0f;
     float xkm = 0.0f, xkp = 0.0f;
@@ -82,8 +82,8 @@ __device__ __forceinline__ void residual_row8_split(const TR *__restrict__ r, co
     const uint32_t ia = __ldg(items + (p ? ng : 0) + g), ib = __ldg(items + (p ? 0 : ng) + g);
     float rv[8], a[4], b[4], n[4][4];
     St<TR>::ld8_any(r + ((size_t)g << 3), rv);
-    St<TZ>::ld4_ro(za, a);
-    St<TZ>::ld4_ro(zb, b);
+    St<TZ>::ld4_in(za, a);
+    St<TZ>::ld4_in(zb, b);
     const bool hip = i + 1 < D.nx, him = i > 0, hjp = j + 1 < D.ny, hjm = j > 0;
 #pragma unroll
     for (int half = 0; half < 2; half++) {
@@ -91,18 +91,18 @@ __device__ __forceinline__ void residual_row8_split(const TR *__restrict__ r, co
         const TZ *zx = half ? zb : za, *zy = half ? za : zb;
         const float *x = half ? b : a, *y = half ? a : b;
         const uint32_t item = half ? ib : ia;
-        St<TZ>::ld4_ro(hip ? zy + si : zx, n[0]);
-        St<TZ>::ld4_ro(him ? zy - si : zx, n[1]);
-        St<TZ>::ld4_ro(hjp ? zy + sj : zx, n[2]);
-        St<TZ>::ld4_ro(hjm ? zy - sj : zx, n[3]);
+        St<TZ>::ld4_in(hip ? zy + si : zx, n[0]);
+        St<TZ>::ld4_in(him ? zy - si : zx, n[1]);
+        St<TZ>::ld4_in(hjp ? zy + sj : zx, n[2]);
+        St<TZ>::ld4_in(hjm ? zy - sj : zx, n[3]);
         float u[4], v[4];
 #pragma unroll
         for (int m = 0; m < 4; m++) u[m] = y[m];
         if (half) {
             v[0] = y[1]; v[1] = y[2]; v[2] = y[3];
-            v[3] = 4 * kg + 4 < hz ? St<TZ>::ld_ro(zy + 4) : x[3];
+            v[3] = 4 * kg + 4 < hz ? St<TZ>::ld_in(zy + 4) : x[3];
         } else {
-            v[0] = kg > 0 ? St<TZ>::ld_ro(zy - 1) : x[0];
+            v[0] = kg > 0 ? St<TZ>::ld_in(zy - 1) : x[0];
             v[1] = y[0]; v[2] = y[1]; v[3] = y[2];
         }
         if (item & kItemSolid) {
@@ -211,7 +211,7 @@ __device__ __forceinline__ void restrict8_pass(TRO *__restrict__ rc, const uint8
 }
 
 template <typename TRI, typename TZI, typename TRO>
-__global__ void __launch_bounds__(256, 4) k_restrict8(const TRI *__restrict__ rf, const TZI *__restrict__ zf,
+__global__ void __launch_bounds__(256, 4) k_restrict8(const TRI *rf, const TZI *zf,
                                                       const uint8_t *__restrict__ cf, const uint16_t *__restrict__ swf,
                                                       TRO *__restrict__ rc,
                                                       const uint8_t *__restrict__ cc, Dims C, float out_scale,
@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(256, 4) k_restrict8(const TRI *__restrict__ rf
 // fluid cells: 127 -> 81 us (32 -> 15 M shared/L1 wavefronts and 70 -> 50 M warp
 // instructions), 0.32 GB of DRAM traffic.
 template <typename TRI, typename TZI, typename TRO>
-__global__ void __launch_bounds__(256, 4) k_restrict8_split(const TRI *__restrict__ rf, const TZI *__restrict__ zf,
+__global__ void __launch_bounds__(256, 4) k_restrict8_split(const TRI *rf, const TZI *zf,
                                                             const uint32_t *__restrict__ items,
                                                             const uint16_t *__restrict__ swf, TRO *__restrict__ rc,
                                                             const uint8_t *__restrict__ cc, Dims C, float out_scale,

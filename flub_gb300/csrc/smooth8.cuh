@@ -148,14 +148,14 @@ __device__ __forceinline__ bool words_have_fluid(const uint4 &u) {
 template <typename TC>
 __device__ __forceinline__ void add_coarse_row8(Row8 &o, const TC *__restrict__ pc, float scale) {
     float cv[4];
-    St<TC>::ld4_ro(pc, cv);
+    St<TC>::ld4_in(pc, cv);
 #pragma unroll
     for (int m = 0; m < 8; m++) o.v[m] = __fadd_rn(o.v[m], __fmul_rn(cv[m >> 1], scale));
 }
 
 template <bool kNC, typename TC>
 __device__ __forceinline__ float coarse_at(const TC *__restrict__ p, float scale) {
-    return __fmul_rn(kNC ? St<TC>::ld_ro(p) : St<TC>::ld_cg(p), scale);
+    return __fmul_rn(kNC ? St<TC>::ld_in(p) : St<TC>::ld_cg(p), scale);
 }
 
 // One cell's red-black update (multigrid/mgpcg.py:72-86 in the reference's
@@ -252,7 +252,7 @@ __device__ __forceinline__ void smooth8_pass(TO *zout, const TI *zin, const TC *
                 const uint4 w8 = words8_from_codes(code, D, i, j, k0, c0);
                 wd = h ? make_uint2(w8.z, w8.w) : make_uint2(w8.x, w8.y);
             }
-            if (kNC) St<TR>::ld4_ro(r + ch, rr); else St<TR>::ld4_cg(r + ch, rr);
+            if (kNC) St<TR>::ld4_in(r + ch, rr); else St<TR>::ld4_cg(r + ch, rr);
             if (!kFromZero) {
                 // z: plain loads (rows of the other colour do not change during the
                 // launch), or L2-only ones where other blocks of the same launch
@@ -275,7 +275,7 @@ __device__ __forceinline__ void smooth8_pass(TO *zout, const TI *zin, const TC *
                     float cv[2];
 #define FLUB_ADD_COARSE(row, p)                                                         \
     {                                                                                   \
-        if (kNC) St<TC>::ld2_ro((p), cv); else St<TC>::ld2_cg((p), cv);                 \
+        if (kNC) St<TC>::ld2_in((p), cv); else St<TC>::ld2_cg((p), cv);                 \
         _Pragma("unroll") for (int mm = 0; mm < 4; mm++)                                \
             row[mm] = __fadd_rn(row[mm], __fmul_rn(cv[mm >> 1], zc_scale));             \
     }

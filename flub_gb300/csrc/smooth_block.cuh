@@ -65,11 +65,11 @@ static inline size_t block_smem(int ti, int h, int ks, int V) {
 template <int V, typename T>
 __device__ __forceinline__ void ld_nat(const T *p, float *o) {
     if constexpr (V == 4)
-        St<T>::ld4_ro(p, o);
+        St<T>::ld4_in(p, o);
     else if constexpr (V == 2)
-        St<T>::ld2_ro(p, o);
+        St<T>::ld2_in(p, o);
     else
-        o[0] = St<T>::ld_ro(p);
+        o[0] = St<T>::ld_in(p);
 }
 template <int V, typename T>
 __device__ __forceinline__ void st_nat(T *p, const float *v) {

@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(256, 4)
             St<TZ>::st4(z + uoff + h, out);
             continue;
         }
-        St<TR>::ld4_ro(rs + uoff + h, rr);
+        St<TR>::ld4_in(rs + uoff + h, rr);
         const bool hip = i + 1 < D.nx, him = i > 0, hjp = j + 1 < D.ny, hjm = j > 0;
         const bool hkm = kg > 0, hkp = 4 * kg + 4 < hz;
         // operands: own z, the other colour's row (i, j) with the element before
@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(256, 4)
             const int cy = D.ny >> 1;  // the coarse level is nx/2 x ny/2 x hz, natural order
             // coarse row (I, J) at K = 4 kg .. 4 kg + 3: the parents of elements h .. h + 3
             auto crow = [&](int ii, int jj, float o[4]) {
-                St<TC>::ld4_ro(zc + ((size_t)((ii >> 1) * cy + (jj >> 1)) * hz + 4 * kg), o);
+                St<TC>::ld4_in(zc + ((size_t)((ii >> 1) * cy + (jj >> 1)) * hz + 4 * kg), o);
             };
             float cc[4], cn[4] = {0.f, 0.f, 0.f, 0.f};
             crow(i, j, cc);
@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(256, 4)
             if (q ? hkp : hkm)
                 edge = __fadd_rn(
                     St<TZI>::ld(zi + voff + h + eo),
-                    __fmul_rn(St<TC>::ld_ro(zc + (size_t)((i >> 1) * cy + (j >> 1)) * hz + 4 * kg + eo), s));
+                    __fmul_rn(St<TC>::ld_in(zc + (size_t)((i >> 1) * cy + (j >> 1)) * hz + 4 * kg + eo), s));
         } else {
             // a neighbour row outside the domain is replaced by the cells
             // themselves: their terms are then 0

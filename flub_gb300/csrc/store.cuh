@@ -1,6 +1,12 @@
 // Storage types of the V-cycle levels: FP32, or FP16 for the mixed-precision
 // preconditioner (values are converted to FP32 on load and all arithmetic is
 // FP32; FP16 rounding happens only on store).
+//
+// ld*_in load what an earlier kernel of the stream wrote: residuals and
+// corrections.  Under programmatic dependent launch a block is resident while
+// that kernel still writes them, so they are not read-only for the kernel's
+// life, as the read-only path (__ldg, and what the compiler makes of const
+// __restrict__ parameters) asks; volatile, they stay behind griddepcontrol.wait.
 #pragma once
 
 #include <cuda_fp16.h>
@@ -15,27 +21,31 @@ struct St;
 template <>
 struct St<float> {
     static __device__ __forceinline__ float ld(const float *p) { return *p; }
-    static __device__ __forceinline__ float ld_ro(const float *p) { return __ldg(p); }
+    static __device__ __forceinline__ float ld_in(const float *p) {
+        float v;
+        asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(__cvta_generic_to_global(p)));
+        return v;
+    }
     static __device__ __forceinline__ void st(float *p, float v) { *p = v; }
     static __device__ __forceinline__ void ld8(const float *p, float o[8]) {
         const float4 a = reinterpret_cast<const float4 *>(p)[0], b = reinterpret_cast<const float4 *>(p)[1];
         o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w; o[4] = b.x; o[5] = b.y; o[6] = b.z; o[7] = b.w;
     }
-    static __device__ __forceinline__ void ld8_ro(const float *p, float o[8]) {
-        const float4 a = __ldg(reinterpret_cast<const float4 *>(p)), b = __ldg(reinterpret_cast<const float4 *>(p) + 1);
-        o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w; o[4] = b.x; o[5] = b.y; o[6] = b.z; o[7] = b.w;
+    static __device__ __forceinline__ void ld8_in(const float *p, float o[8]) {
+        ld4_in(p, o);
+        ld4_in(p + 4, o + 4);
     }
-    static __device__ __forceinline__ void ld4_ro(const float *p, float o[4]) {
-        const float4 a = __ldg(reinterpret_cast<const float4 *>(p));
-        o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w;
+    static __device__ __forceinline__ void ld4_in(const float *p, float *o) {
+        asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
+                     : "=f"(o[0]), "=f"(o[1]), "=f"(o[2]), "=f"(o[3])
+                     : "l"(__cvta_generic_to_global(p)));
     }
     static __device__ __forceinline__ void ld4(const float *p, float o[4]) {
         const float4 a = *reinterpret_cast<const float4 *>(p);
         o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w;
     }
-    static __device__ __forceinline__ void ld2_ro(const float *p, float o[2]) {
-        const float2 a = __ldg(reinterpret_cast<const float2 *>(p));
-        o[0] = a.x; o[1] = a.y;
+    static __device__ __forceinline__ void ld2_in(const float *p, float o[2]) {
+        asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(o[0]), "=f"(o[1]) : "l"(__cvta_generic_to_global(p)));
     }
     static __device__ __forceinline__ void ld2(const float *p, float o[2]) {
         const float2 a = *reinterpret_cast<const float2 *>(p);
@@ -87,7 +97,11 @@ struct St<float> {
 template <>
 struct St<__half> {
     static __device__ __forceinline__ float ld(const __half *p) { return __half2float(*p); }
-    static __device__ __forceinline__ float ld_ro(const __half *p) { return __half2float(__ldg(p)); }
+    static __device__ __forceinline__ float ld_in(const __half *p) {
+        unsigned short u;
+        asm volatile("ld.global.u16 %0, [%1];" : "=h"(u) : "l"(__cvta_generic_to_global(p)));
+        return __half2float(__ushort_as_half(u));
+    }
     static __device__ __forceinline__ void st(__half *p, float v) { *p = __float2half_rn(v); }
     static __device__ __forceinline__ void unpack8(uint4 u, float o[8]) {
         const __half2 *h = reinterpret_cast<const __half2 *>(&u);
@@ -101,12 +115,17 @@ struct St<__half> {
     static __device__ __forceinline__ void ld8(const __half *p, float o[8]) {
         unpack8(*reinterpret_cast<const uint4 *>(p), o);
     }
-    static __device__ __forceinline__ void ld8_ro(const __half *p, float o[8]) {
-        unpack8(__ldg(reinterpret_cast<const uint4 *>(p)), o);
+    static __device__ __forceinline__ void ld8_in(const __half *p, float o[8]) {
+        uint4 u;
+        asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(u.x), "=r"(u.y), "=r"(u.z), "=r"(u.w)
+                     : "l"(__cvta_generic_to_global(p)));
+        unpack8(u, o);
     }
     static __device__ __forceinline__ void ld8_any(const __half *p, float o[8]) { ld8(p, o); }
-    static __device__ __forceinline__ void ld4_ro(const __half *p, float o[4]) {
-        const uint2 u = __ldg(reinterpret_cast<const uint2 *>(p));
+    static __device__ __forceinline__ void ld4_in(const __half *p, float o[4]) {
+        uint2 u;
+        asm volatile("ld.global.v2.u32 {%0, %1}, [%2];" : "=r"(u.x), "=r"(u.y) : "l"(__cvta_generic_to_global(p)));
         const __half2 *h = reinterpret_cast<const __half2 *>(&u);
         const float2 a = __half22float2(h[0]), b = __half22float2(h[1]);
         o[0] = a.x; o[1] = a.y; o[2] = b.x; o[3] = b.y;
@@ -117,8 +136,10 @@ struct St<__half> {
         const float2 a = __half22float2(h[0]), b = __half22float2(h[1]);
         o[0] = a.x; o[1] = a.y; o[2] = b.x; o[3] = b.y;
     }
-    static __device__ __forceinline__ void ld2_ro(const __half *p, float o[2]) {
-        const float2 a = __half22float2(__ldg(reinterpret_cast<const __half2 *>(p)));
+    static __device__ __forceinline__ void ld2_in(const __half *p, float o[2]) {
+        unsigned int u;
+        asm volatile("ld.global.u32 %0, [%1];" : "=r"(u) : "l"(__cvta_generic_to_global(p)));
+        const float2 a = __half22float2(*reinterpret_cast<const __half2 *>(&u));
         o[0] = a.x; o[1] = a.y;
     }
     static __device__ __forceinline__ void ld2(const __half *p, float o[2]) {
