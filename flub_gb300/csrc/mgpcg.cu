@@ -166,9 +166,9 @@ static inline int block_tiles(const Dims D, int ti) {
 }
 
 // Planes of a tile of the blocked smoothing on level l, or 0 where it is not
-// used: level 0 of a mixed-precision handle (its post-smoothing stores FP32),
-// levels one block of the coarse kernel holds, and rows of
-// odd pairs so long that a block has fewer threads than a tile has rows.
+// used: the bottom level (so that rows are 4 k cells), level 0 of a mixed-precision
+// handle (its post-smoothing stores FP32) and levels one block of the coarse kernel
+// holds.
 // Not above 256 tiles either: a tile takes 6 us for four half-sweeps (13,000
 // cycles: 3,000 to load, 7,000 of sweeps bound by shared-memory bandwidth), so
 // on a larger level, full of fluid, waves of them take longer than four
@@ -176,11 +176,9 @@ static inline int block_tiles(const Dims D, int ti) {
 // colour-split storage).
 static int block_planes(const flub_mg *mg, int l) {
     const Dims D{mg->nx >> l, mg->ny >> l, mg->nz >> l};
-    if (mg->tile_ok || D.n() <= kBlockCells || D.n() >= (int64_t)1 << 30 || D.nz % 2 != 0) return 0;
+    if (mg->tile_ok || l + 1 >= mg->levels || D.n() <= kBlockCells || D.n() >= (int64_t)1 << 30) return 0;
     if (D.nx > 4 * 2047 || D.ny > kTJb * 2047 || D.nz > kKB * 1023) return 0;  // packed tile coordinates
-    if (l == 0 && (mg->precision == FLUB_PRECISION_MIXED || mg->levels < 2)) return 0;
-    const int V = row_vector(D.nz);
-    if (kBlockThreads / (block_row(D) / V) < kTJb + 6) return 0;
+    if (l == 0 && mg->precision == FLUB_PRECISION_MIXED) return 0;
     return block_tiles(D, 4) <= 256 ? 4 : 0;
 }
 
@@ -889,22 +887,22 @@ static int tile_side(flub_mg *mg, const LaunchCtx &c, int l, bool post, int iter
 
 // ---------------------------------------------------------------- blocked smoothing (smooth_block.cuh)
 
-template <int V, typename T, int TI, int S>
+template <int V, typename T, int TI, int S, bool kAnyR>
 static int block_launch(const LaunchCtx &c, const Level &L, const BlockArgs &A) {
     const size_t smem = block_smem(TI, S, A.ks, V);
     if (!A.tiles) {  // block_prepare: the kernel's shared-memory limit on this device
-        FLUB_CHECK_CUDA(cudaFuncSetAttribute(k_smooth_block<V, T, TI, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        FLUB_CHECK_CUDA(cudaFuncSetAttribute(k_smooth_block<V, T, TI, S, kAnyR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)block_smem(TI, S, (kKB + 2 * kKHalo) / 2, V)));
         return FLUB_OK;
     }
     const int blocks = L.b_tiles < kNumSMs ? L.b_tiles : kNumSMs;
-    return launch_pdl(k_smooth_block<V, T, TI, S>, dim3(blocks), dim3(kBlockThreads), smem, c, A, c.kc);
+    return launch_pdl(k_smooth_block<V, T, TI, S, kAnyR>, dim3(blocks), dim3(kBlockThreads), smem, c, A, c.kc);
 }
 
-// One launch of `its` red-black iterations (1 or 2).
+// One launch of `its` red-black iterations (1 or 2); top: level 0.
 template <typename T>
-static int block_iterations(const LaunchCtx &c, const Level &L, int its, int mode, bool post, const T *r, const T *zin,
-                            T *zout, const T *zc, float zc_scale, bool prepare = false) {
+static int block_iterations(const LaunchCtx &c, const Level &L, bool top, int its, int mode, bool post, const T *r,
+                            const T *zin, T *zout, const T *zc, float zc_scale, bool prepare = false) {
     BlockArgs A = {};
     A.D = L.D;
     A.tiles = prepare ? nullptr : L.b_list;
@@ -920,13 +918,19 @@ static int block_iterations(const LaunchCtx &c, const Level &L, int its, int mod
     A.first_odd = post ? 0 : 1;
     A.ks = block_row(L.D);
     const int V = row_vector(L.D.nz);
-    if (V == 4) {
-        return its == 2 ? block_launch<4, T, 4, 4>(c, L, A) : block_launch<4, T, 4, 2>(c, L, A);
-    }
+    auto launch = [&](auto v, auto any) {
+        constexpr int kV = decltype(v)::value;
+        constexpr bool kAny = decltype(any)::value;
+        return its == 2 ? block_launch<kV, T, 4, 4, kAny>(c, L, A) : block_launch<kV, T, 4, 2, kAny>(c, L, A);
+    };
+    using std::integral_constant;
     if constexpr (std::is_same<T, float>::value) {
-        if (V == 2) return its == 2 ? block_launch<2, T, 4, 4>(c, L, A) : block_launch<2, T, 4, 2>(c, L, A);
-        return its == 2 ? block_launch<1, T, 4, 4>(c, L, A) : block_launch<1, T, 4, 2>(c, L, A);
+        if (V == 2)
+            return top ? launch(integral_constant<int, 2>{}, std::true_type{})
+                       : launch(integral_constant<int, 2>{}, std::false_type{});
+        if (top) return launch(integral_constant<int, 4>{}, std::true_type{});
     }
+    if (V == 4) return launch(integral_constant<int, 4>{}, std::false_type{});
     return FLUB_ERR_UNSUPPORTED;
 }
 
@@ -937,11 +941,11 @@ static int block_prepare(flub_mg *mg) {
         for (int its = 1; its <= 2 && mg->lv[l].b_ti; its++) {
             if (mg->precision == FLUB_PRECISION_MIXED) {
                 if (mg->lv[l].D.nz % 8 == 0)
-                    FLUB_TRY(block_iterations<__half>(c, mg->lv[l], its, 0, false, nullptr, nullptr, nullptr, nullptr,
-                                                      1.0f, true));
+                    FLUB_TRY(block_iterations<__half>(c, mg->lv[l], l == 0, its, 0, false, nullptr, nullptr, nullptr,
+                                                      nullptr, 1.0f, true));
             } else {
-                FLUB_TRY(block_iterations<float>(c, mg->lv[l], its, 0, false, nullptr, nullptr, nullptr, nullptr, 1.0f,
-                                                 true));
+                FLUB_TRY(block_iterations<float>(c, mg->lv[l], l == 0, its, 0, false, nullptr, nullptr, nullptr,
+                                                 nullptr, 1.0f, true));
             }
         }
     return FLUB_OK;
@@ -952,14 +956,14 @@ static int block_prepare(flub_mg *mg) {
 // z_fin, two iterations a launch; the launches alternate between z_fin and z3
 // so that the last one writes z_fin.
 template <typename T>
-static int block_side(const LaunchCtx &c, const Level &L, bool post, int iters, const T *r, const T *z_pre, T *z_fin,
-                      T *z3, const T *zc, float zc_scale) {
+static int block_side(const LaunchCtx &c, const Level &L, bool top, bool post, int iters, const T *r, const T *z_pre,
+                      T *z_fin, T *z3, const T *zc, float zc_scale) {
     const int launches = (iters + 1) / 2;
     const T *prev = z_pre;
     for (int t = 0; t < launches; t++) {
         T *w = ((launches - 1 - t) % 2 == 0) ? z_fin : z3;
         const int mode = t ? kBlockPlain : (post ? kBlockProlong : kBlockFromZero);
-        FLUB_TRY(block_iterations<T>(c, L, t + 1 == launches && iters % 2 ? 1 : 2, mode, post, r, prev, w, zc,
+        FLUB_TRY(block_iterations<T>(c, L, top, t + 1 == launches && iters % 2 ? 1 : 2, mode, post, r, prev, w, zc,
                                      zc_scale));
         prev = w;
     }
@@ -1052,7 +1056,7 @@ static int enqueue_vcycle(flub_mg *mg, const LaunchCtx &c, const float *r0, floa
         if (TILED_PRE(l)) {
             FLUB_TRY(tile_side(mg, c, l, false, iters, R(l), nullptr, ZP(l), nullptr));
         } else if (BLOCK(l)) {
-            FLUB_TRY(block_side<float>(c, L, false, iters, R(l), nullptr, ZP(l), L.z3, nullptr, 1.0f));
+            FLUB_TRY(block_side<float>(c, L, l == 0, false, iters, R(l), nullptr, ZP(l), L.z3, nullptr, 1.0f));
         } else {
             for (int it = 0; it < iters; it++) {
                 FLUB_TRY(sweep(c, L, 0, it == 0 ? kSweepFromZero : kSweepInPlace, sk, R(l), ZP(l), ZP(l), nullptr));
@@ -1113,7 +1117,7 @@ static int enqueue_vcycle(flub_mg *mg, const LaunchCtx &c, const float *r0, floa
         if (BLOCK(l)) {
             // only tiles with fluid are written: a caller's z0 gets 0 everywhere else first
             if (l == 0 && !z0_clean) FLUB_CHECK_CUDA(cudaMemsetAsync(z0, 0, sizeof(float) * (size_t)mg->n, c.s));
-            FLUB_TRY(block_side<float>(c, L, true, iters, R(l), ZP(l), ZF(l), L.z3, mg->lv[l + 1].z, 1.0f));
+            FLUB_TRY(block_side<float>(c, L, l == 0, true, iters, R(l), ZP(l), ZF(l), L.z3, mg->lv[l + 1].z, 1.0f));
             continue;
         }
         for (int it = 0; it < iters; it++) {
@@ -1153,7 +1157,7 @@ static int enqueue_vcycle_mixed(flub_mg *mg, const LaunchCtx &c, float *z0, bool
             continue;
         }
         if (L.b_ti && sk == 1) {
-            FLUB_TRY(block_side<__half>(c, L, false, iters, L.rh, nullptr, L.z2h, L.z3h, nullptr, 1.0f));
+            FLUB_TRY(block_side<__half>(c, L, l == 0, false, iters, L.rh, nullptr, L.z2h, L.z3h, nullptr, 1.0f));
         } else for (int it = 0; it < iters; it++) {
             FLUB_TRY(sweep8<__half, __half, __half, __half>(c, L, 0, it == 0 ? kSweepFromZero : kSweepInPlace, sk,
                                                             L.rh, L.z2h, L.z2h, nullptr, 1.0f));
@@ -1217,7 +1221,7 @@ static int enqueue_vcycle_mixed(flub_mg *mg, const LaunchCtx &c, float *z0, bool
             continue;
         }
         if (l > 0 && L.b_ti && sk == 1) {
-            FLUB_TRY(block_side<__half>(c, L, true, iters, L.rh, L.z2h, L.zh, L.z3h, zc, 8.0f));
+            FLUB_TRY(block_side<__half>(c, L, l == 0, true, iters, L.rh, L.z2h, L.zh, L.z3h, zc, 8.0f));
             continue;
         }
         for (int it = 0; it < iters; it++) {
@@ -1581,12 +1585,7 @@ static int enqueue_tile_lists(flub_mg *mg, const LaunchCtx &c) {
         q.count = L.b_n;
         tile_blocks += L.b_tiles;
         if (L.sw) continue;  // its items came with its words
-        const int V = row_vector(L.D.nz);
-        const unsigned blocks = blocks_for(L.D.n() / (2 * V), 256);
-        if (V == 2)
-            k_block_items<2><<<blocks, 256, 0, c.s>>>(L.cw, L.D, L.b_items);
-        else
-            k_block_items<1><<<blocks, 256, 0, c.s>>>(L.cw, L.D, L.b_items);
+        k_block_items<2><<<blocks_for(L.D.n() / 4, 256), 256, 0, c.s>>>(L.cw, L.D, l == 0, L.b_items);
         FLUB_CHECK_LAUNCH();
     }
     if (T.n) FLUB_TRY(launch_pdl(k_setup_tiles, dim3(tile_blocks), dim3(128), 0, c, T));
@@ -1919,6 +1918,7 @@ int flub_mg_set_tags(flub_mg *mg, const int32_t *tag, void *stream) {
         q.act = L.act;
         q.act_n = L.act_n;
         q.first = P.blocks;
+        q.part = l == 0;
         P.blocks += (int)((L.D.n() / 8 + kSetupThreads - 1) / kSetupThreads);
     }
     if (P.n) {

@@ -26,6 +26,7 @@ struct SetupLevel {
     uint32_t *items;     // item words (NULL: not kept)
     int *act, *act_n;    // active groups, ascending, and their number
     int first;           // the level's first block
+    bool part;           // items with kItemPart: level 0
 };
 
 struct SetupParams {
@@ -72,7 +73,7 @@ __global__ void __launch_bounds__(kSetupThreads) k_setup_words(const __grid_cons
         }
         if (L.items) {
             uint32_t out[2];
-            item_words<4>(wd, D, i, j, kg << 3, out);
+            item_words<4>(wd, D, i, j, kg << 3, L.part, out);
             L.items[g] = out[0];
             L.items[ng + g] = out[1];
         }

@@ -36,11 +36,14 @@ enum BlockMode { kBlockFromZero = 0, kBlockPlain = 1, kBlockProlong = 2 };
 // What a half-sweep has to know of an item (V cells of one colour in a row),
 // in one word per colour: a nibble per cell with its diagonal count (0: never
 // updated), kItemAny when a count is not 0, kItemSolid when a neighbour does not
-// count although it lies in the domain, and kItemAir when one is air.  Built once by set_tags; an
+// count although it lies in the domain, kItemAir when one is air, and at level 0,
+// whose residual can hold anything off the fluid, kItemPart when some counts are 0 and
+// others not.  Built once by set_tags; an
 // item without kItemSolid needs no stencil words: a neighbour outside the
 // domain is replaced by the cell itself, whose term is then 0.
 constexpr uint32_t kAllCount = 0x1554u;  // sw_ns of a cell whose six neighbours all count
-constexpr uint32_t kItemAny = 1u << 16, kItemSolid = 1u << 17, kItemAir = 1u << 18;
+constexpr uint32_t kItemAny = 1u << 16, kItemSolid = 1u << 17, kItemAir = 1u << 18,
+                   kItemPart = 1u << 19;
 
 struct BlockArgs {
     Dims D;
@@ -66,10 +69,8 @@ template <int V, typename T>
 __device__ __forceinline__ void ld_nat(const T *p, float *o) {
     if constexpr (V == 4)
         St<T>::ld4_in(p, o);
-    else if constexpr (V == 2)
-        St<T>::ld2_in(p, o);
     else
-        o[0] = St<T>::ld_in(p);
+        St<T>::ld2_in(p, o);
 }
 template <int V, typename T>
 __device__ __forceinline__ void st_nat(T *p, const float *v) {
@@ -87,7 +88,8 @@ template <int V>
 __device__ __forceinline__ void block_update(uint32_t item, float *xc, const float *ip, const float *im,
                                              const float *jp, const float *jm, const float *va, const float *vb,
                                              const float *r, const float2 *lut) {
-    constexpr int h = V > 1 ? 1 : 0;
+    static_assert(V % 2 == 0, "two cells at a time");
+    constexpr int h = 1;
 #pragma unroll
     for (int m = 0; m < V; m += 2) {
         const F2 x = f2(xc[m], xc[m + h]);
@@ -108,8 +110,10 @@ __device__ __forceinline__ float as_stored(float v) {
 }
 
 // T: storage of r, z and zc (float, or __half in mixed precision: each update
-// is rounded to it).  TI: planes of a tile.  S: half-sweeps.
-template <int V, typename T, int TI, int S>
+// is rounded to it).  TI: planes of a tile.  S: half-sweeps.  kAnyR: level 0, whose
+// residual can hold anything off the fluid (elsewhere the restriction leaves 0); its
+// test in the other levels' kernels cost 1 % of a solve on rows of 4 k cells.
+template <int V, typename T, int TI, int S, bool kAnyR>
 __global__ void __launch_bounds__(kBlockThreads, 1) k_smooth_block(const BlockArgs A, unsigned long long *kc) {
     constexpr int RI = TI + 2 * S, RJ = kTJb + 2 * S;
     extern __shared__ __align__(16) unsigned char block_smem_[];
@@ -182,10 +186,17 @@ __global__ void __launch_bounds__(kBlockThreads, 1) k_smooth_block(const BlockAr
                 for (int m = 0; m < V; m++) {
                     ze[m] = par ? zn[u][2 * m + 1] : zn[u][2 * m];
                     zo[m] = par ? zn[u][2 * m] : zn[u][2 * m + 1];
+                    re[m] = par ? rn[u][2 * m + 1] : rn[u][2 * m];
+                    ro[m] = par ? rn[u][2 * m] : rn[u][2 * m + 1];
+                }
+                if (kAnyR && ((we[u] | wo[u]) & kItemPart)) {
                     // 0 on the cells that are never updated: their factor 0 would turn a
                     // caller's infinity there into NaN, and an air cell's z is read
-                    re[m] = (we[u] >> (4 * m)) & 7u ? (par ? rn[u][2 * m + 1] : rn[u][2 * m]) : 0.0f;
-                    ro[m] = (wo[u] >> (4 * m)) & 7u ? (par ? rn[u][2 * m] : rn[u][2 * m + 1]) : 0.0f;
+#pragma unroll
+                    for (int m = 0; m < V; m++) {
+                        re[m] = (we[u] >> (4 * m)) & 7u ? re[m] : 0.0f;
+                        ro[m] = (wo[u] >> (4 * m)) & 7u ? ro[m] : 0.0f;
+                    }
                 }
                 if (A.mode == kBlockProlong && in) {
                     // z stays 0 on the cells that are never updated
@@ -320,12 +331,13 @@ __global__ void __launch_bounds__(kBlockThreads, 1) k_smooth_block(const BlockAr
 }
 
 // The item words of the 2 V cells of a row from k0 on, from their stencil words
-// (two in each element of wd).
+// (two in each element of wd).  part: kItemPart is kept.
 template <int V>
-__device__ __forceinline__ void item_words(const uint32_t (&wd)[V], const Dims D, int i, int j, int k0,
+__device__ __forceinline__ void item_words(const uint32_t (&wd)[V], const Dims D, int i, int j, int k0, bool part,
                                            uint32_t (&out)[2]) {
     const int par = (i + j) & 1;
     uint32_t ab[2] = {0u, 0u};  // of the cells k0 + 0, 2, .. and k0 + 1, 3, ..
+    int updated[2] = {0, 0};
 #pragma unroll
     for (int m = 0; m < 2 * V; m++) {
         const uint32_t w = (wd[m >> 1] >> (16 * (m & 1))) & 0xffffu;
@@ -341,24 +353,31 @@ __device__ __forceinline__ void item_words(const uint32_t (&wd)[V], const Dims D
         if (k == 0) inside &= ~4096u;
         uint32_t &o = ab[m & 1];
         o |= d << (4 * (m >> 1));
-        if (d) o |= kItemAny;
+        if (d) {
+            o |= kItemAny;
+            updated[m & 1]++;
+        }
         if (d && ns != inside) o |= kItemSolid;
         if (d && (w & kAllCount)) o |= kItemAir;  // the low bit of a neighbour's code
     }
+#pragma unroll
+    for (int c = 0; c < 2; c++)
+        if (part && updated[c] > 0 && updated[c] < V) ab[c] |= kItemPart;
     out[0] = par ? ab[1] : ab[0];
     out[1] = par ? ab[0] : ab[1];
 }
 
-// The item words of a level whose rows are not whole 8-cell groups (V = 2 or 1).
+// The item words of a level whose rows are not whole 8-cell groups (V = 2).
 template <int V>
-__global__ void __launch_bounds__(256) k_block_items(const uint16_t *__restrict__ cw, Dims D, uint32_t *__restrict__ items) {
+__global__ void __launch_bounds__(256) k_block_items(const uint16_t *__restrict__ cw, Dims D, bool part,
+                                                     uint32_t *__restrict__ items) {
     const int lsegs = D.nz / (2 * V), n = D.nx * D.ny * lsegs;
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
         const int seg = e % lsegs, row = e / lsegs, j = row % D.ny, i = row / D.ny;
         uint32_t wd[V], out[2];
 #pragma unroll
         for (int m = 0; m < V; m++) wd[m] = __ldg(reinterpret_cast<const uint32_t *>(cw) + (int64_t)e * V + m);
-        item_words<V>(wd, D, i, j, 2 * V * seg, out);
+        item_words<V>(wd, D, i, j, 2 * V * seg, part, out);
         items[e] = out[0];
         items[n + e] = out[1];
     }
