@@ -429,6 +429,9 @@ struct BottomCache {
     int upd0;  // bit q: in phase 0 the odd-k cell of pair q is updated
 };
 
+// Whether the cell of stencil word w is updated.
+__device__ __forceinline__ bool bottom_updated(uint32_t w) { return (w & 3u) == kCodeFluid && sw_ns(w) != 0u; }
+
 // r + the fluid neighbours' z of cell c (mask m), in the order above.  All six
 // neighbours are loaded (an excluded one reads the cell itself) so the loads
 // issue together.
@@ -474,24 +477,55 @@ __device__ __forceinline__ void bottom_half64(double *z, const BottomCache &tc, 
     coarse_sync(nthr);
 }
 
+// Where a thread has several of the FP64 bottom's pairs, those with a cell that is
+// updated are listed before the wait on the previous kernel and dealt out from the
+// list: the FP64 pipe takes as long for a warp with one such pair as for a full one,
+// and a warp's pairs run one after the other.  V(2,2) cycles in mixed precision, dam /
+// full of fluid: 96 x 48 x 48 on 3 levels 114 -> 91 / 153 -> 154 us, 64^3 on 3 levels
+// 104 -> 85 / 160 -> 161, 128^3 on 4 levels 144 -> 124 / 228 -> 228.
+// list: room for an index per pair and their number.
+__device__ __forceinline__ void bottom_list(int *list, const uint16_t *cw, int npairs) {
+    const uint32_t *words = reinterpret_cast<const uint32_t *>(cw);
+    int *listed = list + npairs;
+    if (threadIdx.x == 0) *listed = 0;
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    uint32_t next = __ldg(words + threadIdx.x);
+#pragma unroll 1
+    for (int t = threadIdx.x; t - lane < npairs; t += kCoarseThreads) {  // whole warps
+        const uint32_t w2 = next;
+        next = t + kCoarseThreads < npairs ? __ldg(words + t + kCoarseThreads) : 0u;
+        const bool on = bottom_updated(w2 & 0xffffu) || bottom_updated(w2 >> 16);
+        const unsigned who = __ballot_sync(0xffffffffu, on);
+        int at = 0;
+        if (lane == 0) at = atomicAdd(listed, __popc(who));
+        at = __shfl_sync(0xffffffffu, at, 0) + __popc(who & ((1u << lane) - 1u));
+        if (on) list[at] = t;
+    }
+}
+
 // The bottom's 2 x nbottom red-black iterations in FP64, starting from z = 0,
 // then z rounded to FP32 into the split halves.  Not inlined: its FP64
-// registers would otherwise count against the FP32 sweeps.
+// registers would otherwise count against the FP32 sweeps.  list: bottom_list's,
+// of a bottom with more pairs than threads.
 __device__ __noinline__ void coarse_bottom64(double *zd, float *zs, const float *r, int hn, const uint16_t *cw,
-                                             const Dims D, int nbottom) {
+                                             const Dims D, int nbottom, const int *list) {
     const int n = (int)D.n(), hz = D.nz >> 1, npairs = n >> 1;
+    const bool deal = npairs > kCoarseThreads;
     for (int q = threadIdx.x; q < n; q += blockDim.x) zd[q] = 0.0;
+    const uint32_t *words = reinterpret_cast<const uint32_t *>(cw);
+    const int total = deal ? list[npairs] : npairs;
     BottomCache tc;
     tc.upd0 = 0;
 #pragma unroll
     for (int q = 0; q < kBottomPairs; q++) {
-        const int t = threadIdx.x + q * kCoarseThreads;
+        const int e = threadIdx.x + q * kCoarseThreads;
         tc.idx[q] = -1;
         tc.msk[q] = 0;
         tc.r0[q] = tc.r1[q] = 0.0f;
-        if (t < npairs) {
-            const int c = 2 * t, qq = t / hz, j = qq % D.ny, i = qq / D.ny;
-            const uint32_t w2 = __ldg(reinterpret_cast<const uint32_t *>(cw) + t);
+        if (e < total) {
+            const int t = deal ? list[e] : e, c = 2 * t, qq = t / hz, j = qq % D.ny, i = qq / D.ny;
+            const uint32_t w2 = __ldg(words + t);
             tc.idx[q] = c;
             tc.msk[q] = bottom_mask(w2 & 0xffffu) | (bottom_mask(w2 >> 16) << 16);
             tc.r0[q] = r[c];
@@ -501,7 +535,7 @@ __device__ __noinline__ void coarse_bottom64(double *zd, float *zs, const float 
         }
     }
     __syncthreads();
-    const int w = (npairs + 31) & ~31, nthr = w < kCoarseThreads ? w : kCoarseThreads;
+    const int w = (total + 31) & ~31, nthr = w < kCoarseThreads ? w : kCoarseThreads;
     if ((int)threadIdx.x < nthr)
         for (int it = 0; it < 2 * nbottom; it++) {
             const int first = it < nbottom ? 0 : 1;
@@ -827,6 +861,12 @@ __global__ void __launch_bounds__(kCoarseThreads, 1) k_coarse_vcycle(const __gri
     for (int t = 0; t < P.nl; t++) {
         if (t >= P.nd && rank != 0) break;
         const CoarseLevel &L = P.lv[t];
+        if (P.bottom64 && t + 1 == P.nl) {
+            // no weights: their place takes the list of the bottom's pairs (block 0 holds it)
+            const int npairs = (int)(L.D.n() >> 1);
+            if (npairs > kCoarseThreads) bottom_list(reinterpret_cast<int *>(smem + L.off_w), L.cw, npairs);
+            break;
+        }
         const int first = t < P.nd ? (int)rank * L.P : 0, yz = L.D.ny * L.D.nz;
         const int pairs = (max(0, min(L.P, L.D.nx - first)) * yz) >> 1;
         const uint32_t *w2 = reinterpret_cast<const uint32_t *>(L.cw) + ((first * yz) >> 1);
@@ -885,7 +925,7 @@ __global__ void __launch_bounds__(kCoarseThreads, 1) k_coarse_vcycle(const __gri
                 coarse_bottom64(reinterpret_cast<double *>(smem + P.off_zd),
                                 reinterpret_cast<float *>(smem + P.lv[t].off_z),
                                 reinterpret_cast<const float *>(smem + P.lv[t].off_r), P.lv[t].hn, P.lv[t].cw,
-                                P.lv[t].D, P.nbottom);
+                                P.lv[t].D, P.nbottom, reinterpret_cast<const int *>(smem + P.lv[t].off_w));
             else
                 S = coarse_dispatch<kV, kMixed>(P, t, mode, smem, 0u, S);
         }
