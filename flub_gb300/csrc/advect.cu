@@ -12,10 +12,12 @@
 // touches one or two cache lines.  The kernels are bound by instruction issue
 // and L1 gathers, not by HBM: a MacCormack element whose bounds leave no room
 // for the correction takes 144 loads (one trace and one tricubic), else 257.
-// Samples away from the array's ends address their rows from one base.
-// Measured on 256 x 64 x 256 (advect_phi and three face arrays): 1204 us with
-// both traces always taken and every index clamped on its own, 750 us now.
+// On long rows samples away from the array's ends address their rows from one base
+// (by_row).  Measured on 256 x 64 x 256: advect_phi and three face arrays 1207 us with
+// both traces always taken and every index clamped on its own, 754 now; the face arrays
+// alone with minmax_h = 1, where the bounds admit the second trace, 1031 and 912.
 #include <cmath>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -92,6 +94,7 @@ __device__ __forceinline__ float adv_tri8_in(const float *__restrict__ q, int sp
 
 // utils/util.py:34-88 sample_velocity_3d.  The three components share their
 // clamped index pairs where their arrays share an extent.
+template <bool kIn>
 __device__ __forceinline__ AdvF3 adv_velocity(const AdvVel &M, AdvF3 p) {
     const int nx = M.nx, ny = M.ny, nz = M.nz;
     const float s = __fsub_rn(p.x, 0.5f), t = __fsub_rn(p.y, 0.5f), r = __fsub_rn(p.z, 0.5f);
@@ -101,7 +104,7 @@ __device__ __forceinline__ AdvF3 adv_velocity(const AdvVel &M, AdvF3 p) {
     const int is = adv_floor(s), it = adv_floor(t), ir = adv_floor(r);
     AdvF3 o;
     // s = x - 1/2 rounded: is <= iu, so these bound all six indices
-    if (is >= 0 && iu < nx - 1 && it >= 0 && iv < ny - 1 && ir >= 0 && iw < nz - 1) {
+    if (kIn && is >= 0 && iu < nx - 1 && it >= 0 && iv < ny - 1 && ir >= 0 && iw < nz - 1) {
         o.x = adv_tri8_in(M.u, ny * nz, nz, iu, it, ir, fu, ft, fr);
         o.y = adv_tri8_in(M.v, (ny + 1) * nz, nz, is, iv, ir, fs, fv, fr);
         o.z = adv_tri8_in(M.w, ny * (nz + 1), nz + 1, is, it, iw, fs, ft, fw);
@@ -118,14 +121,15 @@ __device__ __forceinline__ AdvF3 adv_velocity(const AdvVel &M, AdvF3 p) {
 
 // advect.py:10-22 backtrace from p with its first velocity sample v1 given
 // (c1, c2, c3: the step factors of the direction traced).
+template <bool kIn>
 __device__ __forceinline__ AdvF3 adv_backtrace_v1(const AdvVel &M, AdvF3 p, AdvF3 v1, float c1, float c2, float c3) {
     const float k1 = 2.0f / 9.0f, k2 = 1.0f / 3.0f, k3 = 4.0f / 9.0f;
     const AdvF3 p1 = {__fsub_rn(p.x, __fmul_rn(c1, v1.x)), __fsub_rn(p.y, __fmul_rn(c1, v1.y)),
                       __fsub_rn(p.z, __fmul_rn(c1, v1.z))};
-    const AdvF3 v2 = adv_velocity(M, p1);
+    const AdvF3 v2 = adv_velocity<kIn>(M, p1);
     const AdvF3 p2 = {__fsub_rn(p.x, __fmul_rn(c2, v2.x)), __fsub_rn(p.y, __fmul_rn(c2, v2.y)),
                       __fsub_rn(p.z, __fmul_rn(c2, v2.z))};
-    const AdvF3 v3 = adv_velocity(M, p2);
+    const AdvF3 v3 = adv_velocity<kIn>(M, p2);
     AdvF3 o;
     o.x = __fsub_rn(p.x, __fmul_rn(c3, __fadd_rn(__fadd_rn(__fmul_rn(k1, v1.x), __fmul_rn(k2, v2.x)),
                                                  __fmul_rn(k3, v3.x))));
@@ -170,10 +174,11 @@ __device__ __forceinline__ void adv_quad(int i0, int hi, int stride, int o[4]) {
 // utils/util.py:148-160 _tricubic (with _bicubic :139-146 and _cubic
 // :131-137) at (s, t, r): cubics along the first axis innermost, then the
 // second, then the third.
+template <bool kIn>
 __device__ __forceinline__ float adv_tricubic(const AdvVol &Q, float s, float t, float r) {
     const AdvW4 wu = adv_cubic_w(adv_fract(s)), wv = adv_cubic_w(adv_fract(t)), ww = adv_cubic_w(adv_fract(r));
     const int is = adv_floor(s), it = adv_floor(t), ir = adv_floor(r);
-    if (is >= 1 && is < Q.gx - 2 && it >= 1 && it < Q.gy - 2 && ir >= 1 && ir < Q.gz - 2) {
+    if (kIn && is >= 1 && is < Q.gx - 2 && it >= 1 && it < Q.gy - 2 && ir >= 1 && ir < Q.gz - 2) {
         // no index is clamped: 16 row addresses, the third axis in immediate offsets
         const int sr = Q.gz, sp = Q.gy * Q.gz;
         const float *base = Q.q + (is * sp + it * sr + ir);
@@ -209,8 +214,9 @@ __device__ __forceinline__ float adv_tricubic(const AdvVol &Q, float s, float t,
 }
 
 // utils/util.py:98-104 trilerp_stagger: the tricubic at p - stagger.
+template <bool kIn>
 __device__ __forceinline__ float adv_sample_stagger(const AdvVol &Q, AdvF3 p, AdvF3 st) {
-    return adv_tricubic(Q, __fsub_rn(p.x, st.x), __fsub_rn(p.y, st.y), __fsub_rn(p.z, st.z));
+    return adv_tricubic<kIn>(Q, __fsub_rn(p.x, st.x), __fsub_rn(p.y, st.y), __fsub_rn(p.z, st.z));
 }
 
 __device__ __forceinline__ float adv_min(float a, float b) { return a < b ? a : b; }
@@ -249,16 +255,16 @@ __device__ __forceinline__ void adv_minmax(const AdvVol &Q, AdvF3 p, float mh, f
 // values stages 1 and 2 wrote, so recomputing them in registers gives the
 // same result without q_tmp).  The traces over dt and -dt start with the
 // same velocity sample, taken once.  One element (i, j, k).
-template <int STAGE>
+template <int STAGE, bool kIn>
 __device__ __forceinline__ void advect_mc_element(const AdvVel &M, const AdvVol &Q, float *__restrict__ q_out,
                                                   float *__restrict__ q_tmp, AdvF3 st, const AdvSteps &C, float mh,
                                                   float inv_mh, int i, int j, int k) {
     const int f = (i * Q.gy + j) * Q.gz + k;
     const AdvF3 p = {__fadd_rn((float)i, st.x), __fadd_rn((float)j, st.y), __fadd_rn((float)k, st.z)};
-    const AdvF3 v1 = adv_velocity(M, p);
+    const AdvF3 v1 = adv_velocity<kIn>(M, p);
     if (STAGE == 1 || STAGE == 2) {
         const int s = STAGE - 1;
-        const float q = adv_sample_stagger(Q, adv_backtrace_v1(M, p, v1, C.c1[s], C.c2[s], C.c3[s]), st);
+        const float q = adv_sample_stagger<kIn>(Q, adv_backtrace_v1<kIn>(M, p, v1, C.c1[s], C.c2[s], C.c3[s]), st);
         (STAGE == 1 ? q_out : q_tmp)[f] = q;
         return;
     }
@@ -271,8 +277,8 @@ __device__ __forceinline__ void advect_mc_element(const AdvVel &M, const AdvVol 
     float q_sl = 0.0f, q_bk = 0.0f, mn = 0.0f, mx = 0.0f;
 #pragma unroll 1
     for (int s = 0; s < (STAGE == 0 ? 2 : 1); s++) {
-        const AdvF3 e = adv_backtrace_v1(M, p, v1, s ? C.c1[1] : C.c1[0], s ? C.c2[1] : C.c2[0], s ? C.c3[1] : C.c3[0]);
-        const float q = adv_sample_stagger(Q, e, st);
+        const AdvF3 e = adv_backtrace_v1<kIn>(M, p, v1, s ? C.c1[1] : C.c1[0], s ? C.c2[1] : C.c2[0], s ? C.c3[1] : C.c3[0]);
+        const float q = adv_sample_stagger<kIn>(Q, e, st);
         if (s == 0) {
             q_sl = q;
             adv_minmax(Q, e, mh, inv_mh, st, mn, mx);
@@ -297,12 +303,12 @@ __device__ __forceinline__ void advect_mc_element(const AdvVel &M, const AdvVol 
 }
 
 // One field.  Grid: row_grid(qx, qy, qz).
-template <int STAGE>
+template <int STAGE, bool kIn>
 __global__ void __launch_bounds__(kRowThreads) k_advect_mc(const AdvVel M, const AdvVol Q, float *__restrict__ q_out,
                                                           float *__restrict__ q_tmp, AdvF3 st, const AdvSteps C,
                                                           float mh, float inv_mh) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < Q.gz) advect_mc_element<STAGE>(M, Q, q_out, q_tmp, st, C, mh, inv_mh, blockIdx.z, blockIdx.y, k);
+    if (k < Q.gz) advect_mc_element<STAGE, kIn>(M, Q, q_out, q_tmp, st, C, mh, inv_mh, blockIdx.z, blockIdx.y, k);
 }
 
 // The three face arrays of the velocity itself in one launch, in planes along
@@ -310,6 +316,7 @@ __global__ void __launch_bounds__(kRowThreads) k_advect_mc(const AdvVel M, const
 // three launches is the latency of one element's chain (with the level set's launch
 // 24 x 12 x 12 45 -> 34 us, 64 x 33 x 41 79 -> 58, 200 x 90 x 201 749 -> 739).
 // Grid: row_grid(3 nx + 1, ny + 1, nz + 1).
+template <bool kIn>
 __global__ void __launch_bounds__(kRowThreads) k_advect_velocity(const AdvVel M, float *__restrict__ u_out,
                                                                 float *__restrict__ v_out, float *__restrict__ w_out,
                                                                 const AdvSteps C, float mh, float inv_mh) {
@@ -321,32 +328,34 @@ __global__ void __launch_bounds__(kRowThreads) k_advect_velocity(const AdvVel M,
                    M.nz + (d == 2 ? 1 : 0)};
     if (j >= Q.gy || k >= Q.gz) return;
     const AdvF3 st = {d == 0 ? 0.0f : 0.5f, d == 1 ? 0.0f : 0.5f, d == 2 ? 0.0f : 0.5f};
-    advect_mc_element<0>(M, Q, d == 0 ? u_out : (d == 1 ? v_out : w_out), nullptr, st, C, mh, inv_mh, i, j, k);
+    advect_mc_element<0, kIn>(M, Q, d == 0 ? u_out : (d == 1 ? v_out : w_out), nullptr, st, C, mh, inv_mh, i, j, k);
 }
 
 // advect.py:39-54 advect_phi: the tricubic sample at the foot of the trace
 // where it lies inside [0, extent) on every axis, else `outside` (the
 // reference writes h0).  Grid: row_grid(px, py, pz).
+template <bool kIn>
 __global__ void __launch_bounds__(kRowThreads) k_advect_phi(const AdvVel M, const AdvVol Q, float *__restrict__ out,
                                                            AdvF3 st, const AdvSteps C, float outside) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, i = blockIdx.z;
     if (k >= Q.gz) return;
     const AdvF3 p0 = {__fadd_rn((float)i, st.x), __fadd_rn((float)j, st.y), __fadd_rn((float)k, st.z)};
-    const AdvF3 p = adv_backtrace_v1(M, p0, adv_velocity(M, p0), C.c1[0], C.c2[0], C.c3[0]);
+    const AdvF3 p = adv_backtrace_v1<kIn>(M, p0, adv_velocity<kIn>(M, p0), C.c1[0], C.c2[0], C.c3[0]);
     const bool in = 0.0f <= p.x && p.x < (float)Q.gx && 0.0f <= p.y && p.y < (float)Q.gy && 0.0f <= p.z &&
                     p.z < (float)Q.gz;
-    out[(i * Q.gy + j) * Q.gz + k] = in ? adv_sample_stagger(Q, p, st) : outside;
+    out[(i * Q.gy + j) * Q.gz + k] = in ? adv_sample_stagger<kIn>(Q, p, st) : outside;
 }
 
 // advect.py:24-37 advect_simple_3d: a cell-centred q traced back from
 // (i+0.5, j+0.5, k+0.5) and sampled trilinearly (utils/util.py:91-96
 // trilerp).  Grid: row_grid(qx, qy, qz).
+template <bool kIn>
 __global__ void __launch_bounds__(kRowThreads) k_advect_simple(const AdvVel M, const AdvVol Q, float *__restrict__ out,
                                                               const AdvSteps C) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, i = blockIdx.z;
     if (k >= Q.gz) return;
     const AdvF3 p0 = {__fadd_rn((float)i, 0.5f), __fadd_rn((float)j, 0.5f), __fadd_rn((float)k, 0.5f)};
-    const AdvF3 p = adv_backtrace_v1(M, p0, adv_velocity(M, p0), C.c1[0], C.c2[0], C.c3[0]);
+    const AdvF3 p = adv_backtrace_v1<kIn>(M, p0, adv_velocity<kIn>(M, p0), C.c1[0], C.c2[0], C.c3[0]);
     const float s = __fsub_rn(p.x, 0.5f), t = __fsub_rn(p.y, 0.5f), r = __fsub_rn(p.z, 0.5f);
     out[(i * Q.gy + j) * Q.gz + k] =
         adv_tri8(Q.q, Q.gy * Q.gz, Q.gz, adv_pair(adv_floor(s), Q.gx - 1), adv_pair(adv_floor(t), Q.gy - 1),
@@ -385,18 +394,36 @@ static inline bool adv_shape_ok(int x, int y, int z) {
     return x > 0 && y > 0 && z > 0 && x < 65536 && y < 65536 && (int64_t)x * y * z < ((int64_t)1 << 31);
 }
 
+// The kernels come with and without the second path for samples away from the array's
+// ends (kIn), whose rows are addressed from one base without clamps.  A warp at either
+// end of a row runs both paths, so it is for long rows: face arrays and a level set of
+// nz = 128 (128 x 96 x 128) 347 us without it and 359 with it, of 201 (200 x 90 x 201)
+// 779 and 738, of 256 (256 x 64 x 256) 818 and 754; 64 x 33 x 41 46 and 56.
+constexpr int kInRow = 160;
+
+template <typename F>
+static void by_row(int nz, F f) {
+    if (nz >= kInRow)
+        f(std::true_type{});
+    else
+        f(std::false_type{});
+}
+
 static int launch_mc(const AdvVel &M, const float *q_in, float *q_out, float *q_tmp, int qx, int qy, int qz, AdvF3 st,
                      float dt, float h, float mh, int stage, cudaStream_t s) {
     const AdvVol Q{q_in, qx, qy, qz};
     const dim3 g = row_grid(qx, qy, qz);
     const AdvSteps C = make_steps(dt, h);
     const float inv = pow2_inverse(mh);
-    switch (stage) {
-        case 0: k_advect_mc<0><<<g, kRowThreads, 0, s>>>(M, Q, q_out, q_tmp, st, C, mh, inv); break;
-        case 1: k_advect_mc<1><<<g, kRowThreads, 0, s>>>(M, Q, q_out, q_tmp, st, C, mh, inv); break;
-        case 2: k_advect_mc<2><<<g, kRowThreads, 0, s>>>(M, Q, q_out, q_tmp, st, C, mh, inv); break;
-        default: k_advect_mc<3><<<g, kRowThreads, 0, s>>>(M, Q, q_out, q_tmp, st, C, mh, inv); break;
-    }
+    by_row(qz, [&](auto in) {
+        constexpr bool kIn = decltype(in)::value;
+        switch (stage) {
+            case 0: k_advect_mc<0, kIn><<<g, kRowThreads, 0, s>>>(M, Q, q_out, q_tmp, st, C, mh, inv); break;
+            case 1: k_advect_mc<1, kIn><<<g, kRowThreads, 0, s>>>(M, Q, q_out, q_tmp, st, C, mh, inv); break;
+            case 2: k_advect_mc<2, kIn><<<g, kRowThreads, 0, s>>>(M, Q, q_out, q_tmp, st, C, mh, inv); break;
+            default: k_advect_mc<3, kIn><<<g, kRowThreads, 0, s>>>(M, Q, q_out, q_tmp, st, C, mh, inv); break;
+        }
+    });
     FLUB_CHECK_LAUNCH();
     return FLUB_OK;
 }
@@ -433,8 +460,10 @@ int flub_advect_velocity_mc(const float *u, const float *v, const float *w, floa
     const AdvVel M = make_vel(u, v, w, nx, ny, nz);
     cudaStream_t s = as_stream(stream);
     if (nx <= 21844) {  // 3 nx + 1 planes fit the grid's third extent
-        k_advect_velocity<<<row_grid(3 * nx + 1, ny + 1, nz + 1), kRowThreads, 0, s>>>(
-            M, u_out, v_out, w_out, make_steps(dt, h), minmax_h, pow2_inverse(minmax_h));
+        by_row(nz, [&](auto in) {
+            k_advect_velocity<decltype(in)::value><<<row_grid(3 * nx + 1, ny + 1, nz + 1), kRowThreads, 0, s>>>(
+                M, u_out, v_out, w_out, make_steps(dt, h), minmax_h, pow2_inverse(minmax_h));
+        });
         FLUB_CHECK_LAUNCH();
         return FLUB_OK;
     }
@@ -454,9 +483,11 @@ int flub_advect_phi(const float *u, const float *v, const float *w, int nx, int 
     FLUB_REQUIRE(adv_shape_ok(nx + 1, ny + 1, nz + 1), "flub_advect_phi: bad velocity grid %dx%dx%d", nx, ny, nz);
     FLUB_REQUIRE(adv_shape_ok(px, py, pz), "flub_advect_phi: bad field shape %dx%dx%d", px, py, pz);
     FLUB_REQUIRE(h > 0.0f, "flub_advect_phi: h must be > 0");
-    k_advect_phi<<<row_grid(px, py, pz), kRowThreads, 0, as_stream(stream)>>>(
-        make_vel(u, v, w, nx, ny, nz), AdvVol{phi, px, py, pz}, phi_out, AdvF3{sx, sy, sz}, make_steps(dt, h),
-        outside);
+    by_row(pz, [&](auto in) {
+        k_advect_phi<decltype(in)::value><<<row_grid(px, py, pz), kRowThreads, 0, as_stream(stream)>>>(
+            make_vel(u, v, w, nx, ny, nz), AdvVol{phi, px, py, pz}, phi_out, AdvF3{sx, sy, sz}, make_steps(dt, h),
+            outside);
+    });
     FLUB_CHECK_LAUNCH();
     return FLUB_OK;
 }
@@ -468,8 +499,10 @@ int flub_advect_simple(const float *u, const float *v, const float *w, int nx, i
     FLUB_REQUIRE(adv_shape_ok(nx + 1, ny + 1, nz + 1), "flub_advect_simple: bad velocity grid %dx%dx%d", nx, ny, nz);
     FLUB_REQUIRE(adv_shape_ok(qx, qy, qz), "flub_advect_simple: bad field shape %dx%dx%d", qx, qy, qz);
     FLUB_REQUIRE(h > 0.0f, "flub_advect_simple: h must be > 0");
-    k_advect_simple<<<row_grid(qx, qy, qz), kRowThreads, 0, as_stream(stream)>>>(
-        make_vel(u, v, w, nx, ny, nz), AdvVol{q, qx, qy, qz}, q_out, make_steps(dt, h));
+    by_row(qz, [&](auto in) {
+        k_advect_simple<decltype(in)::value><<<row_grid(qx, qy, qz), kRowThreads, 0, as_stream(stream)>>>(
+            make_vel(u, v, w, nx, ny, nz), AdvVol{q, qx, qy, qz}, q_out, make_steps(dt, h));
+    });
     FLUB_CHECK_LAUNCH();
     return FLUB_OK;
 }
