@@ -121,6 +121,7 @@ __global__ void __launch_bounds__(kTj * kTk) k_extrapolate_tile(float *__restric
 constexpr int kPi = 8, kPj = 8, kPk = 128, kPWords = kPk / 32;
 constexpr int kPRows = (kPi + 2) * (kPj + 2);
 constexpr int kPThreads = kPi * kPj * kPWords;  // one word each in the second step
+constexpr int64_t kFusedCells = 1 << 22;        // above: see flub_extrapolate
 
 struct ExtrapArgs {
     float *q[3];
@@ -236,8 +237,9 @@ __global__ void __launch_bounds__(kPThreads) k_extrapolate_phi(const ExtrapArgs 
             patched = last;
         }
         const int fx = A.nx + (d == 0), fy = A.ny + (d == 1), fz = A.nz + (d == 2);
-        float *q = A.q[d];
-        int32_t *t = A.t[d];
+        // (indexed by d the parameters went through local memory)
+        float *q = d == 0 ? A.q[0] : (d == 1 ? A.q[1] : A.q[2]);
+        int32_t *t = d == 0 ? A.t[0] : (d == 1 ? A.t[1] : A.t[2]);
         for (int o = warp; o < kPi * kPj; o += kPThreads / 32) {
             const int i = i0 + o / kPj, j = j0 + o % kPj;
             if (i >= fx || j >= fy) continue;
@@ -255,7 +257,8 @@ __global__ void __launch_bounds__(kPThreads) k_extrapolate_phi(const ExtrapArgs 
                 if (!((td & nr) >> lane & 1u)) continue;
                 int n = 0;
                 float s = 0.0f;
-                // nine loads at a time in flight, summed in (ii, jj, kk) order
+                // nine loads at a time in flight, summed in (ii, jj, kk) order; a face that is
+                // not known adds +0, which leaves the sum (never -0) as it is
 #pragma unroll 1
                 for (int ii = -1; ii <= 1; ii++) {
                     float v[9];
@@ -263,9 +266,8 @@ __global__ void __launch_bounds__(kPThreads) k_extrapolate_phi(const ExtrapArgs 
 #pragma unroll
                     for (int jj = -1; jj <= 1; jj++) {
                         const uint32_t *r = T.known[rc + ii * (kPj + 2) + jj] + w;
-                        const uint64_t bits =
-                            (uint64_t)(r[0] >> 31) | ((uint64_t)r[1] << 1) | ((uint64_t)(r[2] & 1u) << 33);
-                        const unsigned b3 = (unsigned)(bits >> lane) & 7u;  // the row's faces k - 1, k, k + 1
+                        const unsigned b3 =  // the row's faces k - 1, k, k + 1
+                            __funnelshift_r(__funnelshift_l(r[0], r[1], 1), __funnelshift_l(r[1], r[2], 1), lane) & 7u;
                         const float *qr = q + f + 32 * w + ((int64_t)ii * fy + jj) * fz;
                         have |= b3 << (3 * (jj + 1));
 #pragma unroll
@@ -273,8 +275,7 @@ __global__ void __launch_bounds__(kPThreads) k_extrapolate_phi(const ExtrapArgs 
                     }
                     n += __popc(have);
 #pragma unroll
-                    for (int m = 0; m < 9; m++)
-                        if (have & (1u << m)) s = __fadd_rn(s, v[m]);
+                    for (int m = 0; m < 9; m++) s = __fadd_rn(s, v[m]);
                 }
                 q[f + 32 * w] = __fdiv_rn(s, (float)n);
             }
@@ -335,15 +336,25 @@ int flub_extrapolate(float *u, float *v, float *w, int32_t *tu, int32_t *tv, int
     // 1), never writes a known face and reads no other, so every further pass
     // writes the values the first one wrote: one pass gives the result of
     // n_passes >= 1 for any input.
-    if (phi && n_passes > 0) {
+    //
+    // The fused kernel reads the level set once and touches few faces away from the
+    // interface, but near it loads every neighbour from the caches, with few blocks on
+    // a small grid; the tiles have them in shared memory.  Set-up and tiles against
+    // fused, a dam / white noise (an interface everywhere): 64^3 38 / 40 us and 64 / 72,
+    // 128 x 96 x 128 64 / 87 and 97 / 147, 256 x 64 x 256 116 / 178 and 108 / 233,
+    // 172^3 150 / 228 and 110 / 232, 256^3 383 / 619 and 199 / 628.
+    if (phi && n_passes > 0 && (int64_t)nx * ny * nz > kFusedCells) {
         ExtrapArgs A{{u, v, w}, {tu, tv, tw}, phi, nx, ny, nz};
         k_extrapolate_phi<<<dim3((unsigned)(nz / kPk + 1), (unsigned)(ny / kPj + 1), (unsigned)(nx / kPi + 1)),
                             kPThreads, 0, s>>>(A);
         FLUB_CHECK_LAUNCH();
-    } else if (phi) {
+        return FLUB_OK;
+    }
+    if (phi) {
         k_set_unknown<<<row_grid(nx, ny, nz), kRowThreads, 0, s>>>(phi, tu, tv, tw, nx, ny, nz);
         FLUB_CHECK_LAUNCH();
-    } else if (n_passes > 0) {
+    }
+    if (n_passes > 0) {
         k_extrapolate_tile<false><<<tile_grid(nx + 1, ny, nz), dim3(kTk, kTj), 0, s>>>(u, tu, nx + 1, ny, nz);
         FLUB_CHECK_LAUNCH();
         k_extrapolate_tile<false><<<tile_grid(nx, ny + 1, nz), dim3(kTk, kTj), 0, s>>>(v, tv, nx, ny + 1, nz);
