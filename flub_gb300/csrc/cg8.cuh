@@ -16,8 +16,6 @@
 
 namespace flub {
 
-__device__ __forceinline__ bool group_has_fluid(uint2 c) { return ((c.x | c.y) & 0x02020202u) != 0u; }
-
 // L x for the 8 cells of the row starting at c0 (group g), same operation
 // order as lap_at, from the stencil words of the row (sw, or the codes when sw
 // is NULL).  Non-fluid cells get 0.

@@ -262,11 +262,7 @@ __device__ __forceinline__ void group_ijk(int g, const Dims D, int &i, int &j, i
 // (in the 256^3 dam break 20 % of the groups are active).  Built once per
 // set_tags in three deterministic passes (setup_levels.cuh): per-block counts,
 // one-block scan, ordered write.
-__device__ __forceinline__ bool group_active(const uint8_t *__restrict__ code, int g) {
-    const uint2 c = __ldg(reinterpret_cast<const uint2 *>(code + ((int64_t)g << 3)));
-    return ((c.x | c.y) & 0x02020202u) != 0u;  // a fluid byte (code 2) among the 8
-}
-
+//
 // Loop over the groups a kernel works on: the active list when act is not
 // NULL (its length read from *act_n on the device), else every group 0..ng-1.
 #define FLUB_ACT_LOOP(g, act, act_n, ng)                                                                   \

@@ -58,7 +58,7 @@ __global__ void __launch_bounds__(kSetupThreads) k_setup_words(const __grid_cons
     if (g < ng) {
         int i, j, kg;
         group_ijk(g, D, i, j, kg);
-        const uint4 u = words8_from_codes(L.code, D, i, j, kg << 3, g << 3);
+        const uint4 u = words8_from_codes<true>(L.code, D, i, j, kg << 3, g << 3);
         fluid = words_have_fluid(u);
         *reinterpret_cast<uint4 *>(L.sw + ((int64_t)g << 3)) = u;
         const uint32_t wd[4] = {u.x, u.y, u.z, u.w};
@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(kSetupThreads) k_setup_write(const __grid_cons
     setup_open();
     const SetupLevel &L = P.lv[setup_level(P, blockIdx.x)];
     const int g = ((int)blockIdx.x - L.first) * kSetupThreads + (int)threadIdx.x;
-    const bool f = g < (int)(L.D.n() >> 3) && group_active(L.code, g);
+    const bool f = g < (int)(L.D.n() >> 3) && group_has_fluid(load_codes8<true>(L.code + ((int64_t)g << 3)));
     const unsigned m = __ballot_sync(0xffffffffu, f);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (lane == 0) wcount[warp] = __popc(m);
@@ -191,8 +191,7 @@ __global__ void __launch_bounds__(kSetupThreads) k_setup_clear(const __grid_cons
 // k_restrict_codes for fine rows of whole 8-cell groups: four coarse cells a
 // thread.  With solid 0, air 1 and fluid 2 the bitwise or of the 8 children has bit
 // 0 for air and bit 1 for fluid.
-__global__ void __launch_bounds__(256) k_restrict_codes8(const uint8_t *__restrict__ cf, uint8_t *__restrict__ cc,
-                                                         Dims C) {
+__global__ void __launch_bounds__(256) k_restrict_codes8(const uint8_t *cf, uint8_t *cc, Dims C) {
     setup_open();
     const int n4 = (int)(C.n() >> 2);
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n4; q += gridDim.x * blockDim.x) {
@@ -200,8 +199,8 @@ __global__ void __launch_bounds__(256) k_restrict_codes8(const uint8_t *__restri
         group_ijk(q, Dims{C.nx, C.ny, C.nz << 1}, I, J, K4);  // the coarse grid read as 4-cell groups
         const int fz = 2 * C.nz, fy = 2 * C.ny;
         const uint8_t *r = cf + ((int64_t)(2 * I) * fy + 2 * J) * fz + 8 * K4;
-        const uint2 a = load_codes8(r), b = load_codes8(r + fz), c = load_codes8(r + (int64_t)fy * fz),
-                    d = load_codes8(r + (int64_t)fy * fz + fz);
+        const uint2 a = load_codes8<true>(r), b = load_codes8<true>(r + fz),
+                    c = load_codes8<true>(r + (int64_t)fy * fz), d = load_codes8<true>(r + (int64_t)fy * fz + fz);
         const uint32_t x = a.x | b.x | c.x | d.x, y = a.y | b.y | c.y | d.y;
         const uint32_t v = __byte_perm(x | (x >> 8), y | (y >> 8), 0x6420);
         const uint32_t air = v & 0x01010101u;

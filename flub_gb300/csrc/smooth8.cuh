@@ -36,9 +36,30 @@ __device__ __forceinline__ void zero_row8(Row8 &o) {
     for (int m = 0; m < 8; m++) o.v[m] = 0.0f;
 }
 
-__device__ __forceinline__ uint2 load_codes8(const uint8_t *__restrict__ p) {
+// kSetup: in a kernel of set_tags, whose blocks may be resident while an earlier one
+// still writes the codes (see St::ld_in in store.cuh).
+template <bool kSetup = false>
+__device__ __forceinline__ uint2 load_codes8(const uint8_t *p) {
+    if constexpr (kSetup) {
+        uint2 v;
+        asm volatile("ld.global.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(__cvta_generic_to_global(p)));
+        return v;
+    }
     return __ldg(reinterpret_cast<const uint2 *>(p));
 }
+
+template <bool kSetup = false>
+__device__ __forceinline__ uint32_t load_code(const uint8_t *p) {
+    if constexpr (kSetup) {
+        uint32_t v;
+        asm volatile("ld.global.u8 %0, [%1];" : "=r"(v) : "l"(__cvta_generic_to_global(p)));
+        return v;
+    }
+    return __ldg(p);
+}
+
+// A fluid byte (code 2) among the 8.
+__device__ __forceinline__ bool group_has_fluid(uint2 c) { return ((c.x | c.y) & 0x02020202u) != 0u; }
 
 __device__ __forceinline__ uint8_t code_at(uint2 c, int m) {
     return (uint8_t)(((m < 4 ? c.x : c.y) >> (8 * (m & 3))) & 0xffu);
@@ -111,17 +132,17 @@ __device__ __forceinline__ uint32_t word_at(const uint4 &u, int m) {
 }
 
 // Words of the 8 cells of the row starting at c0 = (i, j, k0), from the codes.
-__device__ __forceinline__ uint4 words8_from_codes(const uint8_t *__restrict__ code, const Dims D, int i, int j,
-                                                   int k0, int c0) {
+template <bool kSetup = false>
+__device__ __forceinline__ uint4 words8_from_codes(const uint8_t *code, const Dims D, int i, int j, int k0, int c0) {
     const int sj = D.nz, si = D.ny * D.nz;
     const uint2 z2 = make_uint2(0u, 0u);
-    const uint2 cc = load_codes8(code + c0);
-    const uint2 cip = i + 1 < D.nx ? load_codes8(code + c0 + si) : z2;
-    const uint2 cim = i > 0 ? load_codes8(code + c0 - si) : z2;
-    const uint2 cjp = j + 1 < D.ny ? load_codes8(code + c0 + sj) : z2;
-    const uint2 cjm = j > 0 ? load_codes8(code + c0 - sj) : z2;
-    const uint32_t ckm = k0 > 0 ? __ldg(code + c0 - 1) : 0u;
-    const uint32_t ckp = k0 + 8 < D.nz ? __ldg(code + c0 + 8) : 0u;
+    const uint2 cc = load_codes8<kSetup>(code + c0);
+    const uint2 cip = i + 1 < D.nx ? load_codes8<kSetup>(code + c0 + si) : z2;
+    const uint2 cim = i > 0 ? load_codes8<kSetup>(code + c0 - si) : z2;
+    const uint2 cjp = j + 1 < D.ny ? load_codes8<kSetup>(code + c0 + sj) : z2;
+    const uint2 cjm = j > 0 ? load_codes8<kSetup>(code + c0 - sj) : z2;
+    const uint32_t ckm = k0 > 0 ? load_code<kSetup>(code + c0 - 1) : 0u;
+    const uint32_t ckp = k0 + 8 < D.nz ? load_code<kSetup>(code + c0 + 8) : 0u;
     uint32_t w[8];
 #pragma unroll
     for (int m = 0; m < 8; m++)
