@@ -946,13 +946,13 @@ __global__ void __launch_bounds__(kCoarseThreads, 1) k_coarse_vcycle(const __gri
 
 // Stencil words of every cell of a level, natural order, for any nz (the same
 // words as words8_from_codes).
-__global__ void __launch_bounds__(256) k_cell_words(const uint8_t *__restrict__ code, uint16_t *__restrict__ cw,
-                                                    Dims D) {
+__global__ void __launch_bounds__(256) k_cell_words(const uint8_t *code, uint16_t *cw, Dims D) {
+    setup_open();
     const int n = (int)D.n(), sj = D.nz, si = D.ny * D.nz;
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
         const int k = c % D.nz, j = (c / D.nz) % D.ny, i = c / si;
         auto nb = [&](bool in, int off, int q) -> uint32_t {
-            return in ? (uint32_t)__ldg(code + c + off) << (2 * q) : 0u;
+            return in ? (uint32_t)code[c + off] << (2 * q) : 0u;
         };
         cw[c] = (uint16_t)((uint32_t)code[c] | nb(i + 1 < D.nx, si, 1) | nb(i > 0, -si, 2) | nb(j + 1 < D.ny, sj, 3) |
                            nb(j > 0, -sj, 4) | nb(k + 1 < D.nz, 1, 5) | nb(k > 0, -1, 6));

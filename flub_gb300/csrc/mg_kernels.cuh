@@ -96,6 +96,12 @@ __device__ __forceinline__ double dot8_ff(const float *x, const float *y) {
 // and pdl_wait then waits for the previous kernel's results.
 __device__ __forceinline__ void pdl_open() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// The kernels of set_tags, which read what the one before them writes.
+__device__ __forceinline__ void setup_open() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 __device__ __forceinline__ void pdl_wait(unsigned long long *kc) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (kc && (blockIdx.x | blockIdx.y | blockIdx.z | threadIdx.x | threadIdx.y | threadIdx.z) == 0)
@@ -220,7 +226,8 @@ __global__ void k_encode_tags4(const int4 *__restrict__ tag, uint32_t *__restric
 }
 
 // multigrid/mgpcg.py:162-174 restrict_tag on cell codes.
-__global__ void k_restrict_codes(const uint8_t *__restrict__ cf, uint8_t *__restrict__ cc, Dims C) {
+__global__ void k_restrict_codes(const uint8_t *cf, uint8_t *cc, Dims C) {
+    setup_open();
     const int64_t n = C.n();
     const Dims F{2 * C.nx, 2 * C.ny, 2 * C.nz};
     for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.x * blockDim.x) {

@@ -1555,12 +1555,12 @@ static int read_info(flub_mg *mg, cudaStream_t s, flub_solve_info *info) {
 
 // Stencil words of the levels the coarse kernel or the blocked smoothing runs
 // whose rows are not whole 8-cell groups (the others' are Level::sw).
-static int enqueue_cell_words(flub_mg *mg, cudaStream_t s) {
+static int enqueue_cell_words(flub_mg *mg, const LaunchCtx &c) {
     for (int l = 0; l < mg->levels; l++) {
         const Level &L = mg->lv[l];
         if (!L.cw || L.sw || (l < mg->co_start && !L.b_ti)) continue;
-        k_cell_words<<<blocks_for(L.D.n(), 256), 256, 0, s>>>(L.code, L.cw, L.D);
-        FLUB_CHECK_LAUNCH();
+        FLUB_TRY(launch_pdl(k_cell_words, dim3(blocks_for(L.D.n(), 256)), dim3(256), 0, c, (const uint8_t *)L.code,
+                            L.cw, L.D));
     }
     return FLUB_OK;
 }
@@ -1585,8 +1585,8 @@ static int enqueue_tile_lists(flub_mg *mg, const LaunchCtx &c) {
         q.count = L.b_n;
         tile_blocks += L.b_tiles;
         if (L.sw) continue;  // its items came with its words
-        k_block_items<2><<<blocks_for(L.D.n() / 4, 256), 256, 0, c.s>>>(L.cw, L.D, l == 0, L.b_items);
-        FLUB_CHECK_LAUNCH();
+        FLUB_TRY(launch_pdl(k_block_items<2>, dim3(blocks_for(L.D.n() / 4, 256)), dim3(256), 0, c,
+                            (const uint16_t *)L.cw, L.D, l == 0, L.b_items));
     }
     if (T.n) FLUB_TRY(launch_pdl(k_setup_tiles, dim3(tile_blocks), dim3(128), 0, c, T));
     return FLUB_OK;
@@ -1869,10 +1869,10 @@ int flub_mg_set_tags(flub_mg *mg, const int32_t *tag, void *stream) {
                                 (const uint8_t *)mg->lv[l].code, C.code, C.D));
             continue;
         }
-        k_restrict_codes<<<blocks_for(C.D.n(), 256), 256, 0, s>>>(mg->lv[l].code, C.code, C.D);
-        FLUB_CHECK_LAUNCH();
+        FLUB_TRY(launch_pdl(k_restrict_codes, dim3(blocks_for(C.D.n(), 256)), dim3(256), 0, c,
+                            (const uint8_t *)mg->lv[l].code, C.code, C.D));
     }
-    FLUB_TRY(enqueue_cell_words(mg, s));
+    FLUB_TRY(enqueue_cell_words(mg, c));
     // new tags: re-establish z = p = Ap = 0 off the fluid (the kernels skip
     // 8-cell groups without fluid and rely on it), and the tiles' count
     ClearParams clear = {};
@@ -2082,7 +2082,7 @@ int flub_mg_set_bottom_precision(flub_mg *mg, int bits) {
         const LaunchCtx c{nullptr, nullptr, 0, 0};
         for (int l = 0; l < mg->levels; l++)
             if (mg->lv[l].b_n) FLUB_CHECK_CUDA(cudaMemsetAsync(mg->lv[l].b_n, 0, sizeof(int), c.s));
-        FLUB_TRY(enqueue_cell_words(mg, c.s));
+        FLUB_TRY(enqueue_cell_words(mg, c));
         FLUB_TRY(enqueue_tile_lists(mg, c));
         FLUB_CHECK_CUDA(cudaDeviceSynchronize());
     }
@@ -2334,7 +2334,8 @@ extern "C" int flub_vcycle_noalloc(const int32_t *tag, const float *r, float *z,
         k_restrict_codes<<<blocks_for(C.D.n(), 256), 256, 0, s>>>(mg.lv[l].code, C.code, C.D);
         FLUB_CHECK_LAUNCH();
     }
-    FLUB_TRY(enqueue_cell_words(&mg, s));
-    LaunchCtx c{s, nullptr, 0, 0, true};  // follows the words directly
+    LaunchCtx c{s, nullptr, 0, 0};
+    FLUB_TRY(enqueue_cell_words(&mg, c));
+    c.ordinary = true;  // the V-cycle follows the words directly
     return enqueue_vcycle(&mg, c, r, z, false);  // mg.skip_ok is false: every sweep writes every cell
 }

@@ -35,11 +35,6 @@ struct SetupParams {
     int *bcount;    // active groups per block, then their exclusive sums within a level
 };
 
-__device__ __forceinline__ void setup_open() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-
 template <typename P>
 __device__ __forceinline__ int setup_level(const P &p, int block) {
     int l = 0;

@@ -369,14 +369,14 @@ __device__ __forceinline__ void item_words(const uint32_t (&wd)[V], const Dims D
 
 // The item words of a level whose rows are not whole 8-cell groups (V = 2).
 template <int V>
-__global__ void __launch_bounds__(256) k_block_items(const uint16_t *__restrict__ cw, Dims D, bool part,
-                                                     uint32_t *__restrict__ items) {
+__global__ void __launch_bounds__(256) k_block_items(const uint16_t *cw, Dims D, bool part, uint32_t *items) {
+    setup_open();
     const int lsegs = D.nz / (2 * V), n = D.nx * D.ny * lsegs;
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
         const int seg = e % lsegs, row = e / lsegs, j = row % D.ny, i = row / D.ny;
         uint32_t wd[V], out[2];
 #pragma unroll
-        for (int m = 0; m < V; m++) wd[m] = __ldg(reinterpret_cast<const uint32_t *>(cw) + (int64_t)e * V + m);
+        for (int m = 0; m < V; m++) wd[m] = reinterpret_cast<const uint32_t *>(cw)[(int64_t)e * V + m];
         item_words<V>(wd, D, i, j, 2 * V * seg, part, out);
         items[e] = out[0];
         items[n + e] = out[1];
