@@ -91,9 +91,9 @@ struct LaunchCtx {
     // The next launch is an ordinary one, which starts when everything before it
     // on the stream has finished, and clears this.  The solver's kernels read what
     // new tags set up (lists, words, codes) before they wait for the kernel in
-    // front of them; a call that may follow flub_mg_set_tags with no ordinary launch
-    // between would otherwise start while the set-up kernels, which let their
-    // dependents in at once, still write it.
+    // front of them; the first call behind flub_mg_set_tags (behind_tags) would
+    // otherwise start while the set-up kernels, which let their dependents in at
+    // once, still write it.
     mutable bool ordinary = false;
 };
 
@@ -121,6 +121,7 @@ struct flub_mg {
     // FLUB_NO_CLUSTER=1 and FLUB_COARSE_FP16=0 when the handle was created: what
     // they decide is looked at again whenever a graph is captured
     bool no_cluster, no_coarse_fp16;
+    bool tags_new;  // set_tags has run and no V-cycle or sweep has been enqueued since (see behind_tags)
     int cg_blocks;  // blocks of the CG step in one cluster (cg_small.cuh), 0: the four kernels
     bool skip_ok;   // internal z buffers keep z = 0 off the fluid (see k_smooth8)
     bool tile_ok;   // the TMA-tiled smoother runs where a level has tiles (FLUB_TILE=1)
@@ -1592,6 +1593,52 @@ static int enqueue_tile_lists(flub_mg *mg, const LaunchCtx &c) {
     return FLUB_OK;
 }
 
+// Runs f with a context whose first launch is an ordinary one where set_tags may be
+// directly in front of it: behind new tags, and while a graph is captured, which may
+// hold a set_tags and runs at another time.  (On every call it cost 2.7 us of the 10.7
+// of a level-0 iteration of the 256^3 dam break.)
+template <typename F>
+static int behind_tags(flub_mg *mg, void *stream, F f) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    const bool live = cudaStreamIsCapturing(as_stream(stream), &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone;
+    if (!live) cudaGetLastError();
+    const LaunchCtx c{as_stream(stream), nullptr, 0, 0, mg->tags_new || !live};
+    const int st = f(c);
+    if (live && !c.ordinary) mg->tags_new = false;
+    return st;
+}
+
+// flub_mg_smooth_iteration's launches.
+static int smooth_iteration(flub_mg *mg, const LaunchCtx &c, int level, int phase, int *tiled) {
+    const Level &L = mg->lv[level];
+    const bool t = mg->tile_ok && L.n_tiles > 0 && mg->skip_ok;
+    if (tiled) *tiled = t ? 1 : 0;
+    if (!t && level == 0 && L.sws && mg->skip_ok) {
+        // the colour-split kernels the V-cycle runs at level 0, in place on the
+        // post-smoothing buffer with the split residual of the last V-cycle
+        if (tiled) *tiled = 2;
+        for (int ph : {phase, 1 - phase}) {
+            if (mg->precision == FLUB_PRECISION_MIXED)
+                FLUB_TRY((split_sweep<kInPlace, __half, __half, float, float, float>(
+                    c, L, ph, nullptr, L.rsh, nullptr, L.zs, nullptr, 1.0f, nullptr)));
+            else
+                FLUB_TRY((split_sweep<kInPlace, float, float, float, float, float>(c, L, ph, nullptr, L.rs, nullptr,
+                                                                                  L.zs, nullptr, 1.0f, nullptr)));
+        }
+        return FLUB_OK;
+    }
+    if (t) {
+        // z -> z3 and z3 -> z on alternate calls (both keep 0 off the fluid);
+        // the handle's pointers stay as the captured solve graphs know them
+        const bool back = mg->iter_toggle[level];
+        mg->iter_toggle[level] = !back;
+        return tile_iteration(mg, c, level, phase, kTileInPlaceInput, L.r, back ? L.z3 : L.z, back ? L.z : L.z3,
+                              nullptr);
+    }
+    FLUB_TRY(sweep(c, L, phase, kSweepInPlace, mg->skip_ok ? 1 : 0, L.r, L.z, L.z, nullptr));
+    return sweep(c, L, 1 - phase, kSweepInPlace, mg->skip_ok ? 1 : 0, L.r, L.z, L.z, nullptr);
+}
+
 // ---------------------------------------------------------------- warm-start support (no reference counterpart)
 
 __global__ void k_set_x0_scale(MgState *st, double v) { st->x0_scale = v; }
@@ -1853,6 +1900,7 @@ int flub_mg_destroy(flub_mg *mg) {
 
 int flub_mg_set_tags(flub_mg *mg, const int32_t *tag, void *stream) {
     FLUB_REQUIRE(mg && tag, "flub_mg_set_tags: NULL argument");
+    mg->tags_new = true;
     cudaStream_t s = as_stream(stream);
     const LaunchCtx c{s, nullptr, 0, 0};
     if (mg->n % 4 == 0 && (uintptr_t)tag % 16 == 0)
@@ -2164,13 +2212,14 @@ int flub_mg_get_x(flub_mg *mg, float *out, float scale, void *stream) {
 
 int flub_mg_apply_preconditioner(flub_mg *mg, const float *r, float *z, void *stream) {
     FLUB_REQUIRE(mg && r && z, "flub_mg_apply_preconditioner: NULL argument");
-    LaunchCtx c{as_stream(stream), nullptr, 0, 0, true};  // may follow set_tags directly
-    if (mg->precision == FLUB_PRECISION_MIXED) {
-        FLUB_TRY(launch_pdl(k8_to_half, dim3(blocks_for(mg->n / 8, 256)), dim3(256), 0, c, (MgState *)nullptr, r, mg->lv[0].rh, mg->n,
-                            c.kc));
-        return enqueue_vcycle_mixed(mg, c, z, false);
-    }
-    return enqueue_vcycle(mg, c, r, z, false);
+    return behind_tags(mg, stream, [&](const LaunchCtx &c) -> int {
+        if (mg->precision == FLUB_PRECISION_MIXED) {
+            FLUB_TRY(launch_pdl(k8_to_half, dim3(blocks_for(mg->n / 8, 256)), dim3(256), 0, c, (MgState *)nullptr, r,
+                                mg->lv[0].rh, mg->n, c.kc));
+            return enqueue_vcycle_mixed(mg, c, z, false);
+        }
+        return enqueue_vcycle(mg, c, r, z, false);
+    });
 }
 
 int flub_mg_matvec(flub_mg *mg, const float *p, float *Ap, void *stream) {
@@ -2185,9 +2234,10 @@ int flub_mg_smooth(flub_mg *mg, int level, int phase, void *stream) {
     FLUB_REQUIRE(mg, "flub_mg_smooth: NULL handle");
     FLUB_REQUIRE(level >= 0 && level < mg->levels, "flub_mg_smooth: level %d outside [0, %d)", level, mg->levels);
     FLUB_REQUIRE(phase == 0 || phase == 1, "flub_mg_smooth: phase must be 0 or 1");
-    LaunchCtx c{as_stream(stream), nullptr, 0, 0, true};  // may follow set_tags directly
     const Level &L = mg->lv[level];
-    return sweep(c, L, phase, kSweepInPlace, mg->skip_ok ? 1 : 0, L.r, L.z, L.z, nullptr);
+    return behind_tags(mg, stream, [&](const LaunchCtx &c) {
+        return sweep(c, L, phase, kSweepInPlace, mg->skip_ok ? 1 : 0, L.r, L.z, L.z, nullptr);
+    });
 }
 
 int flub_mg_smooth_iteration(flub_mg *mg, int level, int phase, int *tiled, void *stream) {
@@ -2195,34 +2245,7 @@ int flub_mg_smooth_iteration(flub_mg *mg, int level, int phase, int *tiled, void
     FLUB_REQUIRE(level >= 0 && level < mg->levels, "flub_mg_smooth_iteration: level %d outside [0, %d)", level,
                  mg->levels);
     FLUB_REQUIRE(phase == 0 || phase == 1, "flub_mg_smooth_iteration: phase must be 0 or 1");
-    LaunchCtx c{as_stream(stream), nullptr, 0, 0, true};  // may follow set_tags directly
-    const Level &L = mg->lv[level];
-    const bool t = mg->tile_ok && L.n_tiles > 0 && mg->skip_ok;
-    if (tiled) *tiled = t ? 1 : 0;
-    if (!t && level == 0 && L.sws && mg->skip_ok) {
-        // the colour-split kernels the V-cycle runs at level 0, in place on the
-        // post-smoothing buffer with the split residual of the last V-cycle
-        if (tiled) *tiled = 2;
-        for (int ph : {phase, 1 - phase}) {
-            if (mg->precision == FLUB_PRECISION_MIXED)
-                FLUB_TRY((split_sweep<kInPlace, __half, __half, float, float, float>(
-                    c, L, ph, nullptr, L.rsh, nullptr, L.zs, nullptr, 1.0f, nullptr)));
-            else
-                FLUB_TRY((split_sweep<kInPlace, float, float, float, float, float>(c, L, ph, nullptr, L.rs, nullptr,
-                                                                                  L.zs, nullptr, 1.0f, nullptr)));
-        }
-        return FLUB_OK;
-    }
-    if (t) {
-        // z -> z3 and z3 -> z on alternate calls (both keep 0 off the fluid);
-        // the handle's pointers stay as the captured solve graphs know them
-        const bool back = mg->iter_toggle[level];
-        mg->iter_toggle[level] = !back;
-        return tile_iteration(mg, c, level, phase, kTileInPlaceInput, L.r, back ? L.z3 : L.z, back ? L.z : L.z3,
-                              nullptr);
-    }
-    FLUB_TRY(sweep(c, L, phase, kSweepInPlace, mg->skip_ok ? 1 : 0, L.r, L.z, L.z, nullptr));
-    return sweep(c, L, 1 - phase, kSweepInPlace, mg->skip_ok ? 1 : 0, L.r, L.z, L.z, nullptr);
+    return behind_tags(mg, stream, [&](const LaunchCtx &c) { return smooth_iteration(mg, c, level, phase, tiled); });
 }
 
 int flub_mg_kernels_executed(flub_mg *mg, void *stream, int64_t *out) {
