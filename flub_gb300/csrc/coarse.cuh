@@ -336,8 +336,9 @@ __device__ __forceinline__ float half_stored(float v) { return __half2float(__fl
 // z += (r + L z) / d on the item's cells of colour COL, the quotient by
 // Markstein's FMA correction with y = -1/d: q0 = a y, -q = q0 + (a + d q0) y.
 // For d = 1..6 that is IEEE a / d for every finite a but ties between two
-// denormals at d = 6 (tests/test_coarse_div.py checks all 2^32 values), so it
-// needs no guard; a branch here cost 100 ns of a 350 ns half-sweep.  A cell
+// denormals at d = 6, so it needs no guard; a branch here cost 100 ns of a 350 ns
+// half-sweep.  (tests/test_coarse_div.py checks every finite a >= 0 for d = 3, 5 and 6
+// and every 61st for the powers of two; the operations are odd in a.)  A cell
 // that is never updated has y = d = 0: its z stays 0.
 template <int V, int COL, bool kKeep, bool kHalf>
 __device__ __forceinline__ void coarse_half(CoarseItem<V> &t, float *zs, int hn, int ps, int rs) {

@@ -33,9 +33,9 @@
 // stencil words; the prolongation, which adds the correction to air as well, does
 // so next to air too.
 // A half-sweep of 128^3 (FP32, dam break / full): 1.9 / 3.3 us, in natural order
-// 3.0 / 6.7.  Measured through a whole solve (before -> now): 128^3 sphere in mixed
-// precision 8536 -> 7859 us, 256^3 dam break 15880 -> 15310, 256 x 64 x 256
-// 3951 -> 3733, 104 x 72 x 88 2296 -> 2141.
+// 3.0 / 6.7.  Whole projections with these levels in natural order (FLUB_NO_SPLIT=1)
+// and as they are: 128^3 sphere in mixed precision 8.8 and 7.1 ms, 256^3 dam break 15.9
+// and 12.7, 256 x 64 x 256 3.72 and 3.44, 104 x 72 x 88 2.11 and 1.88.
 //
 // Modes of one half-sweep (phase 0 updates the odd cells, phase 1 the even):
 //   kFirst    first pre-smoothing half-sweep (phase 0, from zero): reads the
